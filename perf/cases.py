@@ -250,7 +250,6 @@ def run(state):
     if call == "update":
         return state["solver"].solve(state["b"], values=state["values"])
     if call == "train":
-        state["solver"].set_values(state["values"].detach())  # as after an optimizer's step
         x = sp.sparse_triangular_solve(state["solver"], state["values"], state["b"])
         db, dv = torch.autograd.grad(x, (state["b"], state["values"]), state["gx"])
         return x.detach(), db, dv
