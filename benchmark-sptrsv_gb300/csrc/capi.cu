@@ -53,6 +53,7 @@ struct sptrsv_gb300_handle_s {
   int opt_option = SPTRSV_OPT_WARP_AUTO;  // push, many rhs: the reference's lane mode
   int rhs_tile_option = 0;                // many rhs: right-hand sides per lane (0: automatic)
   int stretch_option = 1;                 // batches in level order: levels stretched to the batch depth
+  int cluster_option = 2;                 // one-cluster executor: 0 off, 1 wherever it fits, 2 by the plan
   unsigned long long user_set = 0;  // options the caller set explicitly (bit = option id)
   // executor settings chosen from the analysis for SPTRSV_SCHED_AUTO (one rhs)
   struct AutoPlan {
@@ -60,6 +61,9 @@ struct sptrsv_gb300_handle_s {
     int order_block = INT_MAX, chunk = 256, block = 256, ctas = 2, backoff = 0, staged = 0, wsync = 1;
     int split_fwd = 0, split_adj = 0;  // split length for the forward / transposed walk (0: none)
     double locality = 0.0;
+    ClusterPlan cluster;       // one-cluster executor (block 0: the cluster cannot hold the system)
+    bool cluster_f64 = false, cluster_f32 = false;  // the device can run it for this element type
+    bool narrow = false;       // few enough dependencies per level for one cluster
     double coarrive = 0.0;  // short lists: share of unknowns with >= 2 dependencies on the preceding level
   } plan;
   // analysis
@@ -834,6 +838,40 @@ double long_share(const std::vector<int>& ptr, int cut) {
   return all ? static_cast<double>(lng) / static_cast<double>(all) : 0.0;
 }
 
+// One-cluster executor (k_pull_cluster, exec_cluster.cu): a single system in
+// level order with at most kClusterDeps dependencies and kClusterWidth unknowns
+// per level on average and no lists to split, whose values fit the cluster's
+// shared memory. Past either line 16 SMs no longer keep up with the whole GPU
+// (FP64, cluster vs level-order executor: 2,973 dependencies per level 299 vs
+// 385 us, 3,628 297 vs 316, 4,368 383 vs 343, 5,294 378 vs 285; 925 unknowns of
+// 4 entries per level 123 vs 95 us, 1,724 of 2 entries 76 vs 56).
+//
+// Threads and runs: below 1,000 dependencies per level 128 threads per CTA and
+// runs of 128 walk indices (10,000 rows, 543 per level: 67.5 us; 75.7 with 256
+// threads and runs of 32), from there 256 threads and runs of 32 (30,000 rows,
+// 1,391 per level: 87.9 vs 112.5 us). Levels of fewer than 24 unknowns: 256
+// threads and runs of 256, so that most hops stay inside a CTA (150,001 rows,
+// 17 per level: 2,786 us; 2,926 with the first rule, 3,506 with runs of 32).
+constexpr double kClusterDeps = 3000.0;
+constexpr long long kClusterWidth = 512;
+
+void plan_cluster(sptrsv_gb300_handle_s* h) {
+  auto& P = h->plan;
+  const int n = h->n, nl = h->nlevels;
+  if (n <= 0 || nl <= 0 || h->batch_count != 1) return;
+  const double deps = static_cast<double>(h->nnz - n) / nl;
+  ClusterPlan& c = P.cluster;
+  const bool wide = deps >= 1000.0, thin = n < 24LL * nl;
+  c.block = wide || thin ? 256 : 128;
+  c.cshift = thin ? 8 : (wide ? 5 : 7);
+  // list buffers: 1.5 x the average segment, fewer entries where values are many
+  const double avg = 32.0 * (h->nnz - n) / n;
+  c.cap = std::min(512, std::max(64, (static_cast<int>(1.5 * avg) + 31) / 32 * 32));
+  P.cluster_f64 = cluster_fits<double>(c, n);
+  P.cluster_f32 = cluster_fits<float>(c, n);
+  P.narrow = deps <= kClusterDeps && n <= kClusterWidth * nl;
+}
+
 int make_plan(sptrsv_gb300_handle_s* h, const std::vector<int>& row_ptr, cudaStream_t s) {
   auto& P = h->plan;
   P = sptrsv_gb300_handle_s::AutoPlan();
@@ -883,6 +921,7 @@ int make_plan(sptrsv_gb300_handle_s* h, const std::vector<int>& row_ptr, cudaStr
       }
     }
   }
+  plan_cluster(h);
   P.valid = true;
   return SPTRSV_OK;
 }
@@ -1015,6 +1054,26 @@ ExecConfig pick_config(const sptrsv_gb300_handle_s* h, int rhs) {
   return c;
 }
 
+// Whether a one-rhs solve (the transposed one for adj) runs the one-cluster
+// executor. It follows the automatic plan unless the caller set an option that
+// selects or shapes another executor; SPTRSV_OPTION_CLUSTER = 1 asks for it
+// wherever a level-order layout fits, 0 turns it off.
+template <typename T>
+bool use_cluster(const sptrsv_gb300_handle_s* h, bool adj) {
+  const auto& P = h->plan;
+  if (h->cluster_option == 0 || !P.valid || h->cfg.exact || h->layout_block < h->n || h->layout_stretched) return false;
+  if (!(sizeof(T) == 8 ? P.cluster_f64 : P.cluster_f32)) return false;
+  if (h->cluster_option == 1) return h->sched_option == SCHED_AUTO || h->sched_option == SCHED_PULL;
+  constexpr unsigned long long shaping =
+      1ull << SPTRSV_OPTION_LANES | 1ull << SPTRSV_OPTION_CHUNK | 1ull << SPTRSV_OPTION_SMEM_TIER |
+      1ull << SPTRSV_OPTION_ORDER_BLOCK | 1ull << SPTRSV_OPTION_BLOCK | 1ull << SPTRSV_OPTION_BACKOFF_NS |
+      1ull << SPTRSV_OPTION_CTAS_PER_SM | 1ull << SPTRSV_OPTION_STAGED | 1ull << SPTRSV_OPTION_STAGE_ENTRIES |
+      1ull << SPTRSV_OPTION_STAGES | 1ull << SPTRSV_OPTION_WARP_SYNC | 1ull << SPTRSV_OPTION_SPLIT |
+      1ull << SPTRSV_OPTION_WSYNC_BATCH | 1ull << SPTRSV_OPTION_IMPORT | 1ull << SPTRSV_OPTION_UNIT_PIPELINE;
+  if (h->sched_option != SCHED_AUTO || (h->user_set & shaping)) return false;
+  return P.narrow && P.order_block >= h->n && (adj ? P.split_adj : P.split_fwd) == 0;
+}
+
 template <typename T>
 int solve_typed(sptrsv_gb300_handle_s* h, const Values<T>& V, int rhs, int layout, const T* b, T* x,
                 cudaStream_t s, const AdjointArgs<T>* adj = nullptr, bool allow_check = true) {
@@ -1034,7 +1093,10 @@ int solve_typed(sptrsv_gb300_handle_s* h, const Values<T>& V, int rhs, int layou
   h->last_sched = c.sched;
   h->last_pipe = false;
   const size_t elems = (size_t)n * (size_t)rhs;
-  if (c.sched == SCHED_PUSH) {
+  const bool cluster = rhs == 1 && !(adj && adj->grad) && use_cluster<T>(h, adj != nullptr);
+  if (cluster) {
+    // values live in the cluster's shared memory: no flag words to clear
+  } else if (c.sched == SCHED_PUSH) {
     ST_TRY(ensure_buf(h, h->left_sum, elems * sizeof(T), 1, s));
     ST_TRY(ensure_buf(h, h->counters, (size_t)n * sizeof(unsigned), 1, s));
   } else {
@@ -1048,7 +1110,9 @@ int solve_typed(sptrsv_gb300_handle_s* h, const Values<T>& V, int rhs, int layou
     }
     CUDA_TRY(cudaEventRecord(h->ev_exec[0], s));
   }
-  if (c.sched == SCHED_PUSH) {
+  if (cluster) {
+    CUDA_TRY(launch_pull_cluster<T>(h->layout, V, v, h->ctl, h->plan.cluster, timeout_ns(h), s, adj != nullptr));
+  } else if (c.sched == SCHED_PUSH) {
     CUDA_TRY(launch_push<T>(h->layout, V, rhs, v, static_cast<T*>(h->left_sum.p),
                             static_cast<unsigned*>(h->counters.p), h->ctl, c, timeout_ns(h), h->num_sms, s));
   } else if (c.sched == SCHED_LEVELSET) {
@@ -1303,6 +1367,10 @@ static int set_option_value(sptrsv_handle_t h, int option, long long value) {
     case SPTRSV_OPTION_STRETCH:
       h->stretch_option = value != 0;
       return SPTRSV_OK;
+    case SPTRSV_OPTION_CLUSTER:
+      if (value < 0 || value > 2) return SPTRSV_ERR_INVALID;
+      h->cluster_option = static_cast<int>(value);
+      return SPTRSV_OK;
     default:
       return SPTRSV_ERR_INVALID;
   }
@@ -1336,6 +1404,7 @@ int sptrsv_gb300_get_option(sptrsv_handle_t h, int option, long long* value) {
     case SPTRSV_OPTION_OPT: *value = h->opt_option; break;
     case SPTRSV_OPTION_RHS_TILE: *value = h->rhs_tile_option; break;
     case SPTRSV_OPTION_STRETCH: *value = h->stretch_option; break;
+    case SPTRSV_OPTION_CLUSTER: *value = h->cluster_option; break;
     default: return SPTRSV_ERR_INVALID;
   }
   return SPTRSV_OK;
@@ -2022,7 +2091,7 @@ int sptrsv_gb300_tune(sptrsv_handle_t h, const void* d_val, int dtype, int rhs, 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   struct Cand {
     int sched, order_block, chunk, staged, backoff, ctas, lanes, stages, wsync, block, split, batch = 0;
-    int smem = 1, opt = SPTRSV_OPT_WARP_AUTO, tile = 0;
+    int smem = 1, opt = SPTRSV_OPT_WARP_AUTO, tile = 0, cluster = 0;
   };
   const int n = h->n;
   const int big = INT_MAX;
@@ -2046,6 +2115,9 @@ int sptrsv_gb300_tune(sptrsv_handle_t h, const void* d_val, int dtype, int rhs, 
   if (rhs == 1) {
     // staged warp-specialised executor, level order
     for (int bo : {0, 256}) cands.push_back({SCHED_PULL, big, 224, 1, bo, 0, 1, 2, 0, 256, sp});
+    // one cluster, all values in its shared memory (where they fit)
+    if (dtype == SPTRSV_DTYPE_F64 ? h->plan.cluster_f64 : h->plan.cluster_f32)
+      cands.push_back({SCHED_PULL, big, 256, 0, 0, 1, 1, 2, 1, 256, 0, 0, 1, SPTRSV_OPT_WARP_AUTO, 0, 1});
     // warp-synchronous executor (long lists split over lanes): level order, and
     // blocked orders for deep narrow DAGs
     for (int ch : {128, 256}) cands.push_back({SCHED_PULL, big, ch, 0, 128, 1, 1, 2, 1, ch, sp});
@@ -2113,6 +2185,7 @@ int sptrsv_gb300_tune(sptrsv_handle_t h, const void* d_val, int dtype, int rhs, 
     h->cfg.smem_tier = c.smem;
     h->opt_option = c.opt;
     h->rhs_tile_option = c.tile;
+    h->cluster_option = c.cluster;
     int st = sptrsv_gb300_solve(h, d_val, dtype, rhs, layout, d_b, d_x, stream);
     if (st == SPTRSV_OK) st = check_device(h, s);
     if (st != SPTRSV_OK) continue;  // a candidate that fails (or times out) is skipped
@@ -2156,6 +2229,7 @@ int sptrsv_gb300_tune(sptrsv_handle_t h, const void* d_val, int dtype, int rhs, 
   h->cfg.smem_tier = c.smem;
   h->opt_option = c.opt;
   h->rhs_tile_option = c.tile;
+  h->cluster_option = c.cluster;
   ST_TRY(ensure_layout(h, s));
   ST_TRY(stage_values(h, d_val, dtype, s, false));
   if (best_ms) *best_ms = best;

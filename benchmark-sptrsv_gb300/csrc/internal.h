@@ -266,6 +266,28 @@ template <typename T>
 cudaError_t launch_levelset(const Layout& L, const Values<T>& V, int rhs, const VecView<T>& v, T* xw,
                             DeviceCtl* ctl, const ExecConfig& cfg, unsigned long long timeout_ns,
                             cudaStream_t s);
+// One-cluster executor (exec_cluster.cu): 16 CTAs of `block` threads; walk
+// indices are dealt to them in runs of 1 << cshift; a warp's list buffer holds
+// `cap` entries.
+struct ClusterPlan {
+  static constexpr int kRankShift = 4;  // 16 CTAs (a non-portable cluster size)
+  int block = 0;                        // 0: not used
+  int cshift = 5;
+  int cap = 0;
+  int slots(int n) const {  // value words per CTA
+    const int run = 1 << cshift, round = run << kRankShift;
+    return static_cast<int>(((long long)n + round - 1) / round) * run;
+  }
+  size_t smem(int n, size_t elem) const {  // values, then two list buffers (weights, positions) per warp
+    return (size_t)slots(n) * elem + (size_t)(block / 32) * 2 * cap * (elem + sizeof(int));
+  }
+};
+// true when the device can run one such cluster for n unknowns
+template <typename T>
+bool cluster_fits(const ClusterPlan& plan, int n);
+template <typename T>
+cudaError_t launch_pull_cluster(const Layout& L, const Values<T>& V, const VecView<T>& v, DeviceCtl* ctl,
+                                const ClusterPlan& plan, unsigned long long timeout_ns, cudaStream_t s, bool adj);
 size_t pull_smem_bytes(int chunk, int rhs, size_t elem);
 size_t imported_smem_bytes(int chunk, int max_imports, size_t elem);
 // warp-synchronous one-rhs forward pull with an importer warp per CTA (blocked layouts)

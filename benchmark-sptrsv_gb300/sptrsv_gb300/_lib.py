@@ -66,6 +66,7 @@ OPTION_FUSED_REFINE = 21
 OPTION_OPT = 22
 OPTION_RHS_TILE = 23
 OPTION_STRETCH = 24
+OPTION_CLUSTER = 25
 
 NOALLOC_MAX_N = 262144  # SPTRSV_NOALLOC_MAX_N
 

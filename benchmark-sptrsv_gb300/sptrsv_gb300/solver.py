@@ -107,7 +107,7 @@ class SyncFreeSolver:
                  warp_sync: bool | None = None, split: int | None = None, wsync_batch: int | None = None,
                  import_deps: bool | None = None, unit_pipeline: int | None = None, fused_grad: bool | None = None,
                  fused_refine: int | None = None, opt: int | None = None, rhs_tile: int | None = None,
-                 stretch: bool | None = None, stream=None):
+                 stretch: bool | None = None, cluster: int | None = None, stream=None):
         torch = _torch()
         self._lib = load()
         self.device = torch.device("cuda", torch.cuda.current_device())
@@ -153,7 +153,7 @@ class SyncFreeSolver:
                        (_lib.OPTION_UNIT_PIPELINE, unit_pipeline),
                        (_lib.OPTION_FUSED_GRAD, fused_grad), (_lib.OPTION_FUSED_REFINE, fused_refine),
                        (_lib.OPTION_OPT, opt), (_lib.OPTION_RHS_TILE, rhs_tile),
-                       (_lib.OPTION_STRETCH, stretch)):
+                       (_lib.OPTION_STRETCH, stretch), (_lib.OPTION_CLUSTER, cluster)):
             if v is not None:
                 self.set_option(opt, int(v))
         self._stream = stream
@@ -319,7 +319,7 @@ class SyncFreeSolver:
         return dval
 
     TUNED_OPTIONS = ("SCHEDULE", "ORDER_BLOCK", "CHUNK", "STAGED", "BACKOFF_NS", "CTAS_PER_SM", "LANES", "STAGES",
-                     "WARP_SYNC", "BLOCK", "SPLIT", "WSYNC_BATCH", "SMEM_TIER", "OPT", "RHS_TILE")
+                     "WARP_SYNC", "BLOCK", "SPLIT", "WSYNC_BATCH", "SMEM_TIER", "OPT", "RHS_TILE", "CLUSTER")
 
     def tune(self, b, values=None, reps: int = 3) -> dict:
         """Autotune the executor on this right-hand side; returns the chosen options and time."""

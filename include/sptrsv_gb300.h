@@ -139,13 +139,19 @@ typedef enum sptrsv_option {
   SPTRSV_OPTION_RHS_TILE = 23,    /* pull executors with several right-hand sides: right-hand sides each
                                      lane covers, 1, 2 or 4 (so 4-32 lanes per unknown); 0 (default) =
                                      one per lane up to 32 right-hand sides, two beyond */
-  SPTRSV_OPTION_STRETCH = 24      /* batches in level order (not the level-set schedule): 1 (default) =
+  SPTRSV_OPTION_STRETCH = 24,     /* batches in level order (not the level-set schedule): 1 (default) =
                                      the schedule key of an unknown is its level stretched to T =
                                      65 % of the batch's depth (or to its system's depth, if deeper),
                                      floor(level * max(T, depth(system)) / depth(system)), so every
                                      system's chain spreads over most of the launch instead of a deep
                                      system waiting behind the shallow systems' wide levels; 0 = global
                                      level order */
+  SPTRSV_OPTION_CLUSTER = 25        /* one-rhs pull solves of one system in level order: 16 CTAs of one
+                                     cluster hold every value in their shared memory. 2 (default) = where
+                                     the automatic plan finds few dependencies per level and no option
+                                     that shapes another executor is set; 1 = wherever the values fit
+                                     (automatic and pull schedules, fast arithmetic); 0 = off. The other
+                                     executor settings do not apply to such a solve */
 } sptrsv_option;
 
 typedef struct sptrsv_info {
