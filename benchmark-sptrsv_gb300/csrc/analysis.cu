@@ -2,6 +2,7 @@
 // prefix scans, a stable radix sort, level sets, and the position-space
 // layouts the executors read.
 #include <algorithm>
+#include <climits>
 #include <cstdio>
 
 #include "internal.h"
@@ -809,56 +810,108 @@ cudaError_t launch_fill_push(const int* perm, const int* iperm, const int* col_p
 }
 
 // ------------------------------------------------------------ value staging
-template <typename TV, typename T>
-__global__ void k_stage_edges(const TV* __restrict__ val, const int* __restrict__ src, T* out, int count) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += stride)
-    out[i] = static_cast<T>(val[src[i]]);
-}
-template <typename TV, typename T>
-__global__ void k_stage_diag(const TV* __restrict__ val, const int* __restrict__ diag_src, T* diag, T* rcp, int n,
-                             int* flags) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += stride) {
-    const T d = static_cast<T>(val[diag_src[p]]);
-    diag[p] = d;
-    rcp[p] = T(1) / d;
-    if (!(d != T(0)) || !isfinite(d)) atomicOr(flags, SF_ZERO_DIAG);
+// Gathers the values of one list set (out[e] = val[src[e]], scaled by the
+// reciprocal of the owning position's diagonal for SCALE: x_p = b_p/d_p - sum_j
+// w_j x_j then needs one fused multiply-add per dependency). DIAG first stages
+// the diagonal and its reciprocal of the same positions.
+//
+// A warp takes 32 positions at a time: their lists are one contiguous range, so
+// its lanes walk entries, coalesced, and find an entry's owner among the 32 list
+// starts they hold by a binary search over shuffles. Bound by the gather of
+// 8-byte values from 32-byte sectors. (One thread per list, as before, strides
+// its loads and stores over 32 lists: the 5M-entry band system's pull weights
+// took 66 us, the FP64 diagonal 11 more.)
+template <typename TV, typename T, bool DIAG, bool SCALE>
+__global__ void __launch_bounds__(256) k_stage_lists(const int* __restrict__ ptr, const int* __restrict__ src,
+                                                     const TV* __restrict__ val, const int* __restrict__ diag_src,
+                                                     T* diag, T* rcp, T* out, int n, int* flags) {
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int U = 4;
+  const int lane = threadIdx.x & 31;
+  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  const long long groups = ((long long)n + 31) / 32;
+  for (long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; g < groups; g += nwarps) {
+    const long long p = g * 32 + lane;
+    T r = T(0);
+    int start = INT_MAX, end = 0;
+    if (p < n) {
+      start = ptr[p];
+      end = ptr[p + 1];
+      if (DIAG) {
+        const T d = static_cast<T>(val[diag_src[p]]);
+        r = T(1) / d;
+        diag[p] = d;
+        rcp[p] = r;
+        if (flags && (!(d != T(0)) || !isfinite(d))) atomicOr(flags, SF_ZERO_DIAG);
+      } else if (SCALE) {
+        r = rcp[p];
+      }
+    }
+    if (!out) continue;
+    // entry indices as unsigned: a batch may reach past the last entry a 32-bit count can hold
+    const unsigned lo = static_cast<unsigned>(__shfl_sync(kFull, start, 0));
+    const unsigned hi = static_cast<unsigned>(__reduce_max_sync(kFull, end));
+    for (unsigned base = lo; base < hi; base += 32 * U) {
+      TV v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const unsigned e = base + u * 32 + lane;
+        v[u] = e < hi ? val[src[e]] : TV(0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const unsigned e = base + u * 32 + lane;
+        T w = static_cast<T>(v[u]);
+        if (SCALE) {
+          // the last list that starts at or before e owns it (empty lists share
+          // their successor's start)
+          int own = 0;
+#pragma unroll
+          for (int step = 16; step > 0; step >>= 1) {
+            const int t = __shfl_sync(kFull, start, own + step);
+            if (static_cast<unsigned>(t) <= e) own += step;
+          }
+          w *= __shfl_sync(kFull, r, own);
+        }
+        if (e < hi) out[e] = w;
+      }
+    }
   }
 }
 
-// w = v * (1/diag of the dependent row): x_p = b_p/d_p - sum_j w_j x_j needs one
-// fused multiply-add per dependency once the reciprocal is folded in. The scaled
-// lists follow the ready order (src_f), the plain ones the serial order.
 template <typename TV, typename T>
-__global__ void k_stage_scaled(const int* __restrict__ ptr, const TV* __restrict__ val, const int* __restrict__ src_f,
-                               const T* __restrict__ rcp, T* w, int n) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += stride) {
-    const T r = rcp[p];
-    for (int e = ptr[p]; e < ptr[p + 1]; ++e) w[e] = static_cast<T>(val[src_f[e]]) * r;
+cudaError_t launch_stage_values(const Layout& L, const TV* val, Values<T>& V, unsigned forms, int* flags,
+                                cudaStream_t s) {
+  if (L.n <= 0) return cudaSuccess;
+  const int grid = grid_for(L.n);
+  const bool dep = (forms & FORM_DEP_W) && L.ndep > 0;
+  // the diagonal with the pull weights where both are wanted
+  if (forms & FORM_DIAG) {
+    k_stage_lists<TV, T, true, true><<<grid, kThreads, 0, s>>>(L.dep_ptr, L.dep_src_f, val, L.diag_src, V.diag, V.rcp,
+                                                               dep ? V.dep_w : nullptr, L.n, flags);
+  } else if (dep) {
+    k_stage_lists<TV, T, false, true><<<grid, kThreads, 0, s>>>(L.dep_ptr, L.dep_src_f, val, nullptr, nullptr, V.rcp,
+                                                                V.dep_w, L.n, nullptr);
   }
-}
-
-template <typename TV, typename T>
-cudaError_t launch_stage_values(const Layout& L, const TV* val, Values<T>& V, int* flags, cudaStream_t s) {
   if (L.ndep > 0) {
-    k_stage_edges<TV, T><<<grid_for(L.ndep), kThreads, 0, s>>>(val, L.dep_src, V.dep_val, L.ndep);
-    k_stage_edges<TV, T><<<grid_for(L.ndep), kThreads, 0, s>>>(val, L.out_src, V.out_val, L.ndep);
-  }
-  if (L.n > 0) k_stage_diag<TV, T><<<grid_for(L.n), kThreads, 0, s>>>(val, L.diag_src, V.diag, V.rcp, L.n, flags);
-  if (L.n > 0 && L.ndep > 0) {
-    k_stage_scaled<TV, T><<<grid_for(L.n), kThreads, 0, s>>>(L.dep_ptr, val, L.dep_src_f, V.rcp, V.dep_w, L.n);
-    k_stage_scaled<TV, T><<<grid_for(L.n), kThreads, 0, s>>>(L.out_ptr, val, L.out_src_f, V.rcp, V.out_w, L.n);
+    if (forms & FORM_OUT_W)
+      k_stage_lists<TV, T, false, true><<<grid, kThreads, 0, s>>>(L.out_ptr, L.out_src_f, val, nullptr, nullptr, V.rcp,
+                                                                  V.out_w, L.n, nullptr);
+    if (forms & FORM_DEP_VAL)
+      k_stage_lists<TV, T, false, false><<<grid, kThreads, 0, s>>>(L.dep_ptr, L.dep_src, val, nullptr, nullptr,
+                                                                   nullptr, V.dep_val, L.n, nullptr);
+    if (forms & FORM_OUT_VAL)
+      k_stage_lists<TV, T, false, false><<<grid, kThreads, 0, s>>>(L.out_ptr, L.out_src, val, nullptr, nullptr,
+                                                                   nullptr, V.out_val, L.n, nullptr);
   }
   return cudaGetLastError();
 }
 
-template cudaError_t launch_stage_values<double, double>(const Layout&, const double*, Values<double>&, int*,
+template cudaError_t launch_stage_values<double, double>(const Layout&, const double*, Values<double>&, unsigned, int*,
                                                           cudaStream_t);
-template cudaError_t launch_stage_values<double, float>(const Layout&, const double*, Values<float>&, int*,
+template cudaError_t launch_stage_values<double, float>(const Layout&, const double*, Values<float>&, unsigned, int*,
                                                          cudaStream_t);
-template cudaError_t launch_stage_values<float, float>(const Layout&, const float*, Values<float>&, int*,
+template cudaError_t launch_stage_values<float, float>(const Layout&, const float*, Values<float>&, unsigned, int*,
                                                         cudaStream_t);
 
 }  // namespace sptrsv

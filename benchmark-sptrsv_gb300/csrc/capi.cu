@@ -108,6 +108,8 @@ struct sptrsv_gb300_handle_s {
   Values<double> v64;
   Values<float> v32;
   bool staged64 = false, staged32 = false;
+  DevBuf vals;          // the values as given (CSC order), for forms staged later
+  int vals_dtype = SPTRSV_DTYPE_F64;
   // workspace
   DevBuf xw, left_sum, counters, r32, d32, stats;
   DevBuf tb, tx;  // row-major staging of column-major blocks of many right-hand sides
@@ -224,6 +226,7 @@ void free_values(Values<T>& V) {
   dev_free(&V.out_val);
   dev_free(&V.diag);
   dev_free(&V.rcp);
+  V.ready = 0;
 }
 
 void free_analysis(sptrsv_gb300_handle_s* h) {
@@ -936,39 +939,99 @@ int ensure_layout(sptrsv_gb300_handle_s* h, cudaStream_t s) {
   return build_layout(h, want, s);
 }
 
-template <typename TV, typename T>
-int stage(sptrsv_gb300_handle_s* h, Values<T>& V, const TV* val, cudaStream_t s, bool check) {
+template <typename T>
+Values<T>& values_of(sptrsv_gb300_handle_s* h);
+template <>
+Values<double>& values_of<double>(sptrsv_gb300_handle_s* h) { return h->v64; }
+template <>
+Values<float>& values_of<float>(sptrsv_gb300_handle_s* h) { return h->v32; }
+
+template <typename T>
+unsigned allocated_forms(const Values<T>& V) {
+  return (V.rcp ? FORM_DIAG : 0u) | (V.dep_w ? FORM_DEP_W : 0u) | (V.out_w ? FORM_OUT_W : 0u) |
+         (V.dep_val ? FORM_DEP_VAL : 0u) | (V.out_val ? FORM_OUT_VAL : 0u);
+}
+
+template <typename T>
+int alloc_forms(sptrsv_gb300_handle_s* h, Values<T>& V, unsigned forms) {
   const Layout& L = h->layout;
-  if (!V.dep_val) {
-    ST_TRY(dev_alloc(h, &V.dep_val, L.ndep));
-    ST_TRY(dev_alloc(h, &V.dep_w, L.ndep));
-    ST_TRY(dev_alloc(h, &V.out_w, L.ndep));
-    ST_TRY(dev_alloc(h, &V.out_val, L.ndep));
-    ST_TRY(dev_alloc(h, &V.diag, L.n));
-    ST_TRY(dev_alloc(h, &V.rcp, L.n));
+  if ((forms & FORM_DIAG) && !V.diag) ST_TRY(dev_alloc(h, &V.diag, L.n));
+  if ((forms & FORM_DIAG) && !V.rcp) ST_TRY(dev_alloc(h, &V.rcp, L.n));
+  if ((forms & FORM_DEP_W) && !V.dep_w) ST_TRY(dev_alloc(h, &V.dep_w, L.ndep));
+  if ((forms & FORM_OUT_W) && !V.out_w) ST_TRY(dev_alloc(h, &V.out_w, L.ndep));
+  if ((forms & FORM_DEP_VAL) && !V.dep_val) ST_TRY(dev_alloc(h, &V.dep_val, L.ndep));
+  if ((forms & FORM_OUT_VAL) && !V.out_val) ST_TRY(dev_alloc(h, &V.out_val, L.ndep));
+  return SPTRSV_OK;
+}
+
+// The given forms of the staged values, in precision T, ready for the work that
+// follows on `s`: those not staged since the last set of values are staged now
+// from the handle's copy. Inside a stream capture the staging becomes part of
+// the graph (and is not recorded as done here, since it runs at replay).
+template <typename T>
+int need_forms(sptrsv_gb300_handle_s* h, unsigned forms, cudaStream_t s) {
+  Values<T>& V = values_of<T>(h);
+  const unsigned missing = (forms | FORM_DIAG) & ~V.ready;
+  if (!missing) return SPTRSV_OK;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  CUDA_TRY(cudaStreamIsCapturing(s, &capture));
+  // an allocation is no stream operation: relaxed mode lets it through a capture
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (capture != cudaStreamCaptureStatusNone) CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+  const int st = alloc_forms(h, V, missing);
+  if (capture != cudaStreamCaptureStatusNone) CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+  ST_TRY(st);
+  if (h->vals_dtype == SPTRSV_DTYPE_F64) {
+    CUDA_TRY(launch_stage_values(h->layout, static_cast<const double*>(h->vals.p), V, missing, nullptr, s));
+  } else if constexpr (sizeof(T) == 4) {
+    CUDA_TRY(launch_stage_values(h->layout, static_cast<const float*>(h->vals.p), V, missing, nullptr, s));
+  } else {
+    return SPTRSV_ERR_STATE;  // FP64 forms of FP32 values
   }
+  if (capture == cudaStreamCaptureStatusNone) V.ready |= missing;
+  return SPTRSV_OK;
+}
+
+// Stages new values: the handle's copy (the caller's array is not kept), the
+// forward pull weights, and every form an earlier call needed; the others wait
+// until one does. (Staging all forms in both precisions took 385 us for the
+// 5M-entry band system, of a 2.4 ms training step.)
+template <typename TV>
+int stage_all(sptrsv_gb300_handle_s* h, const TV* val, cudaStream_t s, bool check) {
+  Values<TV>& V = values_of<TV>(h);
+  ST_TRY(ensure_buf(h, h->vals, sizeof(TV) * std::max<size_t>(h->nnz, 1), 0, s));
+  if (h->nnz > 0)
+    CUDA_TRY(cudaMemcpyAsync(h->vals.p, val, sizeof(TV) * (size_t)h->nnz, cudaMemcpyDeviceToDevice, s));
+  h->vals_dtype = sizeof(TV) == 8 ? SPTRSV_DTYPE_F64 : SPTRSV_DTYPE_F32;
+  const unsigned forms = allocated_forms(V) | FORM_DIAG | FORM_DEP_W;
+  ST_TRY(alloc_forms(h, V, forms));
+  h->v64.ready = h->v32.ready = 0;
   if (check) CUDA_TRY(cudaMemsetAsync(h->flags, 0, sizeof(int), s));
-  CUDA_TRY(launch_stage_values<TV, T>(L, val, V, h->flags, s));
+  CUDA_TRY(launch_stage_values(h->layout, val, V, forms, h->flags, s));
   if (check) {
     int f = 0;
     ST_TRY(read_flags(h, s, &f));
     if (f & SF_ZERO_DIAG) return SPTRSV_ERR_BAD_STRUCTURE;
   }
+  V.ready = forms;
   return SPTRSV_OK;
 }
 
 int stage_values(sptrsv_gb300_handle_s* h, const void* d_val, int dtype, cudaStream_t s, bool check) {
+  if (dtype != SPTRSV_DTYPE_F64 && dtype != SPTRSV_DTYPE_F32) return SPTRSV_ERR_INVALID;
+  h->wsplit_ok = false;
   if (dtype == SPTRSV_DTYPE_F64) {
-    ST_TRY(stage<double, double>(h, h->v64, static_cast<const double*>(d_val), s, check));
-    ST_TRY(stage<double, float>(h, h->v32, static_cast<const double*>(d_val), s, false));
+    ST_TRY(stage_all(h, static_cast<const double*>(d_val), s, check));
+    const unsigned again = allocated_forms(h->v32);
+    if (again) {
+      CUDA_TRY(launch_stage_values(h->layout, static_cast<const double*>(d_val), h->v32, again, nullptr, s));
+      h->v32.ready = again;
+    }
     h->staged64 = h->staged32 = true;
-    h->wsplit_ok = false;
-  } else if (dtype == SPTRSV_DTYPE_F32) {
-    ST_TRY(stage<float, float>(h, h->v32, static_cast<const float*>(d_val), s, check));
+  } else {
+    ST_TRY(stage_all(h, static_cast<const float*>(d_val), s, check));
     h->staged32 = true;
     h->staged64 = false;
-  } else {
-    return SPTRSV_ERR_INVALID;
   }
   return SPTRSV_OK;
 }
@@ -1075,8 +1138,8 @@ bool use_cluster(const sptrsv_gb300_handle_s* h, bool adj) {
 }
 
 template <typename T>
-int solve_typed(sptrsv_gb300_handle_s* h, const Values<T>& V, int rhs, int layout, const T* b, T* x,
-                cudaStream_t s, const AdjointArgs<T>* adj = nullptr, bool allow_check = true) {
+int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x, cudaStream_t s,
+                const AdjointArgs<T>* adj = nullptr, bool allow_check = true) {
   const int n = h->n;
   VecView<T> v{};
   v.b = b;
@@ -1093,6 +1156,11 @@ int solve_typed(sptrsv_gb300_handle_s* h, const Values<T>& V, int rhs, int layou
   h->last_sched = c.sched;
   h->last_pipe = false;
   const size_t elems = (size_t)n * (size_t)rhs;
+  const Values<T>& V = values_of<T>(h);
+  unsigned form = adj ? (c.exact ? FORM_OUT_VAL : FORM_OUT_W) : (c.exact ? FORM_DEP_VAL : FORM_DEP_W);
+  if (c.sched == SCHED_PUSH) form = FORM_OUT_VAL;
+  if (c.sched == SCHED_LEVELSET) form = FORM_DEP_W;
+  ST_TRY(need_forms<T>(h, form, s));
   const bool cluster = rhs == 1 && !(adj && adj->grad) && use_cluster<T>(h, adj != nullptr);
   if (cluster) {
     // values live in the cluster's shared memory: no flag words to clear
@@ -1254,6 +1322,7 @@ int sptrsv_gb300_destroy(sptrsv_handle_t h) {
   free_buf(h->tx);
   free_buf(h->c0);
   free_buf(h->wsplit);
+  free_buf(h->vals);
   if (h->ctl) cudaFree(h->ctl);
   if (h->flags) cudaFree(h->flags);
   if (h->host_pinned) cudaFreeHost(h->host_pinned);
@@ -1760,10 +1829,10 @@ int sptrsv_gb300_solve(sptrsv_handle_t h, const void* d_val, int dtype, int rhs,
   }
   if (dtype == SPTRSV_DTYPE_F64) {
     if (!h->staged64) return SPTRSV_ERR_STATE;
-    return solve_typed<double>(h, h->v64, rhs, layout, static_cast<const double*>(d_b), static_cast<double*>(d_x), s);
+    return solve_typed<double>(h, rhs, layout, static_cast<const double*>(d_b), static_cast<double*>(d_x), s);
   }
   if (!h->staged32) return SPTRSV_ERR_STATE;
-  return solve_typed<float>(h, h->v32, rhs, layout, static_cast<const float*>(d_b), static_cast<float*>(d_x), s);
+  return solve_typed<float>(h, rhs, layout, static_cast<const float*>(d_b), static_cast<float*>(d_x), s);
 }
 
 int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, int layout, const double* d_b,
@@ -1849,6 +1918,8 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
       }
       CUDA_TRY(cudaEventRecord(h->ev_exec[0], s));
     }
+    ST_TRY(need_forms<double>(h, FORM_DEP_W, s));
+    if (h->fused_refine != 2) ST_TRY(need_forms<float>(h, FORM_DEP_W, s));
     const float2* wsplit = nullptr;
     if (h->fused_refine == 2) {
       // the residual in double-float: (hi, lo) pairs of the FP64 weights, once per staging
@@ -1899,7 +1970,7 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
   } else {
     // X_0 = FP32 solve of (float) B
     CUDA_TRY(launch_cast_d2f(d_b, r32, count, s));
-    ST_TRY(solve_typed<float>(h, h->v32, rhs, layout, r32, d32, s, nullptr, false));
+    ST_TRY(solve_typed<float>(h, rhs, layout, r32, d32, s, nullptr, false));
     CUDA_TRY(cudaMemsetAsync(stats, 0, 2 * sizeof(unsigned long long), s));
     CUDA_TRY(launch_update(d_x, d32, count, stats, true, s));
     if (checked) {
@@ -1911,8 +1982,9 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
   }
   int steps = first - 1;  // refinement steps done
   for (it = first; !converged && it <= max_iter; ++it) {
+    ST_TRY(need_forms<double>(h, FORM_DEP_VAL, s));
     CUDA_TRY(launch_residual(h->layout, h->v64, rhs, d_b, d_x, si, sk, r32, s));
-    ST_TRY(solve_typed<float>(h, h->v32, rhs, layout, r32, d32, s, nullptr, false));
+    ST_TRY(solve_typed<float>(h, rhs, layout, r32, d32, s, nullptr, false));
     CUDA_TRY(cudaMemsetAsync(stats, 0, 2 * sizeof(unsigned long long), s));
     CUDA_TRY(launch_update(d_x, d32, count, stats, false, s));
     steps = it;
@@ -1971,7 +2043,7 @@ int sptrsv_gb300_solve_adjoint(sptrsv_handle_t h, const void* d_val, int dtype, 
     adj.xf = static_cast<const double*>(d_x);
     adj.xf_si = si;
     adj.xf_sk = sk;
-    return solve_typed<double>(h, h->v64, rhs, layout, static_cast<const double*>(d_g), static_cast<double*>(d_lambda),
+    return solve_typed<double>(h, rhs, layout, static_cast<const double*>(d_g), static_cast<double*>(d_lambda),
                                s, &adj);
   }
   if (!h->staged32) return SPTRSV_ERR_STATE;
@@ -1980,7 +2052,7 @@ int sptrsv_gb300_solve_adjoint(sptrsv_handle_t h, const void* d_val, int dtype, 
   adj.xf = static_cast<const float*>(d_x);
   adj.xf_si = si;
   adj.xf_sk = sk;
-  return solve_typed<float>(h, h->v32, rhs, layout, static_cast<const float*>(d_g), static_cast<float*>(d_lambda), s,
+  return solve_typed<float>(h, rhs, layout, static_cast<const float*>(d_g), static_cast<float*>(d_lambda), s,
                             &adj);
 }
 

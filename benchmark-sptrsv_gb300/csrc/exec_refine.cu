@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(256) k_pull_refine1(RefineArgs a) {
         row = a.perm[p];
         e = a.dep_ptr[p];
         e1 = a.dep_ptr[p + 1];
-        const float s32 = a.rcp32[p];
+        const float s32 = DF ? 0.f : a.rcp32[p];
         const double s64 = a.rcp64[p];
 #pragma unroll
         for (int r = 0; r < RPL; ++r) {

@@ -160,6 +160,15 @@ struct Layout {
   int* level_ptr = nullptr;  // [nlevels+1] (positions)
 };
 
+// Staged forms of the values (one array set each), staged when an executor
+// first needs them.
+enum ValueForm : unsigned {
+  FORM_DIAG = 1,     // diag, rcp
+  FORM_DEP_W = 2,    // dep_w
+  FORM_OUT_W = 4,    // out_w
+  FORM_DEP_VAL = 8,  // dep_val
+  FORM_OUT_VAL = 16  // out_val
+};
 template <typename T>
 struct Values {
   T* dep_val = nullptr;  // [ndep]
@@ -168,6 +177,7 @@ struct Values {
   T* out_w = nullptr;    // [ndep] values scaled by the reciprocal of the owning position's diagonal (ready order)
   T* diag = nullptr;     // [n]
   T* rcp = nullptr;      // [n] correctly rounded 1/diag
+  unsigned ready = 0;    // forms that hold the current values
 };
 
 // Independent triangles sharing one index space (a batch): unknown c belongs
@@ -243,7 +253,8 @@ cudaError_t launch_coarrival(const int* row_ptr, const int* col, const int* dept
 cudaError_t launch_sort_lists(const int* ptr, const int* pos, const int* src, int n, int count, bool descending,
                               int* pos_out, int* src_out, cudaStream_t s);
 template <typename TV, typename T>
-cudaError_t launch_stage_values(const Layout& L, const TV* val, Values<T>& V, int* flags, cudaStream_t s);
+cudaError_t launch_stage_values(const Layout& L, const TV* val, Values<T>& V, unsigned forms, int* flags,
+                                cudaStream_t s);
 
 // ---------------------------------------------------------------- execution
 // Transposed (adjoint) solve request: optional fused gradient w.r.t. the values.
