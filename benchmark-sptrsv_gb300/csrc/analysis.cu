@@ -813,7 +813,8 @@ cudaError_t launch_fill_push(const int* perm, const int* iperm, const int* col_p
 // Gathers the values of one list set (out[e] = val[src[e]], scaled by the
 // reciprocal of the owning position's diagonal for SCALE: x_p = b_p/d_p - sum_j
 // w_j x_j then needs one fused multiply-add per dependency). DIAG first stages
-// the diagonal and its reciprocal of the same positions.
+// the diagonal and its reciprocal of the same positions; `flags` (a word of
+// pinned host memory, or null) is set to SF_ZERO_DIAG on a zero or non-finite one.
 //
 // A warp takes 32 positions at a time: their lists are one contiguous range, so
 // its lanes walk entries, coalesced, and find an entry's owner among the 32 list
@@ -842,7 +843,7 @@ __global__ void __launch_bounds__(256) k_stage_lists(const int* __restrict__ ptr
         r = T(1) / d;
         diag[p] = d;
         rcp[p] = r;
-        if (flags && (!(d != T(0)) || !isfinite(d))) atomicOr(flags, SF_ZERO_DIAG);
+        if (flags && (!(d != T(0)) || !isfinite(d))) *reinterpret_cast<volatile int*>(flags) = SF_ZERO_DIAG;
       } else if (SCALE) {
         r = rcp[p];
       }

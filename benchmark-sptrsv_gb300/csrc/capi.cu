@@ -118,7 +118,8 @@ struct sptrsv_gb300_handle_s {
   bool wsplit_ok = false;
   DeviceCtl* ctl = nullptr;
   int* flags = nullptr;
-  int* host_pinned = nullptr;  // 4 ints
+  int* host_pinned = nullptr;  // 4 ints the device can write: [0] DeviceCtl::host_code, [1] structure
+                               // flags, [2] level count, [3] value flags
   int last_sched = 0;
   bool last_pipe = false;  // the last one-rhs solve ran the unit pipeline
   size_t device_bytes = 0;
@@ -295,27 +296,37 @@ unsigned long long timeout_ns(const sptrsv_gb300_handle_s* h) {
   return static_cast<unsigned long long>(h->timeout_ms) * 1000000ull;
 }
 
+// A clean control block that reports failures to host_pinned[0].
+cudaError_t init_ctl(sptrsv_gb300_handle_s* h, cudaStream_t s) {
+  DeviceCtl clean{};
+  clean.host_code = h->host_pinned;
+  const cudaError_t e = cudaMemcpyAsync(h->ctl, &clean, sizeof(clean), cudaMemcpyHostToDevice, s);
+  if (e != cudaSuccess) return e;
+  const cudaError_t done = cudaStreamSynchronize(s);
+  h->host_pinned[0] = DEV_OK;
+  return done;
+}
+
 // Clears the control block and the self-cleaning push workspace after a
 // failed launch left them dirty.
 int reset_after_failure(sptrsv_gb300_handle_s* h, cudaStream_t s) {
   cudaGetLastError();
-  CUDA_TRY(cudaMemsetAsync(h->ctl, 0, sizeof(DeviceCtl), s));
+  CUDA_TRY(init_ctl(h, s));
   if (h->left_sum.p) CUDA_TRY(cudaMemsetAsync(h->left_sum.p, 0, h->left_sum.bytes, s));
   if (h->counters.p) CUDA_TRY(cudaMemsetAsync(h->counters.p, 0, h->counters.bytes, s));
   CUDA_TRY(cudaStreamSynchronize(s));
   return SPTRSV_OK;
 }
 
+// Waits for the stream, then reads the code its kernels left in pinned host
+// memory (a 4-byte copy and a second wait cost a small solve ~10 us).
 int read_device_code(sptrsv_gb300_handle_s* h, cudaStream_t s, int* code) {
-  CUDA_TRY(cudaMemcpyAsync(h->host_pinned, &h->ctl->code, sizeof(int), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaStreamSynchronize(s));
-  *code = h->host_pinned[0];
+  *code = *reinterpret_cast<volatile int*>(h->host_pinned);
   return SPTRSV_OK;
 }
 
 int check_device(sptrsv_gb300_handle_s* h, cudaStream_t s) {
-  cudaError_t e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return map_cuda_error(e);
   int code = 0;
   ST_TRY(read_device_code(h, s, &code));
   if (code != DEV_OK) {
@@ -1006,12 +1017,12 @@ int stage_all(sptrsv_gb300_handle_s* h, const TV* val, cudaStream_t s, bool chec
   const unsigned forms = allocated_forms(V) | FORM_DIAG | FORM_DEP_W;
   ST_TRY(alloc_forms(h, V, forms));
   h->v64.ready = h->v32.ready = 0;
-  if (check) CUDA_TRY(cudaMemsetAsync(h->flags, 0, sizeof(int), s));
-  CUDA_TRY(launch_stage_values(h->layout, val, V, forms, h->flags, s));
+  volatile int* flags = check ? h->host_pinned + 3 : nullptr;
+  if (check) *flags = 0;
+  CUDA_TRY(launch_stage_values(h->layout, val, V, forms, const_cast<int*>(flags), s));
   if (check) {
-    int f = 0;
-    ST_TRY(read_flags(h, s, &f));
-    if (f & SF_ZERO_DIAG) return SPTRSV_ERR_BAD_STRUCTURE;
+    CUDA_TRY(cudaStreamSynchronize(s));
+    if (*flags & SF_ZERO_DIAG) return SPTRSV_ERR_BAD_STRUCTURE;
   }
   V.ready = forms;
   return SPTRSV_OK;
@@ -1295,12 +1306,13 @@ int sptrsv_gb300_create(sptrsv_handle_t* handle) {
   cudaError_t e = cudaGetDevice(&h->device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device);
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&h->ctl), sizeof(DeviceCtl));
-  if (e == cudaSuccess) e = cudaMemset(h->ctl, 0, sizeof(DeviceCtl));
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&h->flags), sizeof(int));
   if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&h->host_pinned), 4 * sizeof(int));
+  if (e == cudaSuccess) e = init_ctl(h, nullptr);
   if (e != cudaSuccess) {
     if (h->ctl) cudaFree(h->ctl);
     if (h->flags) cudaFree(h->flags);
+    if (h->host_pinned) cudaFreeHost(h->host_pinned);
     delete h;
     return map_cuda_error(e);
   }

@@ -21,8 +21,20 @@ struct alignas(64) DeviceCtl {
   int where;                // diagnostic: position whose wait ran out
   unsigned int barrier_count;
   unsigned int barrier_gen;
-  unsigned int pad[10];
+  int* host_code;           // pinned host copy of `code` (may be null): read after a
+                            // synchronisation without a copy of its own
+  unsigned int pad[8];
 };
+
+// Records the first failure of a launch, on the device and for the host.
+__device__ __forceinline__ void ctl_raise(DeviceCtl* ctl, int code, int where) {
+  if (atomicCAS(&ctl->code, DEV_OK, code) != DEV_OK) return;
+  ctl->where = where;
+  if (ctl->host_code) {
+    *reinterpret_cast<volatile int*>(ctl->host_code) = code;
+    __threadfence_system();
+  }
+}
 
 // ------------------------------------------------------------------ PTX wrappers
 __device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned* p) {
@@ -143,7 +155,7 @@ struct WaitBudget {
     if (start == 0) { start = now; return true; }
     if (*reinterpret_cast<volatile int*>(&ctl->code) != DEV_OK) return false;
     if (now - start > limit_ns) {
-      if (atomicCAS(&ctl->code, DEV_OK, DEV_TIMEOUT) == DEV_OK) ctl->where = where;
+      ctl_raise(ctl, DEV_TIMEOUT, where);
       return false;
     }
     return true;

@@ -1566,7 +1566,7 @@ cudaError_t launch_grad_values(const int* csc_row, const int* csc_col, int nnz, 
 // flags raised earlier in the stream) nothing is solved and DEV_BAD_INPUT is
 // recorded.
 __device__ __forceinline__ void raise_bad_input(DeviceCtl* ctl, int where) {
-  if (atomicCAS(&ctl->code, DEV_OK, DEV_BAD_INPUT) == DEV_OK) ctl->where = where;
+  ctl_raise(ctl, DEV_BAD_INPUT, where);
 }
 
 template <typename T>

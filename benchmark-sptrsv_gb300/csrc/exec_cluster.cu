@@ -242,11 +242,8 @@ __global__ void __launch_bounds__(512) k_pull_cluster(ClusterArgs<T> a) {
 }
 
 // Launch configuration of the executor; the attribute must outlive it.
-template <typename K>
-cudaError_t cluster_config(K kernel, const ClusterPlan& plan, size_t smem, cudaStream_t s, cudaLaunchConfig_t& cfg,
-                           cudaLaunchAttribute& at) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+void cluster_config(const ClusterPlan& plan, size_t smem, cudaStream_t s, cudaLaunchConfig_t& cfg,
+                    cudaLaunchAttribute& at) {
   at.id = cudaLaunchAttributeClusterDimension;
   at.val.clusterDim.x = 1u << kRankShift;
   at.val.clusterDim.y = 1;
@@ -257,7 +254,6 @@ cudaError_t cluster_config(K kernel, const ClusterPlan& plan, size_t smem, cudaS
   cfg.stream = s;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return e;
 }
 
 template <typename T>
@@ -278,8 +274,13 @@ bool cluster_fits(const ClusterPlan& plan, int n) {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at{};
     int clusters = 0;
-    if (cluster_config(cluster_kernel<T>(adj), plan, smem, nullptr, cfg, at) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&clusters, cluster_kernel<T>(adj), &cfg) != cudaSuccess || clusters < 1) {
+    auto kernel = cluster_kernel<T>(adj);
+    cluster_config(plan, smem, nullptr, cfg, at);
+    // set once per plan, to the device's limit whatever this plan needs, so that
+    // no launch has to set them
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
       cudaGetLastError();
       return false;
     }
@@ -307,8 +308,7 @@ cudaError_t launch_pull_cluster(const Layout& L, const Values<T>& V, const VecVi
   a.timeout_ns = timeout_ns;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at{};
-  const cudaError_t e = cluster_config(cluster_kernel<T>(adj), plan, plan.smem(L.n, sizeof(T)), s, cfg, at);
-  if (e != cudaSuccess) return e;
+  cluster_config(plan, plan.smem(L.n, sizeof(T)), s, cfg, at);
   return cudaLaunchKernelEx(&cfg, cluster_kernel<T>(adj), a);
 }
 template bool cluster_fits<double>(const ClusterPlan&, int);

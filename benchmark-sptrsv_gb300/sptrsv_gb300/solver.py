@@ -202,13 +202,15 @@ class SyncFreeSolver:
         [n, rhs] view (stride (1, n)) is solved in place of layout without a copy. Returns x with
         b's layout and dtype."""
         torch = _torch()
-        if b.dim() == 1:
+        if b.dim() == 1 and b.is_contiguous():
+            b2 = b   # one contiguous right-hand side: no two-dimensional views needed
+        elif b.dim() == 1:
             b2 = b.reshape(-1, 1)
         else:
             b2 = b
         if b2.shape[0] != self.n:
             raise ValueError(f"b has {b2.shape[0]} rows, the matrix has {self.n}")
-        rhs = int(b2.shape[1])
+        rhs = int(b2.shape[1]) if b2.dim() != 1 else 1
         if b2.is_contiguous():
             layout = LAYOUT_ROW_MAJOR
         elif b2.t().is_contiguous():
@@ -227,15 +229,16 @@ class SyncFreeSolver:
                 out = torch.empty_like(b2, memory_format=torch.contiguous_format)
             else:
                 out = torch.empty((rhs, self.n), dtype=b2.dtype, device=b2.device).t()
-        vptr = ctypes.c_void_p(0)
+        vptr = None
         if values is not None:
             v = values.to(self.device).contiguous()
             self.values = v
-            vptr = _ptr(v)
-        st = self._lib.sptrsv_gb300_solve(self._h, vptr, dt, rhs, layout, _ptr(b2), _ptr(out),
+            vptr = v.data_ptr()
+        st = self._lib.sptrsv_gb300_solve(self._h, vptr, dt, rhs, layout, b2.data_ptr(), out.data_ptr(),
                                           _stream_ptr(self._stream))
-        check(st, "solve")
-        return out.reshape(b.shape) if b.dim() == 1 else out
+        if st:
+            check(st, "solve")
+        return out.reshape(b.shape) if b.dim() == 1 and out.shape != b.shape else out
 
     def solve_refine(self, b, values=None, *, tol: float = 1e-12, max_iter: int = 10, out=None):
         """FP32 storage/solve + FP64-residual iterative refinement (b float64). Returns
