@@ -421,6 +421,69 @@ cudaError_t launch_expand_cols(const int* col_ptr, int n, int* col_of, cudaStrea
   return cudaGetLastError();
 }
 
+constexpr int kRankMax = 1024;  // longest list sorted by rank (k_rank_lists)
+
+// Column of every entry, and the entries dealt to their rows in any order:
+// (entry, column) at the next free slot of row r (cursor[r], row pointers on
+// entry). A warp takes 32 columns, whose entries are one contiguous range.
+__global__ void __launch_bounds__(kThreads) k_scatter_rows(const int* __restrict__ col_ptr,
+                                                           const int* __restrict__ row_idx, int n, int* cursor,
+                                                           int* col_of, int* entry_out, int* col_out) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  const long long groups = ((long long)n + 31) / 32;
+  for (long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; g < groups; g += nwarps) {
+    const long long c = g * 32 + lane;
+    const int start = c < n ? col_ptr[c] : INT_MAX;
+    const int end = c < n ? col_ptr[c + 1] : 0;
+    const unsigned lo = static_cast<unsigned>(__shfl_sync(kFull, start, 0));
+    const unsigned hi = static_cast<unsigned>(__reduce_max_sync(kFull, end));
+    for (unsigned base = lo; base < hi; base += 32) {
+      const unsigned e = base + lane;
+      int own = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const int t = __shfl_sync(kFull, start, own + step);
+        if (static_cast<unsigned>(t) <= e) own += step;
+      }
+      if (e >= hi) continue;
+      const int col = static_cast<int>(g * 32) + own;
+      const int slot = atomicAdd(&cursor[row_idx[e]], 1);
+      col_of[e] = col;
+      entry_out[slot] = static_cast<int>(e);
+      col_out[slot] = col;
+    }
+  }
+}
+
+// CSR rows from CSC columns by a counting transpose: scatter, then each row's
+// entries sorted by their CSC index (ascending column). row_ptr = exclusive
+// scan of the row counts, no row longer than kRankMax entries. (The stable
+// radix sort of all entries on their row took 0.65 ms for 3M entries.)
+bool transpose_by_rank(int longest_row) { return longest_row <= kRankMax; }
+
+cudaError_t launch_transpose_pattern(const int* col_ptr, const int* row_idx, const int* row_ptr, int n, int nnz,
+                                     int* col_of, int* src_out, int* col_out, cudaStream_t s) {
+  if (n <= 0 || nnz <= 0) return cudaSuccess;
+  int *cursor = nullptr, *entry = nullptr, *col = nullptr;
+  auto run = [&]() -> cudaError_t {
+    cudaError_t e;
+    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&cursor), sizeof(int) * n, s)) != cudaSuccess) return e;
+    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&entry), sizeof(int) * nnz, s)) != cudaSuccess) return e;
+    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&col), sizeof(int) * nnz, s)) != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(cursor, row_ptr, sizeof(int) * n, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
+    k_scatter_rows<<<grid_for(n), kThreads, 0, s>>>(col_ptr, row_idx, n, cursor, col_of, entry, col);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    return launch_rank_lists(row_ptr, entry, col, n, false, src_out, col_out, s);
+  };
+  const cudaError_t e = run();
+  if (cursor) cudaFreeAsync(cursor, s);
+  if (entry) cudaFreeAsync(entry, s);
+  if (col) cudaFreeAsync(col, s);
+  return e;
+}
+
 __global__ void k_copy_keys(const int* __restrict__ in, unsigned* out, int count) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += stride)
@@ -461,9 +524,60 @@ __global__ void k_owner_keys(const int* __restrict__ owner, const int* __restric
     keys[i] = static_cast<unsigned>(owner[idx[i]]);
 }
 
-cudaError_t launch_sort_lists(const int* ptr, const int* pos, const int* src, int n, int count, bool descending,
-                              int* pos_out, int* src_out, cudaStream_t s) {
+// Lists up to kRankMax entries are sorted by rank: an entry's place in its list
+// is the number of smaller keys there (keys are distinct inside a list). A warp
+// takes the lists of 32 consecutive owners, one contiguous range; its lanes walk
+// the entries and, as neighbours mostly share a list, read each list's keys as
+// broadcasts. Two stable radix sorts of all entries (by position, then by owner)
+// took 0.80 ms for the lists of a 2.7M-entry system and 8.1 ms for those of 33M
+// entries (lists up to 1,000).
+__global__ void __launch_bounds__(kThreads) k_rank_lists(const int* __restrict__ ptr, const int* __restrict__ key,
+                                                         const int* __restrict__ src, int n, int descending,
+                                                         int* key_out, int* src_out) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  const long long groups = ((long long)n + 31) / 32;
+  for (long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; g < groups; g += nwarps) {
+    const long long p = g * 32 + lane;
+    const int start = p < n ? ptr[p] : INT_MAX;
+    const int end = p < n ? ptr[p + 1] : 0;
+    const unsigned lo = static_cast<unsigned>(__shfl_sync(kFull, start, 0));
+    const unsigned hi = static_cast<unsigned>(__reduce_max_sync(kFull, end));
+    for (unsigned base = lo; base < hi; base += 32) {
+      const unsigned e = base + lane;
+      // the last list that starts at or before e owns it (empty lists share
+      // their successor's start)
+      int own = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const int t = __shfl_sync(kFull, start, own + step);
+        if (static_cast<unsigned>(t) <= e) own += step;
+      }
+      const int s0 = __shfl_sync(kFull, start, own), s1 = __shfl_sync(kFull, end, own);
+      if (e >= hi) continue;
+      const int k = key[e];
+      int rank = 0;
+#pragma unroll 4
+      for (int j = s0; j < s1; ++j) rank += key[j] < k ? 1 : 0;
+      if (descending) rank = s1 - s0 - 1 - rank;
+      key_out[s0 + rank] = k;
+      src_out[s0 + rank] = src[e];
+    }
+  }
+}
+
+cudaError_t launch_rank_lists(const int* ptr, const int* key, const int* src, int n, bool descending, int* key_out,
+                              int* src_out, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  k_rank_lists<<<grid_for(n), kThreads, 0, s>>>(ptr, key, src, n, descending ? 1 : 0, key_out, src_out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_sort_lists(const int* ptr, const int* pos, const int* src, int n, int count, int longest,
+                              bool descending, int* pos_out, int* src_out, cudaStream_t s) {
   if (count <= 0 || n <= 0) return cudaSuccess;
+  if (longest <= kRankMax) return launch_rank_lists(ptr, pos, src, n, descending, pos_out, src_out, s);
   int bits = 1;
   while (bits < 31 && (1u << bits) <= static_cast<unsigned>(n - 1)) ++bits;
   unsigned *k1 = nullptr, *k2 = nullptr;
@@ -498,12 +612,71 @@ cudaError_t launch_sort_lists(const int* ptr, const int* pos, const int* src, in
 }
 
 // ------------------------------------------------------------ schedule heuristics
+// The plan's counters (PlanCounter, summed or maximised into count[]). Grids of
+// a few CTAs per SM with one atomic per CTA and counter: with one per warp the
+// same-address atomics took 130-200 us of a 6-10M-entry analysis.
+namespace {
+constexpr int kStatGrid = 152 * 8;
+
+__device__ __forceinline__ unsigned long long block_sum(unsigned long long v, unsigned long long* s_warp) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = v;
+  __syncthreads();
+  unsigned long long t = 0;
+  for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += s_warp[w];
+  return t;
+}
+}  // namespace
+
+// Longest dependency list (CSR rows) and longest dependent list (CSC columns),
+// and the entries of lists longer than `cut` on either side (diagonals excluded).
+__global__ void k_list_stats(const int* __restrict__ row_ptr, const int* __restrict__ col_ptr, int n, int cut,
+                             unsigned long long* count) {
+  __shared__ unsigned long long s_warp[kThreads / 32];
+  __shared__ int s_max[2];
+  if (threadIdx.x < 2) s_max[threadIdx.x] = 0;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  unsigned long long row_long = 0, col_long = 0;
+  int row_max = 0, col_max = 0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
+    const int r = row_ptr[i + 1] - row_ptr[i] - 1, c = col_ptr[i + 1] - col_ptr[i] - 1;
+    row_max = max(row_max, r);
+    col_max = max(col_max, c);
+    if (r > cut) row_long += r;
+    if (c > cut) col_long += c;
+  }
+  row_max = __reduce_max_sync(0xffffffffu, row_max);
+  col_max = __reduce_max_sync(0xffffffffu, col_max);
+  row_long = block_sum(row_long, s_warp);
+  col_long = block_sum(col_long, s_warp);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&s_max[0], row_max);
+    atomicMax(&s_max[1], col_max);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    atomicMax(&count[PC_ROW_MAX], static_cast<unsigned long long>(s_max[0]));
+    atomicMax(&count[PC_COL_MAX], static_cast<unsigned long long>(s_max[1]));
+    if (row_long) atomicAdd(&count[PC_ROW_LONG], row_long);
+    if (col_long) atomicAdd(&count[PC_COL_LONG], col_long);
+  }
+}
+
+cudaError_t launch_list_stats(const int* row_ptr, const int* col_ptr, int n, int cut, unsigned long long* count,
+                              cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  k_list_stats<<<grid_for(n, kThreads, kStatGrid), kThreads, 0, s>>>(row_ptr, col_ptr, n, cut, count);
+  return cudaGetLastError();
+}
+
 // Off-diagonal entries whose row and column fall in the same block of `block`
 // unknowns of the natural execution order (ascending for a forward solve,
 // descending for a backward one): how much of the DAG a blocked order keeps
 // inside one CTA.
 __global__ void k_block_locality(const int* __restrict__ row, const int* __restrict__ col, int nnz, int n,
                                  int block, int backward, unsigned long long* count) {
+  __shared__ unsigned long long s_warp[kThreads / 32];
   const long long stride = (long long)gridDim.x * blockDim.x;
   unsigned local = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nnz; i += stride) {
@@ -512,23 +685,25 @@ __global__ void k_block_locality(const int* __restrict__ row, const int* __restr
     const int pr = backward ? n - 1 - r : r, pc = backward ? n - 1 - c : c;
     local += (pr / block == pc / block) ? 1u : 0u;
   }
-  for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-  if ((threadIdx.x & 31) == 0 && local) atomicAdd(count, (unsigned long long)local);
+  const unsigned long long total = block_sum(local, s_warp);
+  if (threadIdx.x == 0 && total) atomicAdd(&count[PC_LOCAL], total);
 }
 
 cudaError_t launch_block_locality(const int* row, const int* col, int nnz, int n, int block, bool backward,
                                   unsigned long long* count, cudaStream_t s) {
   if (nnz <= 0) return cudaSuccess;
-  k_block_locality<<<grid_for(nnz), kThreads, 0, s>>>(row, col, nnz, n, block, backward ? 1 : 0, count);
+  k_block_locality<<<grid_for(nnz, kThreads, kStatGrid), kThreads, 0, s>>>(row, col, nnz, n, block, backward ? 1 : 0,
+                                                                           count);
   return cudaGetLastError();
 }
 
 // Unknowns with two or more dependencies on the level just before their own
-// (count[0]; in a warp-synchronous loop those dependencies land in the same
-// iteration) and unknowns with any dependency (count[1]), over the CSR rows
-// (diagonal included in each row and skipped here).
+// (in a warp-synchronous loop those dependencies land in the same iteration)
+// and unknowns with any dependency, over the CSR rows (diagonal included in
+// each row and skipped here).
 __global__ void k_coarrival(const int* __restrict__ row_ptr, const int* __restrict__ col,
                             const int* __restrict__ depth, int n, unsigned long long* count) {
+  __shared__ unsigned long long s_warp[kThreads / 32];
   const long long stride = (long long)gridDim.x * blockDim.x;
   unsigned co = 0, any = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -543,20 +718,17 @@ __global__ void k_coarrival(const int* __restrict__ row_ptr, const int* __restri
     co += k >= 2 ? 1u : 0u;
     any += deps > 0 ? 1u : 0u;
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    co += __shfl_xor_sync(0xffffffffu, co, o);
-    any += __shfl_xor_sync(0xffffffffu, any, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (co) atomicAdd(&count[0], (unsigned long long)co);
-    if (any) atomicAdd(&count[1], (unsigned long long)any);
+  const unsigned long long co_total = block_sum(co, s_warp), any_total = block_sum(any, s_warp);
+  if (threadIdx.x == 0) {
+    if (co_total) atomicAdd(&count[PC_COARRIVE], co_total);
+    if (any_total) atomicAdd(&count[PC_DEPENDENT], any_total);
   }
 }
 
 cudaError_t launch_coarrival(const int* row_ptr, const int* col, const int* depth, int n, unsigned long long* count,
                              cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_coarrival<<<grid_for(n), kThreads, 0, s>>>(row_ptr, col, depth, n, count);
+  k_coarrival<<<grid_for(n, kThreads, kStatGrid), kThreads, 0, s>>>(row_ptr, col, depth, n, count);
   return cudaGetLastError();
 }
 

@@ -93,9 +93,10 @@ struct sptrsv_gb300_handle_s {
   int layout_block = -1;
   int layout_stretched = 0;        // the layout's level order is stretched per system (batches)
   std::vector<int> layout_units;   // blocked layouts: start positions of the units (+ n), else empty
-  std::vector<int> dep_cnt_host;   // dependencies per position
+  std::vector<int> dep_cnt_host;   // dependencies per position (list_counts)
   std::vector<int> out_cnt_host;   // dependents per position
   int max_dep_cnt = 0, max_out_cnt = 0;
+  long long long_deps = 0, long_outs = 0;  // entries of long lists (long_cut)
   ChunkTable tab_fwd, tab_adj;
   PieceTable pc_fwd, pc_adj;
   ImportTable imports;
@@ -362,6 +363,8 @@ int build_layout(sptrsv_gb300_handle_s* h, int block, cudaStream_t s) {
   free_values(h->v32);
   h->staged64 = h->staged32 = false;
   h->wsplit_ok = false;
+  h->dep_cnt_host.clear();
+  h->out_cnt_host.clear();
   Layout& L = h->layout;
   const int n = h->n;
   const int ndep = h->nnz - n;
@@ -403,10 +406,13 @@ int build_layout(sptrsv_gb300_handle_s* h, int block, cudaStream_t s) {
       CUDA_TRY(cudaMallocAsync(&temp, radix_sort_temp_bytes(n), s));
       // long dependency lists first inside each level (so chunks of one mode form), then
       // level order, then (blocked orders) the natural block
-      int* rows_ls = nullptr;
-      CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&rows_ls), sizeof(int) * n, s));
-      CUDA_TRY(launch_long_keys(rows_nat, h->in_degree, n, kLongDeps, keys, s));
-      CUDA_TRY(radix_sort_pairs(keys, rows_nat, keys_sorted, rows_ls, n, 1, temp, s));
+      int* rows_ls = rows_nat;
+      if (h->max_dep_cnt > kLongDeps) {
+        rows_ls = nullptr;
+        CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&rows_ls), sizeof(int) * n, s));
+        CUDA_TRY(launch_long_keys(rows_nat, h->in_degree, n, kLongDeps, keys, s));
+        CUDA_TRY(radix_sort_pairs(keys, rows_nat, keys_sorted, rows_ls, n, 1, temp, s));
+      }
       if (stretched) {
         // every system's levels spread over 65 % of the batch's depth (or its
         // own depth, if deeper), so a deep system's chain does not queue behind
@@ -426,7 +432,7 @@ int build_layout(sptrsv_gb300_handle_s* h, int block, cudaStream_t s) {
       }
       CUDA_TRY(radix_sort_pairs(keys, rows_ls, keys_sorted, level_order ? L.perm : rows_lv, n,
                                 bits_for(h->nlevels - 1), temp, s));
-      CUDA_TRY(cudaFreeAsync(rows_ls, s));
+      if (rows_ls != rows_nat) CUDA_TRY(cudaFreeAsync(rows_ls, s));
       if (!level_order) {
         CUDA_TRY(launch_schedule_keys(rows_lv, h->depth, n, sd, block, 1, keys, s));
         int max_sys = 0;
@@ -436,13 +442,17 @@ int build_layout(sptrsv_gb300_handle_s* h, int block, cudaStream_t s) {
         if (max_key > 0xFFFFFFFFLL) return SPTRSV_ERR_UNSUPPORTED;
         CUDA_TRY(radix_sort_pairs(keys, rows_lv, keys_sorted, L.perm, n, bits_for(max_key - 1), temp, s));
         // units of the blocked order (one system's natural block): contiguous
-        // position ranges, the work units of the importer executor
-        std::vector<unsigned> ks(n);
-        CUDA_TRY(cudaMemcpyAsync(ks.data(), keys_sorted, sizeof(unsigned) * (size_t)n, cudaMemcpyDeviceToHost, s));
-        CUDA_TRY(cudaStreamSynchronize(s));
-        h->layout_units.clear();
-        for (int i = 0; i < n; ++i)
-          if (i == 0 || ks[i] != ks[i - 1]) h->layout_units.push_back(i);
+        // position ranges, the work units of the importer executor; block by
+        // block, the systems that reach into it in turn
+        const std::vector<int> single(1, n);
+        const std::vector<int>& sizes = h->sys_n_host.empty() ? single : h->sys_n_host;
+        int at = 0;
+        for (long long lo = 0; lo < max_sys; lo += block)
+          for (int size : sizes)
+            if (size > lo) {
+              h->layout_units.push_back(at);
+              at += static_cast<int>(std::min<long long>(block, size - lo));
+            }
         h->layout_units.push_back(n);
       }
       CUDA_TRY(cudaFreeAsync(keys, s));
@@ -460,25 +470,10 @@ int build_layout(sptrsv_gb300_handle_s* h, int block, cudaStream_t s) {
                               L.dep_pos, L.dep_src, L.dep_col, L.diag_src, s));
     CUDA_TRY(launch_fill_push(L.perm, L.iperm, h->csc_ptr, h->csc_row, L.out_ptr, n, sd, L.out_pos,
                               L.out_src, s));
-    CUDA_TRY(launch_sort_lists(L.dep_ptr, L.dep_pos, L.dep_src, n, ndep, false, L.dep_pos_f, L.dep_src_f, s));
-    CUDA_TRY(launch_sort_lists(L.out_ptr, L.out_pos, L.out_src, n, ndep, true, L.out_pos_f, L.out_src_f, s));
-    std::vector<int> ptr((size_t)n + 1);
-    CUDA_TRY(cudaMemcpyAsync(ptr.data(), L.dep_ptr, sizeof(int) * ((size_t)n + 1), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaStreamSynchronize(s));
-    h->dep_cnt_host.resize(n);
-    h->max_dep_cnt = 0;
-    for (int p = 0; p < n; ++p) {
-      h->dep_cnt_host[p] = ptr[p + 1] - ptr[p];
-      h->max_dep_cnt = std::max(h->max_dep_cnt, h->dep_cnt_host[p]);
-    }
-    CUDA_TRY(cudaMemcpyAsync(ptr.data(), L.out_ptr, sizeof(int) * ((size_t)n + 1), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaStreamSynchronize(s));
-    h->out_cnt_host.resize(n);
-    h->max_out_cnt = 0;
-    for (int p = 0; p < n; ++p) {
-      h->out_cnt_host[p] = ptr[p + 1] - ptr[p];
-      h->max_out_cnt = std::max(h->max_out_cnt, h->out_cnt_host[p]);
-    }
+    CUDA_TRY(launch_sort_lists(L.dep_ptr, L.dep_pos, L.dep_src, n, ndep, h->max_dep_cnt, false,
+                               L.dep_pos_f, L.dep_src_f, s));
+    CUDA_TRY(launch_sort_lists(L.out_ptr, L.out_pos, L.out_src, n, ndep, h->max_out_cnt, true,
+                               L.out_pos_f, L.out_src_f, s));
   }
   if (level_order && !stretched) {
     L.nlevels = h->nlevels;
@@ -491,6 +486,21 @@ int build_layout(sptrsv_gb300_handle_s* h, int block, cudaStream_t s) {
   CUDA_TRY(cudaStreamSynchronize(s));
   h->layout_block = block;
   h->layout_stretched = stretched ? 1 : 0;
+  return SPTRSV_OK;
+}
+
+// List lengths by position, fetched when a table is first built from them.
+int list_counts(sptrsv_gb300_handle_s* h, bool adj, cudaStream_t s, const std::vector<int>** out) {
+  std::vector<int>& counts = adj ? h->out_cnt_host : h->dep_cnt_host;
+  *out = &counts;
+  const int n = h->layout.n;
+  if (static_cast<int>(counts.size()) == n) return SPTRSV_OK;
+  std::vector<int> ptr((size_t)n + 1);
+  CUDA_TRY(cudaMemcpyAsync(ptr.data(), adj ? h->layout.out_ptr : h->layout.dep_ptr, sizeof(int) * ((size_t)n + 1),
+                           cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(cudaStreamSynchronize(s));
+  counts.resize(n);
+  for (int p = 0; p < n; ++p) counts[p] = ptr[p + 1] - ptr[p];
   return SPTRSV_OK;
 }
 
@@ -535,10 +545,12 @@ int build_table(sptrsv_gb300_handle_s* h, ChunkTable& t, const std::vector<int>&
   return SPTRSV_OK;
 }
 
-int ensure_table(sptrsv_gb300_handle_s* h, bool adj, int cmax, int emax) {
+int ensure_table(sptrsv_gb300_handle_s* h, bool adj, int cmax, int emax, cudaStream_t s) {
   ChunkTable& t = adj ? h->tab_adj : h->tab_fwd;
   if (t.start && t.cmax == cmax && t.emax == emax) return SPTRSV_OK;
-  return build_table(h, t, adj ? h->out_cnt_host : h->dep_cnt_host, adj, cmax, emax);
+  const std::vector<int>* counts = nullptr;
+  ST_TRY(list_counts(h, adj, s, &counts));
+  return build_table(h, t, *counts, adj, cmax, emax);
 }
 
 // Piece table over a walk (see PieceTable): lists longer than `split` entries
@@ -635,7 +647,9 @@ int build_pieces(sptrsv_gb300_handle_s* h, PieceTable& t, const std::vector<int>
 int ensure_pieces(sptrsv_gb300_handle_s* h, bool adj, int split, int chunk, cudaStream_t s) {
   PieceTable& t = adj ? h->pc_adj : h->pc_fwd;
   if (t.walk && t.split == split && t.chunk == chunk) return SPTRSV_OK;
-  return build_pieces(h, t, adj ? h->out_cnt_host : h->dep_cnt_host, adj, split, chunk, s);
+  const std::vector<int>* counts = nullptr;
+  ST_TRY(list_counts(h, adj, s, &counts));
+  return build_pieces(h, t, *counts, adj, split, chunk, s);
 }
 
 // Import table of the forward walk for chunks of `chunk` positions (see
@@ -841,17 +855,6 @@ int effective_block(const sptrsv_gb300_handle_s* h) {
 // the wave: 1M-row band 1.109 vs 1.139 ms, 500k-row band 2.21 vs 2.68 ms),
 // two up to 8,192 (4M-row power-law 1.68 vs 1.76 ms forward, 2.19 vs 2.60
 // backward), three beyond (a 4M-row band with 17,468 per level 0.51 vs 0.60).
-double long_share(const std::vector<int>& ptr, int cut) {
-  long long all = 0, lng = 0;
-  for (size_t i = 0; i + 1 < ptr.size(); ++i) {
-    const int c = ptr[i + 1] - ptr[i] - 1;  // entries without the diagonal
-    if (c <= 0) continue;
-    all += c;
-    if (c > cut) lng += c;
-  }
-  return all ? static_cast<double>(lng) / static_cast<double>(all) : 0.0;
-}
-
 // One-cluster executor (k_pull_cluster, exec_cluster.cu): a single system in
 // level order with at most kClusterDeps dependencies and kClusterWidth unknowns
 // per level on average and no lists to split, whose values fit the cluster's
@@ -886,53 +889,74 @@ void plan_cluster(sptrsv_gb300_handle_s* h) {
   P.narrow = deps <= kClusterDeps && n <= kClusterWidth * nl;
 }
 
-int make_plan(sptrsv_gb300_handle_s* h, const std::vector<int>& row_ptr, cudaStream_t s) {
+// Entries in lists of more than this many (diagonal excluded) count as long.
+int long_cut(const sptrsv_gb300_handle_s* h) {
+  return h->n > 0 ? std::max<int>(32, static_cast<int>(4.0 * (double)(h->nnz - h->n) / (double)h->n)) : 32;
+}
+
+// Runs `launch` over the plan's counters and reads them back.
+template <class F>
+int plan_counters(unsigned long long (&count)[PC_COUNT], cudaStream_t s, F launch) {
+  unsigned long long* d_count = nullptr;
+  CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&d_count), sizeof(count), s));
+  cudaError_t e = cudaMemsetAsync(d_count, 0, sizeof(count), s);
+  if (e == cudaSuccess) e = launch(d_count);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(count, d_count, sizeof(count), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaFreeAsync(d_count, s);
+  CUDA_TRY(e);
+  return SPTRSV_OK;
+}
+
+// Longest lists and long entries of the pattern, counted on the device.
+int list_stats(sptrsv_gb300_handle_s* h, cudaStream_t s) {
+  h->max_in_degree = h->max_dep_cnt = h->max_out_cnt = 0;
+  h->long_deps = h->long_outs = 0;
+  if (h->n <= 0) return SPTRSV_OK;
+  unsigned long long count[PC_COUNT] = {};
+  ST_TRY(plan_counters(count, s, [&](unsigned long long* d) {
+    return launch_list_stats(h->csr_ptr, h->csc_ptr, h->n, long_cut(h), d, s);
+  }));
+  h->max_dep_cnt = static_cast<int>(count[PC_ROW_MAX]);
+  h->max_out_cnt = static_cast<int>(count[PC_COL_MAX]);
+  h->max_in_degree = h->max_dep_cnt + 1;
+  h->long_deps = static_cast<long long>(count[PC_ROW_LONG]);
+  h->long_outs = static_cast<long long>(count[PC_COL_LONG]);
+  return SPTRSV_OK;
+}
+
+int make_plan(sptrsv_gb300_handle_s* h, cudaStream_t s) {
   auto& P = h->plan;
   P = sptrsv_gb300_handle_s::AutoPlan();
   const int n = h->n, nnz = h->nnz, nl = h->nlevels;
   if (n > 0) {
-    std::vector<int> col_ptr((size_t)n + 1);
-    CUDA_TRY(cudaMemcpyAsync(col_ptr.data(), h->csc_ptr, sizeof(int) * ((size_t)n + 1), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaStreamSynchronize(s));
-    const int cut = std::max<int>(32, static_cast<int>(4.0 * (double)(nnz - n) / (double)n));
-    P.split_fwd = long_share(row_ptr, cut) > 0.05 ? 32 : 0;
-    P.split_adj = long_share(col_ptr, cut) > 0.05 ? 8 : 0;  // the reverse walk measured best with short pieces
-    if (h->batch_count == 1 && nl > 0) {
-      const long long width = ((long long)n + nl - 1) / nl;
-      P.ctas = width < 1536 ? 1 : (width < 8192 ? 2 : 3);
+    const double deps = static_cast<double>(nnz - n);
+    P.split_fwd = deps > 0 && h->long_deps / deps > 0.05 ? 32 : 0;
+    P.split_adj = deps > 0 && h->long_outs / deps > 0.05 ? 8 : 0;  // the reverse walk measured best with short pieces
+    const long long width = nl > 0 ? ((long long)n + nl - 1) / nl : 0;
+    if (h->batch_count == 1 && nl > 0) P.ctas = width < 1536 ? 1 : (width < 8192 ? 2 : 3);
+    const bool deep = nl >= 256 && h->batch_count == 1 && nnz > n && width <= 4096;
+    const bool short_lists = nnz > n && (long long)(nnz - n) <= 3LL * (long long)n;
+    const int blk = static_cast<int>(std::min<long long>(24576, std::max<long long>(2048, (32 * width + 31) / 32 * 32)));
+    if (deep || short_lists) {
+      unsigned long long count[PC_COUNT] = {};
+      ST_TRY(plan_counters(count, s, [&](unsigned long long* d) {
+        cudaError_t e = cudaSuccess;
+        if (short_lists) e = launch_coarrival(h->csr_ptr, h->csr_col, h->depth, n, d, s);
+        if (e == cudaSuccess && deep)
+          e = launch_block_locality(h->csc_row, h->csc_col, nnz, n, blk, h->substitution == 1, d, s);
+        return e;
+      }));
+      if (count[PC_DEPENDENT])
+        P.coarrive = static_cast<double>(count[PC_COARRIVE]) / static_cast<double>(count[PC_DEPENDENT]);
+      if (deep) P.locality = static_cast<double>(count[PC_LOCAL]) / deps;
     }
-    if (nnz > n && (long long)(nnz - n) <= 3LL * (long long)n) {
-      unsigned long long* d_count = nullptr;
-      CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&d_count), 2 * sizeof(unsigned long long), s));
-      CUDA_TRY(cudaMemsetAsync(d_count, 0, 2 * sizeof(unsigned long long), s));
-      CUDA_TRY(launch_coarrival(h->csr_ptr, h->csr_col, h->depth, n, d_count, s));
-      unsigned long long count[2] = {0, 0};
-      CUDA_TRY(cudaMemcpyAsync(count, d_count, sizeof(count), cudaMemcpyDeviceToHost, s));
-      CUDA_TRY(cudaStreamSynchronize(s));
-      CUDA_TRY(cudaFree(d_count));
-      P.coarrive = count[1] ? static_cast<double>(count[0]) / static_cast<double>(count[1]) : 0.0;
-    }
-  }
-  if (n > 0 && nl >= 256 && h->batch_count == 1 && nnz > n) {
-    const long long width = ((long long)n + nl - 1) / nl;
-    if (width <= 4096) {
-      const int blk = static_cast<int>(std::min<long long>(24576, std::max<long long>(2048, (32 * width + 31) / 32 * 32)));
-      unsigned long long* d_count = nullptr;
-      CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&d_count), sizeof(unsigned long long), s));
-      CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), s));
-      CUDA_TRY(launch_block_locality(h->csc_row, h->csc_col, nnz, n, blk, h->substitution == 1, d_count, s));
-      unsigned long long count = 0;
-      CUDA_TRY(cudaMemcpyAsync(&count, d_count, sizeof(count), cudaMemcpyDeviceToHost, s));
-      CUDA_TRY(cudaStreamSynchronize(s));
-      CUDA_TRY(cudaFree(d_count));
-      P.locality = static_cast<double>(count) / static_cast<double>(nnz - n);
-      if (P.locality >= 0.96) {
-        P.order_block = blk;
-        P.chunk = blk;
-        P.block = 128;
-        P.ctas = 0;
-        P.backoff = 0;
-      }
+    if (P.locality >= 0.96) {
+      P.order_block = blk;
+      P.chunk = blk;
+      P.block = 128;
+      P.ctas = 0;
+      P.backoff = 0;
     }
   }
   plan_cluster(h);
@@ -1200,7 +1224,7 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
              (c.emax > 0 ? fit_emax(c.chunk, sizeof(T), c.stages, c.smem_tier, c.emax) == c.emax
                          : auto_emax(c.chunk, sizeof(T), c.stages, c.smem_tier) > 0)) {
     const int emax = c.emax > 0 ? c.emax : auto_emax(c.chunk, sizeof(T), c.stages, c.smem_tier);
-    ST_TRY(ensure_table(h, adj != nullptr, c.chunk, emax));
+    ST_TRY(ensure_table(h, adj != nullptr, c.chunk, emax, s));
     CUDA_TRY(launch_pull_staged<T>(h->layout, V, adj ? h->tab_adj : h->tab_fwd, v, static_cast<T*>(h->xw.p), h->ctl,
                                    c, timeout_ns(h), h->num_sms, s, adj));
   } else if (rhs == 1 && c.wsync && !c.exact && !adj && h->pipe_option && h->layout_block < n &&
@@ -1524,31 +1548,33 @@ int analyse_core(sptrsv_handle_t h, const int* d_colPtr, const int* d_rowIdx, cu
   CUDA_TRY(cudaMemsetAsync(h->in_degree, 0, sizeof(int) * (size_t)(n > 0 ? n : 1), s));
   CUDA_TRY(launch_in_degree(h->csc_row, n, nnz, h->in_degree, s));
 
-  // 3. CSR transpose by a stable sort of the CSC entries on their row
+  // 3. CSR transpose: a counting transpose, or (rows too long for it) a stable sort of
+  // the CSC entries on their row
   ST_TRY(dev_alloc(h, &h->csr_ptr, (size_t)n + 1));
   ST_TRY(dev_alloc(h, &h->csr_col, nnz));
   ST_TRY(dev_alloc(h, &h->csr_src, nnz));
   CUDA_TRY(exclusive_scan_int(h->in_degree, h->csr_ptr, n, true, s));
-  if (nnz > 0) {
+  ST_TRY(dev_alloc(h, &h->csc_col, nnz));
+  ST_TRY(list_stats(h, s));
+  if (nnz > 0 && transpose_by_rank(h->max_in_degree)) {
+    CUDA_TRY(launch_transpose_pattern(h->csc_ptr, h->csc_row, h->csr_ptr, n, nnz, h->csc_col, h->csr_src, h->csr_col,
+                                      s));
+  } else if (nnz > 0) {
     unsigned *keys = nullptr, *keys_sorted = nullptr;
-    int *iota = nullptr, *col_of = nullptr;
+    int* iota = nullptr;
     void* temp = nullptr;
     CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&keys), sizeof(unsigned) * nnz, s));
     CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&keys_sorted), sizeof(unsigned) * nnz, s));
     CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&iota), sizeof(int) * nnz, s));
-    CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&col_of), sizeof(int) * nnz, s));
     CUDA_TRY(cudaMallocAsync(&temp, radix_sort_temp_bytes(nnz), s));
     CUDA_TRY(launch_copy_keys(h->csc_row, keys, nnz, s));
     CUDA_TRY(launch_iota(iota, nnz, 0, 1, s));
     CUDA_TRY(radix_sort_pairs(keys, iota, keys_sorted, h->csr_src, nnz, bits_for(n - 1), temp, s));
-    CUDA_TRY(launch_expand_cols(h->csc_ptr, n, col_of, s));
-    CUDA_TRY(launch_gather_int(col_of, h->csr_src, h->csr_col, nnz, s));
-    ST_TRY(dev_alloc(h, &h->csc_col, nnz));
-    CUDA_TRY(cudaMemcpyAsync(h->csc_col, col_of, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToDevice, s));
+    CUDA_TRY(launch_expand_cols(h->csc_ptr, n, h->csc_col, s));
+    CUDA_TRY(launch_gather_int(h->csc_col, h->csr_src, h->csr_col, nnz, s));
     CUDA_TRY(cudaFreeAsync(keys, s));
     CUDA_TRY(cudaFreeAsync(keys_sorted, s));
     CUDA_TRY(cudaFreeAsync(iota, s));
-    CUDA_TRY(cudaFreeAsync(col_of, s));
     CUDA_TRY(cudaFreeAsync(temp, s));
   }
 
@@ -1617,17 +1643,9 @@ int analyse_core(sptrsv_handle_t h, const int* d_colPtr, const int* d_rowIdx, cu
     CUDA_TRY(cudaFreeAsync(iota, s));
     CUDA_TRY(cudaFreeAsync(temp, s));
   }
-  // max in-degree, from the CSR row pointers
-  h->max_in_degree = 0;
-  std::vector<int> rp(n > 0 ? (size_t)n + 1 : 0);
-  if (n > 0) {
-    CUDA_TRY(cudaMemcpyAsync(rp.data(), h->csr_ptr, sizeof(int) * ((size_t)n + 1), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaStreamSynchronize(s));
-    for (int i = 0; i < n; ++i) h->max_in_degree = std::max(h->max_in_degree, rp[i + 1] - rp[i]);
-  }
   h->analysed = true;
   // 5. execution plan, schedule and layouts
-  ST_TRY(make_plan(h, rp, s));
+  ST_TRY(make_plan(h, s));
   ST_TRY(build_layout(h, effective_block(h), s));
   CUDA_TRY(cudaEventRecord(e1, s));
   CUDA_TRY(cudaEventSynchronize(e1));

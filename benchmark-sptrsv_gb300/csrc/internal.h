@@ -241,17 +241,35 @@ cudaError_t launch_fill_pull(const int* perm, const int* iperm, const int* csr_p
 cudaError_t launch_fill_push(const int* perm, const int* iperm, const int* col_ptr, const int* row_idx,
                              const int* out_ptr, int n, const SysDesc& sd, int* out_pos, int* out_src,
                              cudaStream_t s);
-// count += off-diagonal entries whose row and column share a block of `block`
-// unknowns in the natural execution order.
+// Counters the plan is made from (device array of PC_COUNT words, zeroed first).
+enum PlanCounter {
+  PC_ROW_MAX,    // longest dependency list
+  PC_ROW_LONG,   // entries of dependency lists longer than the cut
+  PC_COL_MAX,    // longest dependent list
+  PC_COL_LONG,   // entries of dependent lists longer than the cut
+  PC_COARRIVE,   // unknowns with two or more dependencies on the level just before their own
+  PC_DEPENDENT,  // unknowns with any dependency
+  PC_LOCAL,      // off-diagonal entries inside a block of the natural execution order
+  PC_COUNT
+};
+cudaError_t launch_list_stats(const int* row_ptr, const int* col_ptr, int n, int cut, unsigned long long* count,
+                              cudaStream_t s);
 cudaError_t launch_block_locality(const int* row, const int* col, int nnz, int n, int block, bool backward,
                                   unsigned long long* count, cudaStream_t s);
-// count[0] += unknowns with two or more dependencies on the level just before
-// their own, count[1] += unknowns with any dependency (CSR rows, depth per row).
 cudaError_t launch_coarrival(const int* row_ptr, const int* col, const int* depth, int n, unsigned long long* count,
                              cudaStream_t s);
 // Sorts every list [ptr[p], ptr[p+1]) of (pos, src) by pos (descending when asked).
-cudaError_t launch_sort_lists(const int* ptr, const int* pos, const int* src, int n, int count, bool descending,
-                              int* pos_out, int* src_out, cudaStream_t s);
+// `longest` = the longest list.
+cudaError_t launch_sort_lists(const int* ptr, const int* pos, const int* src, int n, int count, int longest,
+                              bool descending, int* pos_out, int* src_out, cudaStream_t s);
+// The same for lists no longer than transpose_by_rank allows: (key, src) by key, distinct inside a list.
+cudaError_t launch_rank_lists(const int* ptr, const int* key, const int* src, int n, bool descending, int* key_out,
+                              int* src_out, cudaStream_t s);
+// Rows of a CSC pattern (src_out = CSC entry of each CSR entry, col_out = its column) and the column of
+// every CSC entry, given the row pointers; only where transpose_by_rank(longest row) holds.
+bool transpose_by_rank(int longest_row);
+cudaError_t launch_transpose_pattern(const int* col_ptr, const int* row_idx, const int* row_ptr, int n, int nnz,
+                                     int* col_of, int* src_out, int* col_out, cudaStream_t s);
 template <typename TV, typename T>
 cudaError_t launch_stage_values(const Layout& L, const TV* val, Values<T>& V, unsigned forms, int* flags,
                                 cudaStream_t s);
