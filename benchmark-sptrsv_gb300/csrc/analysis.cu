@@ -5,6 +5,7 @@
 #include <climits>
 #include <cstdio>
 
+#include "exec_common.cuh"
 #include "internal.h"
 
 namespace sptrsv {
@@ -810,6 +811,150 @@ cudaError_t launch_levels(const int* col_ptr, const int* row_idx, const int* in_
                   (void*)&front_a, (void*)&front_b, (void*)&depth, (void*)&level_sizes, (void*)&ctl,
                   (void*)&timeout_ns, (void*)&tails, (void*)&smin, (void*)&smax};
   return cudaLaunchCooperativeKernel((void*)k_levels, dim3(grid), dim3(kThreads), args, 0, s);
+}
+
+// Level sets without a barrier per level: depth[r] = 1 + the deepest of its
+// dependencies, rows in natural order, one lane per row, a warp's 32 rows in
+// lockstep as in the solve executors (value-as-flag words, -1 = not known yet;
+// chunk-local dependencies through shared memory). A level then costs one poll
+// (or one shared-memory hop) instead of the peeling kernel's chain of dependent
+// accesses and its grid barrier (~4 us a level).
+//
+// Three CTAs of 256 rows per SM and a 100 ns nap after 16 idle iterations: how
+// many rows are in flight bounds systems whose levels spread over all rows (a
+// mesh row is one long chain), and polls of rows far ahead slow the others.
+// Whole analysis, ms, peeling -> 1 / 2 CTAs without naps / 3 with 100 ns / 4
+// with 200: 2M-row mesh (2,827 levels) 15.1 -> 15.6 / 10.9 / 9.2 / 8.5; 1M-row
+// band (1,232) 8.5 -> 4.1 / 4.2 / 4.5 / 5.1; 150k-row narrow band (8,814) 34.9 ->
+// 7.7 / 8.2 / 8.7 / 8.8; 30 independent bands of 39,000 rows one after the other
+// 5.8 -> 6.6 / 5.4 / 5.0 / 5.0; a 300,000-row chain 1,046 -> 80 / 90 / 101 / 107.
+// (Eight CTAs without naps: the pollers starve the rows they wait for.)
+constexpr int kLevelChunk = 256;  // rows per CTA at a time, one per thread
+constexpr int kLevelCtas = 3;
+constexpr unsigned kLevelNap = 100;
+
+__global__ void __launch_bounds__(kLevelChunk) k_levels_pull(const int* __restrict__ row_ptr,
+                                                             const int* __restrict__ col, int n, int backward,
+                                                             int nchunks, int* depth, int* deepest, DeviceCtl* ctl,
+                                                             unsigned long long timeout_ns) {
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int U = 4;
+  __shared__ int s_depth[kLevelChunk];
+  __shared__ unsigned s_chunk;
+  const int last = n - 1;
+  int mine = 0;
+  for (;;) {
+    const unsigned c = next_chunk(ctl, nchunks, &s_chunk);
+    if (c >= (unsigned)nchunks) break;
+    const int base = static_cast<int>(c) * kLevelChunk;
+    volatile int* s_d = s_depth;
+    s_d[threadIdx.x] = -1;
+    __syncthreads();
+    const int w = base + threadIdx.x;  // walk index
+    const int r = backward ? last - w : w;
+    bool done = w >= n, fail = false;
+    // entries e, e + step, ... (left of them): farthest dependency first
+    int e = 0, left = 0;
+    const int step = backward ? -1 : 1;
+    if (!done) {
+      const int b0 = row_ptr[r], b1 = row_ptr[r + 1];
+      left = b1 - b0 - 1;
+      e = backward ? b1 - 1 : b0;
+    }
+    int d = 0, q[U], v[U];
+    unsigned todo = 0u;
+    auto poll = [&](int u) {
+      const int wq = (backward ? last - q[u] : q[u]) - base;
+      v[u] = wq >= 0 ? s_d[wq] : static_cast<int>(ld_relaxed_u32(reinterpret_cast<const unsigned*>(&depth[q[u]])));
+    };
+    auto load = [&]() {
+      todo = 0u;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        q[u] = u < left ? col[e + u * step] : -1;
+        v[u] = -1;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (q[u] >= 0) {
+          poll(u);
+          todo |= 1u << u;
+        }
+    };
+    if (!done) load();
+    WaitBudget wb(timeout_ns);
+    unsigned idle = 0u;
+    bool work = __any_sync(kFull, !done);  // the last chunk may leave a warp without rows
+    while (work) {
+      bool progress = false;
+      if (!done) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if ((todo & (1u << u)) && v[u] >= 0) {
+            d = max(d, v[u] + 1);
+            todo &= ~(1u << u);
+            progress = true;
+          }
+        if (!todo) {
+          e += U * step;
+          left -= U;
+          progress = true;
+          if (left > 0) {
+            load();
+          } else {
+            s_d[threadIdx.x] = d;
+            st_relaxed_u32(reinterpret_cast<unsigned*>(&depth[r]), static_cast<unsigned>(d));
+            mine = max(mine, d);
+            done = true;
+          }
+        } else {
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (todo & (1u << u)) poll(u);
+        }
+      }
+      if (__any_sync(kFull, progress)) {
+        idle = 0u;
+        work = __any_sync(kFull, !done);
+      } else {
+        if (idle >= 16u) __nanosleep(kLevelNap);
+        if ((++idle & 15u) == 0u && __any_sync(kFull, !wb.poll(ctl, r))) {
+          fail = true;
+          break;
+        }
+      }
+    }
+    if (__syncthreads_or(fail)) break;
+  }
+  mine = __reduce_max_sync(kFull, mine);
+  if ((threadIdx.x & 31) == 0 && mine > 0) atomicMax(deepest, mine);
+  leave(ctl);
+}
+
+cudaError_t launch_levels_pull(const int* row_ptr, const int* col, int n, bool backward, int* depth, int* deepest,
+                               DeviceCtl* ctl, unsigned long long timeout_ns, int num_sms, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(depth, 0xFF, sizeof(int) * (size_t)n, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(deepest, 0, sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  const int nchunks = (n + kLevelChunk - 1) / kLevelChunk;
+  const int grid = std::min(nchunks, num_sms * kLevelCtas);
+  k_levels_pull<<<grid, kLevelChunk, 0, s>>>(row_ptr, col, n, backward ? 1 : 0, nchunks, depth, deepest, ctl,
+                                             timeout_ns);
+  return cudaGetLastError();
+}
+
+// level_ptr[l] = first index of key l in the sorted keys (every level is non-empty)
+__global__ void k_level_starts(const unsigned* __restrict__ keys, int n, int nlevels, int* level_ptr) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
+    if (i == 0 || keys[i] != keys[i - 1]) level_ptr[keys[i]] = static_cast<int>(i);
+    if (i == n - 1) level_ptr[nlevels] = n;
+  }
+}
+cudaError_t launch_level_starts(const unsigned* keys, int n, int nlevels, int* level_ptr, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  k_level_starts<<<grid_for(n), kThreads, 0, s>>>(keys, n, nlevels, level_ptr);
+  return cudaGetLastError();
 }
 
 // ------------------------------------------------------------ schedule

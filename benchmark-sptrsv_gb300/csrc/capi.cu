@@ -1518,6 +1518,13 @@ int sptrsv_gb300_get_option(sptrsv_handle_t h, int option, long long* value) {
 }  // extern "C"
 
 namespace {
+// Level sets of a single system whose longest dependency list has at most this
+// many entries come from the sync-free pass (k_levels_pull): one lane walks a
+// row's list, which holds back the lanes behind a far longer one, so those and
+// batches (whose systems would follow one another instead of running side by
+// side) peel level by level (k_levels).
+constexpr int kPullLevelDeps = 256;
+
 // The analysis pipeline on a CSC structure already described by h->n, nnz,
 // substitution and (for batches) the system arrays.
 int analyse_core(sptrsv_handle_t h, const int* d_colPtr, const int* d_rowIdx, cudaStream_t s) {
@@ -1583,51 +1590,52 @@ int analyse_core(sptrsv_handle_t h, const int* d_colPtr, const int* d_rowIdx, cu
   h->nlevels = 0;
   h->level_sizes_host.clear();
   if (n > 0) {
-    int *cnt = nullptr, *fa = nullptr, *fb = nullptr, *sizes = nullptr;
-    CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&cnt), sizeof(int) * n, s));
-    CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&fa), sizeof(int) * n, s));
-    CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&fb), sizeof(int) * n, s));
-    CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&sizes), sizeof(int) * ((size_t)n + 5), s));
-    CUDA_TRY(launch_levels(h->csc_ptr, h->csc_row, h->in_degree, n, cnt, fa, fb, h->depth, sizes, h->ctl,
-                           timeout_ns(h), s));
-    int code = 0;
-    ST_TRY(read_device_code(h, s, &code));
-    if (code != DEV_OK) {
-      ST_TRY(reset_after_failure(h, s));
-      return SPTRSV_ERR_TIMEOUT;
-    }
     int nl = 0;
-    CUDA_TRY(cudaMemcpyAsync(h->host_pinned + 2, sizes + n + 1 + 3, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaStreamSynchronize(s));
-    nl = h->host_pinned[2];
-    if (nl < 1 || nl > n) return SPTRSV_ERR_BAD_STRUCTURE;
-    h->level_sizes_host.resize(nl);
-    CUDA_TRY(cudaMemcpy(h->level_sizes_host.data(), sizes, sizeof(int) * nl, cudaMemcpyDeviceToHost));
-    long long total = 0;
-    for (int l = 0; l < nl; ++l) total += h->level_sizes_host[l];
-    if (total != n) return SPTRSV_ERR_BAD_STRUCTURE;
-    h->nlevels = nl;
-    // findlevel_csc statistics (findlevel.h:123-136)
-    int lo = h->level_sizes_host[0], hi = lo;
-    for (int l = 1; l < nl; ++l) {
-      const int c = h->level_sizes_host[l];
-      if (c > hi) hi = c;
-      else if (c < lo) lo = c;
+    bool found = false;
+    if (h->batch_count == 1 && h->max_dep_cnt <= kPullLevelDeps) {
+      int* deepest = nullptr;
+      CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&deepest), sizeof(int), s));
+      // the bound of a wait is the solves', but at least a second: a long chain
+      // legitimately keeps the rows behind it waiting
+      cudaError_t e = launch_levels_pull(h->csr_ptr, h->csr_col, n, h->substitution == 1, h->depth, deepest, h->ctl,
+                                         std::max(timeout_ns(h), 1000000000ull), h->num_sms, s);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(h->host_pinned + 2, deepest, sizeof(int), cudaMemcpyDeviceToHost, s);
+      cudaFreeAsync(deepest, s);
+      CUDA_TRY(e);
+      int code = 0;
+      ST_TRY(read_device_code(h, s, &code));
+      found = code == DEV_OK;
+      nl = h->host_pinned[2] + 1;
+      if (!found) ST_TRY(reset_after_failure(h, s));  // a wait ran out: peel the levels instead
     }
-    h->pmin = lo;
-    h->pmax = hi;
-    h->pavg = n / nl;
-    CUDA_TRY(cudaFreeAsync(cnt, s));
-    CUDA_TRY(cudaFreeAsync(fa, s));
-    CUDA_TRY(cudaFreeAsync(fb, s));
-    CUDA_TRY(cudaFreeAsync(sizes, s));
+    if (!found) {
+      int *cnt = nullptr, *fa = nullptr, *fb = nullptr, *sizes = nullptr;
+      CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&cnt), sizeof(int) * n, s));
+      CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&fa), sizeof(int) * n, s));
+      CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&fb), sizeof(int) * n, s));
+      CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&sizes), sizeof(int) * ((size_t)n + 5), s));
+      CUDA_TRY(launch_levels(h->csc_ptr, h->csc_row, h->in_degree, n, cnt, fa, fb, h->depth, sizes, h->ctl,
+                             timeout_ns(h), s));
+      CUDA_TRY(cudaMemcpyAsync(h->host_pinned + 2, sizes + n + 1 + 3, sizeof(int), cudaMemcpyDeviceToHost, s));
+      int code = 0;
+      ST_TRY(read_device_code(h, s, &code));
+      if (code != DEV_OK) {
+        ST_TRY(reset_after_failure(h, s));
+        return SPTRSV_ERR_TIMEOUT;
+      }
+      nl = h->host_pinned[2];
+      CUDA_TRY(cudaFreeAsync(cnt, s));
+      CUDA_TRY(cudaFreeAsync(fa, s));
+      CUDA_TRY(cudaFreeAsync(fb, s));
+      CUDA_TRY(cudaFreeAsync(sizes, s));
+    }
+    if (nl < 1 || nl > n) return SPTRSV_ERR_BAD_STRUCTURE;
+    h->nlevels = nl;
 
-    // level items: rows sorted by (level, row)
+    // level items: rows sorted by (level, row); the level starts from the sorted keys
     ST_TRY(dev_alloc(h, &h->level_item, n));
     ST_TRY(dev_alloc(h, &h->level_ptr_nat, (size_t)nl + 1));
-    std::vector<int> lp(nl + 1, 0);
-    for (int l = 0; l < nl; ++l) lp[l + 1] = lp[l] + h->level_sizes_host[l];
-    CUDA_TRY(cudaMemcpyAsync(h->level_ptr_nat, lp.data(), sizeof(int) * (nl + 1), cudaMemcpyHostToDevice, s));
     unsigned *keys = nullptr, *keys_sorted = nullptr;
     int* iota = nullptr;
     void* temp = nullptr;
@@ -1638,10 +1646,26 @@ int analyse_core(sptrsv_handle_t h, const int* d_colPtr, const int* d_rowIdx, cu
     CUDA_TRY(launch_iota(iota, n, 0, 1, s));
     CUDA_TRY(launch_schedule_keys(iota, h->depth, n, SysDesc(), 1, 0, keys, s));
     CUDA_TRY(radix_sort_pairs(keys, iota, keys_sorted, h->level_item, n, bits_for(nl - 1), temp, s));
+    CUDA_TRY(launch_level_starts(keys_sorted, n, nl, h->level_ptr_nat, s));
+    std::vector<int> lp((size_t)nl + 1, 0);
+    CUDA_TRY(cudaMemcpyAsync(lp.data(), h->level_ptr_nat, sizeof(int) * ((size_t)nl + 1), cudaMemcpyDeviceToHost, s));
     CUDA_TRY(cudaFreeAsync(keys, s));
     CUDA_TRY(cudaFreeAsync(keys_sorted, s));
     CUDA_TRY(cudaFreeAsync(iota, s));
     CUDA_TRY(cudaFreeAsync(temp, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    h->level_sizes_host.resize(nl);
+    for (int l = 0; l < nl; ++l) h->level_sizes_host[l] = lp[l + 1] - lp[l];
+    // findlevel_csc statistics (findlevel.h:123-136)
+    int lo = h->level_sizes_host[0], hi = lo;
+    for (int l = 1; l < nl; ++l) {
+      const int c = h->level_sizes_host[l];
+      if (c > hi) hi = c;
+      else if (c < lo) lo = c;
+    }
+    h->pmin = lo;
+    h->pmax = hi;
+    h->pavg = n / nl;
   }
   h->analysed = true;
   // 5. execution plan, schedule and layouts

@@ -222,6 +222,11 @@ cudaError_t launch_gather_int(const int* src, const int* idx, int* out, int coun
 cudaError_t launch_levels(const int* col_ptr, const int* row_idx, const int* in_degree, int n,
                           int* cnt_scratch, int* front_a, int* front_b, int* depth, int* level_sizes,
                           DeviceCtl* ctl, unsigned long long timeout_ns, cudaStream_t s);
+// Level sets of one system by a sync-free pass over the CSR rows (diagonal last in a row of a lower
+// triangle, first in an upper one): depth[n], *deepest = the last level. Bounded waits (ctl->code).
+cudaError_t launch_levels_pull(const int* row_ptr, const int* col, int n, bool backward, int* depth, int* deepest,
+                               DeviceCtl* ctl, unsigned long long timeout_ns, int num_sms, cudaStream_t s);
+cudaError_t launch_level_starts(const unsigned* keys, int n, int nlevels, int* level_ptr, cudaStream_t s);
 // mode 0: level; 1: (natural block, system) of blocked orders; 2: the level
 // stretched to a target of max_depth keys, floor(level * max(D_s, max_depth) /
 // D_s) with D_s = sys_depth[system]

@@ -1,4 +1,5 @@
-"""Analysis of list lengths around the limit of the rank-sorted lists (1,024 entries):
+"""Analysis of list lengths around the limits of the sync-free level pass (256
+dependencies) and of the rank-sorted lists (1,024 entries):
 CSR exactly the transposed pattern, level sets and in-degree exact, and solves that walk
 the sorted lists in both directions (FP64 <= 1e-12 relative, max norm)."""
 from __future__ import annotations
@@ -10,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("lower", [True, False])
-@pytest.mark.parametrize("kind, n", [("star", 2), ("star", 33), ("star", 1024), ("star", 1025), ("star", 1026),
+@pytest.mark.parametrize("kind, n", [("star", 2), ("star", 33), ("star", 257), ("star", 258), ("star", 1024), ("star", 1025), ("star", 1026),
                                      ("dense", 65), ("band", 1), ("band", 31), ("band", 4097), ("diagonal", 100)])
 def test_lists_around_the_rank_limit(cuda, oracle_port, kind, n, lower):
     from sptrsv_gb300 import SyncFreeSolver, matgen
