@@ -63,6 +63,7 @@ struct sptrsv_gb300_handle_s {
     double locality = 0.0;
     ClusterPlan cluster;       // one-cluster executor (block 0: the cluster cannot hold the system)
     bool cluster_f64 = false, cluster_f32 = false;  // the device can run it for this element type
+    bool ahead = false;        // level-order walks stage their lists ahead (use_ahead)
     bool narrow = false;       // few enough dependencies per level for one cluster
     double coarrive = 0.0;  // short lists: share of unknowns with >= 2 dependencies on the preceding level
   } plan;
@@ -859,16 +860,18 @@ int effective_block(const sptrsv_gb300_handle_s* h) {
 // level order with at most kClusterDeps dependencies and kClusterWidth unknowns
 // per level on average and no lists to split, whose values fit the cluster's
 // shared memory. Past either line 16 SMs no longer keep up with the whole GPU
-// (FP64, cluster vs level-order executor: 2,973 dependencies per level 299 vs
-// 385 us, 3,628 297 vs 316, 4,368 383 vs 343, 5,294 378 vs 285; 925 unknowns of
-// 4 entries per level 123 vs 95 us, 1,724 of 2 entries 76 vs 56).
+// (FP64, cluster vs k_pull_ahead: 2,051 dependencies per level 213 vs 301 us,
+// 2,973 288 vs 316, 3,628 281 vs 263, 4,368 358 vs 289; 925 unknowns of 4 entries
+// per level 113 vs 80 us).
 //
-// Threads and runs: below 1,000 dependencies per level 128 threads per CTA and
-// runs of 128 walk indices (10,000 rows, 543 per level: 67.5 us; 75.7 with 256
-// threads and runs of 32), from there 256 threads and runs of 32 (30,000 rows,
-// 1,391 per level: 87.9 vs 112.5 us). Levels of fewer than 24 unknowns: 256
+// Threads and runs (measured before lanes that are done stopped polling): below
+// 1,000 dependencies per level 128 threads per CTA and runs of 128 walk indices
+// (10,000 rows, 543 per level: 67.5 us; 75.7 with 256 threads and runs of 32),
+// from there 256 threads and runs of 32 (30,000 rows, 1,391 per level: 87.9 vs
+// 112.5 us). Levels of fewer than 24 unknowns: 256
 // threads and runs of 256, so that most hops stay inside a CTA (150,001 rows,
 // 17 per level: 2,786 us; 2,926 with the first rule, 3,506 with runs of 32).
+constexpr double kAheadWork = 32000.0;  // use_ahead
 constexpr double kClusterDeps = 3000.0;
 constexpr long long kClusterWidth = 512;
 
@@ -959,6 +962,7 @@ int make_plan(sptrsv_gb300_handle_s* h, cudaStream_t s) {
       P.backoff = 0;
     }
   }
+  P.ahead = n > 0 && nl > 0 && static_cast<double>(nnz - n) + 4.0 * n <= kAheadWork * nl;
   plan_cluster(h);
   P.valid = true;
   return SPTRSV_OK;
@@ -1172,6 +1176,22 @@ bool use_cluster(const sptrsv_gb300_handle_s* h, bool adj) {
   return P.narrow && P.order_block >= h->n && (adj ? P.split_adj : P.split_fwd) == 0;
 }
 
+// Whether a warp-synchronous one-rhs walk in level order without split lists
+// runs k_pull_ahead (exec_ahead.cu), one CTA of 256 threads per SM taking one
+// dependency per iteration. The automatic plan takes it up to kAheadWork units of
+// work per level (dependencies plus 4 per unknown); past that line too few lanes
+// are in flight (us, the plan's other executor -> this one: 4M-row power law,
+// 30,100 units, 1,687 -> 1,484; 1.5M-row band, 31,800, 547 -> 542; 1.5M rows with
+// 3 entries per column, 37,800, 285 -> 299; 2M-row band, 49,700, 508 -> 612). With
+// explicit options it stands in for k_pull_wsync where they ask for just these
+// settings (the tuner's way to it).
+bool use_ahead(const sptrsv_gb300_handle_s* h, const ExecConfig& c) {
+  if (!c.wsync || c.exact || c.staged || !c.smem_tier || h->layout_block < h->n) return false;
+  if (c.block != 256 || c.chunk != 256 || c.sleep_max != 0) return false;
+  if (planned(h, SPTRSV_OPTION_CTAS_PER_SM) && c.wsync_batch == 0) return h->plan.ahead;
+  return c.ctas_per_sm == 1 && c.wsync_batch == 1;
+}
+
 template <typename T>
 int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x, cudaStream_t s,
                 const AdjointArgs<T>* adj = nullptr, bool allow_check = true) {
@@ -1257,9 +1277,14 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
       ST_TRY(ensure_pieces(h, adj != nullptr, c.split, c.chunk, s));
       pc = adj ? &h->pc_adj : &h->pc_fwd;
     }
-    if (c.wsync_batch == 0) c.wsync_batch = auto_wsync_batch(h, adj != nullptr, pc != nullptr);
-    CUDA_TRY(launch_pull<T>(h->layout, V, rhs, v, static_cast<T*>(h->xw.p), h->ctl, c, timeout_ns(h), h->num_sms,
-                            s, adj, pc));
+    if (rhs == 1 && !pc && !(adj && adj->grad) && use_ahead(h, c)) {
+      CUDA_TRY(launch_pull_ahead<T>(h->layout, V, v, static_cast<T*>(h->xw.p), h->ctl, timeout_ns(h), h->num_sms, s,
+                                    adj != nullptr));
+    } else {
+      if (c.wsync_batch == 0) c.wsync_batch = auto_wsync_batch(h, adj != nullptr, pc != nullptr);
+      CUDA_TRY(launch_pull<T>(h->layout, V, rhs, v, static_cast<T*>(h->xw.p), h->ctl, c, timeout_ns(h), h->num_sms,
+                              s, adj, pc));
+    }
   }
   if (h->profile) {
     CUDA_TRY(cudaEventRecord(h->ev_exec[1], s));
@@ -2249,6 +2274,7 @@ int sptrsv_gb300_tune(sptrsv_handle_t h, const void* d_val, int dtype, int rhs, 
     for (int ch : {128, 256}) cands.push_back({SCHED_PULL, big, ch, 0, 128, 1, 1, 2, 1, ch, sp});
     cands.push_back({SCHED_PULL, big, 256, 0, 128, 1, 1, 2, 1, 256, 0});
     for (int bt : {1, 2, 4}) cands.push_back({SCHED_PULL, big, 256, 0, 128, 1, 1, 2, 1, 256, sp, bt});
+    cands.push_back({SCHED_PULL, big, 256, 0, 0, 1, 1, 2, 1, 256, 0, 1});   // lists staged ahead (use_ahead)
     for (int ct : {2, 3}) {
       cands.push_back({SCHED_PULL, big, 256, 0, 0, ct, 1, 2, 1, 256, sp});
       cands.push_back({SCHED_PULL, big, 256, 0, 0, ct, 1, 2, 1, 256, 0});

@@ -1,0 +1,258 @@
+// Level-order executor with lists staged ahead (one right-hand side).
+//
+// As k_pull_wsync with one dependency per iteration: a warp takes 32 consecutive
+// walk indices, one unknown per lane, and advances in lockstep; values are
+// value-as-flag words in global memory. What a level costs is how long a
+// lockstep iteration takes once its last dependency is published, and there a
+// list entry fetched from global memory costs all 32 lanes its latency on top of
+// the poll's. So the warp claims its segments by ticket one ahead (no CTA
+// barrier between them), copies the next segment's lists, one contiguous range,
+// to shared memory with cp.async while it works on the current one, and works
+// out the next entry's address while a poll is in flight. An iteration is then
+// one poll (~285 cycles to L2) plus the multiply-add of the lanes that consumed.
+// Dependencies inside the segment go through a 32-word window in shared memory.
+// Lanes that are done do not poll: a poll of 32 scattered words holds the SM's
+// load path for ~32 cycles, which the other warps' polls wait for. For the same
+// reason one CTA of 8 warps per SM is best (two: 940 -> 1,170 us below).
+//
+// A warp works through its segments in walk order and holds at most two claimed
+// ones it has not started, so the earliest unfinished segment is always being
+// worked on: every dependency lies earlier in the walk.
+//
+// FP64 solves, k_pull_wsync -> this kernel (forward / transposed, us): 1M-row
+// band, 811 unknowns per level, 1,103 / 1,354 -> 918 / 1,048; 4M-row power law,
+// 2,511 per level, 1,687 -> 1,484 (forward); 1M rows with 3 entries per column,
+// 2,358 per level, 384 / 481 -> 314 / 388; 200k rows with 40, 151 per level,
+// 1,187 / 1,383 -> 1,021 / 1,178; 1000 x 1000 mesh in level order 5,179 -> 1,729.
+#include <algorithm>
+
+#include "exec_common.cuh"
+#include "internal.h"
+
+namespace sptrsv {
+
+namespace {
+
+template <typename T>
+struct AheadArgs {
+  int n, nseg, cap;
+  const int* perm;
+  const int* ptr;   // dependency lists in ready order (dependents, for the transposed walk)
+  const int* pos;
+  const T* w;
+  const T* rcp;
+  const T* b;
+  T* x;
+  T* xw;
+  DeviceCtl* ctl;
+  unsigned long long timeout_ns;
+};
+
+// One poll of a value word: from this warp's window when `mine`, else from
+// global memory; lanes that do not `look` get the empty pattern and load nothing.
+__device__ __forceinline__ unsigned long long poll_ahead(unsigned local, const double* word, bool mine, bool look) {
+  unsigned long long v;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tsetp.ne.u32 q, %4, 0;\n\tmov.u64 %0, -1;\n\t"
+      "@p ld.volatile.shared.u64 %0, [%1];\n\t"
+      "@q ld.relaxed.gpu.global.u64 %0, [%2];\n\t}"
+      : "=&l"(v) : "r"(local), "l"(word), "r"((unsigned)(mine && look)), "r"((unsigned)(!mine && look)) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned poll_ahead(unsigned local, const float* word, bool mine, bool look) {
+  unsigned v;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tsetp.ne.u32 q, %4, 0;\n\tmov.u32 %0, -1;\n\t"
+      "@p ld.volatile.shared.u32 %0, [%1];\n\t"
+      "@q ld.relaxed.gpu.global.u32 %0, [%2];\n\t}"
+      : "=&r"(v) : "r"(local), "l"(word), "r"((unsigned)(mine && look)), "r"((unsigned)(!mine && look)) : "memory");
+  return v;
+}
+
+template <typename T, bool ADJ>
+__global__ void __launch_bounds__(256) k_pull_ahead(AheadArgs<T> a) {
+  using F = Flag<T>;
+  using Bits = typename F::Bits;
+  constexpr unsigned kFull = 0xffffffffu;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  // values of the segment in hand, then this warp's two list buffers
+  T* s_win = reinterpret_cast<T*>(smem_raw) + warp * 32;
+  T* s_w = reinterpret_cast<T*>(smem_raw) + nwarps * 32 + (size_t)warp * 2 * a.cap;
+  int* s_q = reinterpret_cast<int*>(reinterpret_cast<T*>(smem_raw) + nwarps * 32 + (size_t)nwarps * 2 * a.cap) +
+             warp * 2 * a.cap;
+  const unsigned s_wina = static_cast<unsigned>(__cvta_generic_to_shared(s_win));
+  const unsigned s_wa = static_cast<unsigned>(__cvta_generic_to_shared(s_w));
+  const unsigned s_qa = static_cast<unsigned>(__cvta_generic_to_shared(s_q));
+  const int last = a.n - 1;
+  unsigned raw = 0u;  // the next segment's number, in lane 0 until it is needed
+  auto claim = [&]() {
+    if (lane == 0) raw = atomicAdd(&a.ctl->ticket, 1u);
+  };
+  auto claimed = [&]() { return static_cast<int>(min(__shfl_sync(kFull, raw, 0), (unsigned)a.nseg)); };
+  int f_row = 0, f_e = 0, f_e1 = 0;
+  auto fetch = [&](int sg) {
+    const int pr = sg < a.nseg ? sg * 32 + lane : a.n;
+    f_e = f_e1 = 0;
+    if (pr < a.n) {
+      const int p = ADJ ? last - pr : pr;
+      f_row = a.perm[p];
+      f_e = a.ptr[p];
+      f_e1 = a.ptr[p + 1];
+    }
+  };
+  int n_row = 0, n_e = 0, n_e1 = 0, n_lo = 0;
+  T n_acc = T(0);
+  auto stage = [&](int sg, int buf) {
+    n_row = f_row;
+    n_e = f_e;
+    n_e1 = f_e1;
+    if (sg >= a.nseg) return;
+    const int pr = sg * 32 + lane;
+    if (pr < a.n) n_acc = a.b[n_row] * a.rcp[ADJ ? last - pr : pr];
+    const int cnt = min(32, a.n - sg * 32);
+    const int lo = __shfl_sync(kFull, f_e, ADJ ? cnt - 1 : 0);
+    const int hi = min(__shfl_sync(kFull, f_e1, ADJ ? 0 : cnt - 1), lo + a.cap);
+    n_lo = lo;
+    for (int e = lo + lane; e < hi; e += 32) {
+      copy_async(s_qa + (unsigned)(buf * a.cap + e - lo) * 4u, a.pos + e);
+      copy_async(s_wa + (unsigned)(buf * a.cap + e - lo) * (unsigned)sizeof(T), a.w + e);
+    }
+  };
+  claim();
+  int sg = claimed();
+  claim();
+  int sg1 = claimed();
+  claim();
+  fetch(sg);
+  stage(sg, 0);
+  fetch(sg1);
+  bool fail = false;
+  for (int buf = 0; sg < a.nseg; buf ^= 1) {
+    const int base = sg * 32, pr = base + lane;
+    bool done = pr >= a.n;
+    const int p = ADJ ? last - pr : pr;
+    const int row = n_row, lo = n_lo;
+    int e = n_e;
+    const int e1 = n_e1;
+    T acc = n_acc;
+    *reinterpret_cast<volatile Bits*>(&s_win[lane]) = F::EMPTY;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    stage(sg1, buf ^ 1);
+    const int sg2 = claimed();
+    claim();
+    fetch(sg2);
+    const T* lw = s_w + buf * a.cap - lo;
+    const int* lq = s_q + buf * a.cap - lo;
+    const int hi = lo + a.cap;
+    const T* word = a.xw;
+    const T* nword = a.xw;
+    unsigned local = s_wina, nlocal = s_wina;
+    bool mine = true, nmine = true;
+    T w = T(0), nw = T(0);
+    int nq = 0;
+    int left = e1 - e - 1;
+    auto next = [&](int ee) {
+      nq = ee < hi ? lq[ee] : a.pos[ee];
+      nw = ee < hi ? lw[ee] : a.w[ee];
+    };
+    auto target = [&](int q) {
+      const int off = (ADJ ? last - q : q) - base;
+      nmine = off >= 0;
+      nlocal = s_wina + (unsigned)(off & 31) * (unsigned)sizeof(T);
+      nword = a.xw + q;
+    };
+    auto publish = [&]() {
+      F::store_shared(&s_win[lane], acc);
+      F::store(&a.xw[p], acc);
+      done = true;
+    };
+    if (!done) {
+      if (left < 0) {
+        publish();
+      } else {
+        next(e);
+        w = nw;
+        target(nq);
+        word = nword;
+        local = nlocal;
+        mine = nmine;
+        if (left > 0) next(++e);
+      }
+    }
+
+    unsigned idle = 0u;
+    WaitBudget wb(a.timeout_ns);
+    while (!__all_sync(kFull, done)) {
+      const Bits bits = poll_ahead(local, word, mine, !done);
+      target(nq);  // in the poll's shadow
+      if (bits != F::EMPTY) {
+        acc = fma(-w, F::value(bits), acc);
+        if (left > 0) {
+          w = nw;
+          word = nword;
+          local = nlocal;
+          mine = nmine;
+          if (--left > 0) next(++e);
+        } else {
+          publish();
+        }
+      }
+      if ((++idle & 255u) == 0u) {
+        if (!wb.poll(a.ctl, p)) fail = true;
+        if (__any_sync(kFull, fail)) {
+          fail = true;
+          break;
+        }
+      }
+    }
+    if (fail) break;
+    if (pr < a.n) a.x[row] = acc;
+    sg = sg1;
+    sg1 = sg2;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  leave(a.ctl);
+}
+
+}  // namespace
+
+template <typename T>
+cudaError_t launch_pull_ahead(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
+                              unsigned long long timeout_ns, int num_sms, cudaStream_t s, bool adj) {
+  if (L.n == 0) return cudaSuccess;
+  // list buffers hold twice the average segment (longer ones read the rest from
+  // global memory), at most 123 KB of them in FP64
+  constexpr int block = 256;
+  const int avg = static_cast<int>(32LL * L.ndep / L.n);
+  const int cap = std::min(640, std::max(64, (2 * avg + 31) / 32 * 32));
+  AheadArgs<T> a{};
+  a.n = L.n;
+  a.nseg = (L.n + 31) / 32;
+  a.cap = cap;
+  a.perm = L.perm;
+  a.ptr = adj ? L.out_ptr : L.dep_ptr;
+  a.pos = adj ? L.out_pos_f : L.dep_pos_f;
+  a.w = adj ? V.out_w : V.dep_w;
+  a.rcp = V.rcp;
+  a.b = v.b;
+  a.x = v.x;
+  a.xw = xw;
+  a.ctl = ctl;
+  a.timeout_ns = timeout_ns;
+  const size_t smem = (size_t)(block / 32) * (32 * sizeof(T) + 2 * cap * (sizeof(T) + sizeof(int)));
+  auto kernel = adj ? k_pull_ahead<T, true> : k_pull_ahead<T, false>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const int grid = std::min(num_sms, (a.nseg + block / 32 - 1) / (block / 32));
+  kernel<<<grid, block, smem, s>>>(a);
+  return cudaGetLastError();
+}
+template cudaError_t launch_pull_ahead<double>(const Layout&, const Values<double>&, const VecView<double>&, double*,
+                                               DeviceCtl*, unsigned long long, int, cudaStream_t, bool);
+template cudaError_t launch_pull_ahead<float>(const Layout&, const Values<float>&, const VecView<float>&, float*,
+                                              DeviceCtl*, unsigned long long, int, cudaStream_t, bool);
+
+}  // namespace sptrsv

@@ -20,10 +20,11 @@
 // works on the segment before, because a list entry fetched from global memory
 // inside the loop stalls all 32 lanes on it.
 //
-// Measured (FP64, kernel and launch, against k_pull_wsync): 10,000 rows / 147
-// levels 67.5 vs 119.7 us; 50,000 rows / 380 levels 145 vs 287; 100,000 rows /
-// 438 levels of 2,051 dependencies 229 vs 370; 150,001 rows / 8,814 levels
-// 2,786 vs 4,993. Bound by the hop: a lockstep iteration is one remote poll
+// Measured (FP64, kernel and launch, forward / transposed, against k_pull_wsync):
+// 10,000 rows / 147 levels 67.2 / 75.7 vs 118.9 / 145.3 us; 50,000 rows / 380
+// levels 145 / 192 vs 295 / 377; 100,000 rows / 438 levels of 2,051 dependencies
+// 213 / 250 vs 369 / 457; 150,001 rows / 8,814 levels 2,921 / 3,721 vs 5,050 /
+// 7,215. Bound by the hop: a lockstep iteration is one remote poll
 // (~220 cycles) plus the multiply-add of the lanes that consumed (64 cycles in
 // FP64; FP32 runs 10 % faster). One CTA instead of 16 loses (10,000 rows: 113
 // us): an FP64 warp instruction holds its sub-partition's pipe for 64 cycles
@@ -64,23 +65,25 @@ __device__ __forceinline__ void cluster_sync() {
 }
 // One poll of a value word: from this CTA's shared memory when `mine`, else
 // from a peer's (one predicated load each, so a warp that holds both kinds
-// waits for the longer of the two, not for their sum).
-__device__ __forceinline__ unsigned long long poll_word(unsigned addr, unsigned remote, bool mine, double) {
+// waits for the longer of the two, not for their sum). Lanes that do not `look`
+// get the empty pattern and load nothing: distributed-shared-memory loads of
+// scattered words are served at well under one a cycle per SM.
+__device__ __forceinline__ unsigned long long poll_word(unsigned addr, unsigned remote, bool mine, bool look, double) {
   unsigned long long v;
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t"
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tsetp.ne.u32 q, %4, 0;\n\tmov.u64 %0, -1;\n\t"
       "@p ld.relaxed.cluster.shared::cta.u64 %0, [%1];\n\t"
-      "@!p ld.relaxed.cluster.shared::cluster.u64 %0, [%2];\n\t}"
-      : "=l"(v) : "r"(addr), "r"(remote), "r"((unsigned)mine) : "memory");
+      "@q ld.relaxed.cluster.shared::cluster.u64 %0, [%2];\n\t}"
+      : "=&l"(v) : "r"(addr), "r"(remote), "r"((unsigned)(mine && look)), "r"((unsigned)(!mine && look)) : "memory");
   return v;
 }
-__device__ __forceinline__ unsigned poll_word(unsigned addr, unsigned remote, bool mine, float) {
+__device__ __forceinline__ unsigned poll_word(unsigned addr, unsigned remote, bool mine, bool look, float) {
   unsigned v;
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t"
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tsetp.ne.u32 q, %4, 0;\n\tmov.u32 %0, -1;\n\t"
       "@p ld.relaxed.cluster.shared::cta.u32 %0, [%1];\n\t"
-      "@!p ld.relaxed.cluster.shared::cluster.u32 %0, [%2];\n\t}"
-      : "=r"(v) : "r"(addr), "r"(remote), "r"((unsigned)mine) : "memory");
+      "@q ld.relaxed.cluster.shared::cluster.u32 %0, [%2];\n\t}"
+      : "=&r"(v) : "r"(addr), "r"(remote), "r"((unsigned)(mine && look)), "r"((unsigned)(!mine && look)) : "memory");
   return v;
 }
 __device__ __forceinline__ void publish_word(unsigned addr, unsigned long long v) {
@@ -88,15 +91,6 @@ __device__ __forceinline__ void publish_word(unsigned addr, unsigned long long v
 }
 __device__ __forceinline__ void publish_word(unsigned addr, unsigned v) {
   asm volatile("st.relaxed.cluster.shared::cta.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-
-__device__ __forceinline__ void copy_async(unsigned dst, const double* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-}
-template <typename V>
-__device__ __forceinline__ void copy_async(unsigned dst, const V* src) {
-  static_assert(sizeof(V) == 4, "4-byte elements");
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 
 template <typename T, bool ADJ>
@@ -210,9 +204,9 @@ __global__ void __launch_bounds__(512) k_pull_cluster(ClusterArgs<T> a) {
     unsigned idle = 0u;
     WaitBudget wb(a.timeout_ns);
     while (!__all_sync(0xffffffffu, done)) {
-      const Bits bits = poll_word(addr, remote, mine, T(0));
+      const Bits bits = poll_word(addr, remote, mine, !done, T(0));
       target(nq);  // in the poll's shadow
-      if (!done && bits != F::EMPTY) {
+      if (bits != F::EMPTY) {
         acc = fma(-w, F::value(bits), acc);
         if (left > 0) {
           w = nw;

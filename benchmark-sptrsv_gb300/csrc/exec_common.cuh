@@ -4,6 +4,16 @@
 
 namespace sptrsv {
 
+// One element to shared memory in the background (cp.async).
+__device__ __forceinline__ void copy_async(unsigned dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+template <typename V>
+__device__ __forceinline__ void copy_async(unsigned dst, const V* src) {
+  static_assert(sizeof(V) == 4, "4-byte elements");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
 // Claim the next chunk for this CTA (uniform across the CTA).
 __device__ __forceinline__ unsigned next_chunk(DeviceCtl* ctl, unsigned nchunks, unsigned* s_chunk) {
   if (threadIdx.x == 0) *s_chunk = ctl_failed(ctl) ? nchunks : atomicAdd(&ctl->ticket, 1u);

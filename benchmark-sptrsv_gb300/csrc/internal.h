@@ -300,6 +300,10 @@ template <typename T>
 cudaError_t launch_levelset(const Layout& L, const Values<T>& V, int rhs, const VecView<T>& v, T* xw,
                             DeviceCtl* ctl, const ExecConfig& cfg, unsigned long long timeout_ns,
                             cudaStream_t s);
+// level-order executor with lists staged ahead, one CTA per SM (exec_ahead.cu)
+template <typename T>
+cudaError_t launch_pull_ahead(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
+                              unsigned long long timeout_ns, int num_sms, cudaStream_t s, bool adj);
 // One-cluster executor (exec_cluster.cu): 16 CTAs of `block` threads; walk
 // indices are dealt to them in runs of 1 << cshift; a warp's list buffer holds
 // `cap` entries.
