@@ -1192,6 +1192,23 @@ bool use_ahead(const sptrsv_gb300_handle_s* h, const ExecConfig& c) {
   return c.ctas_per_sm == 1 && c.wsync_batch == 1;
 }
 
+// The same for several right-hand sides (exec_ahead_multi.cu): level order, lists
+// that the one-rhs plan would not split (one lane walks a whole list: a power-law
+// transposed walk with lists up to 1,000 took 6.0 ms against 4.9), and either the
+// automatic settings or explicit ones that leave tile, chunk and residency open.
+constexpr long long kNarrowWidth = 350;  // unknowns per level (ahead_multi_shape)
+
+bool use_ahead_multi(const sptrsv_gb300_handle_s* h, const ExecConfig& c, int rhs, size_t elem, bool adj) {
+  if (rhs < 2 || !c.wsync || c.exact || !c.smem_tier || h->layout_block < h->n || !h->plan.valid) return false;
+  if (h->rhs_tile_option != 0 || h->chunk_option != 0 || c.block != 256 || c.sleep_max != 0) return false;
+  if (!planned(h, SPTRSV_OPTION_CTAS_PER_SM) && c.ctas_per_sm != 0) return false;
+  if ((adj ? h->plan.split_adj : h->plan.split_fwd) != 0) return false;
+  const int shape = ahead_multi_shape(rhs, elem, false);
+  // pairs over 32 lanes: no gain for the transposed walk (64 right-hand sides, 1M
+  // rows, column-major: 2.27 ms against 2.23)
+  return shape != 0 && !(adj && shape == 32 * 8 + 2);
+}
+
 template <typename T>
 int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x, cudaStream_t s,
                 const AdjointArgs<T>* adj = nullptr, bool allow_check = true) {
@@ -1277,7 +1294,11 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
       ST_TRY(ensure_pieces(h, adj != nullptr, c.split, c.chunk, s));
       pc = adj ? &h->pc_adj : &h->pc_fwd;
     }
-    if (rhs == 1 && !pc && !(adj && adj->grad) && use_ahead(h, c)) {
+    if (!(adj && adj->grad) && use_ahead_multi(h, c, rhs, sizeof(T), adj != nullptr)) {
+      CUDA_TRY(launch_pull_ahead_multi<T>(h->layout, V, rhs, v, static_cast<T*>(h->xw.p), h->ctl,
+                                          n < kNarrowWidth * h->nlevels, timeout_ns(h), h->num_sms, s,
+                                          adj != nullptr));
+    } else if (rhs == 1 && !pc && !(adj && adj->grad) && use_ahead(h, c)) {
       CUDA_TRY(launch_pull_ahead<T>(h->layout, V, v, static_cast<T*>(h->xw.p), h->ctl, timeout_ns(h), h->num_sms, s,
                                     adj != nullptr));
     } else {
@@ -2097,6 +2118,26 @@ int sptrsv_gb300_solve_adjoint(sptrsv_handle_t h, const void* d_val, int dtype, 
   if (!d_g || !d_lambda || (d_dval && !d_x)) return SPTRSV_ERR_INVALID;
   if (h->sched_option == SCHED_LEVELSET) return SPTRSV_ERR_UNSUPPORTED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (!d_dval && stage_col_major(h, rhs, layout, kColMajorStageRhs)) {
+    // through row-major staging, as plain solves (1M rows, 64 right-hand sides:
+    // 2.64 ms walking the columns as they are, 2.36 staged)
+    const size_t bytes = (size_t)h->n * rhs * (dtype == SPTRSV_DTYPE_F64 ? sizeof(double) : sizeof(float));
+    ST_TRY(ensure_buf(h, h->tb, bytes, 0, s));
+    ST_TRY(ensure_buf(h, h->tx, bytes, 0, s));
+    if (dtype == SPTRSV_DTYPE_F64) {
+      CUDA_TRY(launch_transpose<double>(static_cast<const double*>(d_g), static_cast<double*>(h->tb.p), rhs, h->n, s));
+    } else {
+      CUDA_TRY(launch_transpose<float>(static_cast<const float*>(d_g), static_cast<float*>(h->tb.p), rhs, h->n, s));
+    }
+    ST_TRY(sptrsv_gb300_solve_adjoint(h, d_val, dtype, rhs, SPTRSV_LAYOUT_ROW_MAJOR, h->tb.p, h->tx.p, nullptr, nullptr,
+                                      stream));
+    if (dtype == SPTRSV_DTYPE_F64) {
+      CUDA_TRY(launch_transpose<double>(static_cast<const double*>(h->tx.p), static_cast<double*>(d_lambda), h->n, rhs, s));
+    } else {
+      CUDA_TRY(launch_transpose<float>(static_cast<const float*>(h->tx.p), static_cast<float*>(d_lambda), h->n, rhs, s));
+    }
+    return SPTRSV_OK;
+  }
   const int before = h->layout_block;
   ST_TRY(ensure_layout(h, s));
   if (d_val) {
@@ -2303,6 +2344,7 @@ int sptrsv_gb300_tune(sptrsv_handle_t h, const void* d_val, int dtype, int rhs, 
       for (int ct : {1, 2, 3})
         cands.push_back({SCHED_PULL, big, 0, 0, 0, ct, 1, 2, 1, 256, sp, 0, 1, SPTRSV_OPT_WARP_AUTO, tile});
     }
+    cands.push_back({SCHED_PULL, big, 0, 0, 0, 0, 1, 2, 1, 256, sp});         // lists staged ahead (use_ahead_multi)
     cands.push_back({SCHED_PULL, big, 0, 0, 0, 0, 1, 2, 1, 256, sp, 0, 0});   // global-memory tier only
     for (int ob : blocks) cands.push_back({SCHED_PULL, ob, ob, 0, 0, 0, 1, 2, 1, 256, sp});
     cands.push_back({SCHED_PULL, big, 0, 0, 256, 0, 1, 2, 0, 256, sp});

@@ -1,0 +1,356 @@
+// Level-order executor with lists staged ahead, several right-hand sides.
+//
+// The loop of k_pull_ahead (exec_ahead.cu) for blocks: G lanes hold an unknown,
+// each R adjacent right-hand sides (one two-word load per pair), and every lane
+// walks the unknown's list on its own. The next chunk's lists are copied to
+// shared memory with cp.async and its first terms loaded while the CTA works on
+// the current one; the next entry's address is worked out while a poll is in
+// flight, and finished lanes do not poll. Chunks are 256 / G unknowns, claimed
+// two ahead, with a CTA barrier between them: it holds back the warps that
+// would otherwise poll far ahead of the wave. As many CTAs per SM as fit: the
+// lanes of a group poll adjacent words, so polls are cheap and throughput (one
+// dependency per iteration and lane) counts.
+//
+// FP64, 500k-row band of 9 entries per column, k_pull_wsync_multi -> this kernel
+// (forward / transposed, us): 2 right-hand sides 610 / 641 -> 430 / 495, 4 557 /
+// 596 -> 365 / 444, 8 573 / 575 -> 375 / 484, 16 568 / 605 -> 472 / 565, 32 723 /
+// 797 -> 602 / 724, 64 987 / 1,030 -> 945 / 1,018 (there the FP64 pipe: 20 M
+// warp-wide multiply-adds per 1M rows hold it ~1.1 ms); FP32 at 64 840 / 829 ->
+// 534 / 657.
+#include <algorithm>
+
+#include "exec_common.cuh"
+#include "internal.h"
+
+namespace sptrsv {
+
+namespace {
+
+template <typename T>
+struct AheadMultiArgs {
+  int n, rhs, nchunks, cap;
+  const int* perm;
+  const int* ptr;   // dependency lists in ready order (dependents, for the transposed walk)
+  const int* pos;
+  const T* w;
+  const T* rcp;
+  const T* b;
+  T* x;
+  long long b_si, b_sk, x_si, x_sk;
+  T* xw;  // [n * rhs], position-major
+  DeviceCtl* ctl;
+  unsigned long long timeout_ns;
+};
+
+// One poll of the R words of a dependency (R = 2: adjacent, one 2-word load):
+// from the chunk's window when `mine`, else from global memory; lanes that do
+// not `look` get the empty pattern and load nothing.
+__device__ __forceinline__ void poll_words(unsigned long long (&v)[1], unsigned local, const double* word, bool mine,
+                                           bool look) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tsetp.ne.u32 q, %4, 0;\n\tmov.u64 %0, -1;\n\t"
+      "@p ld.volatile.shared.u64 %0, [%1];\n\t@q ld.relaxed.gpu.global.u64 %0, [%2];\n\t}"
+      : "=&l"(v[0])
+      : "r"(local), "l"(word), "r"((unsigned)(mine && look)), "r"((unsigned)(!mine && look))
+      : "memory");
+}
+__device__ __forceinline__ void poll_words(unsigned long long (&v)[2], unsigned local, const double* word, bool mine,
+                                           bool look) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %4, 0;\n\tsetp.ne.u32 q, %5, 0;\n\tmov.u64 %0, -1;\n\tmov.u64 %1, -1;\n\t"
+      "@p ld.volatile.shared.v2.u64 {%0, %1}, [%2];\n\t@q ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%3];\n\t}"
+      : "=&l"(v[0]), "=&l"(v[1])
+      : "r"(local), "l"(word), "r"((unsigned)(mine && look)), "r"((unsigned)(!mine && look))
+      : "memory");
+}
+__device__ __forceinline__ void poll_words(unsigned (&v)[1], unsigned local, const float* word, bool mine, bool look) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tsetp.ne.u32 q, %4, 0;\n\tmov.u32 %0, -1;\n\t"
+      "@p ld.volatile.shared.u32 %0, [%1];\n\t@q ld.relaxed.gpu.global.u32 %0, [%2];\n\t}"
+      : "=&r"(v[0])
+      : "r"(local), "l"(word), "r"((unsigned)(mine && look)), "r"((unsigned)(!mine && look))
+      : "memory");
+}
+__device__ __forceinline__ void poll_words(unsigned (&v)[2], unsigned local, const float* word, bool mine, bool look) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %4, 0;\n\tsetp.ne.u32 q, %5, 0;\n\tmov.u32 %0, -1;\n\tmov.u32 %1, -1;\n\t"
+      "@p ld.volatile.shared.v2.u32 {%0, %1}, [%2];\n\t@q ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%3];\n\t}"
+      : "=&r"(v[0]), "=&r"(v[1])
+      : "r"(local), "l"(word), "r"((unsigned)(mine && look)), "r"((unsigned)(!mine && look))
+      : "memory");
+}
+__device__ __forceinline__ void publish_words(double* p, const unsigned long long (&v)[1]) {
+  st_relaxed_u64(reinterpret_cast<unsigned long long*>(p), v[0]);
+}
+__device__ __forceinline__ void publish_words(float* p, const unsigned (&v)[1]) {
+  st_relaxed_u32(reinterpret_cast<unsigned*>(p), v[0]);
+}
+__device__ __forceinline__ void publish_words(double* p, const unsigned long long (&v)[2]) {
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(v[0]), "l"(v[1]) : "memory");
+}
+__device__ __forceinline__ void publish_words(float* p, const unsigned (&v)[2]) {
+  asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(v[0]), "r"(v[1]) : "memory");
+}
+
+template <typename B, typename T>
+__device__ __forceinline__ void poll_words(B (&v)[4], unsigned local, const T* word, bool mine, bool look) {
+  B lo[2], hi[2];
+  poll_words(lo, local, word, mine, look);
+  poll_words(hi, local + 2u * (unsigned)sizeof(T), word + 2, mine, look);
+  v[0] = lo[0];
+  v[1] = lo[1];
+  v[2] = hi[0];
+  v[3] = hi[1];
+}
+template <typename B, typename T>
+__device__ __forceinline__ void publish_words(T* p, const B (&v)[4]) {
+  const B lo[2] = {v[0], v[1]}, hi[2] = {v[2], v[3]};
+  publish_words(p, lo);
+  publish_words(p + 2, hi);
+}
+
+// G lanes per unknown, R adjacent right-hand sides per lane (R = 2 needs an
+// even number of them), 256 / G unknowns per chunk.
+template <typename T, bool ADJ, int G, int R>
+__global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a) {
+  using F = Flag<T>;
+  using Bits = typename F::Bits;
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int kUnknowns = 256 / G;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ unsigned s_ticket;
+  T* s_win = reinterpret_cast<T*>(smem_raw);  // [kUnknowns * G * R] values of the chunk in hand
+  T* s_w = s_win + kUnknowns * G * R;         // [2][cap]
+  int* s_q = reinterpret_cast<int*>(s_w + 2 * a.cap);
+  const unsigned s_wina = static_cast<unsigned>(__cvta_generic_to_shared(s_win));
+  const unsigned s_wa = static_cast<unsigned>(__cvta_generic_to_shared(s_w));
+  const unsigned s_qa = static_cast<unsigned>(__cvta_generic_to_shared(s_q));
+  const int j = threadIdx.x / G, k = (threadIdx.x % G) * R;  // unknown of the chunk, first right-hand side
+  const int last = a.n - 1, rhs = a.rhs;
+  const bool col = k < rhs;
+  // two chunks ahead: rows and list bounds
+  int f_row = 0, f_e = 0, f_e1 = 0, f_lo = 0, f_hi = 0;
+  auto fetch = [&](int c) {
+    f_e = f_e1 = f_lo = f_hi = 0;
+    if (c >= a.nchunks) return;
+    const int base = c * kUnknowns, end = min(base + kUnknowns, a.n);
+    const int pr = base + j;
+    if (pr < a.n) {
+      const int p = ADJ ? last - pr : pr;
+      f_row = a.perm[p];
+      f_e = a.ptr[p];
+      f_e1 = a.ptr[p + 1];
+    }
+    f_lo = a.ptr[ADJ ? last - (end - 1) : base];
+    f_hi = a.ptr[ADJ ? last - base + 1 : end];
+  };
+  // one chunk ahead: first terms, and the lists on their way to shared memory
+  int n_row = 0, n_e = 0, n_e1 = 0, n_lo = 0;
+  T n_acc[R];
+  auto stage = [&](int c, int buf) {
+    n_row = f_row;
+    n_e = f_e;
+    n_e1 = f_e1;
+    n_lo = f_lo;
+    if (c >= a.nchunks) return;
+    const int pr = c * kUnknowns + j;
+    if (pr < a.n && col) {
+      const T r = a.rcp[ADJ ? last - pr : pr];
+#pragma unroll
+      for (int i = 0; i < R; ++i) n_acc[i] = a.b[(long long)n_row * a.b_si + (long long)(k + i) * a.b_sk] * r;
+    }
+    const int hi = min(f_hi, f_lo + a.cap);
+    for (int e = f_lo + threadIdx.x; e < hi; e += 256) {
+      copy_async(s_qa + (unsigned)(buf * a.cap + e - f_lo) * 4u, a.pos + e);
+      copy_async(s_wa + (unsigned)(buf * a.cap + e - f_lo) * (unsigned)sizeof(T), a.w + e);
+    }
+  };
+  // chunks are claimed two ahead; the earliest unfinished one is always in hand
+  auto claim = [&]() {
+    if (threadIdx.x == 0) s_ticket = ctl_failed(a.ctl) ? a.nchunks : atomicAdd(&a.ctl->ticket, 1u);
+  };
+  auto claimed = [&]() { return static_cast<int>(min(s_ticket, (unsigned)a.nchunks)); };
+  claim();
+  __syncthreads();
+  int c = claimed();
+  __syncthreads();
+  claim();
+  __syncthreads();
+  int c1 = claimed();
+  __syncthreads();
+  claim();
+  fetch(c);
+  stage(c, 0);
+  fetch(c1);
+  for (int buf = 0; c < a.nchunks; buf ^= 1) {
+    const int base = c * kUnknowns, pr = base + j;
+    bool done = pr >= a.n || !col;
+    const int p = ADJ ? last - pr : pr;
+    const int row = n_row, lo = n_lo;
+    int e = n_e;
+    const int e1 = n_e1;
+    T acc[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      acc[i] = n_acc[i];
+      *reinterpret_cast<volatile Bits*>(&s_win[threadIdx.x * R + i]) = F::EMPTY;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const int c2 = claimed();
+    stage(c1, buf ^ 1);
+    fetch(c2);
+    const T* lw = s_w + buf * a.cap - lo;
+    const int* lq = s_q + buf * a.cap - lo;
+    const int hi = lo + a.cap;
+    const T *word = a.xw, *nword = a.xw;
+    unsigned local = s_wina, nlocal = s_wina;
+    bool mine = true, nmine = true;
+    T w = T(0), nw = T(0);
+    int nq = 0;
+    int left = e1 - e - 1;
+    auto next = [&](int ee) {
+      nq = ee < hi ? lq[ee] : a.pos[ee];
+      nw = ee < hi ? lw[ee] : a.w[ee];
+    };
+    auto target = [&](int q) {
+      const int off = (ADJ ? last - q : q) - base;
+      nmine = off >= 0;
+      nlocal = s_wina + (unsigned)((off & (kUnknowns - 1)) * (G * R) + k) * (unsigned)sizeof(T);
+      nword = a.xw + (long long)q * rhs + k;
+    };
+    auto publish = [&]() {
+      Bits v[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        v[i] = F::bits(acc[i]);
+        F::store_shared(&s_win[threadIdx.x * R + i], acc[i]);
+      }
+      publish_words(&a.xw[(long long)p * rhs + k], v);
+      done = true;
+    };
+    if (!done) {
+      if (left < 0) {
+        publish();
+      } else {
+        next(e);
+        w = nw;
+        target(nq);
+        word = nword;
+        local = nlocal;
+        mine = nmine;
+        if (left > 0) next(++e);
+      }
+    }
+    bool fail = false;
+    unsigned idle = 0u;
+    WaitBudget wb(a.timeout_ns);
+    while (!__all_sync(kFull, done)) {
+      Bits bits[R];
+      poll_words(bits, local, word, mine, !done);
+      target(nq);  // in the poll's shadow
+      bool hit = true;
+#pragma unroll
+      for (int i = 0; i < R; ++i) hit = hit && bits[i] != F::EMPTY;
+      if (hit) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) acc[i] = fma(-w, F::value(bits[i]), acc[i]);
+        if (left > 0) {
+          w = nw;
+          word = nword;
+          local = nlocal;
+          mine = nmine;
+          if (--left > 0) next(++e);
+        } else {
+          publish();
+        }
+      }
+      if ((++idle & 255u) == 0u) {
+        if (!wb.poll(a.ctl, p)) fail = true;
+        if (__any_sync(kFull, fail)) {
+          fail = true;
+          break;
+        }
+      }
+    }
+    if (!fail && pr < a.n && col) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) a.x[(long long)row * a.x_si + (long long)(k + i) * a.x_sk] = acc[i];
+    }
+    if (__syncthreads_or(fail)) break;
+    claim();
+    c = c1;
+    c1 = c2;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  leave(a.ctl);
+}
+
+}  // namespace
+
+template <typename T, bool ADJ>
+cudaError_t launch_ahead_multi(AheadMultiArgs<T>& a, int avg, bool narrow, int num_sms, cudaStream_t s) {
+  auto run = [&](auto kernel, int g, int r) -> cudaError_t {
+    const int unknowns = 256 / g;
+    a.nchunks = (a.n + unknowns - 1) / unknowns;
+    // twice the average chunk's lists (longer ones read the rest from global memory)
+    a.cap = std::min(1024, std::max(64, (2 * avg * unknowns / 32 + 31) / 32 * 32));
+    const size_t smem = (size_t)256 * r * sizeof(T) + (size_t)2 * a.cap * (sizeof(T) + sizeof(int));
+    cudaError_t e = cudaSuccess;
+    if (smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    int per = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 256, smem);
+    if (per < 1) per = 1;
+    const int grid = static_cast<int>(std::min<long long>((long long)num_sms * per, a.nchunks));
+    kernel<<<grid, 256, smem, s>>>(a);
+    return cudaGetLastError();
+  };
+  switch (ahead_multi_shape(a.rhs, sizeof(T), narrow)) {
+    case 2 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 2, 1>, 2, 1);
+    case 4 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 4, 1>, 4, 1);
+    case 8 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 8, 1>, 8, 1);
+    case 16 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 16, 1>, 16, 1);
+    case 8 * 8 + 2: return run(k_pull_ahead_multi<T, ADJ, 8, 2>, 8, 2);
+    case 16 * 8 + 2: return run(k_pull_ahead_multi<T, ADJ, 16, 2>, 16, 2);
+    case 16 * 8 + 4: return run(k_pull_ahead_multi<T, ADJ, 16, 4>, 16, 4);
+    case 32 * 8 + 2: return run(k_pull_ahead_multi<T, ADJ, 32, 2>, 32, 2);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+template <typename T>
+cudaError_t launch_pull_ahead_multi(const Layout& L, const Values<T>& V, int rhs, const VecView<T>& v, T* xw,
+                                    DeviceCtl* ctl, bool narrow, unsigned long long timeout_ns, int num_sms,
+                                    cudaStream_t s, bool adj) {
+  if (L.n == 0) return cudaSuccess;
+  AheadMultiArgs<T> a{};
+  a.n = L.n;
+  a.rhs = rhs;
+  a.perm = L.perm;
+  a.ptr = adj ? L.out_ptr : L.dep_ptr;
+  a.pos = adj ? L.out_pos_f : L.dep_pos_f;
+  a.w = adj ? V.out_w : V.dep_w;
+  a.rcp = V.rcp;
+  a.b = v.b;
+  a.x = v.x;
+  a.b_si = v.b_si;
+  a.b_sk = v.b_sk;
+  a.x_si = v.x_si;
+  a.x_sk = v.x_sk;
+  a.xw = xw;
+  a.ctl = ctl;
+  a.timeout_ns = timeout_ns;
+  const int avg = static_cast<int>(32LL * L.ndep / L.n);
+  return adj ? launch_ahead_multi<T, true>(a, avg, narrow, num_sms, s)
+             : launch_ahead_multi<T, false>(a, avg, narrow, num_sms, s);
+}
+template cudaError_t launch_pull_ahead_multi<double>(const Layout&, const Values<double>&, int, const VecView<double>&,
+                                                     double*, DeviceCtl*, bool, unsigned long long, int, cudaStream_t,
+                                                     bool);
+template cudaError_t launch_pull_ahead_multi<float>(const Layout&, const Values<float>&, int, const VecView<float>&,
+                                                    float*, DeviceCtl*, bool, unsigned long long, int, cudaStream_t,
+                                                    bool);
+
+}  // namespace sptrsv

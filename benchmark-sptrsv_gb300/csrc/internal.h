@@ -304,6 +304,27 @@ cudaError_t launch_levelset(const Layout& L, const Values<T>& V, int rhs, const 
 template <typename T>
 cudaError_t launch_pull_ahead(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
                               unsigned long long timeout_ns, int num_sms, cudaStream_t s, bool adj);
+// The same for several right-hand sides (exec_ahead_multi.cu): lanes per unknown
+// times 8 plus right-hand sides per lane, or 0 where the general executor serves
+// the block (an odd number above 16 leaves every pair split: 32 lanes of one took
+// 789 us against 723 on the 500k-row band). Pairs beat single right-hand sides
+// from 9 on (16: 472 vs 555 us) but for levels of fewer than 350 unknowns, where
+// more lanes per unknown win (30k rows: 104 vs 86); quadruples only in FP32 (64:
+// 534 vs 749 us; in FP64 1,043 vs 945).
+inline int ahead_multi_shape(int rhs, size_t elem, bool narrow) {
+  if (rhs < 2 || rhs > 64) return 0;
+  if (rhs <= 2) return 2 * 8 + 1;
+  if (rhs <= 4) return 4 * 8 + 1;
+  if (rhs <= 8) return 8 * 8 + 1;
+  if (rhs <= 16) return rhs % 2 || narrow ? 16 * 8 + 1 : 8 * 8 + 2;
+  if (rhs % 2) return 0;
+  if (rhs <= 32) return 16 * 8 + 2;
+  return elem == 4 && rhs % 4 == 0 ? 16 * 8 + 4 : 32 * 8 + 2;
+}
+template <typename T>
+cudaError_t launch_pull_ahead_multi(const Layout& L, const Values<T>& V, int rhs, const VecView<T>& v, T* xw,
+                                    DeviceCtl* ctl, bool narrow, unsigned long long timeout_ns, int num_sms,
+                                    cudaStream_t s, bool adj);
 // One-cluster executor (exec_cluster.cu): 16 CTAs of `block` threads; walk
 // indices are dealt to them in runs of 1 << cshift; a warp's list buffer holds
 // `cap` entries.
