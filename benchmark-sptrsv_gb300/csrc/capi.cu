@@ -1196,7 +1196,6 @@ bool use_ahead(const sptrsv_gb300_handle_s* h, const ExecConfig& c) {
 // that the one-rhs plan would not split (one lane walks a whole list: a power-law
 // transposed walk with lists up to 1,000 took 6.0 ms against 4.9), and either the
 // automatic settings or explicit ones that leave tile, chunk and residency open.
-constexpr long long kNarrowWidth = 350;  // unknowns per level (ahead_multi_shape)
 
 bool use_ahead_multi(const sptrsv_gb300_handle_s* h, const ExecConfig& c, int rhs, size_t elem, bool adj) {
   if (rhs < 2 || !c.wsync || c.exact || !c.smem_tier || h->layout_block < h->n || !h->plan.valid) return false;
@@ -1990,6 +1989,11 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
   }
   if (fuse) {
     // X_0, the FP64 residual and the first FP32 correction in one pass: X = X_0 + D_1
+    // level order with the plan's settings: lists staged ahead
+    const bool refine_ahead =
+        rhs == 1 ? fc.wsync && fc.smem_tier && h->layout_block >= h->n && fc.block == 256 && fc.chunk == 256 &&
+                       fc.sleep_max == 0 && fc.wsync_batch == 0 && planned(h, SPTRSV_OPTION_CTAS_PER_SM)
+                 : planned(h, SPTRSV_OPTION_CTAS_PER_SM) && use_ahead_multi(h, fc, rhs, sizeof(double), false);
     // the plain solve's rule (160k-row bands with 1 / 2 entries per column and a
     // 1M-row band with 3: 0.101 / 1.95 / 6.40 ms refined with two dependencies
     // per iteration, 0.082 / 1.54 / 5.62 with one; the mesh triangle with two:
@@ -2044,6 +2048,10 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
       CUDA_TRY(launch_refine_fused_imported(h->layout, h->v64, wsplit, d_b, d_x,
                                             static_cast<unsigned long long*>(h->xw.p), stats, h->ctl, fc,
                                             timeout_ns(h), h->num_sms, s, h->imports));
+    } else if (wsplit && refine_ahead) {
+      CUDA_TRY(launch_refine_ahead(h->layout, h->v64, rhs, d_b, d_x, si, sk,
+                                   static_cast<unsigned long long*>(h->xw.p), stats, h->ctl,
+                                   h->n / std::max(1, h->nlevels), timeout_ns(h), h->num_sms, s, wsplit));
     } else {
       CUDA_TRY(launch_refine_fused(h->layout, h->v32, h->v64, rhs, d_b, d_x, si, sk,
                                    static_cast<unsigned long long*>(h->xw.p), stats, h->ctl, fc, timeout_ns(h),

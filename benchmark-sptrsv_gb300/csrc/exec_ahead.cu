@@ -26,7 +26,7 @@
 // 1,187 / 1,383 -> 1,021 / 1,178; 1000 x 1000 mesh in level order 5,179 -> 1,729.
 #include <algorithm>
 
-#include "exec_common.cuh"
+#include "exec_ahead.cuh"
 #include "internal.h"
 
 namespace sptrsv {
@@ -47,27 +47,6 @@ struct AheadArgs {
   DeviceCtl* ctl;
   unsigned long long timeout_ns;
 };
-
-// One poll of a value word: from this warp's window when `mine`, else from
-// global memory; lanes that do not `look` get the empty pattern and load nothing.
-__device__ __forceinline__ unsigned long long poll_ahead(unsigned local, const double* word, bool mine, bool look) {
-  unsigned long long v;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tsetp.ne.u32 q, %4, 0;\n\tmov.u64 %0, -1;\n\t"
-      "@p ld.volatile.shared.u64 %0, [%1];\n\t"
-      "@q ld.relaxed.gpu.global.u64 %0, [%2];\n\t}"
-      : "=&l"(v) : "r"(local), "l"(word), "r"((unsigned)(mine && look)), "r"((unsigned)(!mine && look)) : "memory");
-  return v;
-}
-__device__ __forceinline__ unsigned poll_ahead(unsigned local, const float* word, bool mine, bool look) {
-  unsigned v;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tsetp.ne.u32 q, %4, 0;\n\tmov.u32 %0, -1;\n\t"
-      "@p ld.volatile.shared.u32 %0, [%1];\n\t"
-      "@q ld.relaxed.gpu.global.u32 %0, [%2];\n\t}"
-      : "=&r"(v) : "r"(local), "l"(word), "r"((unsigned)(mine && look)), "r"((unsigned)(!mine && look)) : "memory");
-  return v;
-}
 
 template <typename T, bool ADJ>
 __global__ void __launch_bounds__(256) k_pull_ahead(AheadArgs<T> a) {
@@ -185,10 +164,11 @@ __global__ void __launch_bounds__(256) k_pull_ahead(AheadArgs<T> a) {
     unsigned idle = 0u;
     WaitBudget wb(a.timeout_ns);
     while (!__all_sync(kFull, done)) {
-      const Bits bits = poll_ahead(local, word, mine, !done);
+      Bits bits[1];
+      poll_words(bits, local, word, mine, !done);
       target(nq);  // in the poll's shadow
-      if (bits != F::EMPTY) {
-        acc = fma(-w, F::value(bits), acc);
+      if (bits[0] != F::EMPTY) {
+        acc = fma(-w, F::value(bits[0]), acc);
         if (left > 0) {
           w = nw;
           word = nword;

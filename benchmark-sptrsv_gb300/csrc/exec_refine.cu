@@ -48,7 +48,9 @@
 // the residual: rho is exact to about 2^-44 relative to x, far below what the
 // FP32 correction resolves. FP64 work is left only once per unknown: b/d at
 // the start (product, split into the pair) and x = x0 + d at the end.
-#include "exec_common.cuh"
+#include <algorithm>
+
+#include "exec_ahead.cuh"
 #include "internal.h"
 
 namespace sptrsv {
@@ -60,6 +62,7 @@ constexpr unsigned long long kPairNaN = 0x7FC000007FC00000ull;
 
 struct RefineArgs {
   int n, rhs, chunk, nchunks, smem_tier, ctas_per_sm;
+  int cap;                    // k_refine_ahead: entries of a list buffer
   const int* perm;
   const int* dep_ptr;
   const int* dep_pos_f;
@@ -505,6 +508,211 @@ __global__ void __launch_bounds__(288) k_pull_refine1_imp(RefineArgs a) {
   leave(a.ctl);
 }
 
+// ------------------------------------------------------------------ fused step, lists staged ahead
+// The double-float pass in level order with the loop of k_pull_ahead_multi (there
+// for why): G lanes per unknown, each R adjacent right-hand sides walking the
+// list on its own, the next chunk's lists copied ahead, finished lanes not
+// polling. k_pull_refine1 -> this kernel, us with the pass's transposes: 1M-row
+// band, 1 / 16 (column-major) right-hand sides 1,149 / 1,203 -> 955 / 958; 500k-row
+// band, 4 / 8 / 32 / 64 575 / 598 / 793 / 1,077 -> 358 / 373 / 643 / 1,048; 700k
+// rows, 3,004 per level, 1 / 16 259 / 478 -> 180 / 380. Bound by the hop at few
+// right-hand sides, by FP32 issue at 64.
+template <int G, int R>
+__global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a) {
+  using Bits = unsigned long long;
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int kUnknowns = 256 / G;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ unsigned s_ticket;
+  Bits* s_win = reinterpret_cast<Bits*>(smem_raw);                    // [256 * R] pairs of the chunk in hand
+  float2* s_w = reinterpret_cast<float2*>(s_win + kUnknowns * G * R);  // [2][cap]
+  int* s_q = reinterpret_cast<int*>(s_w + 2 * a.cap);
+  const unsigned s_wina = static_cast<unsigned>(__cvta_generic_to_shared(s_win));
+  const unsigned s_wa = static_cast<unsigned>(__cvta_generic_to_shared(s_w));
+  const unsigned s_qa = static_cast<unsigned>(__cvta_generic_to_shared(s_q));
+  const int j = threadIdx.x / G, k = (threadIdx.x % G) * R;  // unknown of the chunk, first right-hand side
+  const int rhs = a.rhs;
+  const bool col = k < rhs;
+  float mx_d = 0.f, mx_x = 0.f, mx_x0 = 0.f;  // stopping-estimate maxima
+  // two chunks ahead: rows and list bounds
+  int f_row = 0, f_e = 0, f_e1 = 0, f_lo = 0, f_hi = 0;
+  auto fetch = [&](int c) {
+    f_e = f_e1 = f_lo = f_hi = 0;
+    if (c >= a.nchunks) return;
+    const int base = c * kUnknowns, end = min(base + kUnknowns, a.n);
+    const int pr = base + j;
+    if (pr < a.n) {
+      const int p = pr;
+      f_row = a.perm[p];
+      f_e = a.dep_ptr[p];
+      f_e1 = a.dep_ptr[p + 1];
+    }
+    f_lo = a.dep_ptr[base];
+    f_hi = a.dep_ptr[end];
+  };
+  // one chunk ahead: first terms, and the lists on their way to shared memory
+  int n_row = 0, n_e = 0, n_e1 = 0, n_lo = 0;
+  float n_hi[R], n_lo2[R];
+  auto stage = [&](int c, int buf) {
+    n_row = f_row;
+    n_e = f_e;
+    n_e1 = f_e1;
+    n_lo = f_lo;
+    if (c >= a.nchunks) return;
+    const int pr = c * kUnknowns + j;
+    if (pr < a.n && col) {
+      const double s64 = a.rcp64[pr];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        // b/d as a float pair: hi = RN32(b*s), lo = RN32(b*s - hi)
+        const double bv = a.b[(long long)n_row * a.b_si + (long long)(k + i) * a.b_sk];
+        n_hi[i] = __double2float_rn(bv * s64);
+        n_lo2[i] = __double2float_rn(__fma_rn(bv, s64, -widen(n_hi[i])));
+      }
+    }
+    const int hi = min(f_hi, f_lo + a.cap);
+    for (int e = f_lo + threadIdx.x; e < hi; e += 256) {
+      copy_async(s_qa + (unsigned)(buf * a.cap + e - f_lo) * 4u, a.dep_pos_f + e);
+      copy_async(s_wa + (unsigned)(buf * a.cap + e - f_lo) * 8u, reinterpret_cast<const double*>(a.wsplit) + e);
+    }
+  };
+  // chunks are claimed two ahead; the earliest unfinished one is always in hand
+  auto claim = [&]() {
+    if (threadIdx.x == 0) s_ticket = ctl_failed(a.ctl) ? a.nchunks : atomicAdd(&a.ctl->ticket, 1u);
+  };
+  auto claimed = [&]() { return static_cast<int>(min(s_ticket, (unsigned)a.nchunks)); };
+  claim();
+  __syncthreads();
+  int c = claimed();
+  __syncthreads();
+  claim();
+  __syncthreads();
+  int c1 = claimed();
+  __syncthreads();
+  claim();
+  fetch(c);
+  stage(c, 0);
+  fetch(c1);
+  for (int buf = 0; c < a.nchunks; buf ^= 1) {
+    const int base = c * kUnknowns, pr = base + j;
+    bool done = pr >= a.n || !col;
+    const int p = pr;
+    const int row = n_row, lo = n_lo;
+    int e = n_e;
+    const int e1 = n_e1;
+    float acc0[R], rlo[R], accd[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      acc0[i] = n_hi[i];
+      rlo[i] = n_lo2[i];
+      accd[i] = 0.f;
+      *reinterpret_cast<volatile Bits*>(&s_win[threadIdx.x * R + i]) = kPairEmpty;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const int c2 = claimed();
+    stage(c1, buf ^ 1);
+    fetch(c2);
+    const float2* lw = s_w + buf * a.cap - lo;
+    const int* lq = s_q + buf * a.cap - lo;
+    const int hi = lo + a.cap;
+    const double* const xw = reinterpret_cast<const double*>(a.xw);
+    const double *word = xw, *nword = xw;
+    unsigned local = s_wina, nlocal = s_wina;
+    bool mine = true, nmine = true;
+    float2 w = make_float2(0.f, 0.f), nw = w;
+    int nq = 0;
+    int left = e1 - e - 1;
+    auto next = [&](int ee) {
+      nq = ee < hi ? lq[ee] : a.dep_pos_f[ee];
+      nw = ee < hi ? lw[ee] : a.wsplit[ee];
+    };
+    auto target = [&](int q) {
+      const int off = (q) - base;
+      nmine = off >= 0;
+      nlocal = s_wina + (unsigned)((off & (kUnknowns - 1)) * (G * R) + k) * 8u;
+      nword = xw + (long long)q * rhs + k;
+    };
+    auto publish = [&]() {
+      Bits v[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        accd[i] = __fadd_rn(rlo[i], accd[i]);  // rho = S - x0 is the pair's low part; accd holds d from here on
+        v[i] = pack_pair(acc0[i], accd[i]);
+        st_shared_u64(&s_win[threadIdx.x * R + i], v[i]);
+      }
+      publish_words(reinterpret_cast<double*>(&a.xw[(long long)p * rhs + k]), v);
+      done = true;
+    };
+    if (!done) {
+      if (left < 0) {
+        publish();
+      } else {
+        next(e);
+        w = nw;
+        target(nq);
+        word = nword;
+        local = nlocal;
+        mine = nmine;
+        if (left > 0) next(++e);
+      }
+    }
+    bool fail = false;
+    unsigned idle = 0u;
+    WaitBudget wb(a.timeout_ns);
+    while (!__all_sync(kFull, done)) {
+      Bits bits[R];
+      poll_words(bits, local, word, mine, !done);
+      target(nq);  // in the poll's shadow
+      bool hit = true;
+#pragma unroll
+      for (int i = 0; i < R; ++i) hit = hit && bits[i] != kPairEmpty;
+      if (hit) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          df_sub_product(acc0[i], rlo[i], w.x, w.y, pair_x0(bits[i]));
+          accd[i] = fmaf(-w.x, pair_d(bits[i]), accd[i]);
+        }
+        if (left > 0) {
+          w = nw;
+          word = nword;
+          local = nlocal;
+          mine = nmine;
+          if (--left > 0) next(++e);
+        } else {
+          publish();
+        }
+      }
+      if ((++idle & 255u) == 0u) {
+        if (!wb.poll(a.ctl, p)) fail = true;
+        if (__any_sync(kFull, fail)) {
+          fail = true;
+          break;
+        }
+      }
+    }
+    if (!fail && pr < a.n && col) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        a.x[(long long)row * a.x_si + (long long)(k + i) * a.x_sk] = widen(acc0[i]) + widen(accd[i]);
+        mx_d = fmaxf(mx_d, fabsf(accd[i]));
+        mx_x = fmaxf(mx_x, fabsf(acc0[i] + accd[i]));
+        mx_x0 = fmaxf(mx_x0, fabsf(acc0[i]));
+      }
+    }
+    if (__syncthreads_or(fail)) break;
+    claim();
+    c = c1;
+    c1 = c2;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  stats_max(&a.stats[0], mx_d);
+  stats_max(&a.stats[1], mx_x);
+  stats_max(&a.stats[2], mx_x0);
+  __syncthreads();
+  leave(a.ctl);
+}
+
 template <int G, int RPL, int UD, bool DF>
 cudaError_t run_refine1(const RefineArgs& a, int block, size_t smem, int num_sms, cudaStream_t s) {
   auto kernel = k_pull_refine1<G, RPL, UD, DF>;
@@ -579,6 +787,61 @@ cudaError_t launch_refine_fused(const Layout& L, const Values<float>& v32, const
   if (rhs <= 16) return run_refine1<16, 1, 2, false>(a, block, smem, num_sms, s);
   if (rhs <= 32) return run_refine1<32, 1, 2, false>(a, block, smem, num_sms, s);
   return run_refine1<32, 2, 2, false>(a, block, smem, num_sms, s);
+}
+
+cudaError_t launch_refine_ahead(const Layout& L, const Values<double>& v64, int rhs, const double* b, double* x,
+                                long long si, long long sk, unsigned long long* xw, unsigned long long* stats,
+                                DeviceCtl* ctl, long long width, unsigned long long timeout_ns, int num_sms,
+                                cudaStream_t s, const float2* wsplit) {
+  if (L.n == 0) return cudaSuccess;
+  RefineArgs a{};
+  a.n = L.n;
+  a.rhs = rhs;
+  a.perm = L.perm;
+  a.dep_ptr = L.dep_ptr;
+  a.dep_pos_f = L.dep_pos_f;
+  a.rcp64 = v64.rcp;
+  a.wsplit = wsplit;
+  a.b = b;
+  a.x = x;
+  a.b_si = a.x_si = si;
+  a.b_sk = a.x_sk = sk;
+  a.xw = xw;
+  a.stats = stats;
+  a.ctl = ctl;
+  a.timeout_ns = timeout_ns;
+  const int avg = static_cast<int>(32LL * L.ndep / L.n);
+  // one right-hand side: one CTA per SM on levels of fewer than 1,536 unknowns
+  // (the 1M-row band, 811: 955 us; 1,045 with two), two beyond (3,004: 180 vs 232)
+  const int ctas = rhs > 1 ? 0 : (width < 1536 ? 1 : 2);
+  auto run = [&](auto kernel, int g, int r) -> cudaError_t {
+    const int unknowns = 256 / g;
+    a.nchunks = (a.n + unknowns - 1) / unknowns;
+    // twice the average chunk's lists (longer ones read the rest from global memory)
+    a.cap = std::min(g == 1 ? 4096 : 1024, std::max(64, (2 * avg * unknowns / 32 + 31) / 32 * 32));
+    const size_t smem = (size_t)256 * r * 8 + (size_t)2 * a.cap * 12;
+    cudaError_t e = cudaSuccess;
+    if (smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    int per = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 256, smem);
+    if (per < 1) per = 1;
+    if (ctas > 0) per = std::min(per, ctas);
+    const int grid = static_cast<int>(std::min<long long>((long long)num_sms * per, a.nchunks));
+    kernel<<<grid, 256, smem, s>>>(a);
+    return cudaGetLastError();
+  };
+  if (rhs == 1) return run(k_refine_ahead<1, 1>, 1, 1);
+  switch (ahead_multi_shape(rhs, 8, width < kNarrowWidth)) {
+    case 2 * 8 + 1: return run(k_refine_ahead<2, 1>, 2, 1);
+    case 4 * 8 + 1: return run(k_refine_ahead<4, 1>, 4, 1);
+    case 8 * 8 + 1: return run(k_refine_ahead<8, 1>, 8, 1);
+    case 16 * 8 + 1: return run(k_refine_ahead<16, 1>, 16, 1);
+    case 8 * 8 + 2: return run(k_refine_ahead<8, 2>, 8, 2);
+    case 16 * 8 + 2: return run(k_refine_ahead<16, 2>, 16, 2);
+    case 32 * 8 + 2: return run(k_refine_ahead<32, 2>, 32, 2);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 cudaError_t launch_refine_fused_imported(const Layout& L, const Values<double>& v64, const float2* wsplit,

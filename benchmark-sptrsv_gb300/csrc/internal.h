@@ -304,6 +304,7 @@ cudaError_t launch_levelset(const Layout& L, const Values<T>& V, int rhs, const 
 template <typename T>
 cudaError_t launch_pull_ahead(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
                               unsigned long long timeout_ns, int num_sms, cudaStream_t s, bool adj);
+constexpr long long kNarrowWidth = 350;  // unknowns per level (ahead_multi_shape)
 // The same for several right-hand sides (exec_ahead_multi.cu): lanes per unknown
 // times 8 plus right-hand sides per lane, or 0 where the general executor serves
 // the block (an odd number above 16 leaves every pair split: 32 lanes of one took
@@ -387,6 +388,12 @@ cudaError_t launch_refine_fused(const Layout& L, const Values<float>& v32, const
                                 unsigned long long* stats, DeviceCtl* ctl, const ExecConfig& cfg,
                                 unsigned long long timeout_ns, int num_sms, cudaStream_t s,
                                 const float2* wsplit = nullptr);
+// the fused step in double-float on a level-order layout, lists staged ahead (1 right-hand side, or a block
+// ahead_multi_shape has a shape for)
+cudaError_t launch_refine_ahead(const Layout& L, const Values<double>& v64, int rhs, const double* b, double* x,
+                                long long si, long long sk, unsigned long long* xw, unsigned long long* stats,
+                                DeviceCtl* ctl, long long width, unsigned long long timeout_ns, int num_sms,
+                                cudaStream_t s, const float2* wsplit);
 cudaError_t launch_split_weights(const double* w, long long count, float2* out, cudaStream_t s);
 // The same fused step (double-float residual, one right-hand side, b and x
 // vectors) on a blocked layout, with an importer warp per CTA (the table of

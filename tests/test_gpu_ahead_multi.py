@@ -70,3 +70,20 @@ def test_infinities_and_nan_stay_in_their_column(cuda):
         assert np.array_equal(np.isinf(out[0]), np.isinf(out[1]))
         ok = np.isfinite(out[0])
         assert relerr(out[1][ok], out[0][ok]) <= 1e-12
+
+
+@pytest.mark.parametrize("rhs", [1, 2, 4, 7, 8, 15, 16, 18, 31, 32, 34, 63, 64])
+@pytest.mark.parametrize("kind, n", [("band", 33), ("band", 5001), ("chain", 300), ("dense", 300), ("wide", 60_000)])
+def test_refined_blocks(cuda, oracle_port, kind, n, rhs):
+    """The fused first refinement step over the same lane shapes (1e-10, the refinement's tolerance)."""
+    from sptrsv_gb300 import SyncFreeSolver, matgen
+    m = {"band": lambda: matgen.poisson_band(n, 7.0, max(n // 3, 2), seed=n), "chain": lambda: matgen.chain(n),
+         "dense": lambda: matgen.dense_lower(n), "wide": lambda: matgen.poisson_band(n, 3.0, n // 2, seed=n)}[kind]()
+    b = np.random.default_rng(rhs).standard_normal((m.n, rhs))
+    ref = oracle_port.solve(m.col_ptr, m.row_idx, m.val, m.n, m.substitution, b)
+    s = SyncFreeSolver(m.col_ptr, m.row_idx, m.n, m.substitution, values=m.val)
+    bd = cuda.from_numpy(b).cuda()
+    for _ in range(2):
+        x, iters, est = s.solve_refine(bd)
+        assert 1 <= iters <= 4 and est <= 1e-12
+        assert relerr(x.cpu().numpy(), ref) <= 1e-10
