@@ -63,7 +63,6 @@ struct sptrsv_gb300_handle_s {
     double locality = 0.0;
     ClusterPlan cluster;       // one-cluster executor (block 0: the cluster cannot hold the system)
     bool cluster_f64 = false, cluster_f32 = false;  // the device can run it for this element type
-    bool ahead = false;        // level-order walks stage their lists ahead (use_ahead)
     bool narrow = false;       // few enough dependencies per level for one cluster
     double coarrive = 0.0;  // short lists: share of unknowns with >= 2 dependencies on the preceding level
   } plan;
@@ -100,6 +99,7 @@ struct sptrsv_gb300_handle_s {
   long long long_deps = 0, long_outs = 0;  // entries of long lists (long_cut)
   ChunkTable tab_fwd, tab_adj;
   PieceTable pc_fwd, pc_adj;
+  SplitTable sp_fwd, sp_adj;
   ImportTable imports;
   int import_option = 1;   // importer warp on blocked layouts (SPTRSV_OPTION_IMPORT)
   ImportTable pipe;        // unit pipeline tables (ring slots, stages)
@@ -191,6 +191,11 @@ void free_pieces(PieceTable& t) {
   t = PieceTable();
 }
 
+void free_split(SplitTable& t) {
+  if (t.walk) cudaFree(t.walk);
+  t = SplitTable();
+}
+
 void free_imports(ImportTable& t) {
   if (t.start) cudaFree(t.start);
   if (t.ptr) cudaFree(t.ptr);
@@ -256,6 +261,8 @@ void free_analysis(sptrsv_gb300_handle_s* h) {
   free_table(h->tab_adj);
   free_pieces(h->pc_fwd);
   free_pieces(h->pc_adj);
+  free_split(h->sp_fwd);
+  free_split(h->sp_adj);
   free_imports(h->imports);
   free_imports(h->pipe);
   free_values(h->v64);
@@ -358,6 +365,8 @@ int build_layout(sptrsv_gb300_handle_s* h, int block, cudaStream_t s) {
   free_table(h->tab_adj);
   free_pieces(h->pc_fwd);
   free_pieces(h->pc_adj);
+  free_split(h->sp_fwd);
+  free_split(h->sp_adj);
   free_imports(h->imports);
   free_imports(h->pipe);
   free_values(h->v64);
@@ -653,6 +662,30 @@ int ensure_pieces(sptrsv_gb300_handle_s* h, bool adj, int split, int chunk, cuda
   return build_pieces(h, t, *counts, adj, split, chunk, s);
 }
 
+// Split table of a walk, packed on the device.
+int ensure_split(sptrsv_gb300_handle_s* h, bool adj, int split, cudaStream_t s) {
+  SplitTable& t = adj ? h->sp_adj : h->sp_fwd;
+  if (t.walk && t.split == split) return SPTRSV_OK;
+  free_split(t);
+  const Layout& L = h->layout;
+  const int* ptr = adj ? L.out_ptr : L.dep_ptr;
+  const int blocks = pack_blocks(L.n);
+  int *count = nullptr, nseg = 0;
+  CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&count), sizeof(int) * ((size_t)blocks + 1), s));
+  cudaError_t e = launch_pack_count(ptr, L.n, split, adj, count, s);
+  if (e == cudaSuccess) e = exclusive_scan_int(count, count, blocks, true, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&nseg, count + blocks, sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&t.walk), sizeof(int) * 32 * (size_t)nseg);
+  if (e == cudaSuccess) e = launch_pack_fill(ptr, L.n, split, adj, count, t.walk, s);
+  cudaFreeAsync(count, s);
+  CUDA_TRY(e);
+  t.split = split;
+  t.nseg = nseg;
+  h->device_bytes += sizeof(int) * 32 * (size_t)nseg;
+  return SPTRSV_OK;
+}
+
 // Import table of the forward walk for chunks of `chunk` positions (see
 // ImportTable). When a chunk's window and imports do not fit one CTA's shared
 // memory only the sizes are recorded (no device arrays; the caller checks).
@@ -871,7 +904,6 @@ int effective_block(const sptrsv_gb300_handle_s* h) {
 // 112.5 us). Levels of fewer than 24 unknowns: 256
 // threads and runs of 256, so that most hops stay inside a CTA (150,001 rows,
 // 17 per level: 2,786 us; 2,926 with the first rule, 3,506 with runs of 32).
-constexpr double kAheadWork = 32000.0;  // use_ahead
 constexpr double kClusterDeps = 3000.0;
 constexpr long long kClusterWidth = 512;
 
@@ -962,7 +994,6 @@ int make_plan(sptrsv_gb300_handle_s* h, cudaStream_t s) {
       P.backoff = 0;
     }
   }
-  P.ahead = n > 0 && nl > 0 && static_cast<double>(nnz - n) + 4.0 * n <= kAheadWork * nl;
   plan_cluster(h);
   P.valid = true;
   return SPTRSV_OK;
@@ -1176,21 +1207,20 @@ bool use_cluster(const sptrsv_gb300_handle_s* h, bool adj) {
   return P.narrow && P.order_block >= h->n && (adj ? P.split_adj : P.split_fwd) == 0;
 }
 
-// Whether a warp-synchronous one-rhs walk in level order without split lists
-// runs k_pull_ahead (exec_ahead.cu), one CTA of 256 threads per SM taking one
-// dependency per iteration. The automatic plan takes it up to kAheadWork units of
-// work per level (dependencies plus 4 per unknown); past that line too few lanes
-// are in flight (us, the plan's other executor -> this one: 4M-row power law,
-// 30,100 units, 1,687 -> 1,484; 1.5M-row band, 31,800, 547 -> 542; 1.5M rows with
-// 3 entries per column, 37,800, 285 -> 299; 2M-row band, 49,700, 508 -> 612). With
-// explicit options it stands in for k_pull_wsync where they ask for just these
-// settings (the tuner's way to it).
+// Whether a warp-synchronous one-rhs walk in level order runs k_pull_ahead
+// (exec_ahead.cu, which picks entries per iteration and CTAs per SM itself), or
+// with split lists k_pull_ahead_split: under the automatic plan, or where
+// explicit options leave nothing else to k_pull_wsync (one CTA of 256 threads per
+// SM, one dependency per iteration: the tuner's way to it).
 bool use_ahead(const sptrsv_gb300_handle_s* h, const ExecConfig& c) {
   if (!c.wsync || c.exact || c.staged || !c.smem_tier || h->layout_block < h->n) return false;
   if (c.block != 256 || c.chunk != 256 || c.sleep_max != 0) return false;
-  if (planned(h, SPTRSV_OPTION_CTAS_PER_SM) && c.wsync_batch == 0) return h->plan.ahead;
+  if (planned(h, SPTRSV_OPTION_CTAS_PER_SM) && c.wsync_batch == 0) return true;
   return c.ctas_per_sm == 1 && c.wsync_batch == 1;
 }
+// Units of work per level (dependencies plus 4 per unknown) up to which split
+// lists are staged ahead: 13,300 215 -> 191 us, 25,000 614 -> 856 (exec_ahead_split.cu).
+constexpr double kSplitAheadWork = 16000.0;
 
 // The same for several right-hand sides (exec_ahead_multi.cu): level order, lists
 // that the one-rhs plan would not split (one lane walks a whole list: a power-law
@@ -1289,17 +1319,26 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
     const PieceTable* pc = nullptr;
     if (rhs == 1 && planned(h, SPTRSV_OPTION_SPLIT)) c.split = adj ? h->plan.split_adj : h->plan.split_fwd;
     const int longest = adj ? h->max_out_cnt : h->max_dep_cnt;
-    if (rhs == 1 && c.wsync && !c.exact && c.split > 0 && longest > c.split && !(adj && adj->grad)) {
+    const bool cut = rhs == 1 && c.wsync && !c.exact && c.split > 0 && longest > c.split && !(adj && adj->grad);
+    const bool split_ahead = cut && (planned(h, SPTRSV_OPTION_SPLIT) || c.split == 32) && use_ahead(h, c) &&
+                             static_cast<double>(h->nnz - n) + 4.0 * n <= kSplitAheadWork * h->nlevels;
+    if (split_ahead) {
+      ST_TRY(ensure_split(h, adj != nullptr, 32, s));
+      CUDA_TRY(launch_pull_ahead_split<T>(h->layout, V, v, static_cast<T*>(h->xw.p), h->ctl,
+                                          adj ? h->sp_adj : h->sp_fwd, timeout_ns(h), h->num_sms, s, adj != nullptr));
+    } else if (cut) {
       ST_TRY(ensure_pieces(h, adj != nullptr, c.split, c.chunk, s));
       pc = adj ? &h->pc_adj : &h->pc_fwd;
     }
-    if (!(adj && adj->grad) && use_ahead_multi(h, c, rhs, sizeof(T), adj != nullptr)) {
+    if (split_ahead) {
+      // launched above
+    } else if (!(adj && adj->grad) && use_ahead_multi(h, c, rhs, sizeof(T), adj != nullptr)) {
       CUDA_TRY(launch_pull_ahead_multi<T>(h->layout, V, rhs, v, static_cast<T*>(h->xw.p), h->ctl,
                                           n < kNarrowWidth * h->nlevels, timeout_ns(h), h->num_sms, s,
                                           adj != nullptr));
     } else if (rhs == 1 && !pc && !(adj && adj->grad) && use_ahead(h, c)) {
-      CUDA_TRY(launch_pull_ahead<T>(h->layout, V, v, static_cast<T*>(h->xw.p), h->ctl, timeout_ns(h), h->num_sms, s,
-                                    adj != nullptr));
+      CUDA_TRY(launch_pull_ahead<T>(h->layout, V, v, static_cast<T*>(h->xw.p), h->ctl, h->nlevels, timeout_ns(h),
+                                    h->num_sms, s, adj != nullptr));
     } else {
       if (c.wsync_batch == 0) c.wsync_batch = auto_wsync_batch(h, adj != nullptr, pc != nullptr);
       CUDA_TRY(launch_pull<T>(h->layout, V, rhs, v, static_cast<T*>(h->xw.p), h->ctl, c, timeout_ns(h), h->num_sms,
@@ -2323,7 +2362,7 @@ int sptrsv_gb300_tune(sptrsv_handle_t h, const void* d_val, int dtype, int rhs, 
     for (int ch : {128, 256}) cands.push_back({SCHED_PULL, big, ch, 0, 128, 1, 1, 2, 1, ch, sp});
     cands.push_back({SCHED_PULL, big, 256, 0, 128, 1, 1, 2, 1, 256, 0});
     for (int bt : {1, 2, 4}) cands.push_back({SCHED_PULL, big, 256, 0, 128, 1, 1, 2, 1, 256, sp, bt});
-    cands.push_back({SCHED_PULL, big, 256, 0, 0, 1, 1, 2, 1, 256, 0, 1});   // lists staged ahead (use_ahead)
+    for (int spl : {0, sp}) cands.push_back({SCHED_PULL, big, 256, 0, 0, 1, 1, 2, 1, 256, spl, 1});  // lists staged ahead (use_ahead)
     for (int ct : {2, 3}) {
       cands.push_back({SCHED_PULL, big, 256, 0, 0, ct, 1, 2, 1, 256, sp});
       cands.push_back({SCHED_PULL, big, 256, 0, 0, ct, 1, 2, 1, 256, 0});

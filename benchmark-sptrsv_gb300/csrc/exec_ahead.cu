@@ -1,29 +1,37 @@
 // Level-order executor with lists staged ahead (one right-hand side).
 //
-// As k_pull_wsync with one dependency per iteration: a warp takes 32 consecutive
-// walk indices, one unknown per lane, and advances in lockstep; values are
-// value-as-flag words in global memory. What a level costs is how long a
-// lockstep iteration takes once its last dependency is published, and there a
-// list entry fetched from global memory costs all 32 lanes its latency on top of
-// the poll's. So the warp claims its segments by ticket one ahead (no CTA
-// barrier between them), copies the next segment's lists, one contiguous range,
-// to shared memory with cp.async while it works on the current one, and works
-// out the next entry's address while a poll is in flight. An iteration is then
-// one poll (~285 cycles to L2) plus the multiply-add of the lanes that consumed.
-// Dependencies inside the segment go through a 32-word window in shared memory.
-// Lanes that are done do not poll: a poll of 32 scattered words holds the SM's
-// load path for ~32 cycles, which the other warps' polls wait for. For the same
-// reason one CTA of 8 warps per SM is best (two: 940 -> 1,170 us below).
+// As k_pull_wsync: a warp takes 32 consecutive walk indices, one unknown per lane,
+// and advances in lockstep; values are value-as-flag words in global memory.
+// What a level costs is how long a lockstep iteration takes once its last
+// dependency is published, and there a list entry fetched from global memory
+// costs all 32 lanes its latency on top of the poll's. So the warp claims its
+// segments by ticket one ahead (no CTA barrier between them) and copies the next
+// segment's lists, one contiguous range, to shared memory with cp.async while it
+// works on the current one. An iteration is then one poll (~285 cycles to L2)
+// plus the multiply-add of the lanes that consumed. Dependencies inside the
+// segment go through a 32-word window in shared memory. Lanes that are done do
+// not poll: a poll of 32 scattered words holds the SM's load path for ~32 cycles,
+// which the other warps' polls wait for, and a 128-byte line of L1 each, so the
+// list buffers must leave L1 room (two CTAs with 107 KB of buffers each: 2,767 us
+// on a split power-law walk, 2,127 with 86 KB).
+//
+// U = entries polled per iteration. One (the next entry's address is worked out
+// during the poll) is the shortest iteration; two consume lists that have
+// largely arrived twice as fast. Work per level, t = dependencies + 4 per unknown,
+// decides how many lanes are needed (us, forward / transposed):
+//   t < 21,000        one CTA per SM, U = 1 forward, 2 transposed: 1M-row band
+//                     (9,700) 893 / 897, with U the other way 905 / 1,011; 200k rows
+//                     of 40 entries (6,700) 1,010 / 1,084 vs 1,073 / 1,181
+//   t <= 34,000       one CTA, U = 2: 4M-row power law (30,100) 1,363 forward, 1,459
+//                     with U = 1, 1,403 with two CTAs; FP32, 25,000, 373 vs 410
+//   t <= 120,000      two CTAs, U = 2: 2M-row band (49,700) 413 / 479, one CTA 496 / 548
+//   beyond            three CTAs: 4M rows of 4 entries (230,000) 270 / 279, two 299 / 313
+// k_pull_wsync on these: 1,103 / 1,354, 1,187 / 1,383, 1,687, 490 (FP32), 510 / 578,
+// 323 / 297.
 //
 // A warp works through its segments in walk order and holds at most two claimed
 // ones it has not started, so the earliest unfinished segment is always being
 // worked on: every dependency lies earlier in the walk.
-//
-// FP64 solves, k_pull_wsync -> this kernel (forward / transposed, us): 1M-row
-// band, 811 unknowns per level, 1,103 / 1,354 -> 918 / 1,048; 4M-row power law,
-// 2,511 per level, 1,687 -> 1,484 (forward); 1M rows with 3 entries per column,
-// 2,358 per level, 384 / 481 -> 314 / 388; 200k rows with 40, 151 per level,
-// 1,187 / 1,383 -> 1,021 / 1,178; 1000 x 1000 mesh in level order 5,179 -> 1,729.
 #include <algorithm>
 
 #include "exec_ahead.cuh"
@@ -48,7 +56,7 @@ struct AheadArgs {
   unsigned long long timeout_ns;
 };
 
-template <typename T, bool ADJ>
+template <typename T, bool ADJ, int U>
 __global__ void __launch_bounds__(256) k_pull_ahead(AheadArgs<T> a) {
   using F = Flag<T>;
   using Bits = typename F::Bits;
@@ -125,22 +133,32 @@ __global__ void __launch_bounds__(256) k_pull_ahead(AheadArgs<T> a) {
     const T* lw = s_w + buf * a.cap - lo;
     const int* lq = s_q + buf * a.cap - lo;
     const int hi = lo + a.cap;
-    const T* word = a.xw;
-    const T* nword = a.xw;
-    unsigned local = s_wina, nlocal = s_wina;
-    bool mine = true, nmine = true;
-    T w = T(0), nw = T(0);
-    int nq = 0;
-    int left = e1 - e - 1;
-    auto next = [&](int ee) {
-      nq = ee < hi ? lq[ee] : a.pos[ee];
-      nw = ee < hi ? lw[ee] : a.w[ee];
-    };
-    auto target = [&](int q) {
+    // the U entries polled, in list order, and for U = 1 the one after it
+    const T *word0 = a.xw, *word1 = a.xw;
+    unsigned local0 = s_wina, local1 = s_wina;
+    bool mine0 = true, mine1 = true;
+    T w0 = T(0), w1 = T(0);
+    int q1 = 0;
+    int left = e1 - e;  // entries from the first polled on
+    auto target = [&](int q, const T*& word, unsigned& local, bool& mine) {
       const int off = (ADJ ? last - q : q) - base;
-      nmine = off >= 0;
-      nlocal = s_wina + (unsigned)(off & 31) * (unsigned)sizeof(T);
-      nword = a.xw + q;
+      mine = off >= 0;
+      local = s_wina + (unsigned)(off & 31) * (unsigned)sizeof(T);
+      word = a.xw + q;
+    };
+    auto entry = [&](int ee, int& q, T& w) {
+      q = ee < hi ? lq[ee] : a.pos[ee];
+      w = ee < hi ? lw[ee] : a.w[ee];
+    };
+    auto second = [&]() {
+      entry(e + 1, q1, w1);
+      if (U == 2) target(q1, word1, local1, mine1);
+    };
+    auto first = [&]() {
+      int q0;
+      entry(e, q0, w0);
+      target(q0, word0, local0, mine0);
+      if (left > 1) second();
     };
     auto publish = [&]() {
       F::store_shared(&s_win[lane], acc);
@@ -148,36 +166,33 @@ __global__ void __launch_bounds__(256) k_pull_ahead(AheadArgs<T> a) {
       done = true;
     };
     if (!done) {
-      if (left < 0) {
-        publish();
-      } else {
-        next(e);
-        w = nw;
-        target(nq);
-        word = nword;
-        local = nlocal;
-        mine = nmine;
-        if (left > 0) next(++e);
-      }
+      if (left <= 0) publish();
+      else first();
     }
-
     unsigned idle = 0u;
     WaitBudget wb(a.timeout_ns);
     while (!__all_sync(kFull, done)) {
-      Bits bits[1];
-      poll_words(bits, local, word, mine, !done);
-      target(nq);  // in the poll's shadow
-      if (bits[0] != F::EMPTY) {
-        acc = fma(-w, F::value(bits[0]), acc);
-        if (left > 0) {
-          w = nw;
-          word = nword;
-          local = nlocal;
-          mine = nmine;
-          if (--left > 0) next(++e);
+      Bits bits0[1], bits1[1];
+      poll_words(bits0, local0, word0, mine0, !done);
+      if (U == 2) poll_words(bits1, local1, word1, mine1, !done && left > 1);
+      if (U == 1) target(q1, word1, local1, mine1);  // in the poll's shadow
+      if (bits0[0] != F::EMPTY) {
+        acc = fma(-w0, F::value(bits0[0]), acc);
+        if (U == 2 && bits1[0] != F::EMPTY) {
+          acc = fma(-w1, F::value(bits1[0]), acc);
+          left -= 2;
+          e += 2;
+          if (left > 0) first();
         } else {
-          publish();
+          --left;
+          ++e;
+          w0 = w1;
+          word0 = word1;
+          local0 = local1;
+          mine0 = mine1;
+          if (left > 1) second();
         }
+        if (left <= 0) publish();
       }
       if ((++idle & 255u) == 0u) {
         if (!wb.poll(a.ctl, p)) fail = true;
@@ -201,13 +216,16 @@ __global__ void __launch_bounds__(256) k_pull_ahead(AheadArgs<T> a) {
 
 template <typename T>
 cudaError_t launch_pull_ahead(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
-                              unsigned long long timeout_ns, int num_sms, cudaStream_t s, bool adj) {
+                              int nlevels, unsigned long long timeout_ns, int num_sms, cudaStream_t s, bool adj) {
   if (L.n == 0) return cudaSuccess;
-  // list buffers hold twice the average segment (longer ones read the rest from
-  // global memory), at most 123 KB of them in FP64
   constexpr int block = 256;
+  const double t = (static_cast<double>(L.ndep) + 4.0 * L.n) / std::max(1, nlevels);
+  const int ctas = t <= 34000.0 ? 1 : (t <= 120000.0 ? 2 : 3);
+  const bool one = !adj && t < 21000.0;
+  // list buffers hold twice the average segment (longer ones read the rest from
+  // global memory), as far as the CTAs and L1 leave room
   const int avg = static_cast<int>(32LL * L.ndep / L.n);
-  const int cap = std::min(640, std::max(64, (2 * avg + 31) / 32 * 32));
+  const int cap = std::min(ctas == 1 ? 640 : (ctas == 2 ? 400 : 200), std::max(64, (2 * avg + 31) / 32 * 32));
   AheadArgs<T> a{};
   a.n = L.n;
   a.nseg = (L.n + 31) / 32;
@@ -223,16 +241,19 @@ cudaError_t launch_pull_ahead(const Layout& L, const Values<T>& V, const VecView
   a.ctl = ctl;
   a.timeout_ns = timeout_ns;
   const size_t smem = (size_t)(block / 32) * (32 * sizeof(T) + 2 * cap * (sizeof(T) + sizeof(int)));
-  auto kernel = adj ? k_pull_ahead<T, true> : k_pull_ahead<T, false>;
+  auto kernel = one ? k_pull_ahead<T, false, 1> : (adj ? k_pull_ahead<T, true, 2> : k_pull_ahead<T, false, 2>);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const int grid = std::min(num_sms, (a.nseg + block / 32 - 1) / (block / 32));
+  int per = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, block, smem);
+  per = std::max(1, std::min(per, ctas));
+  const int grid = std::min(num_sms * per, (a.nseg + block / 32 - 1) / (block / 32));
   kernel<<<grid, block, smem, s>>>(a);
   return cudaGetLastError();
 }
 template cudaError_t launch_pull_ahead<double>(const Layout&, const Values<double>&, const VecView<double>&, double*,
-                                               DeviceCtl*, unsigned long long, int, cudaStream_t, bool);
+                                               DeviceCtl*, int, unsigned long long, int, cudaStream_t, bool);
 template cudaError_t launch_pull_ahead<float>(const Layout&, const Values<float>&, const VecView<float>&, float*,
-                                              DeviceCtl*, unsigned long long, int, cudaStream_t, bool);
+                                              DeviceCtl*, int, unsigned long long, int, cudaStream_t, bool);
 
 }  // namespace sptrsv

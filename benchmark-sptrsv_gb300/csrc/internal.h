@@ -300,10 +300,24 @@ template <typename T>
 cudaError_t launch_levelset(const Layout& L, const Values<T>& V, int rhs, const VecView<T>& v, T* xw,
                             DeviceCtl* ctl, const ExecConfig& cfg, unsigned long long timeout_ns,
                             cudaStream_t s);
-// level-order executor with lists staged ahead, one CTA per SM (exec_ahead.cu)
+// level-order executor with lists staged ahead (exec_ahead.cu)
 template <typename T>
 cudaError_t launch_pull_ahead(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
-                              unsigned long long timeout_ns, int num_sms, cudaStream_t s, bool adj);
+                              int nlevels, unsigned long long timeout_ns, int num_sms, cudaStream_t s, bool adj);
+// Segments of the split-list form (exec_ahead_split.cu): lists longer than `split`
+// take up to 32 adjacent lanes of a segment, interleaved (lane j of k takes
+// entries j, j + k, ...); no unknown straddles two segments.
+struct SplitTable {
+  int split = 0, nseg = 0;
+  int* walk = nullptr;  // device [nseg*32] walk index of each lane's unknown (-1: padding)
+};
+int pack_blocks(int n);  // blocks the packing counts and fills
+cudaError_t launch_pack_count(const int* ptr, int n, int split, bool adj, int* count, cudaStream_t s);
+cudaError_t launch_pack_fill(const int* ptr, int n, int split, bool adj, const int* first, int* walk, cudaStream_t s);
+template <typename T>
+cudaError_t launch_pull_ahead_split(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
+                                    const SplitTable& tab, unsigned long long timeout_ns, int num_sms, cudaStream_t s,
+                                    bool adj);
 constexpr long long kNarrowWidth = 350;  // unknowns per level (ahead_multi_shape)
 // The same for several right-hand sides (exec_ahead_multi.cu): lanes per unknown
 // times 8 plus right-hand sides per lane, or 0 where the general executor serves

@@ -50,6 +50,37 @@ def test_staged_ahead_solves_match_the_oracle(cuda, oracle_port, kind, n, lower,
         s.close()
 
 
+@pytest.mark.parametrize("lower", [True, False])
+@pytest.mark.parametrize("kind, n", [("star", 40), ("star", 70), ("star", 3000), ("power", 2000), ("power", 20_000),
+                                     ("few", 1025), ("few", 5000)])
+def test_split_lists_match_the_oracle(cuda, oracle_port, kind, n, lower):
+    """Lists of up to 3,000 entries over 2 to 32 lanes, whole and partial segments, packing blocks of 1,024."""
+    from sptrsv_gb300 import SyncFreeSolver, matgen
+    if kind == "star":
+        m = matgen.star(n, lower=lower)
+    elif kind == "power":
+        m = matgen.power_law_band(n, 9 * n, n // 4, seed=n, lower=lower)
+    else:   # a few long columns among columns of two entries
+        counts = np.where(np.arange(n) % 97 == 0, 200, 2)
+        m = matgen.banded_random_lower(n, counts, n // 2, n, lower=lower)
+    s64 = SyncFreeSolver(m.col_ptr, m.row_idx, m.n, m.substitution, values=m.val, cluster=0)
+    if not lower:
+        assert s64.info()["split"] == 32
+    s64.close()
+    rng = np.random.default_rng(n)
+    b = rng.standard_normal(m.n)
+    ref = oracle_port.solve(m.col_ptr, m.row_idx, m.val, m.n, m.substitution, b)
+    t = m.transpose()
+    tref = oracle_port.solve(t.col_ptr, t.row_idx, t.val, m.n, t.substitution, b)
+    for dtype, tol in ((np.float64, 1e-12), (np.float32, 1e-5)):
+        s = SyncFreeSolver(m.col_ptr, m.row_idx, m.n, m.substitution, values=m.val.astype(dtype), cluster=0)
+        bd = cuda.from_numpy(b.astype(dtype)).cuda()
+        for _ in range(2):
+            assert relerr(s.solve(bd).cpu().numpy(), ref) <= tol
+            assert relerr(s.solve_adjoint(bd)[0].cpu().numpy(), tref) <= tol
+        s.close()
+
+
 def test_infinities_and_nan_reach_the_same_unknowns(cuda):
     """Against the executor that reads its lists from global memory (128 threads per CTA)."""
     from sptrsv_gb300 import SyncFreeSolver
