@@ -101,6 +101,7 @@ struct sptrsv_gb300_handle_s {
   PieceTable pc_fwd, pc_adj;
   SplitTable sp_fwd, sp_adj;
   ImportTable imports;
+  UnitTable units;
   int import_option = 1;   // importer warp on blocked layouts (SPTRSV_OPTION_IMPORT)
   ImportTable pipe;        // unit pipeline tables (ring slots, stages)
   int pipe_option = 0;     // SPTRSV_OPTION_UNIT_PIPELINE: 0 off, 1 on, else the ring cap
@@ -207,6 +208,12 @@ void free_imports(ImportTable& t) {
   t = ImportTable();
 }
 
+void free_units(UnitTable& t) {
+  for (int* p : {t.start, t.seg_ptr, t.seg})
+    if (p) cudaFree(p);
+  t = UnitTable();
+}
+
 void free_layout(Layout& L) {
   dev_free(&L.perm);
   dev_free(&L.iperm);
@@ -264,6 +271,7 @@ void free_analysis(sptrsv_gb300_handle_s* h) {
   free_split(h->sp_fwd);
   free_split(h->sp_adj);
   free_imports(h->imports);
+  free_units(h->units);
   free_imports(h->pipe);
   free_values(h->v64);
   free_values(h->v32);
@@ -368,6 +376,7 @@ int build_layout(sptrsv_gb300_handle_s* h, int block, cudaStream_t s) {
   free_split(h->sp_fwd);
   free_split(h->sp_adj);
   free_imports(h->imports);
+  free_units(h->units);
   free_imports(h->pipe);
   free_values(h->v64);
   free_values(h->v32);
@@ -686,13 +695,11 @@ int ensure_split(sptrsv_gb300_handle_s* h, bool adj, int split, cudaStream_t s) 
   return SPTRSV_OK;
 }
 
-// Import table of the forward walk for chunks of `chunk` positions (see
-// ImportTable). When a chunk's window and imports do not fit one CTA's shared
-// memory only the sizes are recorded (no device arrays; the caller checks).
-// ring_cap = 0: the importer kernel's table (a window as wide as the longest
-// unit). ring_cap > 0: the unit pipeline's (ring slots, far dependencies
-// imported, stages of at most pmax positions and emax entries).
-int build_import_table(sptrsv_gb300_handle_s* h, ImportTable& t, int chunk, size_t elem, int ring_cap, int pmax,
+// The unit pipeline's import table (see ImportTable): ring slots, far dependencies
+// imported, stages of at most pmax positions and emax entries. When a unit's
+// window and imports do not fit one CTA's shared memory only the sizes are
+// recorded (no device arrays; the caller checks).
+int build_pipe_table(sptrsv_gb300_handle_s* h, ImportTable& t, int chunk, size_t elem, int ring_cap, int pmax,
                        int emax, int stages, cudaStream_t s) {
   free_imports(t);
   const int smax = std::max(4, pmax / 8);  // segments per stage
@@ -713,16 +720,12 @@ int build_import_table(sptrsv_gb300_handle_s* h, ImportTable& t, int chunk, size
   const int nchunks = static_cast<int>(starts.size()) - 1;
   int width = 1;  // shared-memory window: the longest unit
   for (int c = 0; c < nchunks; ++c) width = std::max(width, starts[c + 1] - starts[c]);
-  int ring = 0;
-  if (ring_cap > 0) {
-    ring = 64;
-    while (ring < width && ring < ring_cap) ring *= 2;
-  }
-  const int win = ring > 0 ? ring : width;  // first import slot
+  int ring = 64;
+  while (ring < width && ring < ring_cap) ring *= 2;
   // a dependency reads the ring when it is in the unit and (with wrapping) fewer
   // than ring - 32 positions back
   auto in_ring = [&](int p, int qe, int base, int len) {
-    return qe >= base && (ring == 0 || len <= ring || p - qe < ring - 32);
+    return qe >= base && (len <= ring || p - qe < ring - 32);
   };
   std::vector<int> cptr((size_t)nchunks + 1, 0), q, slot((size_t)std::max(ndep, 1) + 16, -1), ext;
   std::vector<int> ustage, segs, useg;
@@ -741,49 +744,47 @@ int build_import_table(sptrsv_gb300_handle_s* h, ImportTable& t, int chunk, size
       for (int e = ptr[p]; e < ptr[p + 1]; ++e) {
         const int qe = pos[e];
         slot[e] = in_ring(p, qe, base, len)
-                      ? (ring > 0 ? (qe - base) & (ring - 1) : qe - base)
-                      : win + static_cast<int>(std::lower_bound(ext.begin(), ext.end(), qe) - ext.begin());
+                      ? (qe - base) & (ring - 1)
+                      : ring + static_cast<int>(std::lower_bound(ext.begin(), ext.end(), qe) - ext.begin());
       }
     q.insert(q.end(), ext.begin(), ext.end());
     cptr[c + 1] = static_cast<int>(q.size());
     max_imp = std::max(max_imp, static_cast<int>(ext.size()));
-    if (ring > 0) {
-      // segments: runs of at most 32 consecutive positions (one lane each) whose
-      // lists fit a stage buffer. (Ending runs early at level boundaries was
-      // measured: no faster on 32-wide levels, slower on narrower ones.)
-      useg.clear();
-      int first = base;
-      for (int p = base + 1; p < end; ++p) {
-        if (p - first >= 32 || ptr[p + 1] - ptr[first] > emax) {
-          useg.push_back(first);
-          first = p;
-        }
+    // segments: runs of at most 32 consecutive positions (one lane each) whose
+    // lists fit a stage buffer. (Ending runs early at level boundaries was
+    // measured: no faster on 32-wide levels, slower on narrower ones.)
+    useg.clear();
+    int first = base;
+    for (int p = base + 1; p < end; ++p) {
+      if (p - first >= 32 || ptr[p + 1] - ptr[first] > emax) {
+        useg.push_back(first);
+        first = p;
       }
-      useg.push_back(first);
-      // stages: runs of whole segments with at most pmax positions, emax list
-      // entries and smax segments
-      ustage.push_back(static_cast<int>(stab.size() / 2));
-      const int sg_base = static_cast<int>(segs.size());
-      const int nsu = static_cast<int>(useg.size());
-      for (int i = 0; i < nsu;) {
-        const int lo = useg[i];
-        int j = i;
-        while (j < nsu) {
-          const int hi = j + 1 < nsu ? useg[j + 1] : end;
-          if (hi - lo > pmax || ptr[hi] - ptr[lo] > emax || j + 1 - i > smax) break;
-          ++j;
-        }
-        if (j == i) {  // one segment's lists exceed a stage buffer
-          stages_fit = false;
-          break;
-        }
-        const int hi = j < nsu ? useg[j] : end;
-        stab.push_back(make_int4(lo, hi, ptr[lo], ptr[hi]));
-        stab.push_back(make_int4(sg_base + i, sg_base + j, 0, 0));
-        i = j;
-      }
-      segs.insert(segs.end(), useg.begin(), useg.end());
     }
+    useg.push_back(first);
+    // stages: runs of whole segments with at most pmax positions, emax list
+    // entries and smax segments
+    ustage.push_back(static_cast<int>(stab.size() / 2));
+    const int sg_base = static_cast<int>(segs.size());
+    const int nsu = static_cast<int>(useg.size());
+    for (int i = 0; i < nsu;) {
+      const int lo = useg[i];
+      int j = i;
+      while (j < nsu) {
+        const int hi = j + 1 < nsu ? useg[j + 1] : end;
+        if (hi - lo > pmax || ptr[hi] - ptr[lo] > emax || j + 1 - i > smax) break;
+        ++j;
+      }
+      if (j == i) {  // one segment's lists exceed a stage buffer
+        stages_fit = false;
+        break;
+      }
+      const int hi = j < nsu ? useg[j] : end;
+      stab.push_back(make_int4(lo, hi, ptr[lo], ptr[hi]));
+      stab.push_back(make_int4(sg_base + i, sg_base + j, 0, 0));
+      i = j;
+    }
+    segs.insert(segs.end(), useg.begin(), useg.end());
   }
   t.chunk = chunk;
   t.width = width;
@@ -794,14 +795,10 @@ int build_import_table(sptrsv_gb300_handle_s* h, ImportTable& t, int chunk, size
   t.emax = emax;
   t.stages = stages;
   t.smax = smax;
-  if (ring > 0) {
-    ustage.push_back(static_cast<int>(stab.size() / 2));
-    segs.push_back(n);
-    if (!stages_fit || unit_smem_bytes(ring, max_imp, pmax, emax, smax, stages, elem) > 220 * 1024)
-      return SPTRSV_OK;  // recorded: does not fit
-  } else if (imported_smem_bytes(width, max_imp, elem) > 220 * 1024) {
+  ustage.push_back(static_cast<int>(stab.size() / 2));
+  segs.push_back(n);
+  if (!stages_fit || unit_smem_bytes(ring, max_imp, pmax, emax, smax, stages, elem) > 220 * 1024)
     return SPTRSV_OK;  // recorded: does not fit
-  }
   CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.start), sizeof(int) * starts.size()));
   CUDA_TRY(cudaMemcpy(t.start, starts.data(), sizeof(int) * starts.size(), cudaMemcpyHostToDevice));
   CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.ptr), sizeof(int) * cptr.size()));
@@ -810,17 +807,15 @@ int build_import_table(sptrsv_gb300_handle_s* h, ImportTable& t, int chunk, size
   CUDA_TRY(cudaMemcpy(t.ptr, cptr.data(), sizeof(int) * cptr.size(), cudaMemcpyHostToDevice));
   if (!q.empty()) CUDA_TRY(cudaMemcpy(t.q, q.data(), sizeof(int) * q.size(), cudaMemcpyHostToDevice));
   CUDA_TRY(cudaMemcpy(t.dep_slot, slot.data(), sizeof(int) * slot.size(), cudaMemcpyHostToDevice));
-  if (ring > 0) {
-    CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.ustage), sizeof(int) * ustage.size()));
-    CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.stab), sizeof(int4) * std::max<size_t>(stab.size(), 2)));
-    segs.resize(segs.size() + 16, n);  // bulk copies read up to 16 bytes past a slice
-    CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.segs), sizeof(int) * segs.size()));
-    CUDA_TRY(cudaMemcpy(t.ustage, ustage.data(), sizeof(int) * ustage.size(), cudaMemcpyHostToDevice));
-    if (!stab.empty()) CUDA_TRY(cudaMemcpy(t.stab, stab.data(), sizeof(int4) * stab.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(t.segs, segs.data(), sizeof(int) * segs.size(), cudaMemcpyHostToDevice));
-    t.nstages = static_cast<int>(stab.size() / 2);
-    h->device_bytes += sizeof(int) * (ustage.size() + segs.size()) + sizeof(int4) * stab.size();
-  }
+  CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.ustage), sizeof(int) * ustage.size()));
+  CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.stab), sizeof(int4) * std::max<size_t>(stab.size(), 2)));
+  segs.resize(segs.size() + 16, n);  // bulk copies read up to 16 bytes past a slice
+  CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.segs), sizeof(int) * segs.size()));
+  CUDA_TRY(cudaMemcpy(t.ustage, ustage.data(), sizeof(int) * ustage.size(), cudaMemcpyHostToDevice));
+  if (!stab.empty()) CUDA_TRY(cudaMemcpy(t.stab, stab.data(), sizeof(int4) * stab.size(), cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpy(t.segs, segs.data(), sizeof(int) * segs.size(), cudaMemcpyHostToDevice));
+  t.nstages = static_cast<int>(stab.size() / 2);
+  h->device_bytes += sizeof(int) * (ustage.size() + segs.size()) + sizeof(int4) * stab.size();
   t.chunk = chunk;
   t.nchunks = nchunks;
   t.max_imports = max_imp;
@@ -828,8 +823,137 @@ int build_import_table(sptrsv_gb300_handle_s* h, ImportTable& t, int chunk, size
   return SPTRSV_OK;
 }
 
+// The units of a blocked layout with their level segments.
+int ensure_units(sptrsv_gb300_handle_s* h, cudaStream_t s) {
+  UnitTable& t = h->units;
+  if (t.seg) return SPTRSV_OK;
+  free_units(t);
+  const std::vector<int>& starts = h->layout_units;
+  const Layout& L = h->layout;
+  UnitTable made;  // becomes the table once complete
+  made.count = static_cast<int>(starts.size()) - 1;
+  for (int c = 0; c < made.count; ++c) made.width = std::max(made.width, starts[c + 1] - starts[c]);
+  int* levels = nullptr;
+  auto alloc = [&](int** p, size_t items) { return cudaMalloc(reinterpret_cast<void**>(p), sizeof(int) * items); };
+  auto build = [&]() -> cudaError_t {
+    cudaError_t e;
+    if ((e = alloc(&made.start, starts.size())) != cudaSuccess) return e;
+    if ((e = alloc(&made.seg_ptr, starts.size())) != cudaSuccess) return e;
+    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&levels), sizeof(int), s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(levels, 0, sizeof(int), s)) != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(made.start, starts.data(), sizeof(int) * starts.size(), cudaMemcpyHostToDevice, s)) !=
+        cudaSuccess)
+      return e;
+    if ((e = launch_unit_segments(L.perm, h->depth, made.start, made.count, nullptr, made.seg_ptr, levels, nullptr,
+                                  s)) != cudaSuccess)
+      return e;
+    if ((e = exclusive_scan_int(made.seg_ptr, made.seg_ptr, made.count, true, s)) != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(&made.segments, made.seg_ptr + made.count, sizeof(int), cudaMemcpyDeviceToHost, s)) !=
+        cudaSuccess)
+      return e;
+    if ((e = cudaMemcpyAsync(&made.levels, levels, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+    if ((e = alloc(&made.seg, (size_t)made.segments + 1)) != cudaSuccess) return e;
+    if ((e = launch_unit_segments(L.perm, h->depth, made.start, made.count, made.seg_ptr, nullptr, nullptr, made.seg,
+                                  s)) != cudaSuccess)
+      return e;
+    if ((e = cudaMemcpyAsync(made.seg + made.segments, &L.n, sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess)
+      return e;
+    return cudaStreamSynchronize(s);
+  };
+  const cudaError_t err = build();
+  if (levels) cudaFreeAsync(levels, s);
+  if (err != cudaSuccess) {
+    free_units(made);
+    return map_cuda_error(err);
+  }
+  t = made;
+  h->device_bytes += sizeof(int) * (2 * starts.size() + (size_t)t.segments + 1);
+  return SPTRSV_OK;
+}
+
+// The importer executors' table, built on the device (the host loops took 13 ms
+// on the 2M-row mesh).
 int build_imports(sptrsv_gb300_handle_s* h, int chunk, size_t elem, cudaStream_t s) {
-  return build_import_table(h, h->imports, chunk, elem, 0, 0, 0, 0, s);
+  ImportTable& t = h->imports;
+  free_imports(t);
+  const Layout& L = h->layout;
+  const int n = L.n;
+  std::vector<int> starts = h->layout_units;
+  if (starts.empty())
+    for (int b = 0; b <= n; b += chunk) starts.push_back(std::min(b, n));
+  if (starts.back() != n) starts.push_back(n);
+  const int nunits = static_cast<int>(starts.size()) - 1;
+  int width = 1;  // shared-memory window: the longest unit
+  for (int c = 0; c < nunits; ++c) width = std::max(width, starts[c + 1] - starts[c]);
+  t.chunk = chunk;
+  t.nchunks = nunits;
+  t.width = width;
+  if (imported_smem_bytes(width, 0, elem) > 220 * 1024) return SPTRSV_OK;  // recorded: does not fit
+  ImportTable made;  // becomes the table once complete
+  int *count = nullptr, *ext_u = nullptr, *ext_e = nullptr;
+  unsigned* ext_q = nullptr;
+  std::vector<int> ptr((size_t)nunits + 1, 0);
+  auto alloc = [&](auto** p, size_t items) {
+    return cudaMalloc(reinterpret_cast<void**>(p), sizeof(int) * std::max<size_t>(items, 1));
+  };
+  auto build = [&]() -> cudaError_t {
+    cudaError_t e;
+    if ((e = alloc(&made.start, starts.size())) != cudaSuccess) return e;
+    if ((e = alloc(&made.ptr, starts.size())) != cudaSuccess) return e;
+    if ((e = alloc(&made.dep_slot, (size_t)L.ndep + 16)) != cudaSuccess) return e;
+    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&count), sizeof(int), s)) != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(made.start, starts.data(), sizeof(int) * starts.size(), cudaMemcpyHostToDevice, s)) !=
+        cudaSuccess)
+      return e;
+    if ((e = cudaMemsetAsync(count, 0, sizeof(int), s)) != cudaSuccess) return e;
+    if ((e = launch_import_split(L, made.start, nunits, made.dep_slot, count, nullptr, nullptr, nullptr, s)) !=
+        cudaSuccess)
+      return e;
+    int next = 0;
+    if ((e = cudaMemcpyAsync(&next, count, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+    if ((e = alloc(&made.q, next)) != cudaSuccess) return e;  // at most one import per entry
+    if (next > 0) {
+      const size_t bytes = sizeof(int) * (size_t)next;
+      if ((e = cudaMallocAsync(reinterpret_cast<void**>(&ext_q), bytes, s)) != cudaSuccess) return e;
+      if ((e = cudaMallocAsync(reinterpret_cast<void**>(&ext_u), bytes, s)) != cudaSuccess) return e;
+      if ((e = cudaMallocAsync(reinterpret_cast<void**>(&ext_e), bytes, s)) != cudaSuccess) return e;
+      if ((e = cudaMemsetAsync(count, 0, sizeof(int), s)) != cudaSuccess) return e;
+      if ((e = launch_import_split(L, made.start, nunits, made.dep_slot, count, ext_q, ext_u, ext_e, s)) != cudaSuccess)
+        return e;
+    }
+    if ((e = launch_import_tables(ext_q, ext_u, ext_e, next, n, nunits, width, made.ptr, made.q, made.dep_slot, s)) !=
+        cudaSuccess)
+      return e;
+    if ((e = cudaMemcpyAsync(ptr.data(), made.ptr, sizeof(int) * ptr.size(), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+      return e;
+    return cudaStreamSynchronize(s);
+  };
+  const cudaError_t err = build();
+  for (void* b : {(void*)count, (void*)ext_q, (void*)ext_u, (void*)ext_e})
+    if (b) cudaFreeAsync(b, s);
+  if (err != cudaSuccess) {
+    free_imports(made);
+    free_imports(t);
+    return map_cuda_error(err);
+  }
+  int max_imp = 0;
+  for (int c = 0; c < nunits; ++c) max_imp = std::max(max_imp, ptr[c + 1] - ptr[c]);
+  t.max_imports = max_imp;
+  if (imported_smem_bytes(width, max_imp, elem) > 220 * 1024) {
+    free_imports(made);
+    return SPTRSV_OK;  // recorded: does not fit
+  }
+  made.chunk = chunk;
+  made.nchunks = nunits;
+  made.width = width;
+  made.max_imports = max_imp;
+  t = made;
+  h->device_bytes += sizeof(int) * (2 * starts.size() + (size_t)ptr[nunits] + (size_t)L.ndep + 16);
+  // a solve captured after a refinement alone has run
+  if (h->max_dep_cnt <= 4 && !h->layout_units.empty()) ST_TRY(ensure_units(h, s));
+  return SPTRSV_OK;
 }
 
 // Largest per-chunk entry budget whose ring of stage buffers (plus the
@@ -1116,7 +1240,7 @@ bool pipe_ready(sptrsv_gb300_handle_s* h, int chunk, cudaStream_t s) {
   const int stages = (h->user_set & (1ull << SPTRSV_OPTION_STAGES)) ? h->stages_option : 3;
   ImportTable& t = h->pipe;
   if (t.chunk != chunk || t.ring_cap != ring_cap || t.emax != emax || t.pmax != pmax || t.stages != stages) {
-    if (build_import_table(h, t, chunk, sizeof(T), ring_cap, pmax, emax, stages, s) != SPTRSV_OK) {
+    if (build_pipe_table(h, t, chunk, sizeof(T), ring_cap, pmax, emax, stages, s) != SPTRSV_OK) {
       free_imports(t);
       return false;
     }
@@ -1218,6 +1342,30 @@ bool use_ahead(const sptrsv_gb300_handle_s* h, const ExecConfig& c) {
   if (planned(h, SPTRSV_OPTION_CTAS_PER_SM) && c.wsync_batch == 0) return true;
   return c.ctas_per_sm == 1 && c.wsync_batch == 1;
 }
+
+// Whether the one-rhs forward walk of a blocked layout may run k_pull_block
+// (exec_block.cu): lists of at most 4 entries (more make a level longer and the
+// ring wider; they stay with k_pull_wsync_imp), whole units in shared memory
+// beside the ring, and the importer executor not asked for (its entries per
+// iteration or SPTRSV_OPTION_IMPORT set). Its one
+// consumer warp takes the 32-wide segments of a level in turn where the importer
+// executor has several warps, so it is used up to 1 + 0.75 x the longest list
+// segments per level (k_pull_wsync_imp vs k_pull_block, 1M rows in chains of 300:
+// lists of one entry, 1 segment per level 78 vs 58 us, 2 segments 85 vs 97, 3
+// segments 105 vs 141; lists of two, 2 segments 132 vs 115, 3 segments 173 vs 168;
+// lists of four, 3 segments 341 vs 236).
+template <typename T>
+bool use_block(const sptrsv_gb300_handle_s* h, const ExecConfig& c) {
+  if (!c.wsync || c.exact || c.staged || !c.smem_tier || c.wsync_batch != 0) return false;
+  if (!h->import_option || (h->user_set & (1ull << SPTRSV_OPTION_IMPORT))) return false;
+  if (h->layout_block >= h->n || c.chunk != h->layout_block || h->layout_units.size() < 2) return false;
+  if (h->max_dep_cnt < 1 || h->max_dep_cnt > 4 || (c.split > 0 && h->max_dep_cnt > c.split)) return false;
+  int width = 0;
+  for (size_t i = 1; i < h->layout_units.size(); ++i)
+    width = std::max(width, h->layout_units[i] - h->layout_units[i - 1]);
+  return block_smem_bytes<T>(width, h->max_dep_cnt) <= 226 * 1024;
+}
+
 // Units of work per level (dependencies plus 4 per unknown) up to which split
 // lists are staged ahead: 13,300 215 -> 191 us, 25,000 614 -> 856 (exec_ahead_split.cu).
 constexpr double kSplitAheadWork = 16000.0;
@@ -1272,6 +1420,11 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
     ST_TRY(ensure_buf(h, h->xw, elems * sizeof(T), 0, s));
     if (c.sched != SCHED_LEVELSET) CUDA_TRY(cudaMemsetAsync(h->xw.p, 0xFF, elems * sizeof(T), s));
   }
+  bool block = !cluster && c.sched == SCHED_PULL && rhs == 1 && !adj && !h->pipe_option && use_block<T>(h, c);
+  if (block) {
+    ST_TRY(ensure_units(h, s));
+    block = 4LL * h->units.segments <= (4LL + 3 * h->max_dep_cnt) * h->units.levels;
+  }
   if (h->profile) {
     if (!h->ev_exec[0]) {
       CUDA_TRY(cudaEventCreate(&h->ev_exec[0]));
@@ -1303,6 +1456,9 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
     CUDA_TRY(launch_pull_unit<T>(h->layout, V, v, static_cast<T*>(h->xw.p), static_cast<T*>(h->c0.p), h->ctl, c,
                                  timeout_ns(h), h->num_sms, s, h->pipe));
     h->last_pipe = true;
+  } else if (block) {
+    CUDA_TRY(launch_pull_block<T>(h->layout, V, v, static_cast<T*>(h->xw.p), h->ctl, h->units, h->max_dep_cnt,
+                                  timeout_ns(h), h->num_sms, s));
   } else if (rhs == 1 && c.wsync && !c.exact && !adj && h->import_option && h->layout_block < n &&
              c.chunk == h->layout_block && c.smem_tier &&
              !(c.split > 0 && h->max_dep_cnt > c.split) &&

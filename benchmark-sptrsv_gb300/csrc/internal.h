@@ -120,6 +120,17 @@ struct ImportTable {
   int* segs = nullptr;      // device [segments+1 + padding] first position of each segment
 };
 
+// Units of a blocked layout and their level segments (k_pull_block): unit c starts
+// at position start[c] and owns segments seg_ptr[c] .. seg_ptr[c+1]-1; segment g
+// covers positions [seg[g], seg[g+1]), at most 32 of one level.
+struct UnitTable {
+  int count = 0, width = 0;  // units, positions of the longest
+  int segments = 0, levels = 0;  // of all units
+  int* start = nullptr;      // device [count+1]
+  int* seg_ptr = nullptr;    // device [count+1]
+  int* seg = nullptr;        // device [segments+1]
+};
+
 // Solve-time description of one right-hand-side block. Element (i, k) of b
 // (x) lives at i*si + k*sk.
 template <typename T>
@@ -362,6 +373,23 @@ bool cluster_fits(const ClusterPlan& plan, int n);
 template <typename T>
 cudaError_t launch_pull_cluster(const Layout& L, const Values<T>& V, const VecView<T>& v, DeviceCtl* ctl,
                                 const ClusterPlan& plan, unsigned long long timeout_ns, cudaStream_t s, bool adj);
+// Blocked layouts (exec_block.cu). In-unit slots and the number of imported
+// entries (ext_q null), or those entries as (position, unit, entry); then the
+// import tables from them. Level segments of the units: count per unit and levels of
+// all units (seg null), then their starts.
+cudaError_t launch_import_split(const Layout& L, const int* unit, int nunits, int* dep_slot, int* count,
+                                unsigned* ext_q, int* ext_u, int* ext_e, cudaStream_t s);
+cudaError_t launch_import_tables(const unsigned* ext_q, const int* ext_u, const int* ext_e, int count, int n,
+                                 int nunits, int width, int* im_ptr, int* im_q, int* dep_slot, cudaStream_t s);
+cudaError_t launch_unit_segments(const int* perm, const int* depth, const int* unit, int nunits, const int* first,
+                                 int* count, int* levels, int* seg, cudaStream_t s);
+// one consumer warp per unit, level by level; lists of at most 4 entries (longest)
+template <typename T>
+size_t block_smem_bytes(int width, int longest);
+template <typename T>
+cudaError_t launch_pull_block(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
+                              const UnitTable& units, int longest, unsigned long long timeout_ns, int num_sms,
+                              cudaStream_t s);
 size_t pull_smem_bytes(int chunk, int rhs, size_t elem);
 size_t imported_smem_bytes(int chunk, int max_imports, size_t elem);
 // warp-synchronous one-rhs forward pull with an importer warp per CTA (blocked layouts)
