@@ -1411,14 +1411,17 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
   if (c.sched == SCHED_LEVELSET) form = FORM_DEP_W;
   ST_TRY(need_forms<T>(h, form, s));
   const bool cluster = rhs == 1 && !(adj && adj->grad) && use_cluster<T>(h, adj != nullptr);
+  const bool multi = c.sched == SCHED_PULL && !(adj && adj->grad) && use_ahead_multi(h, c, rhs, sizeof(T), adj != nullptr);
   if (cluster) {
     // values live in the cluster's shared memory: no flag words to clear
   } else if (c.sched == SCHED_PUSH) {
     ST_TRY(ensure_buf(h, h->left_sum, elems * sizeof(T), 1, s));
     ST_TRY(ensure_buf(h, h->counters, (size_t)n * sizeof(unsigned), 1, s));
   } else {
-    ST_TRY(ensure_buf(h, h->xw, elems * sizeof(T), 0, s));
-    if (c.sched != SCHED_LEVELSET) CUDA_TRY(cudaMemsetAsync(h->xw.p, 0xFF, elems * sizeof(T), s));
+    const size_t bytes = sizeof(T) * (multi ? (size_t)n * ahead_multi_words(rhs, sizeof(T), n < kNarrowWidth * h->nlevels)
+                                            : elems);
+    ST_TRY(ensure_buf(h, h->xw, bytes, 0, s));
+    if (c.sched != SCHED_LEVELSET) CUDA_TRY(cudaMemsetAsync(h->xw.p, 0xFF, bytes, s));
   }
   bool block = !cluster && c.sched == SCHED_PULL && rhs == 1 && !adj && !h->pipe_option && use_block<T>(h, c);
   if (block) {
@@ -1488,7 +1491,7 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
     }
     if (split_ahead) {
       // launched above
-    } else if (!(adj && adj->grad) && use_ahead_multi(h, c, rhs, sizeof(T), adj != nullptr)) {
+    } else if (multi) {
       CUDA_TRY(launch_pull_ahead_multi<T>(h->layout, V, rhs, v, static_cast<T*>(h->xw.p), h->ctl,
                                           n < kNarrowWidth * h->nlevels, timeout_ns(h), h->num_sms, s,
                                           adj != nullptr));
@@ -2205,8 +2208,11 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
     // 2.43 ms with four)
     if (h->sched_option == SCHED_AUTO && planned(h, SPTRSV_OPTION_CTAS_PER_SM) && h->layout_block >= h->n)
       fc.ctas_per_sm = rhs <= 4 ? (rhs == 1 && h->batch_count == 1 ? 1 : 2) : (h->fused_refine == 2 ? 0 : 3);
-    ST_TRY(ensure_buf(h, h->xw, sizeof(unsigned long long) * count, 0, s));
-    CUDA_TRY(cudaMemsetAsync(h->xw.p, 0xFF, sizeof(unsigned long long) * count, s));
+    const long long width = h->n / std::max(1, h->nlevels);
+    const size_t bytes = sizeof(unsigned long long) *
+                         (refine_ahead ? (size_t)h->n * ahead_multi_words(rhs, 8, width < kNarrowWidth) : (size_t)count);
+    ST_TRY(ensure_buf(h, h->xw, bytes, 0, s));
+    CUDA_TRY(cudaMemsetAsync(h->xw.p, 0xFF, bytes, s));
     CUDA_TRY(cudaMemsetAsync(stats, 0, 3 * sizeof(unsigned long long), s));
     h->last_sched = SCHED_PULL;
     h->last_pipe = false;
@@ -2245,8 +2251,7 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
                                             timeout_ns(h), h->num_sms, s, h->imports));
     } else if (wsplit && refine_ahead) {
       CUDA_TRY(launch_refine_ahead(h->layout, h->v64, rhs, d_b, d_x, si, sk,
-                                   static_cast<unsigned long long*>(h->xw.p), stats, h->ctl,
-                                   h->n / std::max(1, h->nlevels), timeout_ns(h), h->num_sms, s, wsplit));
+                                   static_cast<unsigned long long*>(h->xw.p), stats, h->ctl, width, timeout_ns(h), h->num_sms, s, wsplit));
     } else {
       CUDA_TRY(launch_refine_fused(h->layout, h->v32, h->v64, rhs, d_b, d_x, si, sk,
                                    static_cast<unsigned long long*>(h->xw.p), stats, h->ctl, fc, timeout_ns(h),

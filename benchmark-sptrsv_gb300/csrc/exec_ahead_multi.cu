@@ -37,15 +37,15 @@ struct AheadMultiArgs {
   const T* b;
   T* x;
   long long b_si, b_sk, x_si, x_sk;
-  T* xw;  // [n * rhs], position-major
+  T* xw;  // [n * rhs in whole lanes], position-major
   DeviceCtl* ctl;
   unsigned long long timeout_ns;
 };
 
-// G lanes per unknown, R adjacent right-hand sides per lane (R = 2 needs an
-// even number of them), 256 / G unknowns per chunk.
-template <typename T, bool ADJ, int G, int R>
-__global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a) {
+// G lanes per unknown, R adjacent right-hand sides per lane, 256 / G unknowns per
+// chunk. PAD: not whole lanes; words past the last right-hand side repeat it.
+template <typename T, bool ADJ, int G, int R, bool PAD>
+__global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, int words) {
   using F = Flag<T>;
   using Bits = typename F::Bits;
   constexpr unsigned kFull = 0xffffffffu;
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a) {
   const unsigned s_wa = static_cast<unsigned>(__cvta_generic_to_shared(s_w));
   const unsigned s_qa = static_cast<unsigned>(__cvta_generic_to_shared(s_q));
   const int j = threadIdx.x / G, k = (threadIdx.x % G) * R;  // unknown of the chunk, first right-hand side
-  const int last = a.n - 1, rhs = a.rhs;
+  const int last = a.n - 1, rhs = PAD ? words : a.rhs;
   const bool col = k < rhs;
   // two chunks ahead: rows and list bounds
   int f_row = 0, f_e = 0, f_e1 = 0, f_lo = 0, f_hi = 0;
@@ -90,7 +90,8 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a) {
     if (pr < a.n && col) {
       const T r = a.rcp[ADJ ? last - pr : pr];
 #pragma unroll
-      for (int i = 0; i < R; ++i) n_acc[i] = a.b[(long long)n_row * a.b_si + (long long)(k + i) * a.b_sk] * r;
+      for (int i = 0; i < R; ++i)
+        n_acc[i] = a.b[(long long)n_row * a.b_si + (long long)(PAD ? min(k + i, a.rhs - 1) : k + i) * a.b_sk] * r;
     }
     const int hi = min(f_hi, f_lo + a.cap);
     for (int e = f_lo + threadIdx.x; e < hi; e += 256) {
@@ -208,7 +209,8 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a) {
     }
     if (!fail && pr < a.n && col) {
 #pragma unroll
-      for (int i = 0; i < R; ++i) a.x[(long long)row * a.x_si + (long long)(k + i) * a.x_sk] = acc[i];
+      for (int i = 0; i < R; ++i)
+        a.x[(long long)row * a.x_si + (long long)(PAD ? min(k + i, a.rhs - 1) : k + i) * a.x_sk] = acc[i];
     }
     if (__syncthreads_or(fail)) break;
     claim();
@@ -224,6 +226,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a) {
 
 template <typename T, bool ADJ>
 cudaError_t launch_ahead_multi(AheadMultiArgs<T>& a, int avg, bool narrow, int num_sms, cudaStream_t s) {
+  const int words = ahead_multi_words(a.rhs, sizeof(T), narrow);
   auto run = [&](auto kernel, int g, int r) -> cudaError_t {
     const int unknowns = 256 / g;
     a.nchunks = (a.n + unknowns - 1) / unknowns;
@@ -237,18 +240,23 @@ cudaError_t launch_ahead_multi(AheadMultiArgs<T>& a, int avg, bool narrow, int n
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 256, smem);
     if (per < 1) per = 1;
     const int grid = static_cast<int>(std::min<long long>((long long)num_sms * per, a.nchunks));
-    kernel<<<grid, 256, smem, s>>>(a);
+    kernel<<<grid, 256, smem, s>>>(a, words);
     return cudaGetLastError();
   };
+  const bool pad = a.rhs != words;
   switch (ahead_multi_shape(a.rhs, sizeof(T), narrow)) {
-    case 2 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 2, 1>, 2, 1);
-    case 4 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 4, 1>, 4, 1);
-    case 8 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 8, 1>, 8, 1);
-    case 16 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 16, 1>, 16, 1);
-    case 8 * 8 + 2: return run(k_pull_ahead_multi<T, ADJ, 8, 2>, 8, 2);
-    case 16 * 8 + 2: return run(k_pull_ahead_multi<T, ADJ, 16, 2>, 16, 2);
-    case 16 * 8 + 4: return run(k_pull_ahead_multi<T, ADJ, 16, 4>, 16, 4);
-    case 32 * 8 + 2: return run(k_pull_ahead_multi<T, ADJ, 32, 2>, 32, 2);
+    case 2 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 2, 1, false>, 2, 1);
+    case 4 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 4, 1, false>, 4, 1);
+    case 8 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 8, 1, false>, 8, 1);
+    case 16 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 16, 1, false>, 16, 1);
+    case 8 * 8 + 2: return pad ? run(k_pull_ahead_multi<T, ADJ, 8, 2, true>, 8, 2)
+                           : run(k_pull_ahead_multi<T, ADJ, 8, 2, false>, 8, 2);
+    case 16 * 8 + 2: return pad ? run(k_pull_ahead_multi<T, ADJ, 16, 2, true>, 16, 2)
+                           : run(k_pull_ahead_multi<T, ADJ, 16, 2, false>, 16, 2);
+    case 16 * 8 + 4: return pad ? run(k_pull_ahead_multi<T, ADJ, 16, 4, true>, 16, 4)
+                           : run(k_pull_ahead_multi<T, ADJ, 16, 4, false>, 16, 4);
+    case 32 * 8 + 2: return pad ? run(k_pull_ahead_multi<T, ADJ, 32, 2, true>, 32, 2)
+                           : run(k_pull_ahead_multi<T, ADJ, 32, 2, false>, 32, 2);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(288) k_pull_refine1_imp(RefineArgs a) {
 // band, 4 / 8 / 32 / 64 575 / 598 / 793 / 1,077 -> 358 / 373 / 643 / 1,048; 700k
 // rows, 3,004 per level, 1 / 16 259 / 478 -> 180 / 380. Bound by the hop at few
 // right-hand sides, by FP32 issue at 64.
-template <int G, int R>
+template <int G, int R, bool PAD>
 __global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a) {
   using Bits = unsigned long long;
   constexpr unsigned kFull = 0xffffffffu;
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a) {
   const unsigned s_wa = static_cast<unsigned>(__cvta_generic_to_shared(s_w));
   const unsigned s_qa = static_cast<unsigned>(__cvta_generic_to_shared(s_q));
   const int j = threadIdx.x / G, k = (threadIdx.x % G) * R;  // unknown of the chunk, first right-hand side
-  const int rhs = a.rhs;
+  const int rhs = PAD ? (a.rhs + R - 1) / R * R : a.rhs;  // in whole lanes
   const bool col = k < rhs;
   float mx_d = 0.f, mx_x = 0.f, mx_x0 = 0.f;  // stopping-estimate maxima
   // two chunks ahead: rows and list bounds
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a) {
 #pragma unroll
       for (int i = 0; i < R; ++i) {
         // b/d as a float pair: hi = RN32(b*s), lo = RN32(b*s - hi)
-        const double bv = a.b[(long long)n_row * a.b_si + (long long)(k + i) * a.b_sk];
+        const double bv = a.b[(long long)n_row * a.b_si + (long long)(PAD ? min(k + i, a.rhs - 1) : k + i) * a.b_sk];
         n_hi[i] = __double2float_rn(bv * s64);
         n_lo2[i] = __double2float_rn(__fma_rn(bv, s64, -widen(n_hi[i])));
       }
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a) {
     if (!fail && pr < a.n && col) {
 #pragma unroll
       for (int i = 0; i < R; ++i) {
-        a.x[(long long)row * a.x_si + (long long)(k + i) * a.x_sk] = widen(acc0[i]) + widen(accd[i]);
+        a.x[(long long)row * a.x_si + (long long)(PAD ? min(k + i, a.rhs - 1) : k + i) * a.x_sk] = widen(acc0[i]) + widen(accd[i]);
         mx_d = fmaxf(mx_d, fabsf(accd[i]));
         mx_x = fmaxf(mx_x, fabsf(acc0[i] + accd[i]));
         mx_x0 = fmaxf(mx_x0, fabsf(acc0[i]));
@@ -831,15 +831,16 @@ cudaError_t launch_refine_ahead(const Layout& L, const Values<double>& v64, int 
     kernel<<<grid, 256, smem, s>>>(a);
     return cudaGetLastError();
   };
-  if (rhs == 1) return run(k_refine_ahead<1, 1>, 1, 1);
+  if (rhs == 1) return run(k_refine_ahead<1, 1, false>, 1, 1);
+  const bool pad = rhs != ahead_multi_words(rhs, 8, width < kNarrowWidth);
   switch (ahead_multi_shape(rhs, 8, width < kNarrowWidth)) {
-    case 2 * 8 + 1: return run(k_refine_ahead<2, 1>, 2, 1);
-    case 4 * 8 + 1: return run(k_refine_ahead<4, 1>, 4, 1);
-    case 8 * 8 + 1: return run(k_refine_ahead<8, 1>, 8, 1);
-    case 16 * 8 + 1: return run(k_refine_ahead<16, 1>, 16, 1);
-    case 8 * 8 + 2: return run(k_refine_ahead<8, 2>, 8, 2);
-    case 16 * 8 + 2: return run(k_refine_ahead<16, 2>, 16, 2);
-    case 32 * 8 + 2: return run(k_refine_ahead<32, 2>, 32, 2);
+    case 2 * 8 + 1: return run(k_refine_ahead<2, 1, false>, 2, 1);
+    case 4 * 8 + 1: return run(k_refine_ahead<4, 1, false>, 4, 1);
+    case 8 * 8 + 1: return run(k_refine_ahead<8, 1, false>, 8, 1);
+    case 16 * 8 + 1: return run(k_refine_ahead<16, 1, false>, 16, 1);
+    case 8 * 8 + 2: return pad ? run(k_refine_ahead<8, 2, true>, 8, 2) : run(k_refine_ahead<8, 2, false>, 8, 2);
+    case 16 * 8 + 2: return pad ? run(k_refine_ahead<16, 2, true>, 16, 2) : run(k_refine_ahead<16, 2, false>, 16, 2);
+    case 32 * 8 + 2: return pad ? run(k_refine_ahead<32, 2, true>, 32, 2) : run(k_refine_ahead<32, 2, false>, 32, 2);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -332,20 +332,28 @@ cudaError_t launch_pull_ahead_split(const Layout& L, const Values<T>& V, const V
 constexpr long long kNarrowWidth = 350;  // unknowns per level (ahead_multi_shape)
 // The same for several right-hand sides (exec_ahead_multi.cu): lanes per unknown
 // times 8 plus right-hand sides per lane, or 0 where the general executor serves
-// the block (an odd number above 16 leaves every pair split: 32 lanes of one took
-// 789 us against 723 on the 500k-row band). Pairs beat single right-hand sides
-// from 9 on (16: 472 vs 555 us) but for levels of fewer than 350 unknowns, where
-// more lanes per unknown win (30k rows: 104 vs 86); quadruples only in FP32 (64:
-// 534 vs 749 us; in FP64 1,043 vs 945).
+// the block. Pairs beat single right-hand sides from 9 on (16: 472 vs 555 us) but
+// for levels of fewer than 350 unknowns, where more lanes per unknown win (30k
+// rows: 104 vs 86); quadruples only in FP32 (64: 534 vs 749 us; in FP64 1,043 vs
+// 945).
 inline int ahead_multi_shape(int rhs, size_t elem, bool narrow) {
   if (rhs < 2 || rhs > 64) return 0;
   if (rhs <= 2) return 2 * 8 + 1;
   if (rhs <= 4) return 4 * 8 + 1;
   if (rhs <= 8) return 8 * 8 + 1;
-  if (rhs <= 16) return rhs % 2 || narrow ? 16 * 8 + 1 : 8 * 8 + 2;
-  if (rhs % 2) return 0;
+  if (rhs <= 16) return narrow ? 16 * 8 + 1 : 8 * 8 + 2;
   if (rhs <= 32) return 16 * 8 + 2;
-  return elem == 4 && rhs % 4 == 0 ? 16 * 8 + 4 : 32 * 8 + 2;
+  return elem == 4 ? 16 * 8 + 4 : 32 * 8 + 2;
+}
+// Value words per unknown: the right-hand sides rounded up to whole lanes, so that
+// every lane's words are aligned and polled together. Where they are more, the
+// general executor served the block, or single right-hand sides per lane (500k-row
+// band, forward / transposed / refined, us: 15 566 / 672 / 602 -> 480 / 573 / 498,
+// 31 802 / 870 / 905 -> 606 / 726 / 695, 33 1,029 / 1,069 / 1,150 -> 976 / same /
+// 1,119; FP32 33 886 / 855 -> 575 / 690).
+inline int ahead_multi_words(int rhs, size_t elem, bool narrow) {
+  const int per = ahead_multi_shape(rhs, elem, narrow) & 7;
+  return per > 1 ? (rhs + per - 1) / per * per : rhs;
 }
 template <typename T>
 cudaError_t launch_pull_ahead_multi(const Layout& L, const Values<T>& V, int rhs, const VecView<T>& v, T* xw,

@@ -54,6 +54,25 @@ def test_sizes_around_the_chunks(cuda, oracle_port, kind, n, rhs):
     _check(cuda, oracle_port, m, rhs, col_major=False, order_block=2**31 - 1)
 
 
+@pytest.mark.parametrize("rhs", [9, 15, 17, 31, 33, 35, 63])
+def test_counts_that_are_not_whole_lanes(cuda, oracle_port, rhs):
+    """Levels past 350 unknowns; the values around the solution block stay as they are."""
+    from sptrsv_gb300 import SyncFreeSolver, matgen
+    m = matgen.poisson_band(20_001, 3.0, 10_000, seed=rhs)
+    _check(cuda, oracle_port, m, rhs, col_major=rhs % 4 == 1, order_block=2**31 - 1)
+    b = np.random.default_rng(rhs).standard_normal((m.n, rhs))
+    ref = oracle_port.solve(m.col_ptr, m.row_idx, m.val, m.n, m.substitution, b)
+    s = SyncFreeSolver(m.col_ptr, m.row_idx, m.n, m.substitution, values=m.val, order_block=2**31 - 1)
+    room = cuda.full((m.n + 2, rhs), 7.0, dtype=cuda.float64, device="cuda")
+    bd = cuda.from_numpy(b).cuda()
+    s.solve(bd, out=room[1:-1])
+    assert relerr(room[1:-1].cpu().numpy(), ref) <= 1e-12
+    s.solve_refine(bd, out=room[1:-1])
+    assert relerr(room[1:-1].cpu().numpy(), ref) <= 1e-10
+    assert bool((room[0] == 7.0).all()) and bool((room[-1] == 7.0).all())
+    s.close()
+
+
 def test_infinities_and_nan_stay_in_their_column(cuda):
     """Against the executor with an explicit right-hand-side tile."""
     from sptrsv_gb300 import SyncFreeSolver, matgen
