@@ -1386,6 +1386,26 @@ bool use_ahead_multi(const sptrsv_gb300_handle_s* h, const ExecConfig& c, int rh
   return shape != 0 && !(adj && shape == 32 * 8 + 2);
 }
 
+// Column-major blocks of many right-hand sides are solved through row-major
+// staging (transpose in, solve, transpose out): the executors then read and
+// write whole rows of the block with coalesced accesses. Measured worthwhile
+// from 32 right-hand sides for plain solves, and always for refinement
+// (whose FP32 solves and residual run on internal buffers).
+constexpr int kColMajorStageRhs = 32;
+
+bool stage_col_major(const sptrsv_gb300_handle_s* h, int rhs, int layout, int min_rhs) {
+  return layout == SPTRSV_LAYOUT_COL_MAJOR && rhs >= min_rhs && rhs > 1 && h->n > 0;
+}
+
+// Column-major blocks that solve_typed stages itself, scaled on the way in
+// (k_pull_ahead_multi).
+bool stages_columns(const sptrsv_gb300_handle_s* h, int rhs, int layout, size_t elem, bool adj) {
+  ExecConfig c = pick_config(h, rhs);
+  if (adj) c.sched = SCHED_PULL;
+  return stage_col_major(h, rhs, layout, kColMajorStageRhs) && c.sched == SCHED_PULL &&
+         use_ahead_multi(h, c, rhs, elem, adj);
+}
+
 template <typename T>
 int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x, cudaStream_t s,
                 const AdjointArgs<T>* adj = nullptr, bool allow_check = true) {
@@ -1412,14 +1432,23 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
   ST_TRY(need_forms<T>(h, form, s));
   const bool cluster = rhs == 1 && !(adj && adj->grad) && use_cluster<T>(h, adj != nullptr);
   const bool multi = c.sched == SCHED_PULL && !(adj && adj->grad) && use_ahead_multi(h, c, rhs, sizeof(T), adj != nullptr);
+  const int words = multi ? ahead_multi_words(rhs, sizeof(T), n < kNarrowWidth * h->nlevels) : rhs;
+  const bool columns = multi && stage_col_major(h, rhs, layout, kColMajorStageRhs);
+  if (columns) {
+    ST_TRY(ensure_buf(h, h->tb, sizeof(T) * (size_t)n * words, 0, s));
+    CUDA_TRY(launch_columns_in<T>(h->layout, V, b, static_cast<T*>(h->tb.p), rhs, words, s));
+    v.b = static_cast<const T*>(h->tb.p);
+    ST_TRY(ensure_buf(h, h->tx, sizeof(T) * (size_t)n * words, 0, s));
+    v.x = static_cast<T*>(h->tx.p);
+    v.b_si = 0;
+  }
   if (cluster) {
     // values live in the cluster's shared memory: no flag words to clear
   } else if (c.sched == SCHED_PUSH) {
     ST_TRY(ensure_buf(h, h->left_sum, elems * sizeof(T), 1, s));
     ST_TRY(ensure_buf(h, h->counters, (size_t)n * sizeof(unsigned), 1, s));
   } else {
-    const size_t bytes = sizeof(T) * (multi ? (size_t)n * ahead_multi_words(rhs, sizeof(T), n < kNarrowWidth * h->nlevels)
-                                            : elems);
+    const size_t bytes = sizeof(T) * (multi ? (size_t)n * words : elems);
     ST_TRY(ensure_buf(h, h->xw, bytes, 0, s));
     if (c.sched != SCHED_LEVELSET) CUDA_TRY(cudaMemsetAsync(h->xw.p, 0xFF, bytes, s));
   }
@@ -1508,6 +1537,7 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
     CUDA_TRY(cudaEventRecord(h->ev_exec[1], s));
     h->ev_recorded = true;
   }
+  if (columns) CUDA_TRY(launch_columns_out<T>(h->layout, static_cast<const T*>(h->tx.p), x, rhs, words, s));
   if (h->sync_check && allow_check) return check_device(h, s);
   return SPTRSV_OK;
 }
@@ -2077,17 +2107,6 @@ int sptrsv_gb300_set_values(sptrsv_handle_t h, const void* d_val, int dtype, voi
   return stage_values(h, d_val, dtype, s, true);
 }
 
-// Column-major blocks of many right-hand sides are solved through row-major
-// staging (transpose in, solve, transpose out): the executors then read and
-// write whole rows of the block with coalesced accesses. Measured worthwhile
-// from 32 right-hand sides for plain solves, and always for refinement
-// (whose FP32 solves and residual run on internal buffers).
-constexpr int kColMajorStageRhs = 32;
-
-bool stage_col_major(const sptrsv_gb300_handle_s* h, int rhs, int layout, int min_rhs) {
-  return layout == SPTRSV_LAYOUT_COL_MAJOR && rhs >= min_rhs && rhs > 1 && h->n > 0;
-}
-
 int sptrsv_gb300_solve(sptrsv_handle_t h, const void* d_val, int dtype, int rhs, int layout, const void* d_b,
                        void* d_x, void* stream) {
   if (!h) return SPTRSV_ERR_INVALID;
@@ -2098,8 +2117,11 @@ int sptrsv_gb300_solve(sptrsv_handle_t h, const void* d_val, int dtype, int rhs,
   if (!d_b || !d_x) return SPTRSV_ERR_INVALID;
   if ((long long)h->n * rhs > INT_MAX) return SPTRSV_ERR_UNSUPPORTED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (stage_col_major(h, rhs, layout, kColMajorStageRhs)) {
-    const size_t elem = dtype == SPTRSV_DTYPE_F64 ? sizeof(double) : sizeof(float);
+  const size_t elem = dtype == SPTRSV_DTYPE_F64 ? sizeof(double) : sizeof(float);
+  const int before = h->layout_block;
+  ST_TRY(ensure_layout(h, s));
+  if (!d_val && h->layout_block != before) return SPTRSV_ERR_STATE;  // schedule changed since the values were staged
+  if (stage_col_major(h, rhs, layout, kColMajorStageRhs) && !stages_columns(h, rhs, layout, elem, false)) {
     const size_t bytes = (size_t)h->n * rhs * elem;
     ST_TRY(ensure_buf(h, h->tb, bytes, 0, s));
     ST_TRY(ensure_buf(h, h->tx, bytes, 0, s));
@@ -2117,13 +2139,7 @@ int sptrsv_gb300_solve(sptrsv_handle_t h, const void* d_val, int dtype, int rhs,
     }
     return SPTRSV_OK;
   }
-  const int before = h->layout_block;
-  ST_TRY(ensure_layout(h, s));
-  if (d_val) {
-    ST_TRY(stage_values(h, d_val, dtype, s, h->sync_check != 0));
-  } else if (h->layout_block != before) {
-    return SPTRSV_ERR_STATE;  // schedule changed since the values were staged
-  }
+  if (d_val) ST_TRY(stage_values(h, d_val, dtype, s, h->sync_check != 0));
   if (dtype == SPTRSV_DTYPE_F64) {
     if (!h->staged64) return SPTRSV_ERR_STATE;
     return solve_typed<double>(h, rhs, layout, static_cast<const double*>(d_b), static_cast<double*>(d_x), s);
@@ -2326,10 +2342,14 @@ int sptrsv_gb300_solve_adjoint(sptrsv_handle_t h, const void* d_val, int dtype, 
   if (!d_g || !d_lambda || (d_dval && !d_x)) return SPTRSV_ERR_INVALID;
   if (h->sched_option == SCHED_LEVELSET) return SPTRSV_ERR_UNSUPPORTED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (!d_dval && stage_col_major(h, rhs, layout, kColMajorStageRhs)) {
+  const size_t elem = dtype == SPTRSV_DTYPE_F64 ? sizeof(double) : sizeof(float);
+  const int before = h->layout_block;
+  ST_TRY(ensure_layout(h, s));
+  if (!d_val && h->layout_block != before) return SPTRSV_ERR_STATE;
+  if (!d_dval && stage_col_major(h, rhs, layout, kColMajorStageRhs) && !stages_columns(h, rhs, layout, elem, true)) {
     // through row-major staging, as plain solves (1M rows, 64 right-hand sides:
     // 2.64 ms walking the columns as they are, 2.36 staged)
-    const size_t bytes = (size_t)h->n * rhs * (dtype == SPTRSV_DTYPE_F64 ? sizeof(double) : sizeof(float));
+    const size_t bytes = (size_t)h->n * rhs * elem;
     ST_TRY(ensure_buf(h, h->tb, bytes, 0, s));
     ST_TRY(ensure_buf(h, h->tx, bytes, 0, s));
     if (dtype == SPTRSV_DTYPE_F64) {
@@ -2346,13 +2366,7 @@ int sptrsv_gb300_solve_adjoint(sptrsv_handle_t h, const void* d_val, int dtype, 
     }
     return SPTRSV_OK;
   }
-  const int before = h->layout_block;
-  ST_TRY(ensure_layout(h, s));
-  if (d_val) {
-    ST_TRY(stage_values(h, d_val, dtype, s, h->sync_check != 0));
-  } else if (h->layout_block != before) {
-    return SPTRSV_ERR_STATE;
-  }
+  if (d_val) ST_TRY(stage_values(h, d_val, dtype, s, h->sync_check != 0));
   const long long si = layout == SPTRSV_LAYOUT_ROW_MAJOR ? rhs : 1;
   const long long sk = layout == SPTRSV_LAYOUT_ROW_MAJOR ? 1 : h->n;
   if (d_dval && !h->fused_grad) {

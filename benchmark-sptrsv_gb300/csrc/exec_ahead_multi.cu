@@ -42,9 +42,17 @@ struct AheadMultiArgs {
   unsigned long long timeout_ns;
 };
 
+// How a block reaches the kernel: rows or columns of whole lanes; not whole lanes
+// (words past the last right-hand side repeat it); rows of whole lanes that
+// launch_columns_in made of a column-major block, scaled by the diagonal there, where
+// memory is the bound (1M rows of 9 entries, 64 right-hand sides: 1,684 us here
+// instead of 1,772; whole solves 2,148 -> 2,086, at 32 on 500k rows 682 -> 662, FP32
+// 664 -> 638). Laid out like the value words the rows scatter: 90 us longer.
+enum { kWhole, kPad, kStaged };
+
 // G lanes per unknown, R adjacent right-hand sides per lane, 256 / G unknowns per
-// chunk. PAD: not whole lanes; words past the last right-hand side repeat it.
-template <typename T, bool ADJ, int G, int R, bool PAD>
+// chunk.
+template <typename T, bool ADJ, int G, int R, int MODE>
 __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, int words) {
   using F = Flag<T>;
   using Bits = typename F::Bits;
@@ -59,7 +67,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, i
   const unsigned s_wa = static_cast<unsigned>(__cvta_generic_to_shared(s_w));
   const unsigned s_qa = static_cast<unsigned>(__cvta_generic_to_shared(s_q));
   const int j = threadIdx.x / G, k = (threadIdx.x % G) * R;  // unknown of the chunk, first right-hand side
-  const int last = a.n - 1, rhs = PAD ? words : a.rhs;
+  const int last = a.n - 1, rhs = MODE == kWhole ? a.rhs : words;
   const bool col = k < rhs;
   // two chunks ahead: rows and list bounds
   int f_row = 0, f_e = 0, f_e1 = 0, f_lo = 0, f_hi = 0;
@@ -88,10 +96,16 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, i
     if (c >= a.nchunks) return;
     const int pr = c * kUnknowns + j;
     if (pr < a.n && col) {
-      const T r = a.rcp[ADJ ? last - pr : pr];
+      const int p = ADJ ? last - pr : pr;
+      if (MODE == kStaged) {
 #pragma unroll
-      for (int i = 0; i < R; ++i)
-        n_acc[i] = a.b[(long long)n_row * a.b_si + (long long)(PAD ? min(k + i, a.rhs - 1) : k + i) * a.b_sk] * r;
+        for (int i = 0; i < R; ++i) n_acc[i] = a.b[(long long)n_row * rhs + k + i];
+      } else {
+        const T r = a.rcp[p];
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+          n_acc[i] = a.b[(long long)n_row * a.b_si + (long long)(MODE == kPad ? min(k + i, a.rhs - 1) : k + i) * a.b_sk] * r;
+      }
     }
     const int hi = min(f_hi, f_lo + a.cap);
     for (int e = f_lo + threadIdx.x; e < hi; e += 256) {
@@ -209,8 +223,10 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, i
     }
     if (!fail && pr < a.n && col) {
 #pragma unroll
-      for (int i = 0; i < R; ++i)
-        a.x[(long long)row * a.x_si + (long long)(PAD ? min(k + i, a.rhs - 1) : k + i) * a.x_sk] = acc[i];
+      for (int i = 0; i < R; ++i) {
+        if (MODE == kStaged) a.x[(long long)row * rhs + k + i] = acc[i];
+        else a.x[(long long)row * a.x_si + (long long)(MODE == kPad ? min(k + i, a.rhs - 1) : k + i) * a.x_sk] = acc[i];
+      }
     }
     if (__syncthreads_or(fail)) break;
     claim();
@@ -243,23 +259,89 @@ cudaError_t launch_ahead_multi(AheadMultiArgs<T>& a, int avg, bool narrow, int n
     kernel<<<grid, 256, smem, s>>>(a, words);
     return cudaGetLastError();
   };
-  const bool pad = a.rhs != words;
+  const bool pad = a.rhs != words, staged = a.b_si == 0;
   switch (ahead_multi_shape(a.rhs, sizeof(T), narrow)) {
-    case 2 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 2, 1, false>, 2, 1);
-    case 4 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 4, 1, false>, 4, 1);
-    case 8 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 8, 1, false>, 8, 1);
-    case 16 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 16, 1, false>, 16, 1);
-    case 8 * 8 + 2: return pad ? run(k_pull_ahead_multi<T, ADJ, 8, 2, true>, 8, 2)
-                           : run(k_pull_ahead_multi<T, ADJ, 8, 2, false>, 8, 2);
-    case 16 * 8 + 2: return pad ? run(k_pull_ahead_multi<T, ADJ, 16, 2, true>, 16, 2)
-                           : run(k_pull_ahead_multi<T, ADJ, 16, 2, false>, 16, 2);
-    case 16 * 8 + 4: return pad ? run(k_pull_ahead_multi<T, ADJ, 16, 4, true>, 16, 4)
-                           : run(k_pull_ahead_multi<T, ADJ, 16, 4, false>, 16, 4);
-    case 32 * 8 + 2: return pad ? run(k_pull_ahead_multi<T, ADJ, 32, 2, true>, 32, 2)
-                           : run(k_pull_ahead_multi<T, ADJ, 32, 2, false>, 32, 2);
+    case 2 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 2, 1, kWhole>, 2, 1);
+    case 4 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 4, 1, kWhole>, 4, 1);
+    case 8 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 8, 1, kWhole>, 8, 1);
+    case 16 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 16, 1, kWhole>, 16, 1);
+    case 8 * 8 + 2:
+      return pad ? run(k_pull_ahead_multi<T, ADJ, 8, 2, kPad>, 8, 2) : run(k_pull_ahead_multi<T, ADJ, 8, 2, kWhole>, 8, 2);
+    case 16 * 8 + 2:
+      return staged ? run(k_pull_ahead_multi<T, ADJ, 16, 2, kStaged>, 16, 2)
+                    : (pad ? run(k_pull_ahead_multi<T, ADJ, 16, 2, kPad>, 16, 2)
+                           : run(k_pull_ahead_multi<T, ADJ, 16, 2, kWhole>, 16, 2));
+    case 16 * 8 + 4:
+      return staged ? run(k_pull_ahead_multi<T, ADJ, 16, 4, kStaged>, 16, 4)
+                    : (pad ? run(k_pull_ahead_multi<T, ADJ, 16, 4, kPad>, 16, 4)
+                           : run(k_pull_ahead_multi<T, ADJ, 16, 4, kWhole>, 16, 4));
+    case 32 * 8 + 2:
+      return staged ? run(k_pull_ahead_multi<T, ADJ, 32, 2, kStaged>, 32, 2)
+                    : (pad ? run(k_pull_ahead_multi<T, ADJ, 32, 2, kPad>, 32, 2)
+                           : run(k_pull_ahead_multi<T, ADJ, 32, 2, kWhole>, 32, 2));
     default: return cudaErrorInvalidValue;
   }
 }
+
+namespace {
+
+// Columns of a right-hand-side block (n entries each) to rows of `words` first
+// terms b / d, in 32 x 32 tiles through shared memory (whole lines on both sides).
+// Zeros past the last right-hand side.
+template <typename T>
+__global__ void __launch_bounds__(256) k_columns_in(const T* __restrict__ b, const T* __restrict__ rcp,
+                                                    const int* __restrict__ iperm, T* __restrict__ out, int n, int rhs,
+                                                    int words) {
+  __shared__ T tile[32][33];
+  __shared__ T scale[32];
+  const int r0 = blockIdx.x * 32, k0 = blockIdx.y * 32, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp == 0 && r0 + lane < n) scale[lane] = rcp[iperm[r0 + lane]];
+  if (r0 + lane < n) {
+#pragma unroll
+    for (int i = 0; i < 32; i += 8)
+      tile[warp + i][lane] = k0 + warp + i < rhs ? b[(long long)(k0 + warp + i) * n + r0 + lane] : T(0);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = warp; i < 32; i += 8)
+    if (r0 + i < n && k0 + lane < words) out[(long long)(r0 + i) * words + k0 + lane] = tile[lane][i] * scale[i];
+}
+// The solution's columns from rows of `words` values.
+template <typename T>
+__global__ void __launch_bounds__(256) k_columns_out(const T* __restrict__ in, T* __restrict__ x, int n, int rhs,
+                                                     int words) {
+  __shared__ T tile[32][33];
+  const int r0 = blockIdx.x * 32, k0 = blockIdx.y * 32, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = warp; i < 32; i += 8)
+    if (r0 + i < n && k0 + lane < rhs) tile[lane][i] = in[(long long)(r0 + i) * words + k0 + lane];
+  __syncthreads();
+#pragma unroll
+  for (int i = warp; i < 32; i += 8)
+    if (r0 + lane < n && k0 + i < rhs) x[(long long)(k0 + i) * n + r0 + lane] = tile[i][lane];
+}
+
+}  // namespace
+
+template <typename T>
+cudaError_t launch_columns_in(const Layout& L, const Values<T>& V, const T* b, T* out, int rhs, int words,
+                              cudaStream_t s) {
+  if (L.n == 0) return cudaSuccess;
+  k_columns_in<T><<<dim3((L.n + 31) / 32, (words + 31) / 32), 256, 0, s>>>(b, V.rcp, L.iperm, out, L.n, rhs, words);
+  return cudaGetLastError();
+}
+template <typename T>
+cudaError_t launch_columns_out(const Layout& L, const T* in, T* x, int rhs, int words, cudaStream_t s) {
+  if (L.n == 0) return cudaSuccess;
+  k_columns_out<T><<<dim3((L.n + 31) / 32, (rhs + 31) / 32), 256, 0, s>>>(in, x, L.n, rhs, words);
+  return cudaGetLastError();
+}
+template cudaError_t launch_columns_in<double>(const Layout&, const Values<double>&, const double*, double*, int, int,
+                                               cudaStream_t);
+template cudaError_t launch_columns_in<float>(const Layout&, const Values<float>&, const float*, float*, int, int,
+                                              cudaStream_t);
+template cudaError_t launch_columns_out<double>(const Layout&, const double*, double*, int, int, cudaStream_t);
+template cudaError_t launch_columns_out<float>(const Layout&, const float*, float*, int, int, cudaStream_t);
 
 template <typename T>
 cudaError_t launch_pull_ahead_multi(const Layout& L, const Values<T>& V, int rhs, const VecView<T>& v, T* xw,

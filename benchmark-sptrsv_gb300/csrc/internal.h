@@ -355,10 +355,19 @@ inline int ahead_multi_words(int rhs, size_t elem, bool narrow) {
   const int per = ahead_multi_shape(rhs, elem, narrow) & 7;
   return per > 1 ? (rhs + per - 1) / per * per : rhs;
 }
+// v.b_si = 0: v.b holds the rows launch_columns_in wrote, v.x is to hold rows of
+// ahead_multi_words values (shapes of more than 16 right-hand sides).
 template <typename T>
 cudaError_t launch_pull_ahead_multi(const Layout& L, const Values<T>& V, int rhs, const VecView<T>& v, T* xw,
                                     DeviceCtl* ctl, bool narrow, unsigned long long timeout_ns, int num_sms,
                                     cudaStream_t s, bool adj);
+// A column-major block to rows of first terms b / d, and the solution's columns from
+// rows; `words` values per row (ahead_multi_words).
+template <typename T>
+cudaError_t launch_columns_in(const Layout& L, const Values<T>& V, const T* b, T* out, int rhs, int words,
+                              cudaStream_t s);
+template <typename T>
+cudaError_t launch_columns_out(const Layout& L, const T* in, T* x, int rhs, int words, cudaStream_t s);
 // One-cluster executor (exec_cluster.cu): 16 CTAs of `block` threads; walk
 // indices are dealt to them in runs of 1 << cshift; a warp's list buffer holds
 // `cap` entries.
