@@ -1389,12 +1389,21 @@ bool use_ahead_multi(const sptrsv_gb300_handle_s* h, const ExecConfig& c, int rh
 // Column-major blocks of many right-hand sides are solved through row-major
 // staging (transpose in, solve, transpose out): the executors then read and
 // write whole rows of the block with coalesced accesses. Measured worthwhile
-// from 32 right-hand sides for plain solves, and always for refinement
-// (whose FP32 solves and residual run on internal buffers).
+// from 32 right-hand sides for plain solves (1M rows, staged vs columns as they
+// are: 8 700 vs 594 us, 16 812 vs 706, 64 1,861 vs 3,055) and for the fused first
+// refinement step (2 949 vs 861, 16 979 vs 885, 31 1,441 vs 1,358, 64 2,382 vs
+// 3,219; 700k rows, 4 306 vs 245). Refinement steps after it run on rows.
 constexpr int kColMajorStageRhs = 32;
 
 bool stage_col_major(const sptrsv_gb300_handle_s* h, int rhs, int layout, int min_rhs) {
   return layout == SPTRSV_LAYOUT_COL_MAJOR && rhs >= min_rhs && rhs > 1 && h->n > 0;
+}
+
+// Whether the fused first refinement step of a block runs k_refine_ahead.
+bool refine_ahead_blocks(const sptrsv_gb300_handle_s* h, int rhs) {
+  const ExecConfig c = pick_config(h, rhs);
+  return rhs > 1 && rhs <= 64 && h->fused_refine == 2 && c.sched == SCHED_PULL && !c.exact &&
+         planned(h, SPTRSV_OPTION_CTAS_PER_SM) && use_ahead_multi(h, c, rhs, sizeof(double), false);
 }
 
 // Column-major blocks that solve_typed stages itself, scaled on the way in
@@ -2160,7 +2169,16 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
   if (!d_b || !d_x) return SPTRSV_ERR_INVALID;
   if ((long long)h->n * rhs > INT_MAX) return SPTRSV_ERR_UNSUPPORTED;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (stage_col_major(h, rhs, layout, 2)) {
+  const int before = h->layout_block;
+  ST_TRY(ensure_layout(h, s));
+  if (!d_val && h->layout_block != before) return SPTRSV_ERR_STATE;
+  const long long count = (long long)h->n * rhs;
+  // columns as they are through the fused step; a solution over its right-hand side
+  // would leave nothing to refine against
+  const bool as_is = layout == SPTRSV_LAYOUT_COL_MAJOR && rhs > 1 && rhs < kColMajorStageRhs &&
+                     (tol > 0.0 || max_iter == 1) && refine_ahead_blocks(h, rhs) &&
+                     (d_x + count <= d_b || d_b + count <= d_x);
+  if (stage_col_major(h, rhs, layout, 2) && !as_is) {
     const size_t bytes = (size_t)h->n * rhs * sizeof(double);
     ST_TRY(ensure_buf(h, h->tb, bytes, 0, s));
     ST_TRY(ensure_buf(h, h->tx, bytes, 0, s));
@@ -2171,20 +2189,13 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
     CUDA_TRY(launch_transpose<double>(static_cast<const double*>(h->tx.p), d_x, h->n, rhs, s));
     return st;
   }
-  const int before = h->layout_block;
-  ST_TRY(ensure_layout(h, s));
-  if (d_val) {
-    ST_TRY(stage_values(h, d_val, SPTRSV_DTYPE_F64, s, h->sync_check != 0));
-  } else if (h->layout_block != before) {
-    return SPTRSV_ERR_STATE;
-  }
+  if (d_val) ST_TRY(stage_values(h, d_val, SPTRSV_DTYPE_F64, s, h->sync_check != 0));
   if (!h->staged64 || !h->staged32) return SPTRSV_ERR_STATE;
-  const long long count = (long long)h->n * rhs;
   ST_TRY(ensure_buf(h, h->r32, sizeof(float) * count, 0, s));
   ST_TRY(ensure_buf(h, h->d32, sizeof(float) * count, 0, s));
   ST_TRY(ensure_buf(h, h->stats, 4 * sizeof(unsigned long long), 1, s));
-  const long long si = layout == SPTRSV_LAYOUT_ROW_MAJOR ? rhs : 1;
-  const long long sk = layout == SPTRSV_LAYOUT_ROW_MAJOR ? 1 : h->n;
+  long long si = layout == SPTRSV_LAYOUT_ROW_MAJOR ? rhs : 1;
+  long long sk = layout == SPTRSV_LAYOUT_ROW_MAJOR ? 1 : h->n;
   float* r32 = static_cast<float*>(h->r32.p);
   float* d32 = static_cast<float*>(h->d32.p);
   auto* stats = static_cast<unsigned long long*>(h->stats.p);
@@ -2207,7 +2218,7 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
     const bool refine_ahead =
         rhs == 1 ? fc.wsync && fc.smem_tier && h->layout_block >= h->n && fc.block == 256 && fc.chunk == 256 &&
                        fc.sleep_max == 0 && fc.wsync_batch == 0 && planned(h, SPTRSV_OPTION_CTAS_PER_SM)
-                 : planned(h, SPTRSV_OPTION_CTAS_PER_SM) && use_ahead_multi(h, fc, rhs, sizeof(double), false);
+                 : refine_ahead_blocks(h, rhs);
     // the plain solve's rule (160k-row bands with 1 / 2 entries per column and a
     // 1M-row band with 3: 0.101 / 1.95 / 6.40 ms refined with two dependencies
     // per iteration, 0.082 / 1.54 / 5.62 with one; the mesh triangle with two:
@@ -2305,12 +2316,26 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
     }
   }
   int steps = first - 1;  // refinement steps done
+  const bool to_rows = as_is && !converged && first <= max_iter;
+  const double* rb = d_b;
+  double* rx = d_x;
+  const int steps_layout = to_rows ? SPTRSV_LAYOUT_ROW_MAJOR : layout;
+  if (to_rows) {
+    ST_TRY(ensure_buf(h, h->tb, sizeof(double) * count, 0, s));
+    ST_TRY(ensure_buf(h, h->tx, sizeof(double) * count, 0, s));
+    CUDA_TRY(launch_transpose<double>(d_b, static_cast<double*>(h->tb.p), rhs, h->n, s));
+    CUDA_TRY(launch_transpose<double>(d_x, static_cast<double*>(h->tx.p), rhs, h->n, s));
+    rb = static_cast<const double*>(h->tb.p);
+    rx = static_cast<double*>(h->tx.p);
+    si = rhs;
+    sk = 1;
+  }
   for (it = first; !converged && it <= max_iter; ++it) {
     ST_TRY(need_forms<double>(h, FORM_DEP_VAL, s));
-    CUDA_TRY(launch_residual(h->layout, h->v64, rhs, d_b, d_x, si, sk, r32, s));
-    ST_TRY(solve_typed<float>(h, rhs, layout, r32, d32, s, nullptr, false));
+    CUDA_TRY(launch_residual(h->layout, h->v64, rhs, rb, rx, si, sk, r32, s));
+    ST_TRY(solve_typed<float>(h, rhs, steps_layout, r32, d32, s, nullptr, false));
     CUDA_TRY(cudaMemsetAsync(stats, 0, 2 * sizeof(unsigned long long), s));
-    CUDA_TRY(launch_update(d_x, d32, count, stats, false, s));
+    CUDA_TRY(launch_update(rx, d32, count, stats, false, s));
     steps = it;
     if (!checked) continue;
     CUDA_TRY(cudaMemcpyAsync(host_stats, stats, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
@@ -2325,6 +2350,7 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
     }
     prev = dmax;
   }
+  if (to_rows) CUDA_TRY(launch_transpose<double>(rx, d_x, h->n, rhs, s));
   if (iters) *iters = steps;
   if (est) *est = estimate;
   if (h->sync_check || checked) ST_TRY(check_device(h, s));

@@ -106,3 +106,24 @@ def test_refined_blocks(cuda, oracle_port, kind, n, rhs):
         x, iters, est = s.solve_refine(bd)
         assert 1 <= iters <= 4 and est <= 1e-12
         assert relerr(x.cpu().numpy(), ref) <= 1e-10
+
+
+@pytest.mark.parametrize("rhs", [2, 5, 16, 31, 32])
+def test_refined_columns(cuda, oracle_port, rhs):
+    """Column-major blocks through the fused step as they are (below 32), further steps on rows: a tolerance that one
+    step (FP32, about 1e-14 by the estimate) does not reach; the solution over its right-hand side."""
+    from sptrsv_gb300 import SyncFreeSolver, matgen
+    m = matgen.poisson_band(20_001, 3.0, 10_000, seed=rhs)
+    b = np.random.default_rng(rhs).standard_normal((m.n, rhs))
+    ref = oracle_port.solve(m.col_ptr, m.row_idx, m.val, m.n, m.substitution, b)
+    s = SyncFreeSolver(m.col_ptr, m.row_idx, m.n, m.substitution, values=m.val)
+    bd = cuda.from_numpy(b).cuda().t().contiguous().t()
+    x, iters, est = s.solve_refine(bd, tol=1e-12)
+    assert iters == 1 and relerr(x.cpu().numpy(), ref) <= 1e-10
+    for tol, want in ((1e-18, 2), (0.0, 3)):
+        x, iters, _ = s.solve_refine(bd, tol=tol, max_iter=3 if tol == 0.0 else 10)
+        assert iters >= want
+        assert relerr(x.cpu().numpy(), ref) <= 1e-12
+    s.solve_refine(bd, tol=1e-18, out=bd)
+    assert relerr(bd.cpu().numpy(), ref) <= 1e-12
+    s.close()
