@@ -1343,7 +1343,7 @@ bool use_ahead(const sptrsv_gb300_handle_s* h, const ExecConfig& c) {
   return c.ctas_per_sm == 1 && c.wsync_batch == 1;
 }
 
-// Whether the one-rhs forward walk of a blocked layout may run k_pull_block
+// Whether a one-rhs walk of a blocked layout may run k_pull_block
 // (exec_block.cu): lists of at most 4 entries (more make a level longer and the
 // ring wider; they stay with k_pull_wsync_imp), whole units in shared memory
 // beside the ring, and the importer executor not asked for (its entries per
@@ -1355,15 +1355,15 @@ bool use_ahead(const sptrsv_gb300_handle_s* h, const ExecConfig& c) {
 // segments 105 vs 141; lists of two, 2 segments 132 vs 115, 3 segments 173 vs 168;
 // lists of four, 3 segments 341 vs 236).
 template <typename T>
-bool use_block(const sptrsv_gb300_handle_s* h, const ExecConfig& c) {
+bool use_block(const sptrsv_gb300_handle_s* h, const ExecConfig& c, int longest) {
   if (!c.wsync || c.exact || c.staged || !c.smem_tier || c.wsync_batch != 0) return false;
   if (!h->import_option || (h->user_set & (1ull << SPTRSV_OPTION_IMPORT))) return false;
   if (h->layout_block >= h->n || c.chunk != h->layout_block || h->layout_units.size() < 2) return false;
-  if (h->max_dep_cnt < 1 || h->max_dep_cnt > 4 || (c.split > 0 && h->max_dep_cnt > c.split)) return false;
+  if (longest < 1 || longest > 4 || (c.split > 0 && longest > c.split)) return false;
   int width = 0;
   for (size_t i = 1; i < h->layout_units.size(); ++i)
     width = std::max(width, h->layout_units[i] - h->layout_units[i - 1]);
-  return block_smem_bytes<T>(width, h->max_dep_cnt) <= 226 * 1024;
+  return block_smem_bytes<T>(width, longest) <= 226 * 1024;
 }
 
 // Units of work per level (dependencies plus 4 per unknown) up to which split
@@ -1461,10 +1461,12 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
     ST_TRY(ensure_buf(h, h->xw, bytes, 0, s));
     if (c.sched != SCHED_LEVELSET) CUDA_TRY(cudaMemsetAsync(h->xw.p, 0xFF, bytes, s));
   }
-  bool block = !cluster && c.sched == SCHED_PULL && rhs == 1 && !adj && !h->pipe_option && use_block<T>(h, c);
+  const int longest = adj ? h->max_out_cnt : h->max_dep_cnt;
+  bool block = !cluster && c.sched == SCHED_PULL && rhs == 1 && !(adj && adj->grad) && !h->pipe_option &&
+               use_block<T>(h, c, longest);
   if (block) {
     ST_TRY(ensure_units(h, s));
-    block = 4LL * h->units.segments <= (4LL + 3 * h->max_dep_cnt) * h->units.levels;
+    block = 4LL * h->units.segments <= (4LL + 3 * longest) * h->units.levels;
   }
   if (h->profile) {
     if (!h->ev_exec[0]) {
@@ -1498,8 +1500,8 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
                                  timeout_ns(h), h->num_sms, s, h->pipe));
     h->last_pipe = true;
   } else if (block) {
-    CUDA_TRY(launch_pull_block<T>(h->layout, V, v, static_cast<T*>(h->xw.p), h->ctl, h->units, h->max_dep_cnt,
-                                  timeout_ns(h), h->num_sms, s));
+    CUDA_TRY(launch_pull_block<T>(h->layout, V, v, static_cast<T*>(h->xw.p), h->ctl, h->units, longest,
+                                  timeout_ns(h), h->num_sms, s, adj != nullptr));
   } else if (rhs == 1 && c.wsync && !c.exact && !adj && h->import_option && h->layout_block < n &&
              c.chunk == h->layout_block && c.smem_tier &&
              !(c.split > 0 && h->max_dep_cnt > c.split) &&
@@ -1515,7 +1517,6 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
   } else {
     const PieceTable* pc = nullptr;
     if (rhs == 1 && planned(h, SPTRSV_OPTION_SPLIT)) c.split = adj ? h->plan.split_adj : h->plan.split_fwd;
-    const int longest = adj ? h->max_out_cnt : h->max_dep_cnt;
     const bool cut = rhs == 1 && c.wsync && !c.exact && c.split > 0 && longest > c.split && !(adj && adj->grad);
     const bool split_ahead = cut && (planned(h, SPTRSV_OPTION_SPLIT) || c.split == 32) && use_ahead(h, c) &&
                              static_cast<double>(h->nnz - n) + 4.0 * n <= kSplitAheadWork * h->nlevels;

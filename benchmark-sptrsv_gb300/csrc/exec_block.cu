@@ -1,6 +1,6 @@
-// Blocked layouts (deep, narrow DAGs such as a mesh triangle): the forward walk
-// over short lists for one right-hand side (k_pull_block), and the tables of the
-// units, built on the device.
+// Blocked layouts (deep, narrow DAGs such as a mesh triangle): the walks over short
+// lists for one right-hand side (k_pull_block), and the tables of the units, built on
+// the device.
 //
 // A unit is one CTA's work, and a solve costs its levels times what one level
 // takes, plus a hop from unit to unit. With lockstep lanes that poll for their
@@ -22,7 +22,8 @@
 //
 // Whole solves, before (k_pull_wsync_imp) and after: meshes of 300 x 300 185 and
 // 141 us, 1000 x 1000 592 and 447, 1414 x 1414 860 and 664 (FP32 635 and 495),
-// 300 x 3000 1,071 and 738.
+// 300 x 3000 1,071 and 738; transposed (k_pull_wsync before) 300 x 300 323 and 140,
+// 1000 x 1000 1,061 and 446, 1414 x 1414 1,512 and 677.
 #include <algorithm>
 #include <climits>
 
@@ -105,7 +106,9 @@ struct RingSlot {
   unsigned dst[32];
 };
 
-template <typename T, int U>
+// ADJ: the transposed walk, units and segments from the last to the first over the
+// lists of dependents.
+template <typename T, int U, bool ADJ>
 __global__ void __launch_bounds__(kBlockThreads) k_pull_block(BlockArgs<T> a) {
   using F = Flag<T>;
   using Bits = typename F::Bits;
@@ -122,7 +125,13 @@ __global__ void __launch_bounds__(kBlockThreads) k_pull_block(BlockArgs<T> a) {
   for (;;) {
     const unsigned c = next_chunk(a.ctl, a.nunits, &s_chunk);
     if (c >= (unsigned)a.nunits) break;
-    const int base = a.unit[c], g0 = a.useg[c], nseg = a.useg[c + 1] - g0;
+    const int unit = ADJ ? a.nunits - 1 - (int)c : (int)c;
+    const int base = a.unit[unit], end = ADJ ? a.unit[unit + 1] : 0, nseg = a.useg[unit + 1] - a.useg[unit];
+    // first position of the k-th segment, first past it
+    const int g0 = ADJ ? a.useg[unit + 1] - 1 : a.useg[unit];
+    auto lo_of = [&](int k) { return a.seg[ADJ ? g0 - k : g0 + k]; };
+    auto hi_of = [&](int k) { return a.seg[(ADJ ? g0 - k : g0 + k) + 1]; };
+    auto other_unit = [&](int q) { return ADJ ? q >= end && q != INT_MAX : q < base; };
     if (threadIdx.x < kRing) s_ready[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
       s_done = 0;
@@ -195,8 +204,8 @@ __global__ void __launch_bounds__(kBlockThreads) k_pull_block(BlockArgs<T> a) {
       int n_lo = 0, n_hi = 0, b_lo = 0, b_hi = 0, n_row = 0;
       auto bounds = [&](int k) {
         if (k >= nseg) return;
-        b_lo = a.seg[g0 + k];
-        b_hi = a.seg[g0 + k + 1];
+        b_lo = lo_of(k);
+        b_hi = hi_of(k);
       };
       auto fetch = [&]() {
         n_lo = b_lo;
@@ -207,14 +216,14 @@ __global__ void __launch_bounds__(kBlockThreads) k_pull_block(BlockArgs<T> a) {
       fetch();
       bounds(k0 + kStorers);
       for (int k = k0; k < nseg; k += kStorers) {
-        const int p = n_lo + lane, end = n_hi, row = n_row;
+        const int p = n_lo + lane, hi = n_hi, row = n_row;
         if (k + kStorers < nseg) fetch();
         bounds(k + 2 * kStorers);
         while (ld_acquire_shared(&s_done) <= k)
           if (!keep_waiting()) break;
         if (fail) break;
         __syncwarp();
-        if (p < end) {
+        if (p < hi) {
           const T v = ld_word(s_xa + (unsigned)(p - base) * (unsigned)sizeof(T), T(0));
           F::store(&a.xw[p], v);
           a.x[row] = v;
@@ -222,7 +231,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_pull_block(BlockArgs<T> a) {
       }
     } else {
       for (int k = warp / 4 * 3 + warp % 4 - 1; k < nseg; k += kLoaders) {
-        const int p = a.seg[g0 + k] + lane, end = a.seg[g0 + k + 1];
+        const int p = lo_of(k) + lane, hi = hi_of(k);
         T acc = T(0), w[U];
         unsigned src[U];
         int q[U];
@@ -234,7 +243,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_pull_block(BlockArgs<T> a) {
           q[u] = INT_MAX;
           v[u] = 0;
         }
-        if (p < end) {
+        if (p < hi) {
           const int e = a.dep_ptr[p], e1 = a.dep_ptr[p + 1], row = a.perm[p];
 #pragma unroll
           for (int u = 0; u < U; ++u)
@@ -245,40 +254,40 @@ __global__ void __launch_bounds__(kBlockThreads) k_pull_block(BlockArgs<T> a) {
           acc = a.b[row] * a.rcp[p];
 #pragma unroll
           for (int u = 0; u < U; ++u) {
-            if (q[u] < base) v[u] = F::load(&a.xw[q[u]]);
+            if (other_unit(q[u])) v[u] = F::load(&a.xw[q[u]]);
             else if (q[u] != INT_MAX) src[u] = s_xa + (unsigned)(q[u] - base) * (unsigned)sizeof(T);
           }
         }
         unsigned imported[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) imported[u] = __ballot_sync(kFull, q[u] < base);
+        for (int u = 0; u < U; ++u) imported[u] = __ballot_sync(kFull, other_unit(q[u]));
         while (k - ld_acquire_shared(&s_done) >= kRing)
           if (!keep_waiting()) break;
         if (fail) break;
         __syncwarp();
         RingSlot<T, U>& r = ring[k & (kRing - 1)];
-        r.dst[lane] = p < end ? s_xa + (unsigned)(p - base) * (unsigned)sizeof(T) : spare;
+        r.dst[lane] = p < hi ? s_xa + (unsigned)(p - base) * (unsigned)sizeof(T) : spare;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          r.w[u][lane] = q[u] < base ? -T(0) : -w[u];  // -0 x 0 added changes no value
+          r.w[u][lane] = other_unit(q[u]) ? -T(0) : -w[u];  // -0 x 0 added changes no value
           r.src[u][lane] = src[u];
         }
         // imported dependencies come first in ready order
         for (;;) {
           bool pending = false;
 #pragma unroll
-          for (int u = 0; u < U; ++u) pending = pending || (q[u] < base && v[u] == F::EMPTY);
+          for (int u = 0; u < U; ++u) pending = pending || (other_unit(q[u]) && v[u] == F::EMPTY);
           if (!__any_sync(kFull, pending)) break;
 #pragma unroll
           for (int u = 0; u < U; ++u)
-            if (q[u] < base && v[u] == F::EMPTY) v[u] = F::load(&a.xw[q[u]]);
+            if (other_unit(q[u]) && v[u] == F::EMPTY) v[u] = F::load(&a.xw[q[u]]);
           if (!keep_waiting()) break;
         }
         if (fail) break;
 #pragma unroll
         for (int u = 0; u < U; ++u)
           if (imported[u])
-            if (q[u] < base) acc = fma(-w[u], F::value(v[u]), acc);
+            if (other_unit(q[u])) acc = fma(-w[u], F::value(v[u]), acc);
         r.acc[lane] = acc;
         __syncwarp();
         if (lane == 0) st_release_shared(&s_ready[k & (kRing - 1)], k + 1);
@@ -467,7 +476,7 @@ template size_t block_smem_bytes<float>(int, int);
 template <typename T>
 cudaError_t launch_pull_block(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
                               const UnitTable& units, int longest, unsigned long long timeout_ns, int num_sms,
-                              cudaStream_t s) {
+                              cudaStream_t s, bool adj) {
   if (L.n == 0) return cudaSuccess;
   BlockArgs<T> a{};
   a.nunits = units.count;
@@ -476,9 +485,9 @@ cudaError_t launch_pull_block(const Layout& L, const Values<T>& V, const VecView
   a.useg = units.seg_ptr;
   a.seg = units.seg;
   a.perm = L.perm;
-  a.dep_ptr = L.dep_ptr;
-  a.dep_pos = L.dep_pos_f;
-  a.w = V.dep_w;
+  a.dep_ptr = adj ? L.out_ptr : L.dep_ptr;
+  a.dep_pos = adj ? L.out_pos_f : L.dep_pos_f;
+  a.w = adj ? V.out_w : V.dep_w;
   a.rcp = V.rcp;
   a.b = v.b;
   a.x = v.x;
@@ -493,18 +502,18 @@ cudaError_t launch_pull_block(const Layout& L, const Values<T>& V, const VecView
     return cudaGetLastError();
   };
   switch (longest) {
-    case 1: return run(k_pull_block<T, 1>);
-    case 2: return run(k_pull_block<T, 2>);
-    case 3: return run(k_pull_block<T, 3>);
-    case 4: return run(k_pull_block<T, 4>);
+    case 1: return adj ? run(k_pull_block<T, 1, true>) : run(k_pull_block<T, 1, false>);
+    case 2: return adj ? run(k_pull_block<T, 2, true>) : run(k_pull_block<T, 2, false>);
+    case 3: return adj ? run(k_pull_block<T, 3, true>) : run(k_pull_block<T, 3, false>);
+    case 4: return adj ? run(k_pull_block<T, 4, true>) : run(k_pull_block<T, 4, false>);
     default: return cudaErrorInvalidValue;
   }
 }
 template cudaError_t launch_pull_block<double>(const Layout&, const Values<double>&, const VecView<double>&, double*,
                                                DeviceCtl*, const UnitTable&, int, unsigned long long, int,
-                                               cudaStream_t);
+                                               cudaStream_t, bool);
 template cudaError_t launch_pull_block<float>(const Layout&, const Values<float>&, const VecView<float>&, float*,
                                               DeviceCtl*, const UnitTable&, int, unsigned long long, int,
-                                              cudaStream_t);
+                                              cudaStream_t, bool);
 
 }  // namespace sptrsv

@@ -406,7 +406,7 @@ size_t block_smem_bytes(int width, int longest);
 template <typename T>
 cudaError_t launch_pull_block(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
                               const UnitTable& units, int longest, unsigned long long timeout_ns, int num_sms,
-                              cudaStream_t s);
+                              cudaStream_t s, bool adj);
 size_t pull_smem_bytes(int chunk, int rhs, size_t elem);
 size_t imported_smem_bytes(int chunk, int max_imports, size_t elem);
 // warp-synchronous one-rhs forward pull with an importer warp per CTA (blocked layouts)

@@ -42,6 +42,8 @@ def test_blocked_solves_match_the_oracle(cuda, oracle_port, kind, n, lower, bloc
     m = _matrix(kind, n, lower)
     b = np.random.default_rng(n).standard_normal(m.n)
     ref = oracle_port.solve(m.col_ptr, m.row_idx, m.val, m.n, m.substitution, b)
+    t = m.transpose()
+    tref = oracle_port.solve(t.col_ptr, t.row_idx, t.val, m.n, t.substitution, b)
     kw = _blocked(min(block, m.n - 1))
     if batch:
         kw["wsync_batch"] = batch
@@ -50,6 +52,7 @@ def test_blocked_solves_match_the_oracle(cuda, oracle_port, kind, n, lower, bloc
         x = cuda.from_numpy(b.astype(dtype)).cuda()
         for _ in range(2):
             assert relerr(s.solve(x).cpu().numpy(), ref) <= tol
+            assert relerr(s.solve_adjoint(x)[0].cpu().numpy(), tref) <= tol
         s.solve(x, out=x)   # in place
         assert relerr(x.cpu().numpy(), ref) <= tol
         s.close()
@@ -61,10 +64,14 @@ def test_automatic_plan_of_a_mesh(cuda, oracle_port, grid, lower):
     m = _matrix("mesh", grid, lower)
     b = np.random.default_rng(grid).standard_normal(m.n)
     ref = oracle_port.solve(m.col_ptr, m.row_idx, m.val, m.n, m.substitution, b)
+    t = m.transpose()
+    tref = oracle_port.solve(t.col_ptr, t.row_idx, t.val, m.n, t.substitution, b)
     for dtype, tol in ((np.float64, 1e-12), (np.float32, 1e-5)):
         s = SyncFreeSolver(m.col_ptr, m.row_idx, m.n, m.substitution, values=m.val.astype(dtype), cluster=0)
         assert s.info()["order_block"] < m.n
-        assert relerr(s.solve(cuda.from_numpy(b.astype(dtype)).cuda()).cpu().numpy(), ref) <= tol
+        x = cuda.from_numpy(b.astype(dtype)).cuda()
+        assert relerr(s.solve(x).cpu().numpy(), ref) <= tol
+        assert relerr(s.solve_adjoint(x)[0].cpu().numpy(), tref) <= tol
         s.close()
 
 
@@ -78,6 +85,13 @@ def test_batch_in_blocked_order(cuda, oracle_port):
     at = 0
     for m, bi in zip(ms, b):
         ref = oracle_port.solve(m.col_ptr, m.row_idx, m.val, m.n, m.substitution, bi)
+        assert relerr(x[at:at + m.n], ref) <= 1e-12
+        at += m.n
+    x = s.solve_adjoint(cuda.from_numpy(np.concatenate(b)).cuda())[0].cpu().numpy()
+    at = 0
+    for m, bi in zip(ms, b):
+        t = m.transpose()
+        ref = oracle_port.solve(t.col_ptr, t.row_idx, t.val, m.n, t.substitution, bi)
         assert relerr(x[at:at + m.n], ref) <= 1e-12
         at += m.n
     s.close()
