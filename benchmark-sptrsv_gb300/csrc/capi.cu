@@ -209,7 +209,7 @@ void free_imports(ImportTable& t) {
 }
 
 void free_units(UnitTable& t) {
-  for (int* p : {t.start, t.seg_ptr, t.seg})
+  for (int* p : {t.start, t.seg_ptr, t.seg, t.walk})
     if (p) cudaFree(p);
   t = UnitTable();
 }
@@ -827,7 +827,6 @@ int build_pipe_table(sptrsv_gb300_handle_s* h, ImportTable& t, int chunk, size_t
 int ensure_units(sptrsv_gb300_handle_s* h, cudaStream_t s) {
   UnitTable& t = h->units;
   if (t.seg) return SPTRSV_OK;
-  free_units(t);
   const std::vector<int>& starts = h->layout_units;
   const Layout& L = h->layout;
   UnitTable made;  // becomes the table once complete
@@ -867,8 +866,24 @@ int ensure_units(sptrsv_gb300_handle_s* h, cudaStream_t s) {
     free_units(made);
     return map_cuda_error(err);
   }
+  made.walk = t.walk;
   t = made;
   h->device_bytes += sizeof(int) * (2 * starts.size() + (size_t)t.segments + 1);
+  return SPTRSV_OK;
+}
+
+// Positions by level of a blocked layout.
+int ensure_walk(sptrsv_gb300_handle_s* h, cudaStream_t s) {
+  if (h->units.walk) return SPTRSV_OK;
+  int* walk = nullptr;
+  CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&walk), sizeof(int) * (size_t)h->n));
+  const cudaError_t e = launch_level_walk(h->layout.perm, h->depth, h->n, h->nlevels, walk, s);
+  if (e != cudaSuccess) {
+    cudaFree(walk);
+    return map_cuda_error(e);
+  }
+  h->units.walk = walk;
+  h->device_bytes += sizeof(int) * (size_t)h->n;
   return SPTRSV_OK;
 }
 
@@ -1399,11 +1414,25 @@ bool stage_col_major(const sptrsv_gb300_handle_s* h, int rhs, int layout, int mi
   return layout == SPTRSV_LAYOUT_COL_MAJOR && rhs >= min_rhs && rhs > 1 && h->n > 0;
 }
 
+// Whether a block of right-hand sides on a blocked layout walks it in level order
+// (k_pull_ahead_multi, k_refine_ahead): one CTA per unit is too few for many
+// right-hand sides. From 8 in FP64 (1M-row mesh, a CTA per unit vs level order,
+// solve / refined us: 8 1,929 / 2,173 vs 1,579 / 1,601, 16 2,803 / 3,851 vs 1,891 /
+// 1,916, 33 6,945 vs 2,195, 64 6,393 / 10,408 vs 2,035 / 2,138; 300 x 300, 8 438 vs 421;
+// but 5 432 vs 484), from 9 in FP32 (9 2,445 vs 1,692; 300 x 300, 8 328 vs 367).
+bool use_level_walk(const sptrsv_gb300_handle_s* h, const ExecConfig& c, int rhs, size_t elem) {
+  if (rhs < (elem == 8 ? 8 : 9) || rhs > 64 || !c.wsync || c.exact || !c.smem_tier || h->layout_block >= h->n || h->layout_units.empty())
+    return false;
+  return h->plan.valid && h->rhs_tile_option == 0 && planned(h, SPTRSV_OPTION_CHUNK) &&
+         planned(h, SPTRSV_OPTION_CTAS_PER_SM) && c.block == 256 && c.sleep_max == 0;
+}
+
 // Whether the fused first refinement step of a block runs k_refine_ahead.
 bool refine_ahead_blocks(const sptrsv_gb300_handle_s* h, int rhs) {
   const ExecConfig c = pick_config(h, rhs);
   return rhs > 1 && rhs <= 64 && h->fused_refine == 2 && c.sched == SCHED_PULL && !c.exact &&
-         planned(h, SPTRSV_OPTION_CTAS_PER_SM) && use_ahead_multi(h, c, rhs, sizeof(double), false);
+         planned(h, SPTRSV_OPTION_CTAS_PER_SM) &&
+         (use_ahead_multi(h, c, rhs, sizeof(double), false) || use_level_walk(h, c, rhs, sizeof(double)));
 }
 
 // Column-major blocks that solve_typed stages itself, scaled on the way in
@@ -1440,9 +1469,12 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
   if (c.sched == SCHED_LEVELSET) form = FORM_DEP_W;
   ST_TRY(need_forms<T>(h, form, s));
   const bool cluster = rhs == 1 && !(adj && adj->grad) && use_cluster<T>(h, adj != nullptr);
-  const bool multi = c.sched == SCHED_PULL && !(adj && adj->grad) && use_ahead_multi(h, c, rhs, sizeof(T), adj != nullptr);
+  const bool blocks = c.sched == SCHED_PULL && !(adj && adj->grad);
+  const bool walk = blocks && use_level_walk(h, c, rhs, sizeof(T));
+  if (walk) ST_TRY(ensure_walk(h, s));
+  const bool multi = walk || (blocks && use_ahead_multi(h, c, rhs, sizeof(T), adj != nullptr));
   const int words = multi ? ahead_multi_words(rhs, sizeof(T), n < kNarrowWidth * h->nlevels) : rhs;
-  const bool columns = multi && stage_col_major(h, rhs, layout, kColMajorStageRhs);
+  const bool columns = multi && !walk && stage_col_major(h, rhs, layout, kColMajorStageRhs);
   if (columns) {
     ST_TRY(ensure_buf(h, h->tb, sizeof(T) * (size_t)n * words, 0, s));
     CUDA_TRY(launch_columns_in<T>(h->layout, V, b, static_cast<T*>(h->tb.p), rhs, words, s));
@@ -1533,7 +1565,7 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
     } else if (multi) {
       CUDA_TRY(launch_pull_ahead_multi<T>(h->layout, V, rhs, v, static_cast<T*>(h->xw.p), h->ctl,
                                           n < kNarrowWidth * h->nlevels, timeout_ns(h), h->num_sms, s,
-                                          adj != nullptr));
+                                          adj != nullptr, walk ? h->units.walk : nullptr));
     } else if (rhs == 1 && !pc && !(adj && adj->grad) && use_ahead(h, c)) {
       CUDA_TRY(launch_pull_ahead<T>(h->layout, V, v, static_cast<T*>(h->xw.p), h->ctl, h->nlevels, timeout_ns(h),
                                     h->num_sms, s, adj != nullptr));
@@ -2220,6 +2252,8 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
         rhs == 1 ? fc.wsync && fc.smem_tier && h->layout_block >= h->n && fc.block == 256 && fc.chunk == 256 &&
                        fc.sleep_max == 0 && fc.wsync_batch == 0 && planned(h, SPTRSV_OPTION_CTAS_PER_SM)
                  : refine_ahead_blocks(h, rhs);
+    const bool walk = refine_ahead && rhs > 1 && h->layout_block < h->n;
+    if (walk) ST_TRY(ensure_walk(h, s));
     // the plain solve's rule (160k-row bands with 1 / 2 entries per column and a
     // 1M-row band with 3: 0.101 / 1.95 / 6.40 ms refined with two dependencies
     // per iteration, 0.082 / 1.54 / 5.62 with one; the mesh triangle with two:
@@ -2279,7 +2313,8 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
                                             timeout_ns(h), h->num_sms, s, h->imports));
     } else if (wsplit && refine_ahead) {
       CUDA_TRY(launch_refine_ahead(h->layout, h->v64, rhs, d_b, d_x, si, sk,
-                                   static_cast<unsigned long long*>(h->xw.p), stats, h->ctl, width, timeout_ns(h), h->num_sms, s, wsplit));
+                                   static_cast<unsigned long long*>(h->xw.p), stats, h->ctl, width, timeout_ns(h),
+                                   h->num_sms, s, wsplit, walk ? h->units.walk : nullptr));
     } else {
       CUDA_TRY(launch_refine_fused(h->layout, h->v32, h->v64, rhs, d_b, d_x, si, sk,
                                    static_cast<unsigned long long*>(h->xw.p), stats, h->ctl, fc, timeout_ns(h),

@@ -48,12 +48,14 @@ struct AheadMultiArgs {
 // memory is the bound (1M rows of 9 entries, 64 right-hand sides: 1,684 us here
 // instead of 1,772; whole solves 2,148 -> 2,086, at 32 on 500k rows 682 -> 662, FP32
 // 664 -> 638). Laid out like the value words the rows scatter: 90 us longer.
-enum { kWhole, kPad, kStaged };
+// kWalk: a blocked layout in level order, through `walk` (positions by level). Its
+// lists come from global memory, every dependency from the value words.
+enum { kWhole, kPad, kStaged, kWalk };
 
 // G lanes per unknown, R adjacent right-hand sides per lane, 256 / G unknowns per
 // chunk.
 template <typename T, bool ADJ, int G, int R, int MODE>
-__global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, int words) {
+__global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, int words, const int* walk) {
   using F = Flag<T>;
   using Bits = typename F::Bits;
   constexpr unsigned kFull = 0xffffffffu;
@@ -70,33 +72,36 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, i
   const int last = a.n - 1, rhs = MODE == kWhole ? a.rhs : words;
   const bool col = k < rhs;
   // two chunks ahead: rows and list bounds
-  int f_row = 0, f_e = 0, f_e1 = 0, f_lo = 0, f_hi = 0;
+  int f_row = 0, f_e = 0, f_e1 = 0, f_lo = 0, f_hi = 0, f_p = 0;
   auto fetch = [&](int c) {
     f_e = f_e1 = f_lo = f_hi = 0;
     if (c >= a.nchunks) return;
     const int base = c * kUnknowns, end = min(base + kUnknowns, a.n);
     const int pr = base + j;
     if (pr < a.n) {
-      const int p = ADJ ? last - pr : pr;
+      const int p = MODE == kWalk ? walk[ADJ ? last - pr : pr] : (ADJ ? last - pr : pr);
+      if (MODE == kWalk) f_p = p;
       f_row = a.perm[p];
       f_e = a.ptr[p];
       f_e1 = a.ptr[p + 1];
     }
+    if (MODE == kWalk) return;  // no lists to stage
     f_lo = a.ptr[ADJ ? last - (end - 1) : base];
     f_hi = a.ptr[ADJ ? last - base + 1 : end];
   };
   // one chunk ahead: first terms, and the lists on their way to shared memory
-  int n_row = 0, n_e = 0, n_e1 = 0, n_lo = 0;
+  int n_row = 0, n_e = 0, n_e1 = 0, n_lo = 0, n_p = 0;
   T n_acc[R];
   auto stage = [&](int c, int buf) {
     n_row = f_row;
     n_e = f_e;
     n_e1 = f_e1;
     n_lo = f_lo;
+    n_p = f_p;
     if (c >= a.nchunks) return;
     const int pr = c * kUnknowns + j;
     if (pr < a.n && col) {
-      const int p = ADJ ? last - pr : pr;
+      const int p = MODE == kWalk ? n_p : (ADJ ? last - pr : pr);
       if (MODE == kStaged) {
 #pragma unroll
         for (int i = 0; i < R; ++i) n_acc[i] = a.b[(long long)n_row * rhs + k + i];
@@ -104,7 +109,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, i
         const T r = a.rcp[p];
 #pragma unroll
         for (int i = 0; i < R; ++i)
-          n_acc[i] = a.b[(long long)n_row * a.b_si + (long long)(MODE == kPad ? min(k + i, a.rhs - 1) : k + i) * a.b_sk] * r;
+          n_acc[i] = a.b[(long long)n_row * a.b_si + (long long)(MODE == kPad || MODE == kWalk ? min(k + i, a.rhs - 1) : k + i) * a.b_sk] * r;
       }
     }
     const int hi = min(f_hi, f_lo + a.cap);
@@ -133,7 +138,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, i
   for (int buf = 0; c < a.nchunks; buf ^= 1) {
     const int base = c * kUnknowns, pr = base + j;
     bool done = pr >= a.n || !col;
-    const int p = ADJ ? last - pr : pr;
+    const int p = MODE == kWalk ? n_p : (ADJ ? last - pr : pr);
     const int row = n_row, lo = n_lo;
     int e = n_e;
     const int e1 = n_e1;
@@ -158,12 +163,12 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, i
     int nq = 0;
     int left = e1 - e - 1;
     auto next = [&](int ee) {
-      nq = ee < hi ? lq[ee] : a.pos[ee];
-      nw = ee < hi ? lw[ee] : a.w[ee];
+      nq = MODE != kWalk && ee < hi ? lq[ee] : a.pos[ee];
+      nw = MODE != kWalk && ee < hi ? lw[ee] : a.w[ee];
     };
     auto target = [&](int q) {
       const int off = (ADJ ? last - q : q) - base;
-      nmine = off >= 0;
+      nmine = MODE != kWalk && off >= 0;
       nlocal = s_wina + (unsigned)((off & (kUnknowns - 1)) * (G * R) + k) * (unsigned)sizeof(T);
       nword = a.xw + (long long)q * rhs + k;
     };
@@ -225,7 +230,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, i
 #pragma unroll
       for (int i = 0; i < R; ++i) {
         if (MODE == kStaged) a.x[(long long)row * rhs + k + i] = acc[i];
-        else a.x[(long long)row * a.x_si + (long long)(MODE == kPad ? min(k + i, a.rhs - 1) : k + i) * a.x_sk] = acc[i];
+        else a.x[(long long)row * a.x_si + (long long)(MODE == kPad || MODE == kWalk ? min(k + i, a.rhs - 1) : k + i) * a.x_sk] = acc[i];
       }
     }
     if (__syncthreads_or(fail)) break;
@@ -241,13 +246,13 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, i
 }  // namespace
 
 template <typename T, bool ADJ>
-cudaError_t launch_ahead_multi(AheadMultiArgs<T>& a, int avg, bool narrow, int num_sms, cudaStream_t s) {
+cudaError_t launch_ahead_multi(AheadMultiArgs<T>& a, int avg, bool narrow, int num_sms, cudaStream_t s, const int* walk) {
   const int words = ahead_multi_words(a.rhs, sizeof(T), narrow);
   auto run = [&](auto kernel, int g, int r) -> cudaError_t {
     const int unknowns = 256 / g;
     a.nchunks = (a.n + unknowns - 1) / unknowns;
     // twice the average chunk's lists (longer ones read the rest from global memory)
-    a.cap = std::min(1024, std::max(64, (2 * avg * unknowns / 32 + 31) / 32 * 32));
+    a.cap = walk ? 0 : std::min(1024, std::max(64, (2 * avg * unknowns / 32 + 31) / 32 * 32));
     const size_t smem = (size_t)256 * r * sizeof(T) + (size_t)2 * a.cap * (sizeof(T) + sizeof(int));
     cudaError_t e = cudaSuccess;
     if (smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -256,10 +261,21 @@ cudaError_t launch_ahead_multi(AheadMultiArgs<T>& a, int avg, bool narrow, int n
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 256, smem);
     if (per < 1) per = 1;
     const int grid = static_cast<int>(std::min<long long>((long long)num_sms * per, a.nchunks));
-    kernel<<<grid, 256, smem, s>>>(a, words);
+    kernel<<<grid, 256, smem, s>>>(a, words, walk);
     return cudaGetLastError();
   };
   const bool pad = a.rhs != words, staged = a.b_si == 0;
+  if (walk) {
+    switch (ahead_multi_shape(a.rhs, sizeof(T), narrow)) {
+      case 8 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 8, 1, kWalk>, 8, 1);
+      case 16 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 16, 1, kWalk>, 16, 1);
+      case 8 * 8 + 2: return run(k_pull_ahead_multi<T, ADJ, 8, 2, kWalk>, 8, 2);
+      case 16 * 8 + 2: return run(k_pull_ahead_multi<T, ADJ, 16, 2, kWalk>, 16, 2);
+      case 16 * 8 + 4: return run(k_pull_ahead_multi<T, ADJ, 16, 4, kWalk>, 16, 4);
+      case 32 * 8 + 2: return run(k_pull_ahead_multi<T, ADJ, 32, 2, kWalk>, 32, 2);
+      default: return cudaErrorInvalidValue;
+    }
+  }
   switch (ahead_multi_shape(a.rhs, sizeof(T), narrow)) {
     case 2 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 2, 1, kWhole>, 2, 1);
     case 4 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 4, 1, kWhole>, 4, 1);
@@ -346,7 +362,7 @@ template cudaError_t launch_columns_out<float>(const Layout&, const float*, floa
 template <typename T>
 cudaError_t launch_pull_ahead_multi(const Layout& L, const Values<T>& V, int rhs, const VecView<T>& v, T* xw,
                                     DeviceCtl* ctl, bool narrow, unsigned long long timeout_ns, int num_sms,
-                                    cudaStream_t s, bool adj) {
+                                    cudaStream_t s, bool adj, const int* walk) {
   if (L.n == 0) return cudaSuccess;
   AheadMultiArgs<T> a{};
   a.n = L.n;
@@ -366,14 +382,14 @@ cudaError_t launch_pull_ahead_multi(const Layout& L, const Values<T>& V, int rhs
   a.ctl = ctl;
   a.timeout_ns = timeout_ns;
   const int avg = static_cast<int>(32LL * L.ndep / L.n);
-  return adj ? launch_ahead_multi<T, true>(a, avg, narrow, num_sms, s)
-             : launch_ahead_multi<T, false>(a, avg, narrow, num_sms, s);
+  return adj ? launch_ahead_multi<T, true>(a, avg, narrow, num_sms, s, walk)
+             : launch_ahead_multi<T, false>(a, avg, narrow, num_sms, s, walk);
 }
 template cudaError_t launch_pull_ahead_multi<double>(const Layout&, const Values<double>&, int, const VecView<double>&,
                                                      double*, DeviceCtl*, bool, unsigned long long, int, cudaStream_t,
-                                                     bool);
+                                                     bool, const int*);
 template cudaError_t launch_pull_ahead_multi<float>(const Layout&, const Values<float>&, int, const VecView<float>&,
                                                     float*, DeviceCtl*, bool, unsigned long long, int, cudaStream_t,
-                                                    bool);
+                                                    bool, const int*);
 
 }  // namespace sptrsv

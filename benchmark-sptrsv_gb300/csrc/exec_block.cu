@@ -452,6 +452,28 @@ cudaError_t launch_import_tables(const unsigned* ext_q, const int* ext_u, const 
   return e;
 }
 
+cudaError_t launch_level_walk(const int* perm, const int* depth, int n, int nlevels, int* walk, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  unsigned *keys = nullptr, *sorted = nullptr;
+  int* iota = nullptr;
+  void* temp = nullptr;
+  int bits = 1;
+  while (bits < 31 && (1 << bits) < nlevels) ++bits;
+  const size_t bytes = sizeof(int) * (size_t)n;
+  cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&keys), bytes, s);
+  if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void**>(&sorted), bytes, s);
+  if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void**>(&iota), bytes, s);
+  if (e == cudaSuccess) e = cudaMallocAsync(&temp, radix_sort_temp_bytes(n), s);
+  if (e == cudaSuccess) e = launch_iota(iota, n, 0, 1, s);
+  if (e == cudaSuccess) {
+    k_gather_keys<<<grid_1d(n), 256, 0, s>>>(depth, perm, n, keys);
+    e = radix_sort_pairs(keys, iota, sorted, walk, n, bits, temp, s);
+  }
+  for (void* b : {(void*)keys, (void*)sorted, (void*)iota, temp})
+    if (b) cudaFreeAsync(b, s);
+  return e;
+}
+
 cudaError_t launch_unit_segments(const int* perm, const int* depth, const int* unit, int nunits, const int* first,
                                  int* count, int* levels, int* seg, cudaStream_t s) {
   if (nunits <= 0) return cudaSuccess;

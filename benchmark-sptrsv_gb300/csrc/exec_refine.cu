@@ -517,8 +517,10 @@ __global__ void __launch_bounds__(288) k_pull_refine1_imp(RefineArgs a) {
 // band, 4 / 8 / 32 / 64 575 / 598 / 793 / 1,077 -> 358 / 373 / 643 / 1,048; 700k
 // rows, 3,004 per level, 1 / 16 259 / 478 -> 180 / 380. Bound by the hop at few
 // right-hand sides, by FP32 issue at 64.
-template <int G, int R, bool PAD>
-__global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a) {
+// WALK: a blocked layout in level order, through `walk` (positions by level). Its
+// lists come from global memory, every dependency from the value words.
+template <int G, int R, bool PAD, bool WALK = false>
+__global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a, const int* walk) {
   using Bits = unsigned long long;
   constexpr unsigned kFull = 0xffffffffu;
   constexpr int kUnknowns = 256 / G;
@@ -535,33 +537,36 @@ __global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a) {
   const bool col = k < rhs;
   float mx_d = 0.f, mx_x = 0.f, mx_x0 = 0.f;  // stopping-estimate maxima
   // two chunks ahead: rows and list bounds
-  int f_row = 0, f_e = 0, f_e1 = 0, f_lo = 0, f_hi = 0;
+  int f_row = 0, f_e = 0, f_e1 = 0, f_lo = 0, f_hi = 0, f_p = 0;
   auto fetch = [&](int c) {
     f_e = f_e1 = f_lo = f_hi = 0;
     if (c >= a.nchunks) return;
     const int base = c * kUnknowns, end = min(base + kUnknowns, a.n);
     const int pr = base + j;
     if (pr < a.n) {
-      const int p = pr;
+      const int p = WALK ? walk[pr] : pr;
+      if (WALK) f_p = p;
       f_row = a.perm[p];
       f_e = a.dep_ptr[p];
       f_e1 = a.dep_ptr[p + 1];
     }
+    if (WALK) return;  // no lists to stage
     f_lo = a.dep_ptr[base];
     f_hi = a.dep_ptr[end];
   };
   // one chunk ahead: first terms, and the lists on their way to shared memory
-  int n_row = 0, n_e = 0, n_e1 = 0, n_lo = 0;
+  int n_row = 0, n_e = 0, n_e1 = 0, n_lo = 0, n_p = 0;
   float n_hi[R], n_lo2[R];
   auto stage = [&](int c, int buf) {
     n_row = f_row;
     n_e = f_e;
     n_e1 = f_e1;
     n_lo = f_lo;
+    n_p = f_p;
     if (c >= a.nchunks) return;
     const int pr = c * kUnknowns + j;
     if (pr < a.n && col) {
-      const double s64 = a.rcp64[pr];
+      const double s64 = a.rcp64[WALK ? n_p : pr];
 #pragma unroll
       for (int i = 0; i < R; ++i) {
         // b/d as a float pair: hi = RN32(b*s), lo = RN32(b*s - hi)
@@ -596,7 +601,7 @@ __global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a) {
   for (int buf = 0; c < a.nchunks; buf ^= 1) {
     const int base = c * kUnknowns, pr = base + j;
     bool done = pr >= a.n || !col;
-    const int p = pr;
+    const int p = WALK ? n_p : pr;
     const int row = n_row, lo = n_lo;
     int e = n_e;
     const int e1 = n_e1;
@@ -624,12 +629,12 @@ __global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a) {
     int nq = 0;
     int left = e1 - e - 1;
     auto next = [&](int ee) {
-      nq = ee < hi ? lq[ee] : a.dep_pos_f[ee];
-      nw = ee < hi ? lw[ee] : a.wsplit[ee];
+      nq = !WALK && ee < hi ? lq[ee] : a.dep_pos_f[ee];
+      nw = !WALK && ee < hi ? lw[ee] : a.wsplit[ee];
     };
     auto target = [&](int q) {
       const int off = (q) - base;
-      nmine = off >= 0;
+      nmine = !WALK && off >= 0;
       nlocal = s_wina + (unsigned)((off & (kUnknowns - 1)) * (G * R) + k) * 8u;
       nword = xw + (long long)q * rhs + k;
     };
@@ -792,7 +797,7 @@ cudaError_t launch_refine_fused(const Layout& L, const Values<float>& v32, const
 cudaError_t launch_refine_ahead(const Layout& L, const Values<double>& v64, int rhs, const double* b, double* x,
                                 long long si, long long sk, unsigned long long* xw, unsigned long long* stats,
                                 DeviceCtl* ctl, long long width, unsigned long long timeout_ns, int num_sms,
-                                cudaStream_t s, const float2* wsplit) {
+                                cudaStream_t s, const float2* wsplit, const int* walk) {
   if (L.n == 0) return cudaSuccess;
   RefineArgs a{};
   a.n = L.n;
@@ -818,7 +823,7 @@ cudaError_t launch_refine_ahead(const Layout& L, const Values<double>& v64, int 
     const int unknowns = 256 / g;
     a.nchunks = (a.n + unknowns - 1) / unknowns;
     // twice the average chunk's lists (longer ones read the rest from global memory)
-    a.cap = std::min(g == 1 ? 4096 : 1024, std::max(64, (2 * avg * unknowns / 32 + 31) / 32 * 32));
+    a.cap = walk ? 0 : std::min(g == 1 ? 4096 : 1024, std::max(64, (2 * avg * unknowns / 32 + 31) / 32 * 32));
     const size_t smem = (size_t)256 * r * 8 + (size_t)2 * a.cap * 12;
     cudaError_t e = cudaSuccess;
     if (smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -828,9 +833,19 @@ cudaError_t launch_refine_ahead(const Layout& L, const Values<double>& v64, int 
     if (per < 1) per = 1;
     if (ctas > 0) per = std::min(per, ctas);
     const int grid = static_cast<int>(std::min<long long>((long long)num_sms * per, a.nchunks));
-    kernel<<<grid, 256, smem, s>>>(a);
+    kernel<<<grid, 256, smem, s>>>(a, walk);
     return cudaGetLastError();
   };
+  if (walk) {
+    switch (ahead_multi_shape(rhs, 8, width < kNarrowWidth)) {
+      case 8 * 8 + 1: return run(k_refine_ahead<8, 1, true, true>, 8, 1);
+      case 16 * 8 + 1: return run(k_refine_ahead<16, 1, true, true>, 16, 1);
+      case 8 * 8 + 2: return run(k_refine_ahead<8, 2, true, true>, 8, 2);
+      case 16 * 8 + 2: return run(k_refine_ahead<16, 2, true, true>, 16, 2);
+      case 32 * 8 + 2: return run(k_refine_ahead<32, 2, true, true>, 32, 2);
+      default: return cudaErrorInvalidValue;
+    }
+  }
   if (rhs == 1) return run(k_refine_ahead<1, 1, false>, 1, 1);
   const bool pad = rhs != ahead_multi_words(rhs, 8, width < kNarrowWidth);
   switch (ahead_multi_shape(rhs, 8, width < kNarrowWidth)) {

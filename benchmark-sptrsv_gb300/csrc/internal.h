@@ -129,6 +129,7 @@ struct UnitTable {
   int* start = nullptr;      // device [count+1]
   int* seg_ptr = nullptr;    // device [count+1]
   int* seg = nullptr;        // device [segments+1]
+  int* walk = nullptr;       // device [n] positions by level (blocks of many right-hand sides)
 };
 
 // Solve-time description of one right-hand-side block. Element (i, k) of b
@@ -356,11 +357,12 @@ inline int ahead_multi_words(int rhs, size_t elem, bool narrow) {
   return per > 1 ? (rhs + per - 1) / per * per : rhs;
 }
 // v.b_si = 0: v.b holds the rows launch_columns_in wrote, v.x is to hold rows of
-// ahead_multi_words values (shapes of more than 16 right-hand sides).
+// ahead_multi_words values (shapes of more than 16 right-hand sides). walk: positions
+// by level of a blocked layout (shapes of more than 4 right-hand sides).
 template <typename T>
 cudaError_t launch_pull_ahead_multi(const Layout& L, const Values<T>& V, int rhs, const VecView<T>& v, T* xw,
                                     DeviceCtl* ctl, bool narrow, unsigned long long timeout_ns, int num_sms,
-                                    cudaStream_t s, bool adj);
+                                    cudaStream_t s, bool adj, const int* walk);
 // A column-major block to rows of first terms b / d, and the solution's columns from
 // rows; `words` values per row (ahead_multi_words).
 template <typename T>
@@ -400,6 +402,8 @@ cudaError_t launch_import_tables(const unsigned* ext_q, const int* ext_u, const 
                                  int nunits, int width, int* im_ptr, int* im_q, int* dep_slot, cudaStream_t s);
 cudaError_t launch_unit_segments(const int* perm, const int* depth, const int* unit, int nunits, const int* first,
                                  int* count, int* levels, int* seg, cudaStream_t s);
+// positions by level, ties in order
+cudaError_t launch_level_walk(const int* perm, const int* depth, int n, int nlevels, int* walk, cudaStream_t s);
 // one consumer warp per unit, level by level; lists of at most 4 entries (longest)
 template <typename T>
 size_t block_smem_bytes(int width, int longest);
@@ -448,11 +452,11 @@ cudaError_t launch_refine_fused(const Layout& L, const Values<float>& v32, const
                                 unsigned long long timeout_ns, int num_sms, cudaStream_t s,
                                 const float2* wsplit = nullptr);
 // the fused step in double-float on a level-order layout, lists staged ahead (1 right-hand side, or a block
-// ahead_multi_shape has a shape for)
+// ahead_multi_shape has a shape for; on a blocked one through `walk`, 5 and more)
 cudaError_t launch_refine_ahead(const Layout& L, const Values<double>& v64, int rhs, const double* b, double* x,
                                 long long si, long long sk, unsigned long long* xw, unsigned long long* stats,
                                 DeviceCtl* ctl, long long width, unsigned long long timeout_ns, int num_sms,
-                                cudaStream_t s, const float2* wsplit);
+                                cudaStream_t s, const float2* wsplit, const int* walk);
 cudaError_t launch_split_weights(const double* w, long long count, float2* out, cudaStream_t s);
 // The same fused step (double-float residual, one right-hand side, b and x
 // vectors) on a blocked layout, with an importer warp per CTA (the table of

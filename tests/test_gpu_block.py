@@ -75,6 +75,30 @@ def test_automatic_plan_of_a_mesh(cuda, oracle_port, grid, lower):
         s.close()
 
 
+@pytest.mark.parametrize("rhs", [8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("grid, lower, col_major", [(150, True, False), (131, False, True), (400, True, False)])
+def test_blocks_walk_a_mesh_in_level_order(cuda, oracle_port, grid, lower, col_major, rhs):
+    """Blocks of right-hand sides on the automatic plan's blocked layout, narrow and wide levels."""
+    from sptrsv_gb300 import SyncFreeSolver
+    m = _matrix("mesh", grid, lower)
+    b = np.random.default_rng(rhs).standard_normal((m.n, rhs))
+    ref = oracle_port.solve(m.col_ptr, m.row_idx, m.val, m.n, m.substitution, b)
+    t = m.transpose()
+    tref = oracle_port.solve(t.col_ptr, t.row_idx, t.val, m.n, t.substitution, b)
+    for dtype, tol in ((np.float64, 1e-12), (np.float32, 1e-5)):
+        s = SyncFreeSolver(m.col_ptr, m.row_idx, m.n, m.substitution, values=m.val.astype(dtype))
+        assert s.info()["order_block"] < m.n
+        x = cuda.from_numpy(b.astype(dtype)).cuda()
+        if col_major:
+            x = x.t().contiguous().t()
+        for _ in range(2):
+            assert relerr(s.solve(x).cpu().numpy(), ref) <= tol
+            assert relerr(s.solve_adjoint(x)[0].cpu().numpy(), tref) <= tol
+        if dtype == np.float64:
+            assert relerr(s.solve_refine(x)[0].cpu().numpy(), ref) <= 1e-10
+        s.close()
+
+
 def test_batch_in_blocked_order(cuda, oracle_port):
     from sptrsv_gb300 import SyncFreeSolver
     ms = [_matrix(k, n, low) for k, n, low in (("mesh", 30, True), ("chain", 333, False), ("lists4", 1000, False))]
