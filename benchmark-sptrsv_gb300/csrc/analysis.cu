@@ -1138,7 +1138,8 @@ cudaError_t launch_fill_push(const int* perm, const int* iperm, const int* col_p
 // starts they hold by a binary search over shuffles. Bound by the gather of
 // 8-byte values from 32-byte sectors. (One thread per list, as before, strides
 // its loads and stores over 32 lists: the 5M-entry band system's pull weights
-// took 66 us, the FP64 diagonal 11 more.)
+// took 66 us, the FP64 diagonal 11 more; with the copy of the values into the handle
+// and the checks, all of set_values takes 90 us now.)
 template <typename TV, typename T, bool DIAG, bool SCALE>
 __global__ void __launch_bounds__(256) k_stage_lists(const int* __restrict__ ptr, const int* __restrict__ src,
                                                      const TV* __restrict__ val, const int* __restrict__ diag_src,

@@ -576,99 +576,64 @@ int ensure_table(sptrsv_gb300_handle_s* h, bool adj, int cmax, int emax, cudaStr
 // are cut into k = min(32, ceil(len/split)) interleaved slices (piece j takes
 // entries j, j+k, j+2k, ... of the ready-ordered list), so the latest entries
 // spread over all the pieces instead of piling up in the last one.
-int build_pieces(sptrsv_gb300_handle_s* h, PieceTable& t, const std::vector<int>& counts, bool reversed, int split,
-                 int chunk, cudaStream_t s) {
-  free_pieces(t);
-  const int n = static_cast<int>(counts.size());
-  std::vector<long long> start((size_t)n + 1, 0);
-  for (int p = 0; p < n; ++p) start[p + 1] = start[p] + counts[p];
-  std::vector<int> walk, lo, hi;
-  walk.reserve((size_t)n + n / 8 + 32);
-  lo.reserve(walk.capacity());
-  hi.reserve(walk.capacity());
-  auto pad = [&]() {
-    while (walk.size() % 32) {
-      walk.push_back(-1);
-      lo.push_back(0);
-      hi.push_back(0);
-    }
-  };
-  std::vector<int> cseg, cbase;
-  std::vector<unsigned char> seg_split_host;
-  const size_t seg_cap = static_cast<size_t>(std::max(1, (chunk + 31) / 32));
-  // a reverse walk is shifted so that its chunk boundaries fall on multiples of
-  // `chunk` positions (the order blocks of a blocked layout)
-  const int shift = reversed ? (chunk - n % chunk) % chunk : 0;
-  for (int i = 0; i < n; ++i) {
-    const int p = reversed ? n - 1 - i : i;
-    const long long c = counts[p], e0 = start[p];
-    const int k = (split > 0 && c > split) ? static_cast<int>(std::min<long long>(32, (c + split - 1) / split)) : 1;
-    const bool seg_full = walk.size() % 32 + k > 32;
-    const size_t first = seg_full ? (walk.size() + 31) / 32 * 32 : walk.size();
-    const size_t segs_after = (first + k - 1) / 32 + 1;  // segments in use once i is placed
-    if ((i + shift) % chunk == 0 || i == 0 || (!cseg.empty() && segs_after - cseg.back() > seg_cap)) {
-      pad();  // a chunk starts on a fresh segment
-      cseg.push_back(static_cast<int>(walk.size() / 32));
-      cbase.push_back(i);
-    } else if (seg_full) {
-      pad();
-    }
-    if (k > 1) {  // this unknown spans lanes of the segment it starts (after any padding above)
-      const size_t sg = walk.size() / 32;
-      if (seg_split_host.size() <= sg) seg_split_host.resize(sg + 1, 0);
-      seg_split_host[sg] = 1;
-    }
-    for (int j = 0; j < k; ++j) {  // piece j: entries e0 + j, e0 + j + k, ... (interleaved)
-      walk.push_back(i);
-      lo.push_back(static_cast<int>(e0 + j));
-      hi.push_back(static_cast<int>(e0 + c));
-    }
-  }
-  pad();
-  t.split = split;
-  t.chunk = chunk;
-  t.nseg = static_cast<int>(walk.size() / 32);
-  t.nchunks = static_cast<int>(cseg.size());
-  cseg.push_back(t.nseg);
-  const size_t np = walk.size() > 0 ? walk.size() : 1;
-  CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.walk), sizeof(int) * np));
-  CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.row), sizeof(int) * np));
-  CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.lo), sizeof(int) * np));
-  CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.hi), sizeof(int) * np));
-  CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.cseg), sizeof(int) * cseg.size()));
-  CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.cbase), sizeof(int) * (cbase.empty() ? 1 : cbase.size())));
-  seg_split_host.resize(t.nseg > 0 ? t.nseg : 1, 0);
-  CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&t.seg_split), seg_split_host.size()));
-  CUDA_TRY(cudaMemcpy(t.seg_split, seg_split_host.data(), seg_split_host.size(), cudaMemcpyHostToDevice));
-  if (!cbase.empty())
-    CUDA_TRY(cudaMemcpy(t.cbase, cbase.data(), sizeof(int) * cbase.size(), cudaMemcpyHostToDevice));
-  if (!walk.empty()) {
-    CUDA_TRY(cudaMemcpy(t.walk, walk.data(), sizeof(int) * walk.size(), cudaMemcpyHostToDevice));
-    // row of each piece's unknown: perm gathered on the device (padding reads position 0)
-    std::vector<int> posv(walk.size());
-    for (size_t i = 0; i < walk.size(); ++i)
-      posv[i] = walk[i] < 0 ? 0 : (reversed ? n - 1 - walk[i] : walk[i]);
-    int* pos_dev = nullptr;
-    CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&pos_dev), sizeof(int) * posv.size()));
-    cudaError_t err = cudaMemcpyAsync(pos_dev, posv.data(), sizeof(int) * posv.size(), cudaMemcpyHostToDevice, s);
-    if (err == cudaSuccess) err = launch_gather_int(h->layout.perm, pos_dev, t.row, static_cast<int>(posv.size()), s);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(s);
-    cudaFree(pos_dev);
-    CUDA_TRY(err);
-    CUDA_TRY(cudaMemcpy(t.lo, lo.data(), sizeof(int) * walk.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(t.hi, hi.data(), sizeof(int) * walk.size(), cudaMemcpyHostToDevice));
-  }
-  CUDA_TRY(cudaMemcpy(t.cseg, cseg.data(), sizeof(int) * cseg.size(), cudaMemcpyHostToDevice));
-  h->device_bytes += sizeof(int) * (4 * np + cseg.size() + cbase.size());
-  return SPTRSV_OK;
-}
-
 int ensure_pieces(sptrsv_gb300_handle_s* h, bool adj, int split, int chunk, cudaStream_t s) {
   PieceTable& t = adj ? h->pc_adj : h->pc_fwd;
   if (t.walk && t.split == split && t.chunk == chunk) return SPTRSV_OK;
-  const std::vector<int>* counts = nullptr;
-  ST_TRY(list_counts(h, adj, s, &counts));
-  return build_pieces(h, t, *counts, adj, split, chunk, s);
+  free_pieces(t);
+  const Layout& L = h->layout;
+  const int n = L.n;
+  const int* ptr = adj ? L.out_ptr : L.dep_ptr;
+  // a reverse walk is shifted so that its chunk boundaries fall on multiples of
+  // `chunk` positions (the order blocks of a blocked layout)
+  const int shift = adj ? (chunk - n % chunk) % chunk : 0;
+  const int nranges = static_cast<int>(((long long)n + shift + chunk - 1) / chunk);
+  PieceTable made;  // becomes the table once complete
+  int *nseg = nullptr, *nchunk = nullptr;
+  auto alloc = [&](auto** p, size_t items) {
+    return cudaMalloc(reinterpret_cast<void**>(p), sizeof(**p) * std::max<size_t>(items, 1));
+  };
+  auto build = [&]() -> cudaError_t {
+    cudaError_t e;
+    const size_t bytes = sizeof(int) * ((size_t)nranges + 1);
+    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&nseg), bytes, s)) != cudaSuccess) return e;
+    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&nchunk), bytes, s)) != cudaSuccess) return e;
+    if ((e = launch_pieces(ptr, L.perm, n, adj, split, chunk, shift, nranges, nseg, nchunk, made, s)) != cudaSuccess)
+      return e;
+    if ((e = exclusive_scan_int(nseg, nseg, nranges, true, s)) != cudaSuccess) return e;
+    if ((e = exclusive_scan_int(nchunk, nchunk, nranges, true, s)) != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(&made.nseg, nseg + nranges, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(&made.nchunks, nchunk + nranges, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+      return e;
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+    const size_t np = 32 * (size_t)made.nseg;
+    if ((e = alloc(&made.walk, np)) != cudaSuccess || (e = alloc(&made.row, np)) != cudaSuccess ||
+        (e = alloc(&made.lo, np)) != cudaSuccess || (e = alloc(&made.hi, np)) != cudaSuccess ||
+        (e = alloc(&made.cseg, (size_t)made.nchunks + 1)) != cudaSuccess ||
+        (e = alloc(&made.cbase, made.nchunks)) != cudaSuccess || (e = alloc(&made.seg_split, made.nseg)) != cudaSuccess)
+      return e;
+    // padding: no unknown (-1), row 0, an empty list
+    if ((e = cudaMemsetAsync(made.walk, 0xFF, sizeof(int) * np, s)) != cudaSuccess) return e;
+    for (int* z : {made.row, made.lo, made.hi})
+      if ((e = cudaMemsetAsync(z, 0, sizeof(int) * np, s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(made.seg_split, 0, made.nseg, s)) != cudaSuccess) return e;
+    if ((e = launch_pieces(ptr, L.perm, n, adj, split, chunk, shift, nranges, nseg, nchunk, made, s)) != cudaSuccess)
+      return e;
+    if ((e = cudaMemcpyAsync(made.cseg + made.nchunks, &made.nseg, sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess)
+      return e;
+    return cudaStreamSynchronize(s);
+  };
+  const cudaError_t err = build();
+  for (int* b : {nseg, nchunk})
+    if (b) cudaFreeAsync(b, s);
+  if (err != cudaSuccess) {
+    free_pieces(made);
+    return map_cuda_error(err);
+  }
+  made.split = split;
+  made.chunk = chunk;
+  t = made;
+  h->device_bytes += sizeof(int) * (128 * (size_t)t.nseg + 2 * (size_t)t.nchunks + 1);
+  return SPTRSV_OK;
 }
 
 // Split table of a walk, packed on the device.
@@ -1007,7 +972,8 @@ int effective_block(const sptrsv_gb300_handle_s* h) {
 // warps, measured faster than full occupancy). Deep, narrow DAGs whose
 // dependencies stay local in the natural order (>= 96 % of the entries inside
 // blocks of 32 level widths): level order inside such blocks, one CTA per
-// block with in-block hops through shared memory. Measured on 160k-row band
+// block with in-block hops through shared memory (k_pull_block, or the importer
+// executor). Measured with the importer executor on 160k-row band
 // systems with 1-16 entries per column and bands of 100-2000 rows: blocked
 // orders won at 965-976 permille local (band 100: 2.84 vs 4.33 ms with two
 // entries, 13.1 vs 17.5 with twelve), and lost at 925-953 (band 300: 3.83 vs
@@ -1027,7 +993,9 @@ int effective_block(const sptrsv_gb300_handle_s* h) {
 // threads per SM below 1,536 unknowns per level (fewer lanes polling ahead of
 // the wave: 1M-row band 1.109 vs 1.139 ms, 500k-row band 2.21 vs 2.68 ms),
 // two up to 8,192 (4M-row power-law 1.68 vs 1.76 ms forward, 2.19 vs 2.60
-// backward), three beyond (a 4M-row band with 17,468 per level 0.51 vs 0.60).
+// backward), three beyond (a 4M-row band with 17,468 per level 0.51 vs 0.60):
+// k_pull_wsync; k_pull_ahead, which runs these walks, has a rule of its own.
+
 // One-cluster executor (k_pull_cluster, exec_cluster.cu): a single system in
 // level order with at most kClusterDeps dependencies and kClusterWidth unknowns
 // per level on average and no lists to split, whose values fit the cluster's
@@ -1421,8 +1389,8 @@ bool stage_col_major(const sptrsv_gb300_handle_s* h, int rhs, int layout, int mi
 // 1,916, 33 6,945 vs 2,195, 64 6,393 / 10,408 vs 2,035 / 2,138; 300 x 300, 8 438 vs 421;
 // but 5 432 vs 484), from 9 in FP32 (9 2,445 vs 1,692; 300 x 300, 8 328 vs 367).
 bool use_level_walk(const sptrsv_gb300_handle_s* h, const ExecConfig& c, int rhs, size_t elem) {
-  if (rhs < (elem == 8 ? 8 : 9) || rhs > 64 || !c.wsync || c.exact || !c.smem_tier || h->layout_block >= h->n || h->layout_units.empty())
-    return false;
+  if (rhs < (elem == 8 ? 8 : 9) || rhs > 64 || !c.wsync || c.exact || !c.smem_tier) return false;
+  if (h->layout_block >= h->n || h->layout_units.empty()) return false;
   return h->plan.valid && h->rhs_tile_option == 0 && planned(h, SPTRSV_OPTION_CHUNK) &&
          planned(h, SPTRSV_OPTION_CTAS_PER_SM) && c.block == 256 && c.sleep_max == 0;
 }

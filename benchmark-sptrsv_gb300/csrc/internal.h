@@ -326,6 +326,10 @@ struct SplitTable {
 int pack_blocks(int n);  // blocks the packing counts and fills
 cudaError_t launch_pack_count(const int* ptr, int n, int split, bool adj, int* count, cudaStream_t s);
 cudaError_t launch_pack_fill(const int* ptr, int n, int split, bool adj, const int* first, int* walk, cudaStream_t s);
+// pieces of k_pull_wsync_split: segments and chunks of every range of `chunk` walk
+// indices (t.walk null), then their contents from the first ones
+cudaError_t launch_pieces(const int* ptr, const int* perm, int n, bool reversed, int split, int chunk, int shift,
+                          int nranges, int* nseg, int* nchunk, const PieceTable& t, cudaStream_t s);
 template <typename T>
 cudaError_t launch_pull_ahead_split(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
                                     const SplitTable& tab, unsigned long long timeout_ns, int num_sms, cudaStream_t s,

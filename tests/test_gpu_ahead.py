@@ -96,3 +96,26 @@ def test_infinities_and_nan_reach_the_same_unknowns(cuda):
     assert np.array_equal(np.isinf(out[0]), np.isinf(out[1]))
     ok = np.isfinite(out[0])
     assert relerr(out[1][ok], out[0][ok]) <= 1e-12
+
+
+@pytest.mark.parametrize("chunk, split", [(32, 4), (33, 4), (100, 8), (256, 8), (256, 32), (1000, 5)])
+@pytest.mark.parametrize("kind, n", [("star", 33), ("star", 700), ("few", 1025), ("power", 5003), ("chain", 300)])
+def test_pieces_of_split_lists(cuda, oracle_port, kind, n, chunk, split):
+    """Pieces packed on the device for the executor that splits lists in chunks: ranges and segments of every fill,
+    chunks cut at their segment limit, both directions (the transposed walk starts with a partial chunk)."""
+    from sptrsv_gb300 import SyncFreeSolver, matgen
+    m = {"star": lambda: matgen.star(n, lower=False), "chain": lambda: matgen.chain(n, lower=False),
+         "power": lambda: matgen.power_law_band(n, 9 * n, n // 4, seed=n, lower=False),
+         "few": lambda: matgen.banded_random_lower(n, np.where(np.arange(n) % 97 == 0, 200, 2), n // 2, n,
+                                                   lower=False)}[kind]()
+    b = np.random.default_rng(n).standard_normal(m.n)
+    ref = oracle_port.solve(m.col_ptr, m.row_idx, m.val, m.n, m.substitution, b)
+    t = m.transpose()
+    tref = oracle_port.solve(t.col_ptr, t.row_idx, t.val, m.n, t.substitution, b)
+    s = SyncFreeSolver(m.col_ptr, m.row_idx, m.n, m.substitution, values=m.val, schedule=2, staged=False,
+                       warp_sync=True, order_block=2**31 - 1, chunk=chunk, split=split, wsync_batch=2, cluster=0)
+    bd = cuda.from_numpy(b).cuda()
+    for _ in range(2):
+        assert relerr(s.solve(bd).cpu().numpy(), ref) <= 1e-12
+        assert relerr(s.solve_adjoint(bd)[0].cpu().numpy(), tref) <= 1e-12
+    s.close()
