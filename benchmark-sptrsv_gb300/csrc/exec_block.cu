@@ -167,6 +167,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_pull_block(BlockArgs<T> a) {
         return loaded > k;
       };
       auto wait_loaded = [&](int k) {
+        wb.start = 0;  // the budget is a single wait's
         while (!look(k))
           if (!keep_waiting()) break;
       };
@@ -219,6 +220,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_pull_block(BlockArgs<T> a) {
         const int p = n_lo + lane, hi = n_hi, row = n_row;
         if (k + kStorers < nseg) fetch();
         bounds(k + 2 * kStorers);
+        wb.start = 0;
         while (ld_acquire_shared(&s_done) <= k)
           if (!keep_waiting()) break;
         if (fail) break;
@@ -261,6 +263,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_pull_block(BlockArgs<T> a) {
         unsigned imported[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) imported[u] = __ballot_sync(kFull, other_unit(q[u]));
+        wb.start = 0;
         while (k - ld_acquire_shared(&s_done) >= kRing)
           if (!keep_waiting()) break;
         if (fail) break;
@@ -273,6 +276,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_pull_block(BlockArgs<T> a) {
           r.src[u][lane] = src[u];
         }
         // imported dependencies come first in ready order
+        wb.start = 0;
         for (;;) {
           bool pending = false;
 #pragma unroll

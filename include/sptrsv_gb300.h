@@ -111,7 +111,9 @@ typedef enum sptrsv_option {
                                      sptrsv_info.wsync_batch reports the forward walk's value) */
   SPTRSV_OPTION_IMPORT = 19,      /* 1 (default): warp-synchronous one-rhs forward pull on a blocked
                                      layout (chunk = order block) gives each CTA an importer warp that
-                                     copies the chunk's external dependencies into shared memory */
+                                     copies the chunk's external dependencies into shared memory. Left
+                                     unset, lists of at most 4 entries take an executor with one consumer
+                                     warp per block instead */
   SPTRSV_OPTION_UNIT_PIPELINE = 20, /* warp-synchronous one-rhs forward pull on a blocked layout (chunk =
                                      order block): 1 = one consumer warp per unit reading every operand
                                      from shared memory, fed by a bulk-copy loader warp (stages of
