@@ -111,8 +111,8 @@ struct sptrsv_gb300_handle_s {
   Values<double> v64;
   Values<float> v32;
   bool staged64 = false, staged32 = false;
-  DevBuf vals;          // the values as given (CSC order), for forms staged later
-  int vals_dtype = SPTRSV_DTYPE_F64;
+  DevBuf vals;          // the values (CSC order), for forms staged later; FP32 ones widened, so that the
+                        // array's place and type stay as a captured staging found them
   // workspace
   DevBuf xw, left_sum, counters, r32, d32, stats;
   DevBuf tb, tx;  // row-major staging of column-major blocks of many right-hand sides
@@ -1158,13 +1158,7 @@ int need_forms(sptrsv_gb300_handle_s* h, unsigned forms, cudaStream_t s) {
   const int st = alloc_forms(h, V, missing);
   if (capture != cudaStreamCaptureStatusNone) CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
   ST_TRY(st);
-  if (h->vals_dtype == SPTRSV_DTYPE_F64) {
-    CUDA_TRY(launch_stage_values(h->layout, static_cast<const double*>(h->vals.p), V, missing, nullptr, s));
-  } else if constexpr (sizeof(T) == 4) {
-    CUDA_TRY(launch_stage_values(h->layout, static_cast<const float*>(h->vals.p), V, missing, nullptr, s));
-  } else {
-    return SPTRSV_ERR_STATE;  // FP64 forms of FP32 values
-  }
+  CUDA_TRY(launch_stage_values(h->layout, static_cast<const double*>(h->vals.p), V, missing, nullptr, s));
   if (capture == cudaStreamCaptureStatusNone) V.ready |= missing;
   return SPTRSV_OK;
 }
@@ -1176,10 +1170,12 @@ int need_forms(sptrsv_gb300_handle_s* h, unsigned forms, cudaStream_t s) {
 template <typename TV>
 int stage_all(sptrsv_gb300_handle_s* h, const TV* val, cudaStream_t s, bool check) {
   Values<TV>& V = values_of<TV>(h);
-  ST_TRY(ensure_buf(h, h->vals, sizeof(TV) * std::max<size_t>(h->nnz, 1), 0, s));
-  if (h->nnz > 0)
+  ST_TRY(ensure_buf(h, h->vals, sizeof(double) * std::max<size_t>(h->nnz, 1), 0, s));
+  if constexpr (sizeof(TV) == 4) {
+    CUDA_TRY(launch_cast_f2d(val, static_cast<double*>(h->vals.p), h->nnz, s));
+  } else if (h->nnz > 0) {
     CUDA_TRY(cudaMemcpyAsync(h->vals.p, val, sizeof(TV) * (size_t)h->nnz, cudaMemcpyDeviceToDevice, s));
-  h->vals_dtype = sizeof(TV) == 8 ? SPTRSV_DTYPE_F64 : SPTRSV_DTYPE_F32;
+  }
   const unsigned forms = allocated_forms(V) | FORM_DIAG | FORM_DEP_W;
   ST_TRY(alloc_forms(h, V, forms));
   h->v64.ready = h->v32.ready = 0;

@@ -471,6 +471,7 @@ cudaError_t launch_refine_fused_imported(const Layout& L, const Values<double>& 
                                          unsigned long long timeout_ns, int num_sms, cudaStream_t s,
                                          const ImportTable& im);
 cudaError_t launch_cast_d2f(const double* in, float* out, long long count, cudaStream_t s);
+cudaError_t launch_cast_f2d(const float* in, double* out, long long count, cudaStream_t s);
 cudaError_t launch_residual(const Layout& L, const Values<double>& V, int rhs, const double* b, const double* x,
                             long long si, long long sk, float* r, cudaStream_t s);
 cudaError_t launch_update(double* x, const float* d, long long count, unsigned long long* stats, bool first,
