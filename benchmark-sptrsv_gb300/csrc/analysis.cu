@@ -1127,6 +1127,14 @@ cudaError_t launch_fill_push(const int* perm, const int* iperm, const int* col_p
 }
 
 // ------------------------------------------------------------ value staging
+template <typename TV>
+__device__ __forceinline__ TV value_at(const TV* val, int i) {
+  return __ldg(val + i);
+}
+__device__ __forceinline__ float value_at(const LatestValues& val, int i) {
+  return *val.latest ? val.f32[i] : static_cast<float>(val.f64[i]);
+}
+
 // Gathers the values of one list set (out[e] = val[src[e]], scaled by the
 // reciprocal of the owning position's diagonal for SCALE: x_p = b_p/d_p - sum_j
 // w_j x_j then needs one fused multiply-add per dependency). DIAG first stages
@@ -1140,11 +1148,13 @@ cudaError_t launch_fill_push(const int* perm, const int* iperm, const int* col_p
 // its loads and stores over 32 lists: the 5M-entry band system's pull weights
 // took 66 us, the FP64 diagonal 11 more; with the copy of the values into the handle
 // and the checks, all of set_values takes 90 us now.)
-template <typename TV, typename T, bool DIAG, bool SCALE>
+template <typename Source, typename T, bool DIAG, bool SCALE>
 __global__ void __launch_bounds__(256) k_stage_lists(const int* __restrict__ ptr, const int* __restrict__ src,
-                                                     const TV* __restrict__ val, const int* __restrict__ diag_src,
-                                                     T* diag, T* rcp, T* out, int n, int* flags) {
+                                                     const Source val, const int* __restrict__ diag_src, T* diag,
+                                                     T* rcp, T* out, int n, int* flags, int* latest) {
+  using TV = decltype(value_at(val, 0));
   constexpr unsigned kFull = 0xffffffffu;
+  if (DIAG && latest && blockIdx.x == 0 && threadIdx.x == 0) *latest = sizeof(TV) == 4;
   constexpr int U = 4;
   const int lane = threadIdx.x & 31;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -1157,7 +1167,7 @@ __global__ void __launch_bounds__(256) k_stage_lists(const int* __restrict__ ptr
       start = ptr[p];
       end = ptr[p + 1];
       if (DIAG) {
-        const T d = static_cast<T>(val[diag_src[p]]);
+        const T d = static_cast<T>(value_at(val, diag_src[p]));
         r = T(1) / d;
         diag[p] = d;
         rcp[p] = r;
@@ -1175,7 +1185,7 @@ __global__ void __launch_bounds__(256) k_stage_lists(const int* __restrict__ ptr
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const unsigned e = base + u * 32 + lane;
-        v[u] = e < hi ? val[src[e]] : TV(0);
+        v[u] = e < hi ? value_at(val, src[e]) : TV(0);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -1198,39 +1208,41 @@ __global__ void __launch_bounds__(256) k_stage_lists(const int* __restrict__ ptr
   }
 }
 
-template <typename TV, typename T>
-cudaError_t launch_stage_values(const Layout& L, const TV* val, Values<T>& V, unsigned forms, int* flags,
-                                cudaStream_t s) {
+template <typename Source, typename T>
+cudaError_t launch_stage_values(const Layout& L, Source val, Values<T>& V, unsigned forms, int* flags, cudaStream_t s,
+                                int* latest) {
   if (L.n <= 0) return cudaSuccess;
   const int grid = grid_for(L.n);
   const bool dep = (forms & FORM_DEP_W) && L.ndep > 0;
   // the diagonal with the pull weights where both are wanted
   if (forms & FORM_DIAG) {
-    k_stage_lists<TV, T, true, true><<<grid, kThreads, 0, s>>>(L.dep_ptr, L.dep_src_f, val, L.diag_src, V.diag, V.rcp,
-                                                               dep ? V.dep_w : nullptr, L.n, flags);
+    k_stage_lists<Source, T, true, true><<<grid, kThreads, 0, s>>>(L.dep_ptr, L.dep_src_f, val, L.diag_src, V.diag,
+                                                                   V.rcp, dep ? V.dep_w : nullptr, L.n, flags, latest);
   } else if (dep) {
-    k_stage_lists<TV, T, false, true><<<grid, kThreads, 0, s>>>(L.dep_ptr, L.dep_src_f, val, nullptr, nullptr, V.rcp,
-                                                                V.dep_w, L.n, nullptr);
+    k_stage_lists<Source, T, false, true><<<grid, kThreads, 0, s>>>(L.dep_ptr, L.dep_src_f, val, nullptr, nullptr,
+                                                                    V.rcp, V.dep_w, L.n, nullptr, nullptr);
   }
   if (L.ndep > 0) {
     if (forms & FORM_OUT_W)
-      k_stage_lists<TV, T, false, true><<<grid, kThreads, 0, s>>>(L.out_ptr, L.out_src_f, val, nullptr, nullptr, V.rcp,
-                                                                  V.out_w, L.n, nullptr);
+      k_stage_lists<Source, T, false, true><<<grid, kThreads, 0, s>>>(L.out_ptr, L.out_src_f, val, nullptr, nullptr,
+                                                                      V.rcp, V.out_w, L.n, nullptr, nullptr);
     if (forms & FORM_DEP_VAL)
-      k_stage_lists<TV, T, false, false><<<grid, kThreads, 0, s>>>(L.dep_ptr, L.dep_src, val, nullptr, nullptr,
-                                                                   nullptr, V.dep_val, L.n, nullptr);
+      k_stage_lists<Source, T, false, false><<<grid, kThreads, 0, s>>>(L.dep_ptr, L.dep_src, val, nullptr, nullptr,
+                                                                       nullptr, V.dep_val, L.n, nullptr, nullptr);
     if (forms & FORM_OUT_VAL)
-      k_stage_lists<TV, T, false, false><<<grid, kThreads, 0, s>>>(L.out_ptr, L.out_src, val, nullptr, nullptr,
-                                                                   nullptr, V.out_val, L.n, nullptr);
+      k_stage_lists<Source, T, false, false><<<grid, kThreads, 0, s>>>(L.out_ptr, L.out_src, val, nullptr, nullptr,
+                                                                       nullptr, V.out_val, L.n, nullptr, nullptr);
   }
   return cudaGetLastError();
 }
 
-template cudaError_t launch_stage_values<double, double>(const Layout&, const double*, Values<double>&, unsigned, int*,
-                                                          cudaStream_t);
-template cudaError_t launch_stage_values<double, float>(const Layout&, const double*, Values<float>&, unsigned, int*,
-                                                         cudaStream_t);
-template cudaError_t launch_stage_values<float, float>(const Layout&, const float*, Values<float>&, unsigned, int*,
-                                                        cudaStream_t);
+template cudaError_t launch_stage_values<const double*, double>(const Layout&, const double*, Values<double>&,
+                                                                 unsigned, int*, cudaStream_t, int*);
+template cudaError_t launch_stage_values<const double*, float>(const Layout&, const double*, Values<float>&,
+                                                                unsigned, int*, cudaStream_t, int*);
+template cudaError_t launch_stage_values<const float*, float>(const Layout&, const float*, Values<float>&, unsigned,
+                                                               int*, cudaStream_t, int*);
+template cudaError_t launch_stage_values<LatestValues, float>(const Layout&, LatestValues, Values<float>&, unsigned,
+                                                              int*, cudaStream_t, int*);
 
 }  // namespace sptrsv

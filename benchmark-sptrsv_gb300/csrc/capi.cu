@@ -111,8 +111,10 @@ struct sptrsv_gb300_handle_s {
   Values<double> v64;
   Values<float> v32;
   bool staged64 = false, staged32 = false;
-  DevBuf vals;          // the values (CSC order), for forms staged later; FP32 ones widened, so that the
-                        // array's place and type stay as a captured staging found them
+  // the last values given in each precision (CSC order), for forms staged later; their
+  // places stay as a captured staging found them. flags[1]: the precision given last
+  // (1 FP32), as the stream's work sees it
+  DevBuf vals64, vals32;
   // workspace
   DevBuf xw, left_sum, counters, r32, d32, stats;
   DevBuf tb, tx;  // row-major staging of column-major blocks of many right-hand sides
@@ -242,6 +244,7 @@ void free_values(Values<T>& V) {
   dev_free(&V.diag);
   dev_free(&V.rcp);
   V.ready = 0;
+  V.kept = ~0u;
 }
 
 void free_analysis(sptrsv_gb300_handle_s* h) {
@@ -286,11 +289,28 @@ void free_buf(DevBuf& b) {
   b = DevBuf();
 }
 
+cudaError_t is_capturing(cudaStream_t s, bool* capturing) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(s, &status);
+  *capturing = status != cudaStreamCaptureStatusNone;
+  return e;
+}
+
+// Lets allocations through while a stream is captured: an allocation is no stream
+// operation, and relaxed mode allows it.
+struct AllowAllocations {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  AllowAllocations() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~AllowAllocations() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  AllowAllocations(const AllowAllocations&) = delete;
+};
+
 int ensure_buf(sptrsv_gb300_handle_s* h, DevBuf& b, size_t bytes, int fill_zero, cudaStream_t s) {
   if (b.bytes >= bytes && b.p) return SPTRSV_OK;
   // Growing: make sure nothing in flight still uses the old buffer.
-  CUDA_TRY(cudaStreamSynchronize(s));
+  if (b.p || fill_zero) CUDA_TRY(cudaStreamSynchronize(s));
   free_buf(b);
+  AllowAllocations allow;
   CUDA_TRY(cudaMalloc(&b.p, bytes));
   b.bytes = bytes;
   h->device_bytes += bytes;
@@ -1132,6 +1152,7 @@ unsigned allocated_forms(const Values<T>& V) {
 template <typename T>
 int alloc_forms(sptrsv_gb300_handle_s* h, Values<T>& V, unsigned forms) {
   const Layout& L = h->layout;
+  AllowAllocations allow;
   if ((forms & FORM_DIAG) && !V.diag) ST_TRY(dev_alloc(h, &V.diag, L.n));
   if ((forms & FORM_DIAG) && !V.rcp) ST_TRY(dev_alloc(h, &V.rcp, L.n));
   if ((forms & FORM_DEP_W) && !V.dep_w) ST_TRY(dev_alloc(h, &V.dep_w, L.ndep));
@@ -1141,25 +1162,43 @@ int alloc_forms(sptrsv_gb300_handle_s* h, Values<T>& V, unsigned forms) {
   return SPTRSV_OK;
 }
 
+// Which forms hold the current values is known here only as far as the work was
+// issued from here. A captured update runs at every replay, unseen, and refreshes the
+// forms it was captured with: from then on only those (Values::kept) are ever taken
+// as ready, and a later call stages any other form it needs again. Inside a capture
+// nothing becomes ready: the graph has yet to run.
+template <typename T>
+void update_recorded(Values<T>& V, unsigned forms, bool capturing) {
+  if (capturing) V.kept &= forms;
+  V.ready = (capturing ? V.ready : forms) & V.kept;
+}
+
 // The given forms of the staged values, in precision T, ready for the work that
-// follows on `s`: those not staged since the last set of values are staged now
-// from the handle's copy. Inside a stream capture the staging becomes part of
-// the graph (and is not recorded as done here, since it runs at replay).
+// follows on `s`: those that are not are staged now from the handle's copy (FP32
+// forms from the copy of the precision that the stream's work updated last). Inside
+// a stream capture the staging becomes part of the graph.
 template <typename T>
 int need_forms(sptrsv_gb300_handle_s* h, unsigned forms, cudaStream_t s) {
   Values<T>& V = values_of<T>(h);
   const unsigned missing = (forms | FORM_DIAG) & ~V.ready;
   if (!missing) return SPTRSV_OK;
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  CUDA_TRY(cudaStreamIsCapturing(s, &capture));
-  // an allocation is no stream operation: relaxed mode lets it through a capture
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  if (capture != cudaStreamCaptureStatusNone) CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
-  const int st = alloc_forms(h, V, missing);
-  if (capture != cudaStreamCaptureStatusNone) CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
-  ST_TRY(st);
-  CUDA_TRY(launch_stage_values(h->layout, static_cast<const double*>(h->vals.p), V, missing, nullptr, s));
-  if (capture == cudaStreamCaptureStatusNone) V.ready |= missing;
+  bool capturing = false;
+  CUDA_TRY(is_capturing(s, &capturing));
+  ST_TRY(alloc_forms(h, V, missing));
+  const double* wide = static_cast<const double*>(h->vals64.p);
+  if constexpr (sizeof(T) == 8) {
+    CUDA_TRY(launch_stage_values(h->layout, wide, V, missing, nullptr, s));
+  } else {
+    if (capturing || V.kept != ~0u) {  // a replay may turn to either copy
+      const size_t items = std::max<size_t>(h->nnz, 1);
+      ST_TRY(ensure_buf(h, h->vals64, sizeof(double) * items, 0, s));
+      ST_TRY(ensure_buf(h, h->vals32, sizeof(float) * items, 0, s));
+      wide = static_cast<const double*>(h->vals64.p);
+    }
+    const LatestValues latest{wide, static_cast<const float*>(h->vals32.p), h->flags + 1};
+    CUDA_TRY(launch_stage_values(h->layout, latest, V, missing, nullptr, s));
+  }
+  if (!capturing) V.ready |= missing & V.kept;
   return SPTRSV_OK;
 }
 
@@ -1168,41 +1207,39 @@ int need_forms(sptrsv_gb300_handle_s* h, unsigned forms, cudaStream_t s) {
 // until one does. (Staging all forms in both precisions took 385 us for the
 // 5M-entry band system, of a 2.4 ms training step.)
 template <typename TV>
-int stage_all(sptrsv_gb300_handle_s* h, const TV* val, cudaStream_t s, bool check) {
+int stage_all(sptrsv_gb300_handle_s* h, const TV* val, cudaStream_t s, bool check, bool capturing) {
   Values<TV>& V = values_of<TV>(h);
-  ST_TRY(ensure_buf(h, h->vals, sizeof(double) * std::max<size_t>(h->nnz, 1), 0, s));
-  if constexpr (sizeof(TV) == 4) {
-    CUDA_TRY(launch_cast_f2d(val, static_cast<double*>(h->vals.p), h->nnz, s));
-  } else if (h->nnz > 0) {
-    CUDA_TRY(cudaMemcpyAsync(h->vals.p, val, sizeof(TV) * (size_t)h->nnz, cudaMemcpyDeviceToDevice, s));
-  }
+  DevBuf& copy = sizeof(TV) == 8 ? h->vals64 : h->vals32;
+  ST_TRY(ensure_buf(h, copy, sizeof(TV) * std::max<size_t>(h->nnz, 1), 0, s));
+  if (h->nnz > 0)
+    CUDA_TRY(cudaMemcpyAsync(copy.p, val, sizeof(TV) * (size_t)h->nnz, cudaMemcpyDeviceToDevice, s));
   const unsigned forms = allocated_forms(V) | FORM_DIAG | FORM_DEP_W;
   ST_TRY(alloc_forms(h, V, forms));
-  h->v64.ready = h->v32.ready = 0;
+  if (!capturing) V.ready = h->v32.ready = 0;
   volatile int* flags = check ? h->host_pinned + 3 : nullptr;
   if (check) *flags = 0;
-  CUDA_TRY(launch_stage_values(h->layout, val, V, forms, const_cast<int*>(flags), s));
+  CUDA_TRY(launch_stage_values(h->layout, val, V, forms, const_cast<int*>(flags), s, h->flags + 1));
   if (check) {
     CUDA_TRY(cudaStreamSynchronize(s));
     if (*flags & SF_ZERO_DIAG) return SPTRSV_ERR_BAD_STRUCTURE;
   }
-  V.ready = forms;
+  update_recorded(V, forms, capturing);
   return SPTRSV_OK;
 }
 
 int stage_values(sptrsv_gb300_handle_s* h, const void* d_val, int dtype, cudaStream_t s, bool check) {
   if (dtype != SPTRSV_DTYPE_F64 && dtype != SPTRSV_DTYPE_F32) return SPTRSV_ERR_INVALID;
+  bool capturing = false;
+  CUDA_TRY(is_capturing(s, &capturing));
   h->wsplit_ok = false;
   if (dtype == SPTRSV_DTYPE_F64) {
-    ST_TRY(stage_all(h, static_cast<const double*>(d_val), s, check));
+    ST_TRY(stage_all(h, static_cast<const double*>(d_val), s, check, capturing));
     const unsigned again = allocated_forms(h->v32);
-    if (again) {
-      CUDA_TRY(launch_stage_values(h->layout, static_cast<const double*>(d_val), h->v32, again, nullptr, s));
-      h->v32.ready = again;
-    }
+    CUDA_TRY(launch_stage_values(h->layout, static_cast<const double*>(d_val), h->v32, again, nullptr, s));
+    update_recorded(h->v32, again, capturing);
     h->staged64 = h->staged32 = true;
   } else {
-    ST_TRY(stage_all(h, static_cast<const float*>(d_val), s, check));
+    ST_TRY(stage_all(h, static_cast<const float*>(d_val), s, check, capturing));
     h->staged32 = true;
     h->staged64 = false;
   }
@@ -1609,7 +1646,8 @@ int sptrsv_gb300_create(sptrsv_handle_t* handle) {
   cudaError_t e = cudaGetDevice(&h->device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device);
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&h->ctl), sizeof(DeviceCtl));
-  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&h->flags), sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&h->flags), 2 * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(h->flags, 0, 2 * sizeof(int));
   if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&h->host_pinned), 4 * sizeof(int));
   if (e == cudaSuccess) e = init_ctl(h, nullptr);
   if (e != cudaSuccess) {
@@ -1637,7 +1675,8 @@ int sptrsv_gb300_destroy(sptrsv_handle_t h) {
   free_buf(h->tx);
   free_buf(h->c0);
   free_buf(h->wsplit);
-  free_buf(h->vals);
+  free_buf(h->vals64);
+  free_buf(h->vals32);
   if (h->ctl) cudaFree(h->ctl);
   if (h->flags) cudaFree(h->flags);
   if (h->host_pinned) cudaFreeHost(h->host_pinned);

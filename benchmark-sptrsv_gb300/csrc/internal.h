@@ -190,6 +190,13 @@ struct Values {
   T* diag = nullptr;     // [n]
   T* rcp = nullptr;      // [n] correctly rounded 1/diag
   unsigned ready = 0;    // forms that hold the current values
+  unsigned kept = ~0u;   // forms that every captured update of the values refreshes
+};
+// The values of the precision given last, in FP32: f32[i] where *latest is set, else f64[i].
+struct LatestValues {
+  const double* f64;
+  const float* f32;
+  const int* latest;
 };
 
 // Independent triangles sharing one index space (a batch): unknown c belongs
@@ -287,9 +294,11 @@ cudaError_t launch_rank_lists(const int* ptr, const int* key, const int* src, in
 bool transpose_by_rank(int longest_row);
 cudaError_t launch_transpose_pattern(const int* col_ptr, const int* row_idx, const int* row_ptr, int n, int nnz,
                                      int* col_of, int* src_out, int* col_out, cudaStream_t s);
-template <typename TV, typename T>
-cudaError_t launch_stage_values(const Layout& L, const TV* val, Values<T>& V, unsigned forms, int* flags,
-                                cudaStream_t s);
+// The given forms of V from `val` (an array, or LatestValues); `latest` (or null) is set to
+// the array's precision along with the diagonal.
+template <typename Source, typename T>
+cudaError_t launch_stage_values(const Layout& L, Source val, Values<T>& V, unsigned forms, int* flags,
+                                cudaStream_t s, int* latest = nullptr);
 
 // ---------------------------------------------------------------- execution
 // Transposed (adjoint) solve request: optional fused gradient w.r.t. the values.
@@ -471,7 +480,6 @@ cudaError_t launch_refine_fused_imported(const Layout& L, const Values<double>& 
                                          unsigned long long timeout_ns, int num_sms, cudaStream_t s,
                                          const ImportTable& im);
 cudaError_t launch_cast_d2f(const double* in, float* out, long long count, cudaStream_t s);
-cudaError_t launch_cast_f2d(const float* in, double* out, long long count, cudaStream_t s);
 cudaError_t launch_residual(const Layout& L, const Values<double>& V, int rhs, const double* b, const double* x,
                             long long si, long long sk, float* r, cudaStream_t s);
 cudaError_t launch_update(double* x, const float* d, long long count, unsigned long long* stats, bool first,

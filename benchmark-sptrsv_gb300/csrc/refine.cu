@@ -114,11 +114,6 @@ cudaError_t launch_cast_d2f(const double* in, float* out, long long count, cudaS
   k_cast<double, float><<<grid_1d(count), 256, 0, s>>>(in, out, count);
   return cudaGetLastError();
 }
-cudaError_t launch_cast_f2d(const float* in, double* out, long long count, cudaStream_t s) {
-  if (count <= 0) return cudaSuccess;
-  k_cast<float, double><<<grid_1d(count), 256, 0, s>>>(in, out, count);
-  return cudaGetLastError();
-}
 
 cudaError_t launch_residual(const Layout& L, const Values<double>& V, int rhs, const double* b, const double* x,
                             long long si, long long sk, float* r, cudaStream_t s) {
