@@ -1233,6 +1233,8 @@ cudaError_t launch_stage_values(const Layout& L, Source val, Values<T>& V, unsig
       k_stage_lists<Source, T, false, false><<<grid, kThreads, 0, s>>>(L.out_ptr, L.out_src, val, nullptr, nullptr,
                                                                        nullptr, V.out_val, L.n, nullptr, nullptr);
   }
+  if constexpr (sizeof(T) == 8)
+    if (forms & FORM_DEP_SPLIT) return launch_split_weights(V.dep_w, L.ndep, V.dep_split, s);
   return cudaGetLastError();
 }
 

@@ -119,8 +119,6 @@ struct sptrsv_gb300_handle_s {
   DevBuf xw, left_sum, counters, r32, d32, stats;
   DevBuf tb, tx;  // row-major staging of column-major blocks of many right-hand sides
   DevBuf c0;      // unit pipeline: first term b/d of every position
-  DevBuf wsplit;  // fused refinement in double-float: (hi, lo) float pairs of the FP64 weights
-  bool wsplit_ok = false;
   DeviceCtl* ctl = nullptr;
   int* flags = nullptr;
   int* host_pinned = nullptr;  // 4 ints the device can write: [0] DeviceCtl::host_code, [1] structure
@@ -241,6 +239,7 @@ void free_values(Values<T>& V) {
   dev_free(&V.dep_w);
   dev_free(&V.out_w);
   dev_free(&V.out_val);
+  dev_free(&V.dep_split);
   dev_free(&V.diag);
   dev_free(&V.rcp);
   V.ready = 0;
@@ -279,7 +278,6 @@ void free_analysis(sptrsv_gb300_handle_s* h) {
   free_values(h->v64);
   free_values(h->v32);
   h->staged64 = h->staged32 = false;
-  h->wsplit_ok = false;
   h->analysed = false;
   h->layout_block = -1;
 }
@@ -401,7 +399,6 @@ int build_layout(sptrsv_gb300_handle_s* h, int block, cudaStream_t s) {
   free_values(h->v64);
   free_values(h->v32);
   h->staged64 = h->staged32 = false;
-  h->wsplit_ok = false;
   h->dep_cnt_host.clear();
   h->out_cnt_host.clear();
   Layout& L = h->layout;
@@ -1146,7 +1143,8 @@ Values<float>& values_of<float>(sptrsv_gb300_handle_s* h) { return h->v32; }
 template <typename T>
 unsigned allocated_forms(const Values<T>& V) {
   return (V.rcp ? FORM_DIAG : 0u) | (V.dep_w ? FORM_DEP_W : 0u) | (V.out_w ? FORM_OUT_W : 0u) |
-         (V.dep_val ? FORM_DEP_VAL : 0u) | (V.out_val ? FORM_OUT_VAL : 0u);
+         (V.dep_val ? FORM_DEP_VAL : 0u) | (V.out_val ? FORM_OUT_VAL : 0u) |
+         (V.dep_split ? FORM_DEP_SPLIT : 0u);
 }
 
 template <typename T>
@@ -1159,6 +1157,7 @@ int alloc_forms(sptrsv_gb300_handle_s* h, Values<T>& V, unsigned forms) {
   if ((forms & FORM_OUT_W) && !V.out_w) ST_TRY(dev_alloc(h, &V.out_w, L.ndep));
   if ((forms & FORM_DEP_VAL) && !V.dep_val) ST_TRY(dev_alloc(h, &V.dep_val, L.ndep));
   if ((forms & FORM_OUT_VAL) && !V.out_val) ST_TRY(dev_alloc(h, &V.out_val, L.ndep));
+  if ((forms & FORM_DEP_SPLIT) && !V.dep_split) ST_TRY(dev_alloc(h, &V.dep_split, L.ndep));
   return SPTRSV_OK;
 }
 
@@ -1231,7 +1230,6 @@ int stage_values(sptrsv_gb300_handle_s* h, const void* d_val, int dtype, cudaStr
   if (dtype != SPTRSV_DTYPE_F64 && dtype != SPTRSV_DTYPE_F32) return SPTRSV_ERR_INVALID;
   bool capturing = false;
   CUDA_TRY(is_capturing(s, &capturing));
-  h->wsplit_ok = false;
   if (dtype == SPTRSV_DTYPE_F64) {
     ST_TRY(stage_all(h, static_cast<const double*>(d_val), s, check, capturing));
     const unsigned again = allocated_forms(h->v32);
@@ -1674,7 +1672,6 @@ int sptrsv_gb300_destroy(sptrsv_handle_t h) {
   free_buf(h->tb);
   free_buf(h->tx);
   free_buf(h->c0);
-  free_buf(h->wsplit);
   free_buf(h->vals64);
   free_buf(h->vals32);
   if (h->ctl) cudaFree(h->ctl);
@@ -2288,19 +2285,11 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
       }
       CUDA_TRY(cudaEventRecord(h->ev_exec[0], s));
     }
-    ST_TRY(need_forms<double>(h, FORM_DEP_W, s));
-    if (h->fused_refine != 2) ST_TRY(need_forms<float>(h, FORM_DEP_W, s));
-    const float2* wsplit = nullptr;
-    if (h->fused_refine == 2) {
-      // the residual in double-float: (hi, lo) pairs of the FP64 weights, once per staging
-      const long long ndep = h->layout.ndep;
-      if (!h->wsplit_ok) {
-        ST_TRY(ensure_buf(h, h->wsplit, sizeof(float2) * (size_t)(ndep + 16), 0, s));
-        CUDA_TRY(launch_split_weights(h->v64.dep_w, ndep, static_cast<float2*>(h->wsplit.p), s));
-        h->wsplit_ok = true;
-      }
-      wsplit = static_cast<const float2*>(h->wsplit.p);
-    }
+    // the residual in double-float takes the FP64 weights as (hi, lo) float pairs
+    const bool pairs = h->fused_refine == 2;
+    ST_TRY(need_forms<double>(h, pairs ? FORM_DEP_W | FORM_DEP_SPLIT : FORM_DEP_W, s));
+    if (!pairs) ST_TRY(need_forms<float>(h, FORM_DEP_W, s));
+    const float2* wsplit = pairs ? h->v64.dep_split : nullptr;
     // one right-hand side on a blocked layout: the importer-warp variant (as the
     // plain solve's k_pull_wsync_imp) keeps the cross-block polls out of the
     // consumer warps' lockstep iterations

@@ -179,13 +179,15 @@ enum ValueForm : unsigned {
   FORM_DEP_W = 2,    // dep_w
   FORM_OUT_W = 4,    // out_w
   FORM_DEP_VAL = 8,  // dep_val
-  FORM_OUT_VAL = 16  // out_val
+  FORM_OUT_VAL = 16, // out_val
+  FORM_DEP_SPLIT = 32  // dep_split (FP64 only; with FORM_DEP_W)
 };
 template <typename T>
 struct Values {
   T* dep_val = nullptr;  // [ndep]
   T* dep_w = nullptr;    // [ndep] values scaled by the reciprocal of the row's diagonal (ready order)
   T* out_val = nullptr;  // [ndep]
+  float2* dep_split = nullptr;  // [ndep] dep_w as (hi, lo) float pairs, for refinement in double-float
   T* out_w = nullptr;    // [ndep] values scaled by the reciprocal of the owning position's diagonal (ready order)
   T* diag = nullptr;     // [n]
   T* rcp = nullptr;      // [n] correctly rounded 1/diag

@@ -99,6 +99,8 @@ class _System:
                  "push": (lambda: with_option(_lib.OPTION_SCHEDULE, 1, lambda: s.solve(self.bd)), ref, 1e-12),
                  "exact adjoint": (lambda: with_option(_lib.OPTION_EXACT, 1, lambda: s.solve_adjoint(self.bd)[0]), tref,
                                    1e-12),
+                 "refine": (lambda: s.solve_refine(self.bd)[0], ref, 1e-10),
+                 "two steps": (lambda: s.solve_refine(self.bd, tol=0.0, max_iter=2)[0], ref, 1e-10),
                  "solve f32": (lambda: s.solve(self.bf), ref, 1e-5),
                  "adjoint f32": (lambda: s.solve_adjoint(self.bf)[0], tref, 1e-5)}
         for name in names:
@@ -106,11 +108,11 @@ class _System:
             assert relerr(call().cpu().numpy(), r) <= tol, name
 
 
-F64 = ("solve", "adjoint", "exact", "exact adjoint", "push", "solve f32", "adjoint f32")
+F64 = ("solve", "adjoint", "exact", "exact adjoint", "push", "refine", "two steps", "solve f32", "adjoint f32")
 F32 = ("solve f32", "adjoint f32")
 
 
-@pytest.mark.parametrize("names", [F64, F64[::-1], ("adjoint",), ("solve f32",), ("exact adjoint",)])
+@pytest.mark.parametrize("names", [F64, F64[::-1], ("adjoint",), ("solve f32",), ("exact adjoint",), ("refine",), ("two steps",)])
 @pytest.mark.parametrize("n, lower", [(33, True), (3000, False)])
 def test_replayed_update_reaches_every_form(cuda, oracle_port, own_stream, n, lower, names):
     m = _band(n, lower)
@@ -188,3 +190,23 @@ def test_single_precision_update_first_seen_by_a_capture(cuda, oracle_port, own_
             g.replay()
             sy.check(wide, ("adjoint", "exact"))
     sy.s.check()
+
+
+@pytest.mark.parametrize("rhs, steps", [(1, 1), (1, 2), (8, 1)])
+def test_refinement_graph_follows_new_values(cuda, oracle_port, rhs, steps):
+    from sptrsv_gb300 import SyncFreeSolver
+    m = _band(4000)
+    rng = np.random.default_rng(rhs)
+    b = rng.standard_normal((m.n, rhs))
+    s = SyncFreeSolver(m.col_ptr, m.row_idx, m.n, m.substitution, values=m.val)
+    bd = cuda.from_numpy(b).cuda()
+    x = cuda.empty_like(bd)
+    g = s.graph(bd, x, kind=1, count=steps)
+    for _ in range(2):
+        val = m.val * rng.uniform(0.9, 1.1, m.nnz)
+        s.set_values(val)
+        g.replay()
+        s.check()
+        ref = oracle_port.solve(m.col_ptr, m.row_idx, val, m.n, m.substitution, b)
+        assert relerr(x.cpu().numpy(), ref) <= 1e-10
+    g.close()
