@@ -1377,7 +1377,7 @@ bool use_block(const sptrsv_gb300_handle_s* h, const ExecConfig& c, int longest)
   int width = 0;
   for (size_t i = 1; i < h->layout_units.size(); ++i)
     width = std::max(width, h->layout_units[i] - h->layout_units[i - 1]);
-  return block_smem_bytes<T>(width, longest) <= 226 * 1024;
+  return block_smem_bytes<T>(width, longest) <= kSharedLimit;
 }
 
 // Units of work per level (dependencies plus 4 per unknown) up to which split

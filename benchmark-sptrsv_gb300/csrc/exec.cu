@@ -1313,10 +1313,8 @@ cudaError_t launch_persistent(K kernel, const ExecArgs<int>*, int, size_t, int, 
 
 template <typename T, typename K>
 cudaError_t run(K kernel, const ExecArgs<T>& a, int block, size_t smem, int num_sms, cudaStream_t s) {
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = allow_shared(kernel, smem);
+  if (e != cudaSuccess) return e;
   const int grid = persistent_grid(kernel, block, smem, num_sms, a.nchunks, a.ctas_per_sm);
   kernel<<<grid, block, smem, s>>>(a);
   return cudaGetLastError();

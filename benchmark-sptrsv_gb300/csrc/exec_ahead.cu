@@ -242,7 +242,7 @@ cudaError_t launch_pull_ahead(const Layout& L, const Values<T>& V, const VecView
   a.timeout_ns = timeout_ns;
   const size_t smem = (size_t)(block / 32) * (32 * sizeof(T) + 2 * cap * (sizeof(T) + sizeof(int)));
   auto kernel = one ? k_pull_ahead<T, false, 1> : (adj ? k_pull_ahead<T, true, 2> : k_pull_ahead<T, false, 2>);
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_shared(kernel, smem);
   if (e != cudaSuccess) return e;
   int per = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, block, smem);

@@ -254,8 +254,7 @@ cudaError_t launch_ahead_multi(AheadMultiArgs<T>& a, int avg, bool narrow, int n
     // twice the average chunk's lists (longer ones read the rest from global memory)
     a.cap = walk ? 0 : std::min(1024, std::max(64, (2 * avg * unknowns / 32 + 31) / 32 * 32));
     const size_t smem = (size_t)256 * r * sizeof(T) + (size_t)2 * a.cap * (sizeof(T) + sizeof(int));
-    cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_shared(kernel, smem);
     if (e != cudaSuccess) return e;
     int per = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 256, smem);

@@ -388,7 +388,7 @@ cudaError_t launch_pull_ahead_split(const Layout& L, const Values<T>& V, const V
   constexpr int block = 256;
   const size_t smem = (size_t)(block / 32) * (32 * sizeof(T) + 2 * a.cap * (sizeof(T) + sizeof(int)));
   auto kernel = adj ? k_pull_ahead_split<T, true> : k_pull_ahead_split<T, false>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_shared(kernel, smem);
   if (e != cudaSuccess) return e;
   const int grid = std::min(num_sms, (a.nseg + block / 32 - 1) / (block / 32));
   kernel<<<grid, block, smem, s>>>(a);

@@ -522,7 +522,7 @@ cudaError_t launch_pull_block(const Layout& L, const Values<T>& V, const VecView
   a.timeout_ns = timeout_ns;
   const size_t smem = block_smem_bytes<T>(units.width, longest);
   auto run = [&](auto kernel) -> cudaError_t {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_shared(kernel, smem);
     if (e != cudaSuccess) return e;
     kernel<<<std::min(num_sms, a.nunits), kBlockThreads, smem, s>>>(a);
     return cudaGetLastError();

@@ -721,10 +721,8 @@ __global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a, const int* w
 template <int G, int RPL, int UD, bool DF>
 cudaError_t run_refine1(const RefineArgs& a, int block, size_t smem, int num_sms, cudaStream_t s) {
   auto kernel = k_pull_refine1<G, RPL, UD, DF>;
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = allow_shared(kernel, smem);
+  if (e != cudaSuccess) return e;
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
   if (per_sm < 1) per_sm = 1;
@@ -825,8 +823,7 @@ cudaError_t launch_refine_ahead(const Layout& L, const Values<double>& v64, int 
     // twice the average chunk's lists (longer ones read the rest from global memory)
     a.cap = walk ? 0 : std::min(g == 1 ? 4096 : 1024, std::max(64, (2 * avg * unknowns / 32 + 31) / 32 * 32));
     const size_t smem = (size_t)256 * r * 8 + (size_t)2 * a.cap * 12;
-    cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_shared(kernel, smem);
     if (e != cudaSuccess) return e;
     int per = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 256, smem);
@@ -892,10 +889,8 @@ cudaError_t launch_refine_fused_imported(const Layout& L, const Values<double>& 
   const size_t smem = (size_t)(im.width + im.max_imports) * sizeof(unsigned long long);
   const int block = cfg.block + 32;
   auto launch = [&](auto kernel) -> cudaError_t {
-    if (smem > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_shared(kernel, smem);
+    if (e != cudaSuccess) return e;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
     if (per_sm < 1) per_sm = 1;

@@ -281,10 +281,8 @@ template <typename T, bool EXACT, bool ADJ>
 cudaError_t run_staged(const StagedArgs<T>& a, int block, int ctas_per_sm, int num_sms, cudaStream_t s) {
   const size_t smem = (size_t)a.stages * (stage_bytes<T>(a.cmax, a.emax) + (a.smem_tier ? sizeof(T) * (size_t)a.cmax : 0));
   auto kernel = k_pull_staged<T, EXACT, ADJ>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = allow_shared(kernel, smem);
+  if (e != cudaSuccess) return e;
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
   if (per_sm < 1) return cudaErrorInvalidConfiguration;

@@ -327,10 +327,8 @@ __global__ void __launch_bounds__(96) k_pull_unit(UnitArgs<T> a) {
 template <typename T, int U>
 cudaError_t run_unit(const UnitArgs<T>& a, size_t smem, int num_sms, cudaStream_t s) {
   auto kernel = k_pull_unit<T, U>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = allow_shared(kernel, smem);
+  if (e != cudaSuccess) return e;
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 96, smem);
   if (per_sm < 1) per_sm = 1;

@@ -303,6 +303,17 @@ cudaError_t launch_stage_values(const Layout& L, Source val, Values<T>& V, unsig
                                 cudaStream_t s, int* latest = nullptr);
 
 // ---------------------------------------------------------------- execution
+// Dynamic shared memory that a launch of any executor may ask for: the device's
+// limit (227 KB on sm_103) less 1 KB for static arrays.
+constexpr size_t kSharedLimit = 226 * 1024;
+// Lets a launch of `kernel` use `smem` bytes. The attribute belongs to the function,
+// not to a handle, so every launch sets the same value: one that depended on the
+// system would be lowered by another thread's handle between this and the launch.
+template <typename Kernel>
+cudaError_t allow_shared(Kernel kernel, size_t smem) {
+  if (smem <= 48 * 1024) return cudaSuccess;  // allowed as it is
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSharedLimit));
+}
 // Transposed (adjoint) solve request: optional fused gradient w.r.t. the values.
 template <typename T>
 struct AdjointArgs {
