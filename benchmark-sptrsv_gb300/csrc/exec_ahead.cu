@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead(AheadArgs<T> a) {
       else first();
     }
     unsigned idle = 0u;
+    int seen = 0;
     WaitBudget wb(a.timeout_ns);
     while (!__all_sync(kFull, done)) {
       Bits bits0[1], bits1[1];
@@ -195,8 +196,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead(AheadArgs<T> a) {
         if (left <= 0) publish();
       }
       if ((++idle & 255u) == 0u) {
-        if (!wb.poll(a.ctl, p)) fail = true;
-        if (__any_sync(kFull, fail)) {
+        if (!lockstep_wait(wb, left, seen, a.ctl, p)) {
           fail = true;
           break;
         }

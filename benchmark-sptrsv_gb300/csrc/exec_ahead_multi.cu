@@ -197,6 +197,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, i
     }
     bool fail = false;
     unsigned idle = 0u;
+    int seen = 0;
     WaitBudget wb(a.timeout_ns);
     while (!__all_sync(kFull, done)) {
       Bits bits[R];
@@ -219,8 +220,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead_multi(AheadMultiArgs<T> a, i
         }
       }
       if ((++idle & 255u) == 0u) {
-        if (!wb.poll(a.ctl, p)) fail = true;
-        if (__any_sync(kFull, fail)) {
+        if (!lockstep_wait(wb, left - done, seen, a.ctl, p)) {
           fail = true;
           break;
         }

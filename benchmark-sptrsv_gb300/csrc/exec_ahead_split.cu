@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead_split(SplitArgs<T> a) {
       }
     }
     unsigned idle = 0u, waiting = multi;  // split unknowns not yet published
+    int seen = 0;
     WaitBudget wb(a.timeout_ns);
     while (!__all_sync(kFull, done)) {
       Bits bits0[1], bits1[1];
@@ -268,8 +269,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead_split(SplitArgs<T> a) {
         }
       }
       if ((++idle & 255u) == 0u) {
-        if (!wb.poll(a.ctl, p)) fail = true;
-        if (__any_sync(kFull, fail)) {
+        if (!lockstep_wait(wb, left, seen, a.ctl, p)) {
           fail = true;
           break;
         }

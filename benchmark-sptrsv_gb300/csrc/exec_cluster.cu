@@ -202,6 +202,7 @@ __global__ void __launch_bounds__(512) k_pull_cluster(ClusterArgs<T> a) {
       if (left > 0) next(++e);
     }
     unsigned idle = 0u;
+    int seen = 0;
     WaitBudget wb(a.timeout_ns);
     while (!__all_sync(0xffffffffu, done)) {
       const Bits bits = poll_word(addr, remote, mine, !done, T(0));
@@ -220,8 +221,7 @@ __global__ void __launch_bounds__(512) k_pull_cluster(ClusterArgs<T> a) {
         }
       }
       if ((++idle & 255u) == 0u) {
-        if (!wb.poll(a.ctl, p)) fail = true;
-        if (__any_sync(0xffffffffu, fail)) {
+        if (!lockstep_wait(wb, left - done, seen, a.ctl, p)) {
           fail = true;
           break;
         }

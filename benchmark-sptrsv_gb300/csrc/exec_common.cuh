@@ -14,6 +14,16 @@ __device__ __forceinline__ void copy_async(unsigned dst, const V* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 
+// Wait check of a warp's lockstep loop, once in 256 iterations: `left` is what a lane
+// still has to consume. While any lane has consumed something since the last check
+// the warp was not waiting, however long its lists, and the budget starts over. False
+// (in every lane) once the wait must be abandoned.
+__device__ __forceinline__ bool lockstep_wait(WaitBudget& wb, int left, int& seen, DeviceCtl* ctl, int where) {
+  if (__any_sync(0xffffffffu, left != seen)) wb.start = 0;
+  seen = left;
+  return !__any_sync(0xffffffffu, !wb.poll(ctl, where));
+}
+
 // Claim the next chunk for this CTA (uniform across the CTA).
 __device__ __forceinline__ unsigned next_chunk(DeviceCtl* ctl, unsigned nchunks, unsigned* s_chunk) {
   if (threadIdx.x == 0) *s_chunk = ctl_failed(ctl) ? nchunks : atomicAdd(&ctl->ticket, 1u);

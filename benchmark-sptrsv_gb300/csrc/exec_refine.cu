@@ -664,6 +664,7 @@ __global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a, const int* w
     }
     bool fail = false;
     unsigned idle = 0u;
+    int seen = 0;
     WaitBudget wb(a.timeout_ns);
     while (!__all_sync(kFull, done)) {
       Bits bits[R];
@@ -689,8 +690,7 @@ __global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a, const int* w
         }
       }
       if ((++idle & 255u) == 0u) {
-        if (!wb.poll(a.ctl, p)) fail = true;
-        if (__any_sync(kFull, fail)) {
+        if (!lockstep_wait(wb, left - done, seen, a.ctl, p)) {
           fail = true;
           break;
         }
