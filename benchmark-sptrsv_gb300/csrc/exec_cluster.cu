@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(512) k_pull_cluster(ClusterArgs<T> a) {
   stage(warp, 0);
   asm volatile("cp.async.commit_group;" ::: "memory");
   fetch(warp + nwarps);
+  __syncwarp();  // the cluster barrier's aligned form takes whole warps
   cluster_sync();
   bool fail = false;
   int buf = 0;
