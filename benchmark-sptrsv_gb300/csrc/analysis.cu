@@ -918,7 +918,7 @@ __global__ void __launch_bounds__(kLevelChunk) k_levels_pull(const int* __restri
         work = __any_sync(kFull, !done);
       } else {
         if (idle >= 16u) __nanosleep(kLevelNap);
-        if ((++idle & 15u) == 0u && __any_sync(kFull, !wb.poll(ctl, r))) {
+        if ((++idle & 15u) == 0u && __any_sync(kFull, !wb.poll<true>(ctl, r))) {
           fail = true;
           break;
         }

@@ -21,19 +21,17 @@ struct alignas(64) DeviceCtl {
   int where;                // diagnostic: position whose wait ran out
   unsigned int barrier_count;
   unsigned int barrier_gen;
-  int* host_code;           // pinned host copy of `code` (may be null): read after a
-                            // synchronisation without a copy of its own
+  int* host_code;           // pinned host copy of `code` (may be null), written as CTAs leave:
+                            // read after a synchronisation without a copy of its own
   unsigned int pad[8];
 };
 
-// Records the first failure of a launch, on the device and for the host.
-__device__ __forceinline__ void ctl_raise(DeviceCtl* ctl, int code, int where) {
-  if (atomicCAS(&ctl->code, DEV_OK, code) != DEV_OK) return;
-  ctl->where = where;
-  if (ctl->host_code) {
-    *reinterpret_cast<volatile int*>(ctl->host_code) = code;
-    __threadfence_system();
-  }
+// Passes a failure (`code` as read from the block) on to the host, as a CTA leaves or
+// where it is recorded (WaitBudget::poll).
+__device__ __forceinline__ void ctl_report(DeviceCtl* ctl, int code) {
+  if (code == DEV_OK || !ctl->host_code) return;
+  *reinterpret_cast<volatile int*>(ctl->host_code) = code;
+  __threadfence_system();
 }
 
 // ------------------------------------------------------------------ PTX wrappers
@@ -144,6 +142,13 @@ struct WaitBudget {
   unsigned sleep_max;
   __device__ __forceinline__ explicit WaitBudget(unsigned long long limit, unsigned smin = 0, unsigned smax = 0)
       : start(0), limit_ns(limit), iters(0), sleep_ns(smin), sleep_max(smax) {}
+  // REPORT: tells the host at once instead of as the CTA leaves. That code is rarely
+  // run, but it changes the registers of the loop it sits in, for better or worse:
+  // without it k_pull_wsync_multi keeps 60 registers on 16 lanes instead of 48 (a
+  // 1M-row power-law walk with 16 right-hand sides 30.8 ms, 40.9 with it), with it
+  // k_pull_ahead_multi takes 2,053 us on 1M rows with 64 (2,168 without) and
+  // k_pull_wsync_split 2,184 on 4M rows (2,207).
+  template <bool REPORT = false>
   __device__ __forceinline__ bool poll(DeviceCtl* ctl, int where) {
     ++iters;
     if (sleep_max) {
@@ -155,7 +160,10 @@ struct WaitBudget {
     if (start == 0) { start = now; return true; }
     if (*reinterpret_cast<volatile int*>(&ctl->code) != DEV_OK) return false;
     if (now - start > limit_ns) {
-      ctl_raise(ctl, DEV_TIMEOUT, where);
+      if (atomicCAS(&ctl->code, DEV_OK, DEV_TIMEOUT) == DEV_OK) {
+        ctl->where = where;
+        if (REPORT) ctl_report(ctl, DEV_TIMEOUT);
+      }
       return false;
     }
     return true;
@@ -188,6 +196,7 @@ __device__ __forceinline__ bool grid_barrier(DeviceCtl* ctl, unsigned long long 
       while (ld_acquire_u32(&ctl->barrier_gen) == gen) {
         if (!w.poll(ctl, -1)) { ok = 0; break; }
       }
+      if (!ok) ctl_report(ctl, *reinterpret_cast<volatile int*>(&ctl->code));
     }
     s_ok = ok && !ctl_failed(ctl);
   }

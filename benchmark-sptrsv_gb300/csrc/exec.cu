@@ -697,7 +697,7 @@ __device__ __forceinline__ bool wsync_segment(const ExecArgs<T>& a, T* s_x, int 
         nap = nap * 2u < a.sleep_max ? nap * 2u : a.sleep_max;
       }
       bool fail = false;
-      if ((any_global || (++idle & 255u) == 0u) && !wb.poll(a.ctl, p)) fail = true;
+      if ((any_global || (++idle & 255u) == 0u) && !wb.poll<true>(a.ctl, p)) fail = true;
       if (__any_sync(kFull, fail)) return true;
     }
   }
@@ -1587,7 +1587,7 @@ cudaError_t launch_grad_values(const int* csc_row, const int* csc_col, int nnz, 
 // flags raised earlier in the stream) nothing is solved and DEV_BAD_INPUT is
 // recorded.
 __device__ __forceinline__ void raise_bad_input(DeviceCtl* ctl, int where) {
-  ctl_raise(ctl, DEV_BAD_INPUT, where);
+  if (atomicCAS(&ctl->code, DEV_OK, DEV_BAD_INPUT) == DEV_OK) ctl->where = where;
 }
 
 template <typename T>

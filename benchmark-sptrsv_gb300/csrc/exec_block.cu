@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_pull_block(BlockArgs<T> a) {
     unsigned idle = 0u;
     // false once the wait must end; the first failure of any warp ends the others' waits too
     auto keep_waiting = [&]() {
-      if ((++idle & 63u) == 0u && __any_sync(kFull, !wb.poll(a.ctl, base))) fail = true;
+      if ((++idle & 63u) == 0u && __any_sync(kFull, !wb.poll<true>(a.ctl, base))) fail = true;
       return !fail;
     };
     // whether the consumer is through with `count` segments, seen by every lane (each

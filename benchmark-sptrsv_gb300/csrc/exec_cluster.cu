@@ -234,6 +234,7 @@ __global__ void __launch_bounds__(512) k_pull_cluster(ClusterArgs<T> a) {
   // peers may still poll this CTA's words
   __syncwarp();
   cluster_sync();
+  if (rank == 0 && threadIdx.x == 0) ctl_report(a.ctl, *reinterpret_cast<volatile int*>(&a.ctl->code));
 }
 
 // Launch configuration of the executor; the attribute must outlive it.

@@ -21,7 +21,7 @@ __device__ __forceinline__ void copy_async(unsigned dst, const V* src) {
 __device__ __forceinline__ bool lockstep_wait(WaitBudget& wb, int left, int& seen, DeviceCtl* ctl, int where) {
   if (__any_sync(0xffffffffu, left != seen)) wb.start = 0;
   seen = left;
-  return !__any_sync(0xffffffffu, !wb.poll(ctl, where));
+  return !__any_sync(0xffffffffu, !wb.poll<true>(ctl, where));
 }
 
 // Claim the next chunk for this CTA (uniform across the CTA).
@@ -33,9 +33,11 @@ __device__ __forceinline__ unsigned next_chunk(DeviceCtl* ctl, unsigned nchunks,
   return c;
 }
 
-// The last CTA to leave resets the chunk ticket so the next launch starts at 0.
+// The last CTA to leave resets the chunk ticket so the next launch starts at 0. A CTA
+// that recorded a failure passes it on (a barrier lies between).
 __device__ __forceinline__ void leave(DeviceCtl* ctl) {
   if (threadIdx.x == 0) {
+    const int code = *reinterpret_cast<volatile int*>(&ctl->code);
     __threadfence();
     const unsigned d = atomicAdd(&ctl->done, 1u);
     if (d == gridDim.x - 1) {
@@ -43,6 +45,7 @@ __device__ __forceinline__ void leave(DeviceCtl* ctl) {
       ctl->done = 0;
       __threadfence();
     }
+    ctl_report(ctl, code);
   }
 }
 
