@@ -311,7 +311,7 @@ constexpr size_t kSharedLimit = 226 * 1024;
 // system would be lowered by another thread's handle between this and the launch.
 template <typename Kernel>
 cudaError_t allow_shared(Kernel kernel, size_t smem) {
-  if (smem <= 48 * 1024) return cudaSuccess;  // allowed as it is
+  if (smem <= 47 * 1024) return cudaSuccess;  // 48 KB with the static arrays are allowed as it is
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSharedLimit));
 }
 // Transposed (adjoint) solve request: optional fused gradient w.r.t. the values.
