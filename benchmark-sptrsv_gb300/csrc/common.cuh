@@ -146,8 +146,7 @@ struct WaitBudget {
   // run, but it changes the registers of the loop it sits in, for better or worse:
   // without it k_pull_wsync_multi keeps 60 registers on 16 lanes instead of 48 (a
   // 1M-row power-law walk with 16 right-hand sides 30.8 ms, 40.9 with it), with it
-  // k_pull_ahead_multi takes 2,053 us on 1M rows with 64 (2,168 without) and
-  // k_pull_wsync_split 2,184 on 4M rows (2,207).
+  // k_pull_wsync_split takes 2,184 us on 4M rows (2,207 without).
   template <bool REPORT = false>
   __device__ __forceinline__ bool poll(DeviceCtl* ctl, int where) {
     ++iters;

@@ -269,10 +269,7 @@ __global__ void __launch_bounds__(256) k_pull_ahead_split(SplitArgs<T> a) {
         }
       }
       if ((++idle & 255u) == 0u) {
-        if (!lockstep_wait(wb, left, seen, a.ctl, p)) {
-          fail = true;
-          break;
-        }
+        if (!lockstep_wait(wb, left, seen, fail, a.ctl, p)) break;
       }
     }
     if (fail) break;

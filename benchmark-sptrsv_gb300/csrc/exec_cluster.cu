@@ -222,10 +222,7 @@ __global__ void __launch_bounds__(512) k_pull_cluster(ClusterArgs<T> a) {
         }
       }
       if ((++idle & 255u) == 0u) {
-        if (!lockstep_wait(wb, left - done, seen, a.ctl, p)) {
-          fail = true;
-          break;
-        }
+        if (!lockstep_wait(wb, left - done, seen, fail, a.ctl, p)) break;
       }
     }
     if (pr < a.n && !fail) a.x[row] = acc;

@@ -16,12 +16,16 @@ __device__ __forceinline__ void copy_async(unsigned dst, const V* src) {
 
 // Wait check of a warp's lockstep loop, once in 256 iterations: `left` is what a lane
 // still has to consume. While any lane has consumed something since the last check
-// the warp was not waiting, however long its lists, and the budget starts over. False
-// (in every lane) once the wait must be abandoned.
-__device__ __forceinline__ bool lockstep_wait(WaitBudget& wb, int left, int& seen, DeviceCtl* ctl, int where) {
+// the warp was not waiting, however long its lists, and the budget starts over. False,
+// with `fail`, the loop's own flag, set in every lane, once the wait must be abandoned.
+__device__ __forceinline__ bool lockstep_wait(WaitBudget& wb, int left, int& seen, bool& fail, DeviceCtl* ctl,
+                                              int where) {
   if (__any_sync(0xffffffffu, left != seen)) wb.start = 0;
   seen = left;
-  return !__any_sync(0xffffffffu, !wb.poll<true>(ctl, where));
+  if (!wb.poll<true>(ctl, where)) fail = true;
+  if (!__any_sync(0xffffffffu, fail)) return true;
+  fail = true;
+  return false;
 }
 
 // Claim the next chunk for this CTA (uniform across the CTA).

@@ -690,10 +690,7 @@ __global__ void __launch_bounds__(256) k_refine_ahead(RefineArgs a, const int* w
         }
       }
       if ((++idle & 255u) == 0u) {
-        if (!lockstep_wait(wb, left - done, seen, a.ctl, p)) {
-          fail = true;
-          break;
-        }
+        if (!lockstep_wait(wb, left - done, seen, fail, a.ctl, p)) break;
       }
     }
     if (!fail && pr < a.n && col) {
