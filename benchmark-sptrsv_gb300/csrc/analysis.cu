@@ -671,6 +671,40 @@ cudaError_t launch_list_stats(const int* row_ptr, const int* col_ptr, int n, int
   return cudaGetLastError();
 }
 
+// How unlike the lists of neighbouring positions are: over windows of kVarietyWindow
+// segments of 32 positions, the squared deviations of the segments' entries from their
+// window's mean (count[0]) and the squared means (count[1]), rounded per window, so that
+// the sums do not depend on their order. A last part of a segment is left out.
+constexpr int kVarietyWindow = 64;
+__global__ void __launch_bounds__(kVarietyWindow) k_list_variety(const int* __restrict__ ptr, int nseg,
+                                                                 unsigned long long* count) {
+  __shared__ double s_sum[2], s_square[2];
+  const int g = blockIdx.x * kVarietyWindow + threadIdx.x;
+  const double v = g < nseg ? static_cast<double>(ptr[(g + 1) * 32] - ptr[g * 32]) : 0.0;
+  double sum = v, square = v * v;
+  for (int o = 16; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    square += __shfl_xor_sync(0xffffffffu, square, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    s_sum[threadIdx.x >> 5] = sum;
+    s_square[threadIdx.x >> 5] = square;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  const double total = s_sum[0] + s_sum[1];
+  const double mean2 = total * total / min(kVarietyWindow, nseg - static_cast<int>(blockIdx.x) * kVarietyWindow);
+  atomicAdd(&count[0], static_cast<unsigned long long>(llrint(fmax(s_square[0] + s_square[1] - mean2, 0.0))));
+  atomicAdd(&count[1], static_cast<unsigned long long>(llrint(mean2)));
+}
+
+cudaError_t launch_list_variety(const int* ptr, int n, unsigned long long* count, cudaStream_t s) {
+  const int nseg = n / 32;
+  if (nseg <= 0) return cudaSuccess;
+  k_list_variety<<<(nseg + kVarietyWindow - 1) / kVarietyWindow, kVarietyWindow, 0, s>>>(ptr, nseg, count);
+  return cudaGetLastError();
+}
+
 // Off-diagonal entries whose row and column fall in the same block of `block`
 // unknowns of the natural execution order (ascending for a forward solve,
 // descending for a backward one): how much of the DAG a blocked order keeps

@@ -97,6 +97,8 @@ struct sptrsv_gb300_handle_s {
   std::vector<int> out_cnt_host;   // dependents per position
   int max_dep_cnt = 0, max_out_cnt = 0;
   long long long_deps = 0, long_outs = 0;  // entries of long lists (long_cut)
+  double variety[2] = {0.0, 0.0};  // of neighbouring lists' lengths in the layout, dependencies and
+                                   // dependents (launch_list_variety, the root)
   ChunkTable tab_fwd, tab_adj;
   PieceTable pc_fwd, pc_adj;
   SplitTable sp_fwd, sp_adj;
@@ -510,6 +512,17 @@ int build_layout(sptrsv_gb300_handle_s* h, int block, cudaStream_t s) {
                                L.dep_pos_f, L.dep_src_f, s));
     CUDA_TRY(launch_sort_lists(L.out_ptr, L.out_pos, L.out_src, n, ndep, h->max_out_cnt, true,
                                L.out_pos_f, L.out_src_f, s));
+    unsigned long long* d_variety = nullptr;
+    unsigned long long variety[4] = {};
+    CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&d_variety), sizeof(variety), s));
+    CUDA_TRY(cudaMemsetAsync(d_variety, 0, sizeof(variety), s));
+    CUDA_TRY(launch_list_variety(L.dep_ptr, n, d_variety, s));
+    CUDA_TRY(launch_list_variety(L.out_ptr, n, d_variety + 2, s));
+    CUDA_TRY(cudaMemcpyAsync(variety, d_variety, sizeof(variety), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaFreeAsync(d_variety, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    for (int i : {0, 1})
+      h->variety[i] = variety[2 * i + 1] ? std::sqrt(static_cast<double>(variety[2 * i]) / variety[2 * i + 1]) : 0.0;
   }
   if (level_order && !stretched) {
     L.nlevels = h->nlevels;
@@ -1345,15 +1358,47 @@ bool use_cluster(const sptrsv_gb300_handle_s* h, bool adj) {
   return P.narrow && P.order_block >= h->n && (adj ? P.split_adj : P.split_fwd) == 0;
 }
 
+// Whether the executors that stage lists ahead serve a walk under the automatic plan.
+// Their warps (CTAs, for blocks) hold two or three segments claimed ahead, which wait
+// while the one in hand is walked. Where neighbouring segments' lists are much longer
+// and shorter by turns (batches of unlike systems, striped columns), short segments on
+// the critical path wait in CTAs that walk long ones: a variety of 0.27 to 0.76 was
+// slower on wide levels (the executors without claims ahead vs these, us: 64 systems
+// of 3-20 entries a column, 969 unknowns a level, 1 / 4 / 16 right-hand sides 1,778 /
+// 1,880 / 2,405 vs 2,636 / 2,148 / 3,443; 1M rows in stripes of 2 and 18 entries, 778
+// a level, transposed, 8 / 32 1,339 / 1,767 vs 1,931 / 4,056); up to 0.22 nothing was
+// (two classes of 6 and 8 entries 1,262 vs 943; systems of 1,000 to 200,000 rows of 9
+// entries 1,309 vs 1,237), nor 0.31-0.35 on 3,479 a level (0.39 and 0.44 were). On
+// narrow levels the shorter hop wins all the same (269 a level, 3-20 entries, 1 / 4 /
+// 16: 3,678 / 4,061 / 4,102 vs 3,057 / 2,611 / 3,601). The widest levels for unlike
+// lists lie between what was measured on both sides (unknowns a level, gain), forward
+// and refined: 1 right-hand side 527 1.09, 702 0.93; 2 none (969 1.01, 1,429 1.07-1.19,
+// 1,605 0.95, 4,993 1.58); 4 834 1.00, 969 0.81; 8 527 1.14, 702 0.86; 16 269 1.10,
+// 319 0.96 (FP32 527 1.74, 702 0.95); 24-64 187 1.01-1.19, 201 0.83 (FP32 319 1.02-1.2,
+// 412 0.82); transposed: 1 834 1.03, 969 0.90; 2 834 1.01, 969 0.83, 1,605 0.80, 2,762
+// 1.63; 4 527 1.15, 702 0.82; 8 269 1.08, 386 0.91; 16 187 1.19, 201 0.91 (FP32 527
+// 1.46, 702 0.73).
+bool stages_ahead(const sptrsv_gb300_handle_s* h, int rhs, size_t elem, bool adj) {
+  const int width = h->n / std::max(1, h->nlevels);
+  if (h->variety[adj] < (width < 2500 ? 0.25 : 0.36)) return true;
+  if (rhs == 1) return width <= (adj ? 850 : 600);
+  if (rhs == 2) return !adj || width <= 850 || width >= 2500;
+  if (rhs <= 4) return width <= (adj ? 550 : 900);
+  if (rhs <= 8) return width <= (adj ? 300 : 600);
+  if (rhs <= 16) return width <= (elem == 4 ? 600 : (adj ? 190 : 300));
+  return width <= (elem == 4 ? 320 : 190);
+}
+
 // Whether a warp-synchronous one-rhs walk in level order runs k_pull_ahead
 // (exec_ahead.cu, which picks entries per iteration and CTAs per SM itself), or
 // with split lists k_pull_ahead_split: under the automatic plan, or where
 // explicit options leave nothing else to k_pull_wsync (one CTA of 256 threads per
 // SM, one dependency per iteration: the tuner's way to it).
-bool use_ahead(const sptrsv_gb300_handle_s* h, const ExecConfig& c) {
+bool use_ahead(const sptrsv_gb300_handle_s* h, const ExecConfig& c, bool split, bool adj) {
   if (!c.wsync || c.exact || c.staged || !c.smem_tier || h->layout_block < h->n) return false;
   if (c.block != 256 || c.chunk != 256 || c.sleep_max != 0) return false;
-  if (planned(h, SPTRSV_OPTION_CTAS_PER_SM) && c.wsync_batch == 0) return true;
+  if (planned(h, SPTRSV_OPTION_CTAS_PER_SM) && c.wsync_batch == 0)
+    return split || stages_ahead(h, 1, sizeof(double), adj);
   return c.ctas_per_sm == 1 && c.wsync_batch == 1;
 }
 
@@ -1393,7 +1438,7 @@ bool use_ahead_multi(const sptrsv_gb300_handle_s* h, const ExecConfig& c, int rh
   if (rhs < 2 || !c.wsync || c.exact || !c.smem_tier || h->layout_block < h->n || !h->plan.valid) return false;
   if (h->rhs_tile_option != 0 || h->chunk_option != 0 || c.block != 256 || c.sleep_max != 0) return false;
   if (!planned(h, SPTRSV_OPTION_CTAS_PER_SM) && c.ctas_per_sm != 0) return false;
-  if ((adj ? h->plan.split_adj : h->plan.split_fwd) != 0) return false;
+  if ((adj ? h->plan.split_adj : h->plan.split_fwd) != 0 || !stages_ahead(h, rhs, elem, adj)) return false;
   const int shape = ahead_multi_shape(rhs, elem, false);
   // pairs over 32 lanes: no gain for the transposed walk (64 right-hand sides, 1M
   // rows, column-major: 2.27 ms against 2.23)
@@ -1549,7 +1594,8 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
     const PieceTable* pc = nullptr;
     if (rhs == 1 && planned(h, SPTRSV_OPTION_SPLIT)) c.split = adj ? h->plan.split_adj : h->plan.split_fwd;
     const bool cut = rhs == 1 && c.wsync && !c.exact && c.split > 0 && longest > c.split && !(adj && adj->grad);
-    const bool split_ahead = cut && (planned(h, SPTRSV_OPTION_SPLIT) || c.split == 32) && use_ahead(h, c) &&
+    const bool split_ahead = cut && (planned(h, SPTRSV_OPTION_SPLIT) || c.split == 32) &&
+                             use_ahead(h, c, true, adj != nullptr) &&
                              static_cast<double>(h->nnz - n) + 4.0 * n <= kSplitAheadWork * h->nlevels;
     if (split_ahead) {
       ST_TRY(ensure_split(h, adj != nullptr, 32, s));
@@ -1565,7 +1611,7 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
       CUDA_TRY(launch_pull_ahead_multi<T>(h->layout, V, rhs, v, static_cast<T*>(h->xw.p), h->ctl,
                                           n < kNarrowWidth * h->nlevels, timeout_ns(h), h->num_sms, s,
                                           adj != nullptr, walk ? h->units.walk : nullptr));
-    } else if (rhs == 1 && !pc && !(adj && adj->grad) && use_ahead(h, c)) {
+    } else if (rhs == 1 && !pc && !(adj && adj->grad) && use_ahead(h, c, false, adj != nullptr)) {
       CUDA_TRY(launch_pull_ahead<T>(h->layout, V, v, static_cast<T*>(h->xw.p), h->ctl, h->nlevels, timeout_ns(h),
                                     h->num_sms, s, adj != nullptr));
     } else {
@@ -2250,7 +2296,8 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
     // level order with the plan's settings: lists staged ahead
     const bool refine_ahead =
         rhs == 1 ? fc.wsync && fc.smem_tier && h->layout_block >= h->n && fc.block == 256 && fc.chunk == 256 &&
-                       fc.sleep_max == 0 && fc.wsync_batch == 0 && planned(h, SPTRSV_OPTION_CTAS_PER_SM)
+                       fc.sleep_max == 0 && fc.wsync_batch == 0 && planned(h, SPTRSV_OPTION_CTAS_PER_SM) &&
+                       stages_ahead(h, 1, sizeof(double), false)
                  : refine_ahead_blocks(h, rhs);
     const bool walk = refine_ahead && rhs > 1 && h->layout_block < h->n;
     if (walk) ST_TRY(ensure_walk(h, s));

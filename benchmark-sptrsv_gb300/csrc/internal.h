@@ -280,6 +280,9 @@ enum PlanCounter {
 };
 cudaError_t launch_list_stats(const int* row_ptr, const int* col_ptr, int n, int cut, unsigned long long* count,
                               cudaStream_t s);
+// count[0] / count[1] = squared coefficient of variation of the lists' lengths among
+// neighbouring segments of 32 positions (two words, zeroed first)
+cudaError_t launch_list_variety(const int* ptr, int n, unsigned long long* count, cudaStream_t s);
 cudaError_t launch_block_locality(const int* row, const int* col, int nnz, int n, int block, bool backward,
                                   unsigned long long* count, cudaStream_t s);
 cudaError_t launch_coarrival(const int* row_ptr, const int* col, const int* depth, int n, unsigned long long* count,
