@@ -1471,11 +1471,20 @@ bool use_level_walk(const sptrsv_gb300_handle_s* h, const ExecConfig& c, int rhs
          planned(h, SPTRSV_OPTION_CTAS_PER_SM) && c.block == 256 && c.sleep_max == 0;
 }
 
-// Whether the fused first refinement step of a block runs k_refine_ahead.
+// Whether the fused first refinement step runs k_refine_ahead: for a block, where the
+// plain solve stages its lists ahead too (explicit settings and the tuner's included);
+// for one right-hand side, in level order under the plan's settings or the explicit
+// ones that lead plain solves to k_pull_ahead or the one-cluster executor.
+bool refine_ahead_one(const sptrsv_gb300_handle_s* h, const ExecConfig& c) {
+  if (!c.wsync || !c.smem_tier || h->layout_block < h->n) return false;
+  if (c.block != 256 || c.chunk != 256 || c.sleep_max != 0) return false;
+  if (!h->plan.valid || !stages_ahead(h, 1, sizeof(double), false)) return false;
+  if (planned(h, SPTRSV_OPTION_CTAS_PER_SM)) return c.wsync_batch == 0;
+  return c.ctas_per_sm == 1 && (c.wsync_batch == 1 || (c.wsync_batch == 0 && h->cluster_option == 1));
+}
 bool refine_ahead_blocks(const sptrsv_gb300_handle_s* h, int rhs) {
   const ExecConfig c = pick_config(h, rhs);
   return rhs > 1 && rhs <= 64 && h->fused_refine == 2 && c.sched == SCHED_PULL && !c.exact &&
-         planned(h, SPTRSV_OPTION_CTAS_PER_SM) &&
          (use_ahead_multi(h, c, rhs, sizeof(double), false) || use_level_walk(h, c, rhs, sizeof(double)));
 }
 
@@ -2293,12 +2302,7 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
   }
   if (fuse) {
     // X_0, the FP64 residual and the first FP32 correction in one pass: X = X_0 + D_1
-    // level order with the plan's settings: lists staged ahead
-    const bool refine_ahead =
-        rhs == 1 ? fc.wsync && fc.smem_tier && h->layout_block >= h->n && fc.block == 256 && fc.chunk == 256 &&
-                       fc.sleep_max == 0 && fc.wsync_batch == 0 && planned(h, SPTRSV_OPTION_CTAS_PER_SM) &&
-                       stages_ahead(h, 1, sizeof(double), false)
-                 : refine_ahead_blocks(h, rhs);
+    const bool refine_ahead = rhs == 1 ? refine_ahead_one(h, fc) : refine_ahead_blocks(h, rhs);
     const bool walk = refine_ahead && rhs > 1 && h->layout_block < h->n;
     if (walk) ST_TRY(ensure_walk(h, s));
     // the plain solve's rule (160k-row bands with 1 / 2 entries per column and a
