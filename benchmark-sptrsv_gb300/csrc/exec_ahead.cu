@@ -24,7 +24,14 @@
 //                     of 40 entries (6,700) 1,010 / 1,084 vs 1,073 / 1,181
 //   t <= 34,000       one CTA, U = 2: 4M-row power law (30,100) 1,363 forward, 1,459
 //                     with U = 1, 1,403 with two CTAs; FP32, 25,000, 373 vs 410
-//   t <= 120,000      two CTAs, U = 2: 2M-row band (49,700) 413 / 479, one CTA 496 / 548
+//   t <= 120,000      two CTAs, U = 2: 2M-row band (49,700) 413 / 479, one CTA 496 / 548;
+//                     2M rows of 9 entries (66,300) 393 / 493, three 409 / 580. But
+//                     three where the lists leave L1 to the polls: FP32 of more than 6
+//                     entries (the same 385 / 517, two 481 / 641), transposed FP64 of at
+//                     most 6 (2M rows of 4, 38,900, 456, two 605; 2M of 6, 101,000, 335,
+//                     two 439), and from 90,000 on at most 6 (the same 277, two 346);
+//                     and one transposed where a segment is longer than two CTAs' buffers
+//                     (1M rows of 20, 40,700, 704, two 726; FP32 678, two 1,060)
 //   beyond            three CTAs: 4M rows of 4 entries (230,000) 270 / 279, two 299 / 313
 // k_pull_wsync on these: 1,103 / 1,354, 1,187 / 1,383, 1,687, 490 (FP32), 510 / 578,
 // 323 / 297.
@@ -225,7 +232,13 @@ cudaError_t launch_pull_ahead(const Layout& L, const Values<T>& V, const VecView
   if (L.n == 0) return cudaSuccess;
   constexpr int block = 256;
   const double t = (static_cast<double>(L.ndep) + 4.0 * L.n) / std::max(1, nlevels);
-  const int ctas = t <= 34000.0 ? 1 : (t <= 120000.0 ? 2 : 3);
+  int ctas = t <= 34000.0 ? 1 : (t <= 120000.0 ? 2 : 3);
+  if (ctas == 2) {
+    const double segment = 32.0 * L.ndep / L.n;  // entries
+    if (adj && segment > 400.0) ctas = 1;
+    else if (segment > 200.0) ctas = sizeof(T) == 8 ? 2 : 3;
+    else if ((adj && sizeof(T) == 8) || t > 90000.0) ctas = 3;
+  }
   const bool one = !adj && t < 21000.0;
   // list buffers hold twice the average segment (longer ones read the rest from
   // global memory), as far as the CTAs and L1 leave room
