@@ -1471,6 +1471,19 @@ bool use_level_walk(const sptrsv_gb300_handle_s* h, const ExecConfig& c, int rhs
          planned(h, SPTRSV_OPTION_CTAS_PER_SM) && c.block == 256 && c.sleep_max == 0;
 }
 
+// Transposed solves that k_pull_ahead_multi does not scale on the way in go through
+// rows where the copies pay: walking columns as they are costs a sector per element,
+// which large blocks feel (FP64, as they are vs staged us: 300k rows 33 / 64 743 / 760
+// vs 812 / 798; 500k 48 719 vs 755, 56 776 vs 771, 64 822 vs 757; 1M 33 / 48 / 56 / 64
+// 2,161 / 2,259 / 2,420 / 2,711 vs 2,313 / 2,331 / 2,366 / 2,273; 2M 33 4,024 vs 3,792).
+// Level walks of blocked layouts always do (300 x 300 mesh, FP32 64 622 vs 556).
+bool stage_adjoint(const sptrsv_gb300_handle_s* h, int rhs, int layout, size_t elem) {
+  if (!stage_col_major(h, rhs, layout, kColMajorStageRhs)) return false;
+  if (use_level_walk(h, pick_config(h, rhs), rhs, elem)) return true;
+  const double bytes = static_cast<double>(h->n) * rhs * elem;
+  return bytes > 400e6 || (rhs >= 56 && bytes > 200e6);
+}
+
 // Whether the fused first refinement step runs k_refine_ahead: for a block, where the
 // plain solve stages its lists ahead too (explicit settings and the tuner's included);
 // for one right-hand side, in level order under the plan's settings or the explicit
@@ -2451,9 +2464,7 @@ int sptrsv_gb300_solve_adjoint(sptrsv_handle_t h, const void* d_val, int dtype, 
   const int before = h->layout_block;
   ST_TRY(ensure_layout(h, s));
   if (!d_val && h->layout_block != before) return SPTRSV_ERR_STATE;
-  if (!d_dval && stage_col_major(h, rhs, layout, kColMajorStageRhs) && !stages_columns(h, rhs, layout, elem, true)) {
-    // through row-major staging, as plain solves (1M rows, 64 right-hand sides:
-    // 2.64 ms walking the columns as they are, 2.36 staged)
+  if (!d_dval && stage_adjoint(h, rhs, layout, elem) && !stages_columns(h, rhs, layout, elem, true)) {
     const size_t bytes = (size_t)h->n * rhs * elem;
     ST_TRY(ensure_buf(h, h->tb, bytes, 0, s));
     ST_TRY(ensure_buf(h, h->tx, bytes, 0, s));
