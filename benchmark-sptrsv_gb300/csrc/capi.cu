@@ -867,6 +867,16 @@ int ensure_units(sptrsv_gb300_handle_s* h, cudaStream_t s) {
   return SPTRSV_OK;
 }
 
+// Tables are built outside captures only: inside one, a walk whose table is not there yet
+// takes the executor that does without (*use cleared).
+int ready_in_capture(const void* table, cudaStream_t s, bool* use) {
+  if (table) return SPTRSV_OK;
+  bool capturing = false;
+  CUDA_TRY(is_capturing(s, &capturing));
+  if (capturing) *use = false;
+  return SPTRSV_OK;
+}
+
 // Positions by level of a blocked layout.
 int ensure_walk(sptrsv_gb300_handle_s* h, cudaStream_t s) {
   if (h->units.walk) return SPTRSV_OK;
@@ -1536,7 +1546,8 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
   ST_TRY(need_forms<T>(h, form, s));
   const bool cluster = rhs == 1 && !(adj && adj->grad) && use_cluster<T>(h, adj != nullptr);
   const bool blocks = c.sched == SCHED_PULL && !(adj && adj->grad);
-  const bool walk = blocks && use_level_walk(h, c, rhs, sizeof(T));
+  bool walk = blocks && use_level_walk(h, c, rhs, sizeof(T));
+  if (walk) ST_TRY(ready_in_capture(h->units.walk, s, &walk));
   if (walk) ST_TRY(ensure_walk(h, s));
   const bool multi = walk || (blocks && use_ahead_multi(h, c, rhs, sizeof(T), adj != nullptr));
   const int words = multi ? ahead_multi_words(rhs, sizeof(T), n < kNarrowWidth * h->nlevels) : rhs;
@@ -1562,6 +1573,7 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
   const int longest = adj ? h->max_out_cnt : h->max_dep_cnt;
   bool block = !cluster && c.sched == SCHED_PULL && rhs == 1 && !(adj && adj->grad) && !h->pipe_option &&
                use_block<T>(h, c, longest);
+  if (block) ST_TRY(ready_in_capture(h->units.seg, s, &block));
   if (block) {
     ST_TRY(ensure_units(h, s));
     block = 4LL * h->units.segments <= (4LL + 3 * longest) * h->units.levels;
@@ -2315,8 +2327,10 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
   }
   if (fuse) {
     // X_0, the FP64 residual and the first FP32 correction in one pass: X = X_0 + D_1
-    const bool refine_ahead = rhs == 1 ? refine_ahead_one(h, fc) : refine_ahead_blocks(h, rhs);
-    const bool walk = refine_ahead && rhs > 1 && h->layout_block < h->n;
+    bool refine_ahead = rhs == 1 ? refine_ahead_one(h, fc) : refine_ahead_blocks(h, rhs);
+    const bool blocked = rhs > 1 && h->layout_block < h->n;
+    if (refine_ahead && blocked) ST_TRY(ready_in_capture(h->units.walk, s, &refine_ahead));
+    const bool walk = refine_ahead && blocked;
     if (walk) ST_TRY(ensure_walk(h, s));
     // the plain solve's rule (160k-row bands with 1 / 2 entries per column and a
     // 1M-row band with 3: 0.101 / 1.95 / 6.40 ms refined with two dependencies

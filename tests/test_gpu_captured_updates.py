@@ -210,3 +210,51 @@ def test_refinement_graph_follows_new_values(cuda, oracle_port, rhs, steps):
         ref = oracle_port.solve(m.col_ptr, m.row_idx, val, m.n, m.substitution, b)
         assert relerr(x.cpu().numpy(), ref) <= 1e-10
     g.close()
+
+
+@pytest.mark.parametrize("case", ["adjoint", "single precision block", "refined block"])
+def test_tables_first_needed_inside_a_capture(cuda, oracle_port, own_stream, case):
+    """A blocked layout's tables are built outside captures; a walk captured before they
+    exist takes an executor that does without them."""
+    from sptrsv_gb300 import SyncFreeSolver, matgen
+    stream = cuda.cuda.current_stream()
+    if case == "adjoint":    # rows of more than four entries, columns of at most four
+        m = matgen.banded_random_lower(3000, np.random.default_rng(1).integers(0, 5, 3000), 60, 7)
+        kw = dict(schedule=2, staged=False, warp_sync=True, order_block=300, chunk=300, block=128, ctas_per_sm=0,
+                  backoff_ns=0, split=0)
+    else:
+        m, kw = matgen.laplace2d_lower(150), {}
+    s = SyncFreeSolver(m.col_ptr, m.row_idx, m.n, m.substitution, values=m.val, sync_check=False, stream=stream, **kw)
+
+    def block(rhs, dtype):
+        return cuda.from_numpy(np.random.default_rng(rhs).standard_normal((m.n, rhs)).astype(dtype)).cuda()
+
+    b = block(*{"adjoint": (1, np.float64), "single precision block": (14, np.float32),
+                "refined block": (16, np.float64)}[case])
+    x = cuda.empty_like(b)
+    if case == "adjoint":
+        s.solve(b)
+        call = lambda: s.solve_adjoint(b, out=x)   # noqa: E731
+    elif case == "single precision block":
+        s.solve(block(7, np.float64))              # the value words reach for 14 in FP32
+        s.solve(block(1, np.float32))
+        call = lambda: s.solve(b, out=x)           # noqa: E731
+    else:                                          # workspaces and forms from the FP64 residual's step
+        from sptrsv_gb300 import _lib
+        s.set_option(_lib.OPTION_FUSED_REFINE, 1)
+        s.solve_refine(b)
+        s.set_option(_lib.OPTION_FUSED_REFINE, 2)
+        call = lambda: s.solve_refine(b, out=x, tol=0.0, max_iter=1)   # noqa: E731
+    stream.synchronize()
+    g = cuda.cuda.CUDAGraph()
+    with cuda.cuda.graph(g, stream=stream):
+        call()
+    t = m.transpose() if case == "adjoint" else m
+    ref = oracle_port.solve(t.col_ptr, t.row_idx, t.val, m.n, t.substitution, b.double().cpu().numpy())
+    for _ in range(2):
+        x.zero_()
+        g.replay()
+        assert relerr(x.cpu().numpy(), ref) <= {"adjoint": 1e-12, "single precision block": 1e-5,
+                                                "refined block": 1e-10}[case]
+        call()    # the tables are there from now on
+    s.check()
