@@ -318,6 +318,14 @@ int ensure_buf(sptrsv_gb300_handle_s* h, DevBuf& b, size_t bytes, int fill_zero,
   return SPTRSV_OK;
 }
 
+// Bytes kept for a block of right-hand sides in a workspace: rows in whole 16-byte words,
+// which hold the padding of every executor, so that calls on rows of as many bytes use
+// one size and a captured one keeps its buffers when another runs.
+size_t block_bytes(const sptrsv_gb300_handle_s* h, int rhs, size_t elem) {
+  const size_t row = rhs * elem;
+  return (size_t)h->n * (row <= 32 ? row : (row + 15) / 16 * 16);  // up to 32 bytes nothing is padded
+}
+
 SysDesc sys_desc(const sptrsv_gb300_handle_s* h) {
   SysDesc d;
   d.count = h->batch_count;
@@ -1553,10 +1561,10 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
   const int words = multi ? ahead_multi_words(rhs, sizeof(T), n < kNarrowWidth * h->nlevels) : rhs;
   const bool columns = multi && !walk && stage_col_major(h, rhs, layout, kColMajorStageRhs);
   if (columns) {
-    ST_TRY(ensure_buf(h, h->tb, sizeof(T) * (size_t)n * words, 0, s));
+    ST_TRY(ensure_buf(h, h->tb, block_bytes(h, rhs, sizeof(T)), 0, s));
     CUDA_TRY(launch_columns_in<T>(h->layout, V, b, static_cast<T*>(h->tb.p), rhs, words, s));
     v.b = static_cast<const T*>(h->tb.p);
-    ST_TRY(ensure_buf(h, h->tx, sizeof(T) * (size_t)n * words, 0, s));
+    ST_TRY(ensure_buf(h, h->tx, block_bytes(h, rhs, sizeof(T)), 0, s));
     v.x = static_cast<T*>(h->tx.p);
     v.b_si = 0;
   }
@@ -1567,7 +1575,7 @@ int solve_typed(sptrsv_gb300_handle_s* h, int rhs, int layout, const T* b, T* x,
     ST_TRY(ensure_buf(h, h->counters, (size_t)n * sizeof(unsigned), 1, s));
   } else {
     const size_t bytes = sizeof(T) * (multi ? (size_t)n * words : elems);
-    ST_TRY(ensure_buf(h, h->xw, bytes, 0, s));
+    ST_TRY(ensure_buf(h, h->xw, block_bytes(h, rhs, sizeof(T)), 0, s));
     if (c.sched != SCHED_LEVELSET) CUDA_TRY(cudaMemsetAsync(h->xw.p, 0xFF, bytes, s));
   }
   const int longest = adj ? h->max_out_cnt : h->max_dep_cnt;
@@ -2244,9 +2252,8 @@ int sptrsv_gb300_solve(sptrsv_handle_t h, const void* d_val, int dtype, int rhs,
   ST_TRY(ensure_layout(h, s));
   if (!d_val && h->layout_block != before) return SPTRSV_ERR_STATE;  // schedule changed since the values were staged
   if (stage_col_major(h, rhs, layout, kColMajorStageRhs) && !stages_columns(h, rhs, layout, elem, false)) {
-    const size_t bytes = (size_t)h->n * rhs * elem;
-    ST_TRY(ensure_buf(h, h->tb, bytes, 0, s));
-    ST_TRY(ensure_buf(h, h->tx, bytes, 0, s));
+    ST_TRY(ensure_buf(h, h->tb, block_bytes(h, rhs, elem), 0, s));
+    ST_TRY(ensure_buf(h, h->tx, block_bytes(h, rhs, elem), 0, s));
     if (dtype == SPTRSV_DTYPE_F64) {
       CUDA_TRY(launch_transpose<double>(static_cast<const double*>(d_b), static_cast<double*>(h->tb.p), rhs, h->n, s));
     } else {
@@ -2292,9 +2299,8 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
                      (tol > 0.0 || max_iter == 1) && refine_ahead_blocks(h, rhs) &&
                      (d_x + count <= d_b || d_b + count <= d_x);
   if (stage_col_major(h, rhs, layout, 2) && !as_is) {
-    const size_t bytes = (size_t)h->n * rhs * sizeof(double);
-    ST_TRY(ensure_buf(h, h->tb, bytes, 0, s));
-    ST_TRY(ensure_buf(h, h->tx, bytes, 0, s));
+    ST_TRY(ensure_buf(h, h->tb, block_bytes(h, rhs, sizeof(double)), 0, s));
+    ST_TRY(ensure_buf(h, h->tx, block_bytes(h, rhs, sizeof(double)), 0, s));
     CUDA_TRY(launch_transpose<double>(d_b, static_cast<double*>(h->tb.p), rhs, h->n, s));
     const int st = sptrsv_gb300_solve_refine(h, d_val, rhs, SPTRSV_LAYOUT_ROW_MAJOR, static_cast<double*>(h->tb.p),
                                              static_cast<double*>(h->tx.p), tol, max_iter, iters, est, stream);
@@ -2351,7 +2357,7 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
     const long long width = h->n / std::max(1, h->nlevels);
     const size_t bytes = sizeof(unsigned long long) *
                          (refine_ahead ? (size_t)h->n * ahead_multi_words(rhs, 8, width < kNarrowWidth) : (size_t)count);
-    ST_TRY(ensure_buf(h, h->xw, bytes, 0, s));
+    ST_TRY(ensure_buf(h, h->xw, block_bytes(h, rhs, sizeof(unsigned long long)), 0, s));
     CUDA_TRY(cudaMemsetAsync(h->xw.p, 0xFF, bytes, s));
     CUDA_TRY(cudaMemsetAsync(stats, 0, 3 * sizeof(unsigned long long), s));
     h->last_sched = SCHED_PULL;
@@ -2427,8 +2433,8 @@ int sptrsv_gb300_solve_refine(sptrsv_handle_t h, const double* d_val, int rhs, i
   double* rx = d_x;
   const int steps_layout = to_rows ? SPTRSV_LAYOUT_ROW_MAJOR : layout;
   if (to_rows) {
-    ST_TRY(ensure_buf(h, h->tb, sizeof(double) * count, 0, s));
-    ST_TRY(ensure_buf(h, h->tx, sizeof(double) * count, 0, s));
+    ST_TRY(ensure_buf(h, h->tb, block_bytes(h, rhs, sizeof(double)), 0, s));
+    ST_TRY(ensure_buf(h, h->tx, block_bytes(h, rhs, sizeof(double)), 0, s));
     CUDA_TRY(launch_transpose<double>(d_b, static_cast<double*>(h->tb.p), rhs, h->n, s));
     CUDA_TRY(launch_transpose<double>(d_x, static_cast<double*>(h->tx.p), rhs, h->n, s));
     rb = static_cast<const double*>(h->tb.p);
@@ -2479,9 +2485,8 @@ int sptrsv_gb300_solve_adjoint(sptrsv_handle_t h, const void* d_val, int dtype, 
   ST_TRY(ensure_layout(h, s));
   if (!d_val && h->layout_block != before) return SPTRSV_ERR_STATE;
   if (!d_dval && stage_adjoint(h, rhs, layout, elem) && !stages_columns(h, rhs, layout, elem, true)) {
-    const size_t bytes = (size_t)h->n * rhs * elem;
-    ST_TRY(ensure_buf(h, h->tb, bytes, 0, s));
-    ST_TRY(ensure_buf(h, h->tx, bytes, 0, s));
+    ST_TRY(ensure_buf(h, h->tb, block_bytes(h, rhs, elem), 0, s));
+    ST_TRY(ensure_buf(h, h->tx, block_bytes(h, rhs, elem), 0, s));
     if (dtype == SPTRSV_DTYPE_F64) {
       CUDA_TRY(launch_transpose<double>(static_cast<const double*>(d_g), static_cast<double*>(h->tb.p), rhs, h->n, s));
     } else {
