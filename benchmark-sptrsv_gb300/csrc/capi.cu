@@ -2193,12 +2193,23 @@ int sptrsv_gb300_get_info(sptrsv_handle_t h, sptrsv_info* info) {
   if (c.wsync_batch > 0) {
     info->wsync_batch = c.wsync_batch;
   } else {
-    // the forward walk of a plain solve: the importer executor on a blocked
-    // layout, else the level-order executor with or without split lists
+    // the forward FP64 walk of a plain solve: one entry inside a cluster, all of a
+    // list's at once for one consumer per unit, the staged-ahead executor's own rule,
+    // else that of the lockstep executors (importers on a blocked layout, level order
+    // with or without split lists)
+    const bool pull = h->analysed && h->n > 0 && c.sched == SCHED_PULL;
+    const bool cluster = pull && use_cluster<double>(h, false);
+    const bool block = pull && !cluster && !h->pipe_option && use_block<double>(h, c, h->max_dep_cnt) &&
+                       (!h->units.seg || 4LL * h->units.segments <= (4LL + 3 * h->max_dep_cnt) * h->units.levels);
     const bool imported = c.wsync && !c.exact && h->import_option && h->layout_block < h->n &&
                           c.chunk == h->layout_block && c.smem_tier && !(c.split > 0 && h->max_dep_cnt > c.split);
     const bool split = !imported && c.wsync && !c.exact && info->split > 0 && h->max_dep_cnt > info->split;
-    info->wsync_batch = auto_wsync_batch(h, false, split);
+    if (cluster) info->wsync_batch = 1;
+    else if (block) info->wsync_batch = h->max_dep_cnt;
+    else if (pull && !split && use_ahead(h, c, false, false))
+      info->wsync_batch = ahead_entries(h->layout, h->nlevels, false);
+    else
+      info->wsync_batch = auto_wsync_batch(h, false, split);
   }
   info->coarrive_permille = static_cast<int>(h->plan.coarrive * 1000.0 + 0.5);
   return h->analysed ? SPTRSV_OK : SPTRSV_ERR_STATE;

@@ -226,12 +226,21 @@ __global__ void __launch_bounds__(256) k_pull_ahead(AheadArgs<T> a) {
 
 }  // namespace
 
+namespace {
+// Work per level (see above).
+double level_work(const Layout& L, int nlevels) {
+  return (static_cast<double>(L.ndep) + 4.0 * L.n) / std::max(1, nlevels);
+}
+}  // namespace
+
+int ahead_entries(const Layout& L, int nlevels, bool adj) { return !adj && level_work(L, nlevels) < 21000.0 ? 1 : 2; }
+
 template <typename T>
 cudaError_t launch_pull_ahead(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
                               int nlevels, unsigned long long timeout_ns, int num_sms, cudaStream_t s, bool adj) {
   if (L.n == 0) return cudaSuccess;
   constexpr int block = 256;
-  const double t = (static_cast<double>(L.ndep) + 4.0 * L.n) / std::max(1, nlevels);
+  const double t = level_work(L, nlevels);
   int ctas = t <= 34000.0 ? 1 : (t <= 120000.0 ? 2 : 3);
   if (ctas == 2) {
     const double segment = 32.0 * L.ndep / L.n;  // entries
@@ -239,7 +248,7 @@ cudaError_t launch_pull_ahead(const Layout& L, const Values<T>& V, const VecView
     else if (segment > 200.0) ctas = sizeof(T) == 8 ? 2 : 3;
     else if ((adj && sizeof(T) == 8) || t > 90000.0) ctas = 3;
   }
-  const bool one = !adj && t < 21000.0;
+  const bool one = ahead_entries(L, nlevels, adj) == 1;
   // list buffers hold twice the average segment (longer ones read the rest from
   // global memory), as far as the CTAs and L1 leave room
   const int avg = static_cast<int>(32LL * L.ndep / L.n);

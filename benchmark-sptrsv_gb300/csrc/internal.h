@@ -341,6 +341,7 @@ cudaError_t launch_levelset(const Layout& L, const Values<T>& V, int rhs, const 
 template <typename T>
 cudaError_t launch_pull_ahead(const Layout& L, const Values<T>& V, const VecView<T>& v, T* xw, DeviceCtl* ctl,
                               int nlevels, unsigned long long timeout_ns, int num_sms, cudaStream_t s, bool adj);
+int ahead_entries(const Layout& L, int nlevels, bool adj);  // list entries it polls per iteration
 // Segments of the split-list form (exec_ahead_split.cu): lists longer than `split`
 // take up to 32 adjacent lanes of a segment, interleaved (lane j of k takes
 // entries j, j + k, ...); no unknown straddles two segments.

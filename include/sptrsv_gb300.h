@@ -108,7 +108,9 @@ typedef enum sptrsv_option {
                                      averaging more than 3 entries; for shorter ones 2 when at least half
                                      of the unknowns have two or more dependencies on the level just
                                      before their own, else 1; 2 for split lists and the transposed walk;
-                                     sptrsv_info.wsync_batch reports the forward walk's value) */
+                                     the executors with lists staged ahead, one consumer per block or one
+                                     cluster have rules of their own; sptrsv_info.wsync_batch reports the
+                                     forward walk's value, of the executor that runs it) */
   SPTRSV_OPTION_IMPORT = 19,      /* 1 (default): warp-synchronous one-rhs forward pull on a blocked
                                      layout (chunk = order block) gives each CTA an importer warp that
                                      copies the chunk's external dependencies into shared memory. Left
