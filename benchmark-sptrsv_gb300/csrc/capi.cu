@@ -1341,9 +1341,13 @@ ExecConfig pick_config(const sptrsv_gb300_handle_s* h, int rhs) {
     // many rhs: warp-synchronous lane groups (up to 64 rhs), one unknown per group
     // per chunk; two CTAs per SM up to 8 rhs (the 1M-row band system at 4 / 8 rhs:
     // 1.025 / 1.027 ms against 1.073 / 1.064 with one or with every CTA that
-    // fits), every CTA that fits beyond (16 rhs: 1.13 ms against 1.45 with two)
+    // fits), every CTA that fits beyond (16 rhs: 1.13 ms against 1.45 with two), but
+    // four on narrow levels up to 16 rhs (five fit in FP32: a 30,000-row power-law walk
+    // of 152 unknowns per level 2.6-2.9 ms with five, 1.34 with four; on 3,479 per
+    // level 1.43 vs 1.55)
     if (planned(h, SPTRSV_OPTION_WARP_SYNC)) c.wsync = rhs <= 64 ? 1 : 0;
-    if (planned(h, SPTRSV_OPTION_CTAS_PER_SM)) c.ctas_per_sm = rhs <= 8 ? 2 : 0;
+    if (planned(h, SPTRSV_OPTION_CTAS_PER_SM))
+      c.ctas_per_sm = rhs <= 8 ? 2 : (rhs <= 16 && h->n < kNarrowWidth * h->nlevels ? 4 : 0);
     if (planned(h, SPTRSV_OPTION_BACKOFF_NS)) c.sleep_max = 0u;  // spinning measured 1-3 % faster at 16 and 64 rhs
     // a blocked layout: one CTA per order block (small chunks would hand the
     // blocks out one after another); the shared-memory tier does not fit there
