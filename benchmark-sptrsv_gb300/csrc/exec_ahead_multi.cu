@@ -266,19 +266,27 @@ cudaError_t launch_ahead_multi(AheadMultiArgs<T>& a, int avg, bool narrow, int n
     kernel<<<grid, 256, smem, s>>>(a, words, walk);
     return cudaGetLastError();
   };
+  // quadruples are FP32's, pairs over 32 lanes FP64's (forward, or along a level walk),
+  // and a level walk starts at 9 right-hand sides in FP32 (ahead_multi_shape,
+  // use_ahead_multi, use_level_walk)
+  constexpr bool half = sizeof(T) == 4;
   const bool pad = a.rhs != words, staged = a.b_si == 0;
+  const int shape = ahead_multi_shape(a.rhs, sizeof(T), narrow);
   if (walk) {
-    switch (ahead_multi_shape(a.rhs, sizeof(T), narrow)) {
-      case 8 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 8, 1, kWalk>, 8, 1);
+    switch (shape) {
       case 16 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 16, 1, kWalk>, 16, 1);
       case 8 * 8 + 2: return run(k_pull_ahead_multi<T, ADJ, 8, 2, kWalk>, 8, 2);
       case 16 * 8 + 2: return run(k_pull_ahead_multi<T, ADJ, 16, 2, kWalk>, 16, 2);
-      case 16 * 8 + 4: return run(k_pull_ahead_multi<T, ADJ, 16, 4, kWalk>, 16, 4);
-      case 32 * 8 + 2: return run(k_pull_ahead_multi<T, ADJ, 32, 2, kWalk>, 32, 2);
-      default: return cudaErrorInvalidValue;
     }
+    if constexpr (half) {
+      if (shape == 16 * 8 + 4) return run(k_pull_ahead_multi<T, ADJ, 16, 4, kWalk>, 16, 4);
+    } else {
+      if (shape == 8 * 8 + 1) return run(k_pull_ahead_multi<T, ADJ, 8, 1, kWalk>, 8, 1);
+      if (shape == 32 * 8 + 2) return run(k_pull_ahead_multi<T, ADJ, 32, 2, kWalk>, 32, 2);
+    }
+    return cudaErrorInvalidValue;
   }
-  switch (ahead_multi_shape(a.rhs, sizeof(T), narrow)) {
+  switch (shape) {
     case 2 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 2, 1, kWhole>, 2, 1);
     case 4 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 4, 1, kWhole>, 4, 1);
     case 8 * 8 + 1: return run(k_pull_ahead_multi<T, ADJ, 8, 1, kWhole>, 8, 1);
@@ -289,16 +297,19 @@ cudaError_t launch_ahead_multi(AheadMultiArgs<T>& a, int avg, bool narrow, int n
       return staged ? run(k_pull_ahead_multi<T, ADJ, 16, 2, kStaged>, 16, 2)
                     : (pad ? run(k_pull_ahead_multi<T, ADJ, 16, 2, kPad>, 16, 2)
                            : run(k_pull_ahead_multi<T, ADJ, 16, 2, kWhole>, 16, 2));
-    case 16 * 8 + 4:
+  }
+  if constexpr (half) {
+    if (shape == 16 * 8 + 4)
       return staged ? run(k_pull_ahead_multi<T, ADJ, 16, 4, kStaged>, 16, 4)
                     : (pad ? run(k_pull_ahead_multi<T, ADJ, 16, 4, kPad>, 16, 4)
                            : run(k_pull_ahead_multi<T, ADJ, 16, 4, kWhole>, 16, 4));
-    case 32 * 8 + 2:
+  } else if constexpr (!ADJ) {
+    if (shape == 32 * 8 + 2)
       return staged ? run(k_pull_ahead_multi<T, ADJ, 32, 2, kStaged>, 32, 2)
                     : (pad ? run(k_pull_ahead_multi<T, ADJ, 32, 2, kPad>, 32, 2)
                            : run(k_pull_ahead_multi<T, ADJ, 32, 2, kWhole>, 32, 2));
-    default: return cudaErrorInvalidValue;
   }
+  return cudaErrorInvalidValue;
 }
 
 namespace {
